@@ -105,7 +105,7 @@ def prepare(case, seed):
         torch.manual_seed(seed)
         with torch.device("cuda"):
             model = resnet50().to(memory_format=torch.channels_last)
-        dp = DataParallel(model, None, lr=0.01, momentum=0.9)
+        dp = DataParallel(model, None, lr=0.1, momentum=0.9)
         # the running statistics as views of one buffer, so that a step's updated state comes back as one tensor
         bufs = [(m, k, getattr(m, k)) for m in model.modules() for k in ("running_mean", "running_var")
                 if getattr(m, k, None) is not None]
@@ -161,7 +161,10 @@ def run(st):
     if kind == "resnet":
         loss = st["trainer"].step_device(st["x"], st["y"])
         dp = st["trainer"].dp
-        return {"loss": loss, "param": dp.flat_param, "momentum": dp.flat_mom, "stats": st["stats"]}
+        # the momentum is not returned on its own: with a zero-initialised branch scale the branches' gradients are
+        # differences that bf16 rounding shifts by 2-4 % when nothing but the order of the images changes; the updated
+        # parameters carry it at its weight in the step
+        return {"loss": loss, "param": dp.flat_param, "stats": st["stats"]}
     comm = st["comm"]
     if kind == "allreduce":
         if st["inplace"]:
@@ -215,11 +218,13 @@ def work(case):
 def tolerance(case):
     kind = case["kind"]
     if kind == "resnet":
-        return {"rel": 0.03, "max": 0.5}
+        # four times what permuting the images within the batch (another order of every sum) changes after two steps:
+        # parameters 2.1e-4 / 0.05 at batch 8, 1.0e-4 / 0.02 at 24, 2.8e-5 / 0.006 at 256
+        return {"rel": 2.4e-3 / math.sqrt(case["batch"]), "max": 0.57 / math.sqrt(case["batch"])}
     if kind in ("allreduce", "seqpar"):
         if case["dtype"] == "int32":
             return "exact"
         if case["dtype"] == "float32" and not case.get("wire"):
-            return {"rel": 4e-7, "max": 2e-6}      # order of at most 8 fp32 additions
-        return {"rel": 8e-3, "max": 3e-2}          # one or two roundings to 16 bits
+            return {"rel": 4e-7, "max": 2e-6}      # order of at most 8 fp32 additions (5e-8 from 64-bit sums)
+        return {"rel": 8e-3, "max": 3e-2}          # one or two roundings to 16 bits (2.2e-3 from 64-bit sums)
     return "exact"
