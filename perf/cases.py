@@ -228,3 +228,22 @@ def tolerance(case):
             return {"rel": 4e-7, "max": 2e-6}      # order of at most 8 fp32 additions (5e-8 from 64-bit sums)
         return {"rel": 8e-3, "max": 3e-2}          # one or two roundings to 16 bits (2.2e-3 from 64-bit sums)
     return "exact"
+
+
+def exact(case, seed):
+    """What ``run`` returns for these inputs from sums in 64 bits; None where outputs are copies (compared bit by bit)
+    or follow a whole mixed-precision network."""
+    kind = case["kind"]
+    if kind not in ("allreduce", "seqpar") or case["dtype"] == "int32":
+        return None
+    p, dtype = case["p"], getattr(torch, case["dtype"])
+    gen = torch.Generator(device="cuda").manual_seed(seed)
+    n = case["n"] if kind == "allreduce" else case["rows"] * case["width"]
+    total = torch.zeros(n, dtype=torch.float64, device="cuda")
+    for _ in range(p):                              # the draws of prepare(), in its order
+        total += _values(gen, n, dtype).double()
+    if kind == "allreduce":
+        if case["inplace"]:
+            total /= p
+        return [total for _ in range(p)]
+    return {"reduced": list(total.view(p, n // p)), "gathered": None}
