@@ -191,8 +191,8 @@ struct CollParams {
   int pipelined;                 ///< 1: half of the CTAs publish while the other half consumes (large uniform ops)
   size_t slot_elems;             ///< elements moved per slot and chunk (0 = the slot's capacity)
   int n_pub;                     ///< bulk-copy pipeline: number of publishing CTAs (0 = half of the grid)
-  int own_direct;                ///< one-shot allreduce: a rank reads its own contribution from its send buffer instead of
-                                 ///< pushing it into its own slot (same in / wire type, 16-byte aligned send buffer)
+  unsigned char own_direct[kMaxRanks];  ///< 1: what this rank contributes to its own result skips staging (one element type; reductions
+                                 ///< read it from the send buffer, which must be 16-byte aligned there; movement copies it)
 };
 
 /**

@@ -51,6 +51,10 @@ void launch_coll_f64(const CollParams& P, const LaunchCfg& cfg);
 void launch_coll_f16(const CollParams& P, const LaunchCfg& cfg);
 void launch_coll_bf16(const CollParams& P, const LaunchCfg& cfg);
 void launch_coll_int(const CollParams& P, DType dt, const LaunchCfg& cfg);
+void launch_coll_int8(const CollParams& P, DType dt, const LaunchCfg& cfg);
+void launch_coll_int16(const CollParams& P, DType dt, const LaunchCfg& cfg);
+void launch_coll_int32(const CollParams& P, DType dt, const LaunchCfg& cfg);
+void launch_coll_int64(const CollParams& P, DType dt, const LaunchCfg& cfg);
 void launch_coll_bytes(const CollParams& P, const LaunchCfg& cfg);
 /** Mixed-type sum: (in, wire, out) among f32 / f16 / bf16. Returns false when the triple is not compiled. */
 bool launch_coll_mixed(const CollParams& P, DType ti, DType tw, DType to, const LaunchCfg& cfg);

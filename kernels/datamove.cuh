@@ -2,6 +2,8 @@
 // kernels.  Reads of staging memory (local or a peer's) bypass L1 (ld.cg), so a
 // line cached during an earlier operation can never be served stale.
 #pragma once
+#include <type_traits>
+
 #include "common.cuh"
 
 namespace Al {
@@ -92,53 +94,88 @@ __device__ __forceinline__ size_t clamp_len(size_t count, size_t lo, size_t cap)
 // ---------------------------------------------------------------------------
 // copies
 // ---------------------------------------------------------------------------
-template <typename V>
-__device__ __forceinline__ void copy_units(char* dst, const char* src, size_t units, bool src_is_staging,
-                                           unsigned lane, unsigned nlanes) {
-  V* d = (V*)dst;
-  const V* s = (const V*)src;
-  const size_t stride = nlanes;
-  size_t i = lane;
-  // four independent loads in flight per thread
-  for (; i + 3 * stride < units; i += 4 * stride) {
-    V a, b, c, e;
-    if (src_is_staging) { a = __ldcg(s + i); b = __ldcg(s + i + stride); c = __ldcg(s + i + 2 * stride); e = __ldcg(s + i + 3 * stride); }
-    else { a = s[i]; b = s[i + stride]; c = s[i + 2 * stride]; e = s[i + 3 * stride]; }
-    d[i] = a; d[i + stride] = b; d[i + 2 * stride] = c; d[i + 3 * stride] = e;
+// What bounds the loops below is the number of bytes in flight: the staged kernel runs 512 threads per SM (its
+// register count allows one CTA), so with 4 x 16 bytes per thread 148 SMs keep 4.8 MB under way where HBM3e at
+// about 0.8 us of latency wants 6 MB.  Eight loads per thread and an end that is one more round of independent
+// (predicated) loads instead of up to three dependent ones cover that (halo exchange of 8 MiB planes on one GPU
+// 31.4 -> 27.6 us, ring pass of 4 x 25 MB 103.5 -> 90.5 us; conversions, one element at a time before, allreduce of
+// 8 x 3,000,009 fp32 with a bf16 wire 240 -> 116 us).  Loops that are not inlined, or two CTAs of 64 registers, spill
+// inside the loop and were slower (bucket of 4 x 26 MB: 166 and 195 us against 136 us).  Buffers whose addresses differ modulo 16 (rows
+// or slices of an odd number of elements) are read as aligned 16-byte words and shifted into place, so that they
+// move in 16-byte stores too instead of in units of the common alignment.
+constexpr int kUnroll = 8;
+
+/** 16-byte source words at any byte address: word i is bytes [16 i, 16 i + 16) of `src`.  An unaligned word is put
+ *  together from the two aligned words around it; both hold at least one byte of it, so nothing outside the 16-byte
+ *  granules that the caller's bytes occupy is touched. */
+struct WordSource {
+  const uint4* base;
+  unsigned sh;    ///< bytes that `src` lies above `base`
+  bool staging;   ///< read past L1 (staging memory changes under a running kernel)
+
+  __device__ __forceinline__ WordSource(const char* src, bool is_staging)
+      : base((const uint4*)((uintptr_t)src & ~(uintptr_t)15)), sh((unsigned)((uintptr_t)src & 15)), staging(is_staging) {}
+  __device__ __forceinline__ uint4 raw(size_t i) const { return staging ? __ldcg(base + i) : base[i]; }
+  __device__ __forceinline__ uint4 shifted(size_t i) const {
+    const uint4 a = raw(i), b = raw(i + 1);
+    const unsigned q = sh >> 2, bits = (sh & 3) * 8;
+    const uint32_t w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+    uint32_t x[5];
+#pragma unroll
+    for (int k = 0; k < 5; ++k) {
+      const uint32_t lo = q & 1 ? w[k + 1] : w[k];
+      const uint32_t hi = q & 1 ? w[k + 3 < 8 ? k + 3 : 7] : w[k + 2];
+      x[k] = q & 2 ? hi : lo;
+    }
+    return uint4{__funnelshift_r(x[0], x[1], bits), __funnelshift_r(x[1], x[2], bits), __funnelshift_r(x[2], x[3], bits),
+                 __funnelshift_r(x[3], x[4], bits)};
   }
-  for (; i < units; i += stride) d[i] = src_is_staging ? __ldcg(s + i) : s[i];
+};
+
+/** For every i in [0, units): store(i, load(i)), U independent loads per thread before the first store.  A warp takes U
+ *  rows of 32 consecutive units, so that its accesses differ by constants and share one address register. */
+template <int U, typename Load, typename Store>
+__device__ __forceinline__ void batched_units(size_t units, unsigned lane, unsigned nlanes, Load load, Store store) {
+  const unsigned warps = nlanes >> 5;   // (of a group that is no multiple of 32 threads the last few stay idle)
+  if ((lane >> 5) >= warps) return;
+  const size_t step = (size_t)warps * (32 * U);
+  uint4 v[U];
+  for (size_t i = (size_t)(lane >> 5) * (32 * U) + (lane & 31); i < units; i += step) {
+    if (i + 32 * (U - 1) < units) {
+#pragma unroll
+      for (int k = 0; k < U; ++k) v[k] = load(i + 32 * k);
+#pragma unroll
+      for (int k = 0; k < U; ++k) store(i + 32 * k, v[k]);
+    } else {
+      const unsigned left = (unsigned)((units - i + 31) >> 5);
+#pragma unroll
+      for (int k = 0; k < U; ++k)
+        if (k < left) v[k] = load(i + 32 * k);
+#pragma unroll
+      for (int k = 0; k < U; ++k)
+        if (k < left) store(i + 32 * k, v[k]);
+    }
+  }
 }
 
-/**
- * Copy `nbytes` with `nlanes` cooperating threads (this thread is `lane`).  Uses
- * the widest unit both addresses allow (16, 8, 4, 2 or 1 bytes).
- */
+/** Copy `nbytes` with `nlanes` cooperating threads (this thread is `lane`), whatever the two alignments. */
 __device__ __forceinline__ void group_copy(char* dst, const char* src, size_t nbytes, bool src_is_staging,
                                            unsigned lane, unsigned nlanes) {
   if (nbytes == 0) return;
-  const uintptr_t mis = (uintptr_t)dst | (uintptr_t)src;
-  if ((mis & 15) == 0) {
-    const size_t nv = nbytes >> 4;
-    copy_units<uint4>(dst, src, nv, src_is_staging, lane, nlanes);
-    const size_t done = nv << 4;
-    for (size_t k = lane; k < nbytes - done; k += nlanes) dst[done + k] = src[done + k];
-  } else if ((mis & 7) == 0) {
-    const size_t nv = nbytes >> 3;
-    copy_units<uint2>(dst, src, nv, src_is_staging, lane, nlanes);
-    const size_t done = nv << 3;
-    for (size_t k = lane; k < nbytes - done; k += nlanes) dst[done + k] = src[done + k];
-  } else if ((mis & 3) == 0) {
-    const size_t nv = nbytes >> 2;
-    copy_units<uint32_t>(dst, src, nv, src_is_staging, lane, nlanes);
-    const size_t done = nv << 2;
-    for (size_t k = lane; k < nbytes - done; k += nlanes) dst[done + k] = src[done + k];
-  } else if ((mis & 1) == 0) {
-    const size_t nv = nbytes >> 1;
-    copy_units<uint16_t>(dst, src, nv, src_is_staging, lane, nlanes);
-    if ((nbytes & 1) && lane == 0) dst[nbytes - 1] = src[nbytes - 1];
+  size_t head = (0 - (uintptr_t)dst) & 15;  // bytes up to the first 16-byte boundary of the destination
+  if (head > nbytes) head = nbytes;
+  const size_t nv = (nbytes - head) >> 4, done = head + (nv << 4);
+  for (size_t k = lane; k < head; k += nlanes) dst[k] = src_is_staging ? __ldcg(src + k) : src[k];
+  uint4* d = (uint4*)(dst + head);
+  const WordSource s(src + head, src_is_staging);
+  auto store = [&](size_t i, const uint4& v) { d[i] = v; };
+  if (s.sh == 0) {
+    if (src_is_staging) batched_units<kUnroll>(nv, lane, nlanes, [&](size_t i) { return __ldcg(s.base + i); }, store);
+    else batched_units<kUnroll>(nv, lane, nlanes, [&](size_t i) { return s.base[i]; }, store);
   } else {
-    copy_units<uint8_t>(dst, src, nbytes, src_is_staging, lane, nlanes);
+    batched_units<kUnroll / 4>(nv, lane, nlanes, [&](size_t i) { return s.shifted(i); }, store);
   }
+  for (size_t k = done + lane; k < nbytes; k += nlanes) dst[k] = src_is_staging ? __ldcg(src + k) : src[k];
 }
 
 /** Copy with all threads of the CTA. */
@@ -149,99 +186,103 @@ __device__ __forceinline__ void cta_copy(char* dst, const char* src, size_t nbyt
 // ---------------------------------------------------------------------------
 // publish: one local source, several (possibly remote) destinations
 // ---------------------------------------------------------------------------
-template <typename V>
-__device__ __forceinline__ void fanout_units(char* const* dsts, int ndst, size_t dst_off, const char* src, size_t units) {
-  const V* s = (const V*)src;
-  const size_t stride = blockDim.x;
-  size_t i = threadIdx.x;
-  for (; i + 3 * stride < units; i += 4 * stride) {
-    const V a = s[i], b = s[i + stride], c = s[i + 2 * stride], e = s[i + 3 * stride];
-#pragma unroll
-    for (int d = 0; d < kMaxRanks; ++d) {
-      if (d < ndst) {
-        V* o = (V*)(dsts[d] + dst_off);
-        o[i] = a; o[i + stride] = b; o[i + 2 * stride] = c; o[i + 3 * stride] = e;
-      }
-    }
-  }
-  for (; i < units; i += stride) {
-    const V a = s[i];
+/**
+ * Store `nbytes` read once from local `src` to dst(d) of every rank d whose bit is set in `ranks` (peer-mapped
+ * memory: plain stores over NVLink, which do not stall the issuing thread the way remote loads do).  Every
+ * dst(d) is 16-byte aligned; `dst` is called with compile-time ranks.
+ */
+template <typename Dst>
+__device__ __forceinline__ void cta_fanout(unsigned ranks, Dst dst, const char* src, size_t nbytes) {
+  if (nbytes == 0) return;
+  const size_t nv = nbytes >> 4, done = nv << 4;
+  const WordSource s(src, false);
+  auto store = [&](size_t i, const uint4& v) {
 #pragma unroll
     for (int d = 0; d < kMaxRanks; ++d)
-      if (d < ndst) ((V*)(dsts[d] + dst_off))[i] = a;
+      if (ranks >> d & 1) ((uint4*)dst(d))[i] = v;
+  };
+  if (s.sh == 0) batched_units<kUnroll / 2>(nv, threadIdx.x, blockDim.x, [&](size_t i) { return s.base[i]; }, store);
+  else batched_units<kUnroll / 4>(nv, threadIdx.x, blockDim.x, [&](size_t i) { return s.shifted(i); }, store);
+  if (threadIdx.x < nbytes - done) {
+#pragma unroll
+    for (int d = 0; d < kMaxRanks; ++d)
+      if (ranks >> d & 1) ((char*)dst(d))[done + threadIdx.x] = src[done + threadIdx.x];
   }
 }
 
-/**
- * Store `nbytes` read once from local `src` at byte offset `dst_off` of each of
- * `ndst` staging bases (peer-mapped memory: plain stores over NVLink, which do
- * not stall the issuing thread the way remote loads do).
- */
-__device__ __forceinline__ void cta_fanout(char* const* dsts, int ndst, size_t dst_off, const char* src, size_t nbytes) {
-  if (nbytes == 0 || ndst == 0) return;
-  const uintptr_t mis = (uintptr_t)src | (uintptr_t)dst_off;  // staging bases are 256-byte aligned
-  if ((mis & 15) == 0) {
-    const size_t nv = nbytes >> 4;
-    fanout_units<uint4>(dsts, ndst, dst_off, src, nv);
-    const size_t done = nv << 4;
-    if (threadIdx.x < (nbytes - done))
-      for (int d = 0; d < ndst; ++d) dsts[d][dst_off + done + threadIdx.x] = src[done + threadIdx.x];
-  } else if ((mis & 3) == 0) {
-    const size_t nv = nbytes >> 2;
-    fanout_units<uint32_t>(dsts, ndst, dst_off, src, nv);
-    const size_t done = nv << 2;
-    if (threadIdx.x < (nbytes - done))
-      for (int d = 0; d < ndst; ++d) dsts[d][dst_off + done + threadIdx.x] = src[done + threadIdx.x];
-  } else if ((mis & 1) == 0) {
-    const size_t nv = nbytes >> 1;
-    fanout_units<uint16_t>(dsts, ndst, dst_off, src, nv);
-    if ((nbytes & 1) && threadIdx.x == 0)
-      for (int d = 0; d < ndst; ++d) dsts[d][dst_off + nbytes - 1] = src[nbytes - 1];
-  } else {
-    fanout_units<uint8_t>(dsts, ndst, dst_off, src, nbytes);
+/** 16 bytes of wire elements converted from consecutive user elements: one or two 16-byte loads per vector. */
+template <typename Ti, typename Tw>
+struct Converter {
+  static constexpr int VEC = 16 / (int)sizeof(Tw);
+  static constexpr int in_bytes = VEC * (int)sizeof(Ti);
+  struct alignas(in_bytes < 16 ? in_bytes : 16) In { Ti e[VEC]; };
+  union Out { uint4 u; Tw e[VEC]; };
+  static __device__ __forceinline__ Tw one(Ti v) {
+    using Ai = typename Elem<Ti>::Acc;
+    using Aw = typename Elem<Tw>::Acc;
+    return Elem<Tw>::down(acc_cast<Aw, Ai>(Elem<Ti>::up(v)));
   }
-}
+  static __device__ __forceinline__ bool aligned(const Ti* src) { return (uintptr_t)src % alignof(In) == 0; }
+  static __device__ __forceinline__ uint4 word(const Ti* src, size_t i) { return convert(((const In*)src)[i]); }
+  /** The same out of staging memory (past L1). */
+  static __device__ __forceinline__ uint4 word_staged(const Ti* src, size_t i) {
+    using L = std::conditional_t<(in_bytes >= 16), uint4, std::conditional_t<in_bytes == 8, uint2, uint32_t>>;
+    union { In a; L l[in_bytes / sizeof(L)]; } x;
+#pragma unroll
+    for (int k = 0; k < (int)(in_bytes / sizeof(L)); ++k) x.l[k] = __ldcg((const L*)src + i * (in_bytes / sizeof(L)) + k);
+    return convert(x.a);
+  }
+  static __device__ __forceinline__ uint4 convert(const In& a) {
+    Out o;
+#pragma unroll
+    for (int k = 0; k < VEC; ++k) o.e[k] = one(a.e[k]);
+    return o.u;
+  }
+};
 
-/** Single destination, a subset of the CTA's threads: used to serve all peers of a small message at once. */
+/** Single destination (16-byte aligned), a subset of the CTA's threads: used to serve all peers of a small message at once. */
 template <typename Ti, typename Tw>
 __device__ __forceinline__ void group_publish(char* dst, const Ti* src, size_t n, unsigned lane, unsigned nlanes) {
   if constexpr (std::is_same<Ti, Tw>::value) {
     group_copy(dst, (const char*)src, n * sizeof(Ti), false, lane, nlanes);
   } else {
-    using Ai = typename Elem<Ti>::Acc;
-    using Aw = typename Elem<Tw>::Acc;
-    for (size_t i = lane; i < n; i += nlanes) ((Tw*)dst)[i] = Elem<Tw>::down(acc_cast<Aw, Ai>(Elem<Ti>::up(src[i])));
+    using C = Converter<Ti, Tw>;
+    const size_t nv = C::aligned(src) ? n / C::VEC : 0;
+    batched_units<2>(nv, lane, nlanes, [&](size_t i) { return C::word(src, i); }, [&](size_t i, const uint4& v) { ((uint4*)dst)[i] = v; });
+    for (size_t i = nv * C::VEC + lane; i < n; i += nlanes) ((Tw*)dst)[i] = C::one(src[i]);
   }
 }
 
-/** Publish n elements of user type Ti as wire type Tw into every destination (cast fused in). */
-template <typename Ti, typename Tw>
-__device__ __forceinline__ void cta_publish(char* const* dsts, int ndst, size_t dst_off, const Ti* src, size_t n) {
+/** Publish n elements of user type Ti as wire type Tw to dst(d) of every rank d in `ranks` (cast fused in). */
+template <typename Ti, typename Tw, typename Dst>
+__device__ __forceinline__ void cta_publish(unsigned ranks, Dst dst, const Ti* src, size_t n) {
   if constexpr (std::is_same<Ti, Tw>::value) {
-    cta_fanout(dsts, ndst, dst_off, (const char*)src, n * sizeof(Ti));
+    cta_fanout(ranks, dst, (const char*)src, n * sizeof(Ti));
   } else {
-    using Ai = typename Elem<Ti>::Acc;
-    using Aw = typename Elem<Tw>::Acc;
-    for (size_t i = threadIdx.x; i < n; i += blockDim.x) {
-      const Tw v = Elem<Tw>::down(acc_cast<Aw, Ai>(Elem<Ti>::up(src[i])));
+    using C = Converter<Ti, Tw>;
+    const size_t nv = C::aligned(src) ? n / C::VEC : 0;
+    batched_units<4>(nv, threadIdx.x, blockDim.x, [&](size_t i) { return C::word(src, i); }, [&](size_t i, const uint4& v) {
 #pragma unroll
       for (int d = 0; d < kMaxRanks; ++d)
-        if (d < ndst) ((Tw*)(dsts[d] + dst_off))[i] = v;
+        if (ranks >> d & 1) ((uint4*)dst(d))[i] = v;
+    });
+    for (size_t i = nv * C::VEC + threadIdx.x; i < n; i += blockDim.x) {
+      const Tw v = C::one(src[i]);
+#pragma unroll
+      for (int d = 0; d < kMaxRanks; ++d)
+        if (ranks >> d & 1) ((Tw*)dst(d))[i] = v;
     }
   }
 }
 
-/** dst[i] = (Tw)src[i] for i in [0, n): the publish step of an operation whose wire type differs. */
-template <typename Ti, typename Tw>
-__device__ __forceinline__ void cta_convert(Tw* dst, const Ti* src, size_t n) {
-  if constexpr (std::is_same<Ti, Tw>::value) {
-    cta_copy((char*)dst, (const char*)src, n * sizeof(Ti), false);
-  } else {
-    using Ai = typename Elem<Ti>::Acc;
-    using Aw = typename Elem<Tw>::Acc;
-    for (size_t i = threadIdx.x; i < n; i += blockDim.x)
-      dst[i] = Elem<Tw>::down(acc_cast<Aw, Ai>(Elem<Ti>::up(src[i])));
-  }
+/** Copy n staged elements (16-byte aligned) of type Tw out as To. */
+template <typename Tw, typename To>
+__device__ __forceinline__ void cta_expand(To* dst, const Tw* src, size_t n) {
+  using C = Converter<Tw, To>;
+  const size_t nv = (uintptr_t)dst % 16 == 0 ? n / C::VEC : 0;
+  batched_units<4>(nv, threadIdx.x, blockDim.x, [&](size_t i) { return C::word_staged(src, i); },
+                   [&](size_t i, const uint4& v) { ((uint4*)dst)[i] = v; });
+  for (size_t i = nv * C::VEC + threadIdx.x; i < n; i += blockDim.x) dst[i] = C::one(__ldcg(src + i));
 }
 
 // ---------------------------------------------------------------------------
@@ -257,26 +298,25 @@ __device__ __forceinline__ A finish_acc(A a, double scale, int int_div) {
 }
 
 /**
- * out[i] = finish(red(src_0[i], src_1[i], ..., src_{p-1}[i])) for i in [0, n),
- * where src_r = (const Tw*)(bases[r] + byte_off), written to each of the `ndst`
- * destinations dsts[d] (all holding To elements; several destinations are used
- * when a reduced slice is pushed to every peer).  Sources are staging memory
- * (16-byte aligned); contributions are folded in rank order so every rank
- * computes bit-identical results.  A destination may alias one of the sources.  Sources that are
- * not 16-byte aligned are read element by element.
+ * out[i] = finish(red(src(0)[i], src(1)[i], ..., src(p-1)[i])) for i in [0, n), written to dst(d) for every
+ * rank d in `ranks` (several destinations are used when a reduced slice is pushed to every peer).  src(r) gives
+ * the first Tw element of rank r's contribution, dst(d) the first To element of a destination; both are called with
+ * compile-time ranks.  Contributions are folded in rank order so every rank computes
+ * bit-identical results.  A destination may alias one of the sources.  Where an address is not 16-byte aligned
+ * everything is read element by element.
  */
-template <typename Tw, typename To, typename Red>
-__device__ __forceinline__ void cta_reduce(To* const* dsts, int ndst, char* const* bases, size_t byte_off, int p,
-                                           size_t n, Red red, double scale, int int_div) {
+template <typename Tw, typename To, typename Red, typename Src, typename Dst>
+__device__ __forceinline__ void reduce_to(unsigned ranks, Dst dst, Src src, int p, size_t n, Red red, double scale, int int_div) {
   using Aw = typename Elem<Tw>::Acc;
   using Ao = typename Elem<To>::Acc;
   constexpr int VEC = 16 / (int)sizeof(Tw);
   constexpr size_t out_bytes = (size_t)VEC * sizeof(To);
   constexpr size_t out_align = out_bytes < 16 ? out_bytes : 16;
   bool aligned = true;
-  for (int d = 0; d < ndst; ++d) aligned = aligned && ((uintptr_t)dsts[d] % out_align == 0);
-  // staging sources always are 16-byte aligned; registered user buffers (window kernels) need not be
-  for (int r = 0; r < p; ++r) aligned = aligned && ((uintptr_t)(bases[r] + byte_off) % 16 == 0);
+#pragma unroll
+  for (int d = 0; d < kMaxRanks; ++d) aligned = aligned && (!(ranks >> d & 1) || (uintptr_t)dst(d) % out_align == 0);
+#pragma unroll
+  for (int r = 0; r < kMaxRanks; ++r) aligned = aligned && (r >= p || (uintptr_t)src(r) % 16 == 0);
   const size_t nvec = aligned ? n / VEC : 0;
   union InPack { uint4 u; Tw e[VEC]; };
   union OutPack { uint4 u[(out_bytes + 15) / 16]; To e[VEC]; };
@@ -284,65 +324,77 @@ __device__ __forceinline__ void cta_reduce(To* const* dsts, int ndst, char* cons
   auto store = [&](size_t v, const OutPack& o) {
 #pragma unroll
     for (int d = 0; d < kMaxRanks; ++d) {
-      if (d < ndst) {
-        To* dst = dsts[d];
+      if (ranks >> d & 1) {
+        To* out = dst(d);
         if constexpr (out_bytes >= 16) {
 #pragma unroll
-          for (int q = 0; q < (int)(out_bytes / 16); ++q) ((uint4*)dst)[v * (out_bytes / 16) + q] = o.u[q];
+          for (int q = 0; q < (int)(out_bytes / 16); ++q) ((uint4*)out)[v * (out_bytes / 16) + q] = o.u[q];
         } else if constexpr (out_bytes == 8) {
-          ((uint2*)dst)[v] = *(const uint2*)&o.u[0];
+          ((uint2*)out)[v] = *(const uint2*)&o.u[0];
         } else {
-          ((uint32_t*)dst)[v] = *(const uint32_t*)&o.u[0];
+          ((uint32_t*)out)[v] = *(const uint32_t*)&o.u[0];
         }
       }
     }
   };
 
-  for (size_t v = threadIdx.x; v < nvec; v += 2 * (size_t)blockDim.x) {
-    const size_t v2 = v + blockDim.x;
-    const bool has2 = v2 < nvec;
-    Aw acc0[VEC], acc1[VEC];
+  // Every rank's words are under way before the first one is folded (eight 16-byte loads per thread: two vectors of up
+  // to four ranks, one of up to eight): one memory latency per round instead of one per rank.
+  const size_t stride = blockDim.x;
+  auto rounds = [&](auto most, auto vecs) __attribute__((always_inline)) {
+    constexpr int R = decltype(most)::value, U = decltype(vecs)::value;
+    for (size_t v = (size_t)(threadIdx.x >> 5) * (32 * U) + (threadIdx.x & 31); v < nvec; v += stride * U) {
+      InPack in[R][U];
 #pragma unroll
-    for (int r = 0; r < kMaxRanks; ++r) {
-      if (r < p) {
-        const uint4* s = (const uint4*)(bases[r] + byte_off);
-        InPack a, b;
-        a.u = __ldcg(s + v);
-        if (has2) b.u = __ldcg(s + v2);
-#pragma unroll
-        for (int k = 0; k < VEC; ++k) {
-          const Aw x = Elem<Tw>::up(a.e[k]);
-          acc0[k] = r == 0 ? x : red(acc0[k], x);
-          if (has2) {
-            const Aw y = Elem<Tw>::up(b.e[k]);
-            acc1[k] = r == 0 ? y : red(acc1[k], y);
-          }
+      for (int r = 0; r < R; ++r) {
+        if (r < p) {
+          const uint4* s = (const uint4*)src(r) + v;
+          in[r][0].u = __ldcg(s);
+          if constexpr (U == 2) in[r][1].u = v + 32 < nvec ? __ldcg(s + 32) : uint4{0, 0, 0, 0};
         }
       }
-    }
-    OutPack o;
 #pragma unroll
-    for (int k = 0; k < VEC; ++k) o.e[k] = Elem<To>::down(acc_cast<Ao, Aw>(finish_acc(acc0[k], scale, int_div)));
-    store(v, o);
-    if (has2) {
+      for (int u = 0; u < U; ++u) {
+        Aw acc[VEC];
 #pragma unroll
-      for (int k = 0; k < VEC; ++k) o.e[k] = Elem<To>::down(acc_cast<Ao, Aw>(finish_acc(acc1[k], scale, int_div)));
-      store(v2, o);
+        for (int k = 0; k < VEC; ++k) acc[k] = Elem<Tw>::up(in[0][u].e[k]);
+#pragma unroll
+        for (int r = 1; r < R; ++r)
+          if (r < p) {
+#pragma unroll
+            for (int k = 0; k < VEC; ++k) acc[k] = red(acc[k], Elem<Tw>::up(in[r][u].e[k]));
+          }
+        OutPack o;
+#pragma unroll
+        for (int k = 0; k < VEC; ++k) o.e[k] = Elem<To>::down(acc_cast<Ao, Aw>(finish_acc(acc[k], scale, int_div)));
+        if (u == 0 || v + 32 * u < nvec) store(v + 32 * u, o);
+      }
     }
-  }
-  // scalar remainder (and the whole range when a destination is not aligned for vector stores)
-  for (size_t i = nvec * VEC + threadIdx.x; i < n; i += blockDim.x) {
+  };
+  if (p <= kMaxRanks / 2) rounds(std::integral_constant<int, kMaxRanks / 2>(), std::integral_constant<int, 2>());
+  else rounds(std::integral_constant<int, kMaxRanks>(), std::integral_constant<int, 1>());
+  // scalar remainder (and the whole range when an address is not aligned for vector accesses)
+  for (size_t i = nvec * VEC + threadIdx.x; i < n; i += stride) {
     Aw acc = Aw();
 #pragma unroll
     for (int r = 0; r < kMaxRanks; ++r) {
       if (r < p) {
-        const Aw x = Elem<Tw>::up(__ldcg((const Tw*)(bases[r] + byte_off) + i));
+        const Aw x = Elem<Tw>::up(__ldcg((const Tw*)src(r) + i));
         acc = r == 0 ? x : red(acc, x);
       }
     }
     const To out = Elem<To>::down(acc_cast<Ao, Aw>(finish_acc(acc, scale, int_div)));
-    for (int d = 0; d < ndst; ++d) dsts[d][i] = out;
+#pragma unroll
+    for (int d = 0; d < kMaxRanks; ++d)
+      if (ranks >> d & 1) dst(d)[i] = out;
   }
+}
+
+/** One destination, contributions at bases[r] + byte_off. */
+template <typename Tw, typename To, typename Red>
+__device__ __forceinline__ void cta_reduce(To* out, char* const* bases, size_t byte_off, int p, size_t n, Red red, double scale,
+                                           int int_div) {
+  reduce_to<Tw, To>(1u, [&](int) { return out; }, [&](int r) { return bases[r] + byte_off; }, p, n, red, scale, int_div);
 }
 
 }  // namespace device

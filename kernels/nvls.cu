@@ -56,7 +56,7 @@ __device__ __forceinline__ void reduce_vectors(const char* mc_in, char* mc_out, 
 }
 
 template <typename T, NvOp OP>
-__global__ void __launch_bounds__(512) nvls_allreduce_kernel(const __grid_constant__ NvlsParams P) {
+__global__ void __launch_bounds__(512, 2) nvls_allreduce_kernel(const __grid_constant__ NvlsParams P) {
   const Workspace& ws = P.ws;
   const int p = ws.p, rank = P.rank;
   if (poisoned(ws, rank)) return;
@@ -132,7 +132,7 @@ __global__ void __launch_bounds__(512) nvls_allreduce_kernel(const __grid_consta
  * IN only looks at its own, the closing wait looks at all).
  */
 template <typename T, NvOp OP>
-__global__ void __launch_bounds__(512) nvls_allreduce_pipelined_kernel(const __grid_constant__ NvlsParams P) {
+__global__ void __launch_bounds__(512, 2) nvls_allreduce_pipelined_kernel(const __grid_constant__ NvlsParams P) {
   const Workspace& ws = P.ws;
   const int p = ws.p, rank = P.rank;
   if (poisoned(ws, rank)) return;
@@ -217,7 +217,7 @@ __global__ void __launch_bounds__(512) nvls_allreduce_pipelined_kernel(const __g
  * include/aluminum/nccl_impl.hpp:1306.)
  */
 template <typename T, NvOp OP>
-__global__ void __launch_bounds__(512) nvls_reduce_scatter_kernel(const __grid_constant__ NvlsParams P) {
+__global__ void __launch_bounds__(512, 2) nvls_reduce_scatter_kernel(const __grid_constant__ NvlsParams P) {
   constexpr int VEC = 16 / (int)sizeof(T);
   const Workspace& ws = P.ws;
   const int p = ws.p, rank = P.rank;

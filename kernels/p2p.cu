@@ -67,7 +67,7 @@ __device__ __forceinline__ void group_arrive(uint64_t* counter_slot, unsigned gr
   }
 }
 
-__global__ void __launch_bounds__(512) p2p_kernel(const __grid_constant__ P2PParams P) {
+__global__ void __launch_bounds__(512, 2) p2p_kernel(const __grid_constant__ P2PParams P) {
   const Workspace& ws = P.ws;
   const unsigned group = (unsigned)P.ctas_per_item;
   const int item = (int)(blockIdx.x / group);

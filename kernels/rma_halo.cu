@@ -16,7 +16,7 @@ namespace device {
 
 namespace {
 
-__global__ void __launch_bounds__(512) put_kernel(char* dst, const char* src, size_t bytes) {
+__global__ void __launch_bounds__(512, 2) put_kernel(char* dst, const char* src, size_t bytes) {
   size_t lo, hi;
   split_range(bytes, blockIdx.x, gridDim.x, 16, lo, hi);
   if (hi > lo) cta_copy(dst + lo, src + lo, hi - lo, false);
@@ -57,7 +57,7 @@ __device__ __forceinline__ void copy_planes(float* dst, const float* src, size_t
   }
 }
 
-__global__ void __launch_bounds__(512) halo_exchange_kernel(const __grid_constant__ HaloParams P) {
+__global__ void __launch_bounds__(512, 2) halo_exchange_kernel(const __grid_constant__ HaloParams P) {
   const Workspace& ws = P.ws;
   const int rank = P.rank0 + (int)blockIdx.y;
   if (poisoned(ws, rank)) return;
@@ -132,7 +132,7 @@ __global__ void __launch_bounds__(512) halo_exchange_kernel(const __grid_constan
   }
 }
 
-__global__ void __launch_bounds__(512) halo_pack_kernel(float* packed, const float* tensor, size_t nc, size_t d_total,
+__global__ void __launch_bounds__(512, 2) halo_pack_kernel(float* packed, const float* tensor, size_t nc, size_t d_total,
                                                         size_t plane, size_t d_first, size_t depth, int unpack) {
   const size_t seg = depth * plane, total = nc * seg;
   size_t lo, hi;

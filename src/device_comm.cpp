@@ -153,6 +153,48 @@ int slots_cfg() { return std::max(2, std::min(16, tuning().dev_mailbox_slots)); 
 /** Packet slot of the point-to-point path: twice the largest payload (every 8 bytes carry 4 of payload). */
 size_t p2p_ll_slot_cfg() { return 2 * round_up(std::min(tuning().p2p_ll_max_bytes, kP2PLLMaxPayloadBytes), (size_t)4096); }
 
+/**
+ * May rank r's contribution to its own result skip its staging slot?  Staging makes any overlap of the two buffers safe
+ * (everything is read before anything is written), so the direct route is taken only where the bytes that are
+ * written cannot be bytes that another thread still has to read: where the own slice lies on the place it would be
+ * copied or reduced to (in place), or where the ranges do not meet.  A reduction reads the own slice together with
+ * staged ones in 16-byte vectors and wants it aligned.
+ */
+bool own_may_skip_staging(DevColl kind, const RankArgs& a, const CountTable& T, size_t count, int p, int r, int root,
+                          bool two_phase, size_t esz, size_t esz_out) {
+  if (!a.send || !a.recv) return false;
+  const char* send = (const char*)a.send;
+  const char* recv = (const char*)a.recv;
+  auto apart = [](const char* x, size_t nx, const char* y, size_t ny) { return x + nx <= y || y + ny <= x; };
+  auto extent = [&](const size_t* counts, const size_t* displs) {
+    size_t m = 0;
+    for (int i = 0; i < p; ++i)
+      if (counts[i]) m = std::max(m, displs[i] + counts[i]);
+    return m * esz;
+  };
+  switch (kind) {
+    case DevColl::allreduce:
+    case DevColl::reduce:
+      if (kind == DevColl::reduce && r != root) return false;
+      if ((uintptr_t)send % 16 != 0 || (two_phase && (uintptr_t)recv % 16 != 0)) return false;
+      return (send == recv && esz == esz_out) || apart(send, count * esz, recv, count * esz_out);
+    case DevColl::reduce_scatter: {
+      const char* own = send + T.send_displs[r] * esz;
+      const size_t n = T.recv_counts[r] * esz;
+      return (uintptr_t)own % 16 == 0 && ((own == recv && esz == esz_out) || apart(own, n, recv, T.recv_counts[r] * esz_out));
+    }
+    case DevColl::allgather:
+    case DevColl::alltoall: {
+      const bool ag = kind == DevColl::allgather;
+      if (T.send_counts[r] != T.recv_counts[r] || esz != esz_out) return false;
+      const char* own = send + (ag ? 0 : T.send_displs[r] * esz);
+      const size_t all = ag ? T.send_counts[r] * esz : extent(T.send_counts, T.send_displs);
+      return own == recv + T.recv_displs[r] * esz || apart(send, all, recv, extent(T.recv_counts, T.recv_displs));
+    }
+    default: return false;
+  }
+}
+
 void require_device() {
   if (!cuda::device_usable()) throw_al_exception("the device backend needs a CUDA device, none is usable in this process");
 }
@@ -440,13 +482,7 @@ void DeviceCommunicator::collective(const CollDesc& d, const std::vector<RankArg
     }
     if (algo != AllreduceAlgo::nvls) zero_copy = false;
     P.two_phase = algo == AllreduceAlgo::two_shot ? 1 : 0;
-    if (algo == AllreduceAlgo::one_shot && in == wire && p > 1) {
-      bool aligned = true;
-      for (const RankArgs& a : ranks) aligned = aligned && a.send && (uintptr_t)a.send % 16 == 0;
-      P.own_direct = aligned ? 1 : 0;
-    }
   }
-
 
   // Registered buffers: reduce_scatter (send side) and allgather / alltoall / bcast (receive side) run
   // straight on them.  The decision looks at this rank's buffers only; the kernels compare protocols
@@ -548,6 +584,34 @@ void DeviceCommunicator::collective(const CollDesc& d, const std::vector<RankArg
     throw_al_exception("the nvls path serves reduce_scatter (for allreduce use AllreduceAlgo::nvls)");
   }
 
+  for (int lr = 0; lr < I.nlocal; ++lr) {
+    const int r = I.rank0 + lr;
+    const RankArgs& a = ranks[(size_t)lr];
+    P.send[r] = a.send;
+    P.recv[r] = a.recv;
+    CountTable& T = P.tab[r];
+    if (d.vector) {
+      auto fill = [&](size_t* dst, const std::vector<size_t>& src, const char* what) {
+        if (src.empty()) { for (int i = 0; i < p; ++i) dst[i] = 0; return; }
+        if ((int)src.size() != p) throw_al_exception(what, " must have one entry per rank");
+        for (int i = 0; i < p; ++i) dst[i] = src[(size_t)i] * unit;
+      };
+      fill(T.send_counts, a.send_counts, "send counts");
+      fill(T.send_displs, a.send_displs, "send displacements");
+      fill(T.recv_counts, a.recv_counts, "receive counts");
+      fill(T.recv_displs, a.recv_displs, "receive displacements");
+    } else {
+      for (int i = 0; i < p; ++i) {
+        T.send_counts[i] = T.recv_counts[i] = d.count * unit;
+        T.send_displs[i] = T.recv_displs[i] = (size_t)i * d.count * unit;
+      }
+    }
+    P.own_direct[r] = p > 1 && in == wire && (wire == out || !P.two_phase) && algo != AllreduceAlgo::nvls &&
+                              own_may_skip_staging(d.kind, a, T, P.count, p, r, d.root, P.two_phase != 0, dtype_size(in), dtype_size(out))
+                          ? 1
+                          : 0;
+  }
+
   // Large uniform reduce_scatter / allgather / alltoall run pipelined: smaller chunks, half of the
   // grid publishing while the other half consumes.
   // The one-shot allreduce of two ranks joins them: half of the grid pushes chunk c+1 to the peer while the
@@ -571,26 +635,7 @@ void DeviceCommunicator::collective(const CollDesc& d, const std::vector<RankArg
 
   for (int lr = 0; lr < I.nlocal; ++lr) {
     const int r = I.rank0 + lr;
-    const RankArgs& a = ranks[(size_t)lr];
-    P.send[r] = a.send;
-    P.recv[r] = a.recv;
-    CountTable& T = P.tab[r];
-    if (d.vector) {
-      auto fill = [&](size_t* dst, const std::vector<size_t>& src, const char* what) {
-        if (src.empty()) { for (int i = 0; i < p; ++i) dst[i] = 0; return; }
-        if ((int)src.size() != p) throw_al_exception(what, " must have one entry per rank");
-        for (int i = 0; i < p; ++i) dst[i] = src[(size_t)i] * unit;
-      };
-      fill(T.send_counts, a.send_counts, "send counts");
-      fill(T.send_displs, a.send_displs, "send displacements");
-      fill(T.recv_counts, a.recv_counts, "receive counts");
-      fill(T.recv_displs, a.recv_displs, "receive displacements");
-    } else {
-      for (int i = 0; i < p; ++i) {
-        T.send_counts[i] = T.recv_counts[i] = d.count * unit;
-        T.send_displs[i] = T.recv_displs[i] = (size_t)i * d.count * unit;
-      }
-    }
+    const CountTable& T = P.tab[r];
     size_t need = 0, chunk_unit = full_e, work = 0;
     auto mx = [&](const size_t* v) { size_t m = 0; for (int i = 0; i < p; ++i) m = std::max(m, v[i]); return m; };
     switch (d.kind) {
