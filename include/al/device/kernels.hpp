@@ -31,6 +31,11 @@ void launch_collective(const CollParams& P, DType in, DType wire, DType out, int
 /** True when (in, wire, out, op) has a compiled kernel. */
 bool collective_supported(DType in, DType wire, DType out, ReductionOperator op);
 
+// ---- staged operations with all ranks on this GPU, moved by the bulk copy engine (kernels/bulk_staged.cu) ----
+/** Element type and operator; the kernel also wants 16-byte aligned buffers (and slices) and P.own_direct on every rank. */
+bool bulk_staged_supported(DevColl kind, DType dt, ReductionOperator op);
+void launch_bulk_staged(const CollParams& P, DType dt, int ctas, int local_ranks, cudaStream_t stream);
+
 // ---- bulk-copy pipeline (kernels/bulk_pipeline.cu) ------------------------------
 /**
  * Large uniform allgather / alltoall (dt = u8, counts in bytes) and sum

@@ -195,6 +195,9 @@ bool own_may_skip_staging(DevColl kind, const RankArgs& a, const CountTable& T, 
   }
 }
 
+/** Smallest vector (or whole message) that the bulk copy engine moves when all ranks are on one GPU. */
+constexpr size_t kBulkStagedMinBytes = size_t{1} << 20;
+
 void require_device() {
   if (!cuda::device_usable()) throw_al_exception("the device backend needs a CUDA device, none is usable in this process");
 }
@@ -612,6 +615,13 @@ void DeviceCommunicator::collective(const CollDesc& d, const std::vector<RankArg
                           : 0;
   }
 
+  // All ranks on this GPU: large operations are moved by the bulk copy engine, chunked by what staging holds.
+  bool bulk_staged = I.nlocal > 1 && !use_window && !d.vector && d.ctas <= 0 && !tn.bulk_pipeline && in == wire && wire == out &&
+                     bulk_staged_supported(d.kind, wire, d.op) && (d.kind == DevColl::allreduce || P.count * esz % 16 == 0) &&
+                     P.count * esz * (d.kind == DevColl::allreduce ? 1 : (size_t)p) >= kBulkStagedMinBytes;
+  for (int r = 0; bulk_staged && r < p; ++r)
+    bulk_staged = P.own_direct[r] && (uintptr_t)P.send[r] % 16 == 0 && (uintptr_t)P.recv[r] % 16 == 0;
+
   // Large uniform reduce_scatter / allgather / alltoall run pipelined: smaller chunks, half of the
   // grid publishing while the other half consumes.
   // The one-shot allreduce of two ranks joins them: half of the grid pushes chunk c+1 to the peer while the
@@ -622,8 +632,8 @@ void DeviceCommunicator::collective(const CollDesc& d, const std::vector<RankArg
   // (Real ranks also pipeline as soon as a slice does not fit one staging slot: the alternative would be
   // several chunks one after the other, each with its handshakes exposed.)
   const bool slice_exceeds_slot = !I.emulated && P.count > cap_e;
-  if (((d.kind == DevColl::reduce_scatter || d.kind == DevColl::allgather || d.kind == DevColl::alltoall) && !d.vector &&
-       p > 1 && !use_window && (P.count * esz >= X.pipeline_min_bytes || slice_exceeds_slot)) || ar_pipelined) {
+  if (!bulk_staged && (((d.kind == DevColl::reduce_scatter || d.kind == DevColl::allgather || d.kind == DevColl::alltoall) && !d.vector &&
+       p > 1 && !use_window && (P.count * esz >= X.pipeline_min_bytes || slice_exceeds_slot)) || ar_pipelined)) {
     size_t chunk_b = std::max<size_t>(P.count * esz / 8, size_t{4} << 20);
     chunk_b = std::min(chunk_b / 256 * 256, cap_e * esz);
     if (chunk_b >= 256 && chunk_b < P.count * esz) {
@@ -757,6 +767,7 @@ void DeviceCommunicator::collective(const CollDesc& d, const std::vector<RankArg
       return;
     }
   }
+  if (bulk_staged) return launch_bulk_staged(P, wire, I.sm_count / I.nlocal, I.nlocal, stream);
   launch_collective(P, in, wire, out, ctas, threads, I.nlocal, stream);
 }
 

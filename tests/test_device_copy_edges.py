@@ -107,3 +107,42 @@ def test_converted_wire(comm, wire, shift):
             for x in xs:
                 assert torch.equal(x, want)   # integers of at most 48: exact in both 16-bit types
 
+
+@pytest.mark.parametrize("p", [2, 3, 4, 8])
+@pytest.mark.parametrize("stage", [1 << 20, 64 << 20])
+def test_large_operations_in_bulk_copies(al, p, stage):
+    """Around tiles of 32 KiB, shares of a CTA and (small staging) several chunks; ragged vectors, in place and not."""
+    old = al.get_tuning("dev_stage_bytes")
+    al.set_tuning("dev_stage_bytes", stage)
+    comm = al.DeviceComm(emulate=p)
+    al.set_tuning("dev_stage_bytes", old)
+    for dtype, n in ((torch.float32, 262144), (torch.float32, 1310727), (torch.bfloat16, 524288 + 9), (torch.bfloat16, 3000003)):
+        xs = [small_ints(n, dtype, r) for r in range(p)]
+        want = sum(x.float() for x in xs).to(dtype)
+        outs = [torch.empty_like(x) for x in xs]
+        comm.allreduce(xs, outs, algo="two_shot" if p > 2 else "auto")
+        assert all(torch.equal(o, want) for o in outs)
+        comm.allreduce(xs, algo="two_shot" if p > 2 else "one_shot")
+        assert all(torch.equal(x, want) for x in xs)
+    for dtype, n in ((torch.bfloat16, 262144), (torch.float32, 131072 * 3 + 4), (torch.float32, 655360 + 12)):
+        full = [small_ints(p * n, dtype, 50 + r) for r in range(p)]
+        want = sum(f.float() for f in full).to(dtype)
+        outs = [torch.empty(n, device="cuda", dtype=dtype) for _ in range(p)]
+        comm.reduce_scatter(full, outs, algo="staged")
+        assert all(torch.equal(outs[r], want[r * n:(r + 1) * n]) for r in range(p))
+        all_outs = [torch.empty_like(f) for f in full]
+        comm.allgather(outs, all_outs, algo="staged")
+        assert all(torch.equal(o, want) for o in all_outs)
+        comm.alltoall(full, all_outs, algo="staged")
+        moved = [torch.cat([f[r * n:(r + 1) * n] for f in full]) for r in range(p)]
+        assert all(torch.equal(all_outs[r], moved[r]) for r in range(p))
+        both = [f.clone() for f in full]
+        comm.alltoall(both, algo="staged")
+        assert all(torch.equal(both[r], moved[r]) for r in range(p))
+        both = [f.clone() for f in full]
+        comm.reduce_scatter(both, algo="staged")
+        assert all(torch.equal(both[r][:n], want[r * n:(r + 1) * n]) for r in range(p))
+        both = [f.clone() for f in full]
+        comm.allgather(both, algo="staged")
+        assert all(torch.equal(b, torch.cat([full[r][r * n:(r + 1) * n] for r in range(p)])) for b in both)
+    comm.close()
