@@ -21,6 +21,7 @@ ROOT = Path(__file__).resolve().parent.parent
 PKG = ROOT / "aluminum_b200"
 OBJ = ROOT / "build" / "obj"
 LIB = PKG / "lib" / "libal_b200.so"
+TORCH_LIB = PKG / "lib" / "libal_torch.so"  # autograd operators (src/torch), linked against PyTorch
 BIN = PKG / "bin"
 
 CUDA_HOME = Path(os.environ.get("CUDA_HOME", "/usr/local/cuda"))
@@ -68,6 +69,12 @@ def _headers_digest() -> str:
     return h.hexdigest()
 
 
+def _torch_dir() -> Path:
+    """PyTorch's folder, without importing it."""
+    import importlib.util
+    return Path(next(iter(importlib.util.find_spec("torch").submodule_search_locations)))
+
+
 def _needs(obj: Path, src: Path, stamp: str) -> bool:
     tag = obj.with_suffix(obj.suffix + ".stamp")
     if not obj.exists() or not tag.exists():
@@ -93,6 +100,10 @@ def _compile(src: Path, stamp: str) -> Path:
     if _needs(obj, src, stamp):
         if src.suffix == ".cu":
             _run([NVCC] + NVCCFLAGS + ["-c", str(src), "-o", str(obj)])
+        elif src.parent.name == "torch":
+            inc = _torch_dir() / "include"
+            _run([CXX] + [f for f in CXXFLAGS if f not in ("-Wall", "-Wextra")] +
+                 [f"-isystem{inc}", f"-isystem{inc / 'torch' / 'csrc' / 'api' / 'include'}", "-c", str(src), "-o", str(obj)])
         else:
             _run([CXX] + CXXFLAGS + ["-c", str(src), "-o", str(obj)])
         _mark(obj, src, stamp)
@@ -112,15 +123,21 @@ def build(tools: bool = True, jobs: int | None = None, verbose: bool = False) ->
     BIN.mkdir(parents=True, exist_ok=True)
     stamp = _headers_digest() + hashlib.sha1(" ".join(CXXFLAGS + NVCCFLAGS).encode()).hexdigest()
     jobs = jobs or max(1, (os.cpu_count() or 4))
+    torch_srcs = sorted((ROOT / "src" / "torch").glob("*.cpp"))
     srcs = library_sources()
     with ThreadPoolExecutor(jobs) as ex:
-        objs = list(ex.map(lambda s: _compile(s, stamp), srcs))
+        objs = list(ex.map(lambda s: _compile(s, stamp), torch_srcs + srcs))
+    torch_objs, objs = objs[:len(torch_srcs)], objs[len(torch_srcs):]
     newest = max(o.stat().st_mtime_ns for o in objs)
     if not LIB.exists() or LIB.stat().st_mtime_ns < newest:
         _run([NVCC] + GENCODE + ["-shared", "-o", str(LIB)] + [str(o) for o in objs] +
              ["-lpthread", "-ldl", "-lrt"])
         if verbose:
             print(f"linked {LIB}")
+    if not TORCH_LIB.exists() or TORCH_LIB.stat().st_mtime_ns < max(o.stat().st_mtime_ns for o in torch_objs + [LIB]):
+        _run([CXX, "-shared", "-o", str(TORCH_LIB)] + [str(o) for o in torch_objs] +
+             [f"-L{LIB.parent}", "-lal_b200", f"-L{_torch_dir() / 'lib'}", "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-lc10", "-lc10_cuda",
+              "-Wl,-rpath,$ORIGIN"])
     if tools:
         todo = {n: [ROOT / s for s in ss] for n, ss in TOOLS.items() if all((ROOT / s).exists() for s in ss)}
 

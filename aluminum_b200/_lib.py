@@ -83,6 +83,8 @@ def _declare(lib) -> None:
         "al_scale_cast": (i, [vp, i, vp, i, sz, d, vp]),
         "al_sgd_momentum": (i, [vp, vp, vp, sz, C.c_float, C.c_float, C.c_float, C.c_float, i, i, vp]),
         "al_fill_u32": (i, [vp, sz, C.c_uint32, vp]),
+        "al_bn_forward": (i, [i] + [vp] * 12 + [sz, sz, i, C.c_float, C.c_float, vp]),
+        "al_bn_backward": (i, [i] + [vp] * 11 + [sz, sz, i, vp]),
     }
     for name, (res, args) in sig.items():
         fn = getattr(lib, name)
@@ -105,6 +107,23 @@ def load():
         _declare(lib)
         _lib = lib
         return lib
+
+
+_torch_ops = None
+
+
+def torch_ops():
+    """The autograd operators (``torch.ops.aluminum_b200``); their library is part of the build."""
+    global _torch_ops
+    if _torch_ops is None:
+        import torch
+        load()
+        path = _LIB_PATH.with_name("libal_torch.so")
+        if not path.exists():
+            raise AlError(f"native library missing: {path}")
+        torch.ops.load_library(str(path))
+        _torch_ops = torch.ops.aluminum_b200
+    return _torch_ops
 
 
 def check(rc: int) -> None:

@@ -11,6 +11,8 @@ from __future__ import annotations
 import torch
 from torch import nn
 
+from ..ops.batchnorm import batch_norm_act
+
 
 class Bottleneck(nn.Module):
     expansion = 4
@@ -27,11 +29,30 @@ class Bottleneck(nn.Module):
         self.downsample = downsample
 
     def forward(self, x):
-        identity = x if self.downsample is None else self.downsample(x)
-        out = self.relu(self.bn1(self.conv1(x)))
-        out = self.relu(self.bn2(self.conv2(out)))
-        out = self.bn3(self.conv3(out))
-        return self.relu(out + identity)
+        if torch.jit.is_scripting():
+            identity = x if self.downsample is None else self.downsample(x)
+            out = self.relu(self.bn1(self.conv1(x)))
+            out = self.relu(self.bn2(self.conv2(out)))
+            out = self.bn3(self.conv3(out))
+            return self.relu(out + identity)
+        else:
+            # training on the GPU: normalisation, residual addition and ReLU in one pass (the modules otherwise)
+            identity = x if self.downsample is None else self.downsample(x)
+            out = batch_norm_act(self.bn1, self.conv1(x), self.relu)
+            out = batch_norm_act(self.bn2, self.conv2(out), self.relu)
+            return batch_norm_act(self.bn3, self.conv3(out), self.relu, identity)
+
+
+class Shortcut(nn.Sequential):
+    """Convolution and batch norm of a block whose input and output differ in shape."""
+
+    def forward(self, x):
+        if torch.jit.is_scripting():
+            for m in self:
+                x = m(x)
+            return x
+        else:
+            return batch_norm_act(self[1], self[0](x))
 
 
 class ResNet(nn.Module):
@@ -61,15 +82,19 @@ class ResNet(nn.Module):
     def _stage(self, width: int, blocks: int, stride: int) -> nn.Sequential:
         down = None
         if stride != 1 or self.c != width * Bottleneck.expansion:
-            down = nn.Sequential(nn.Conv2d(self.c, width * Bottleneck.expansion, 1, stride=stride, bias=False),
-                                 nn.BatchNorm2d(width * Bottleneck.expansion))
+            down = Shortcut(nn.Conv2d(self.c, width * Bottleneck.expansion, 1, stride=stride, bias=False),
+                            nn.BatchNorm2d(width * Bottleneck.expansion))
         mods = [Bottleneck(self.c, width, stride, down)]
         self.c = width * Bottleneck.expansion
         mods += [Bottleneck(self.c, width) for _ in range(1, blocks)]
         return nn.Sequential(*mods)
 
     def forward(self, x):
-        x = self.maxpool(self.relu(self.bn1(self.conv1(x))))
+        if torch.jit.is_scripting():
+            x = self.relu(self.bn1(self.conv1(x)))
+        else:
+            x = batch_norm_act(self.bn1, self.conv1(x), self.relu)
+        x = self.maxpool(x)
         x = self.layer4(self.layer3(self.layer2(self.layer1(x))))
         return self.fc(torch.flatten(self.avgpool(x), 1))
 

@@ -1,0 +1,61 @@
+"""Training batch norm of channels-last activations with the residual addition and the ReLU behind it fused in
+(``kernels/batchnorm.cu``, autograd in ``src/torch/batchnorm_autograd.cpp``).
+
+:func:`batch_norm_act` takes the modules that a network holds (``nn.BatchNorm2d``, ``nn.ReLU``) and runs the fused kernels
+where they do exactly what the modules would: 16-bit channels-last CUDA activations in training, plain modules without
+hooks, ordinary reverse-mode autograd.  Everything else - evaluation, other types and layouts, hooks, tracing,
+functorch transforms, forward-mode AD - calls the modules.
+"""
+from __future__ import annotations
+
+import torch
+from torch import nn
+from torch.autograd import forward_ad
+
+from .. import _lib
+
+_TYPES = (torch.bfloat16, torch.float16)
+
+
+def _bare(m: nn.Module) -> bool:
+    """No hook would be missed by not calling the module."""
+    return not (m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks)
+
+
+def _activation_ok(x) -> bool:
+    return (type(x) is torch.Tensor and not x.is_inference() and x.dim() == 4 and x.dtype in _TYPES and x.is_cuda
+            and x.is_contiguous(memory_format=torch.channels_last) and x.shape[1] % 8 == 0 and x.data_ptr() % 16 == 0
+            and x.numel() >= 2 * x.shape[1] > 0)
+
+
+def _parameter_ok(t, x) -> bool:
+    return t is not None and not t.is_inference() and t.dtype == torch.float32 and t.is_contiguous() and t.get_device() == x.get_device() and t.data_ptr() % 16 == 0
+
+
+def _modes_off() -> bool:
+    g = nn.modules.module
+    return not (torch.compiler.is_compiling() or torch.jit.is_tracing() or torch.is_inference_mode_enabled() or forward_ad._current_level >= 0
+                or torch._C._functorch.peek_interpreter_stack() is not None or torch._C._len_torch_dispatch_stack()
+                or torch._C._len_torch_function_stack()
+                or g._global_forward_hooks or g._global_forward_pre_hooks or g._global_backward_hooks or g._global_backward_pre_hooks)
+
+
+def _fusable(bn: nn.Module, x) -> bool:
+    return (type(bn) is nn.BatchNorm2d and bn.training and bn.track_running_stats and bn.momentum is not None and _activation_ok(x)
+            and x.shape[1] == bn.num_features and x.get_device() == torch.cuda.current_device() and _bare(bn)
+            and _parameter_ok(bn.weight, x) and _parameter_ok(bn.bias, x) and _parameter_ok(bn.running_mean, x)
+            and _parameter_ok(bn.running_var, x) and (bn.num_batches_tracked is None or bn.num_batches_tracked.get_device() == x.get_device())
+            and _modes_off())
+
+
+def batch_norm_act(bn: nn.Module, x: torch.Tensor, relu: nn.Module | None = None, residual: torch.Tensor | None = None) -> torch.Tensor:
+    """``relu(bn(x) + residual)``; without ``relu`` or ``residual`` the same without that part."""
+    if (_fusable(bn, x) and (relu is None or (type(relu) is nn.ReLU and _bare(relu)))
+            and (residual is None or (_activation_ok(residual) and residual.shape == x.shape and residual.dtype == x.dtype
+                                      and residual.get_device() == x.get_device()))):
+        return _lib.torch_ops().batch_norm_act.default(x, bn.weight, bn.bias, residual, bn.running_mean, bn.running_var,
+                                                       bn.num_batches_tracked, bn.momentum, bn.eps, relu is not None)
+    y = bn(x)
+    if residual is not None:
+        y = y + residual
+    return y if relu is None else relu(y)

@@ -185,6 +185,13 @@ int al_scale_cast(void* out, int out_dt, const void* in, int in_dt, size_t n, do
 int al_sgd_momentum(float* param, float* momentum, float* grad, size_t n, float lr, float mu, float weight_decay,
                     float grad_scale, int first_step, int zero_grad, void* stream);
 int al_fill_u32(void* out, size_t n, uint32_t value, void* stream);
+/* Training batch norm + residual + ReLU over rows x channels (channels-last); residual, mask, running_*, batches may be NULL. */
+int al_bn_forward(int dt, const void* x, const void* residual, void* y, unsigned char* mask, const float* weight, const float* bias,
+                  float* running_mean, float* running_var, long long* batches, float* save_mean, float* save_invstd,
+                  void* workspace, size_t workspace_bytes, size_t rows, int channels, float momentum, float eps, void* stream);
+int al_bn_backward(int dt, const void* x, const void* dy, const unsigned char* mask, void* dx, void* dres, const float* weight,
+                   const float* save_mean, const float* save_invstd, float* grad_weight, float* grad_bias, void* workspace,
+                   size_t workspace_bytes, size_t rows, int channels, void* stream);
 
 #ifdef __cplusplus
 }

@@ -147,6 +147,38 @@ void launch_scale_cast(void* out, DType out_dt, const void* in, DType in_dt, siz
 void launch_sgd_momentum(float* param, float* momentum, float* grad, size_t n, float lr, float mu,
                          float weight_decay, float grad_scale, int first_step, int zero_grad,
                          cudaStream_t stream);
+/**
+ * Training batch norm of a channels-last activation (rows x channels, bf16 or f16; kernels/batchnorm.cu) with the
+ * residual addition and the ReLU behind it.  residual and mask may be null (no addition, no ReLU); mask gets one byte per
+ * 8 channels.  running_mean / running_var / batches (the count of batches) may be null.
+ */
+struct BnForward {
+  const void *x, *residual;
+  void* y;
+  unsigned char* mask;
+  const float *weight, *bias;
+  float *running_mean, *running_var;
+  long long* batches;
+  float *save_mean, *save_invstd;
+  void* workspace;
+  size_t workspace_bytes;
+  size_t rows;
+  int channels;
+  float momentum, eps;
+};
+struct BnBackward {
+  const void *x, *dy;
+  const unsigned char* mask;
+  void *dx, *dres;
+  const float *weight, *save_mean, *save_invstd;
+  float *grad_weight, *grad_bias;
+  void* workspace;
+  size_t workspace_bytes;
+  size_t rows;
+  int channels;
+};
+void launch_bn_forward(const BnForward& a, DType dt, cudaStream_t stream);
+void launch_bn_backward(const BnBackward& a, DType dt, cudaStream_t stream);
 /** Fill with a 32-bit pattern (used by tests and benchmarks to flush L2). */
 void launch_fill_u32(uint32_t* out, size_t n, uint32_t value, cudaStream_t stream);
 

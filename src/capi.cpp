@@ -622,4 +622,21 @@ int al_fill_u32(void* out, size_t n, uint32_t value, void* stream) {
   return guard([&] { device::launch_fill_u32((uint32_t*)out, n, value, (cudaStream_t)stream); });
 }
 
+int al_bn_forward(int dt, const void* x, const void* residual, void* y, unsigned char* mask, const float* weight, const float* bias,
+                  float* running_mean, float* running_var, long long* batches, float* save_mean, float* save_invstd,
+                  void* workspace, size_t workspace_bytes, size_t rows, int channels, float momentum, float eps, void* stream) {
+  return guard([&] {
+    device::launch_bn_forward({x, residual, y, mask, weight, bias, running_mean, running_var, batches, save_mean, save_invstd, workspace,
+                               workspace_bytes, rows, channels, momentum, eps}, (DType)dt, (cudaStream_t)stream);
+  });
+}
+int al_bn_backward(int dt, const void* x, const void* dy, const unsigned char* mask, void* dx, void* dres, const float* weight,
+                   const float* save_mean, const float* save_invstd, float* grad_weight, float* grad_bias, void* workspace,
+                   size_t workspace_bytes, size_t rows, int channels, void* stream) {
+  return guard([&] {
+    device::launch_bn_backward({x, dy, mask, dx, dres, weight, save_mean, save_invstd, grad_weight, grad_bias, workspace, workspace_bytes,
+                                rows, channels}, (DType)dt, (cudaStream_t)stream);
+  });
+}
+
 }  // extern "C"

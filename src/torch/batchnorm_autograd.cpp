@@ -1,0 +1,106 @@
+// Autograd of the fused batch norm (kernels/batchnorm.cu) for PyTorch, in native code: a small network's step is bound by
+// the host, and 53 layers of a Python autograd function cost it 2 ms more than the three framework operations each
+// replaces.  Registered as torch.ops.aluminum_b200.batch_norm_act; aluminum_b200/ops/batchnorm.py decides when it is called.
+#include <ATen/ATen.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/autograd/custom_function.h>
+#include <torch/library.h>
+
+#include "al/al_c.h"
+#include "al/base.hpp"
+
+namespace {
+
+using at::Tensor;
+using torch::autograd::AutogradContext;
+using torch::autograd::variable_list;
+
+constexpr int kArgs = 10;  // of forward()
+
+int type_code(const Tensor& t) { return (int)(t.scalar_type() == at::kBFloat16 ? Al::DType::bf16 : Al::DType::f16); }
+
+/** Partial sums of at most 148 x 3 CTAs of 256 channels (8 bytes each) and 16 bytes per channel. */
+Tensor workspace(const Tensor& x, int64_t channels) { return at::empty({148 * 3 * 256 * 8 + 16 * channels}, x.options().dtype(at::kByte)); }
+
+struct BatchNormAct : public torch::autograd::Function<BatchNormAct> {
+  static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& weight, const Tensor& bias,
+                        const std::optional<Tensor>& residual, const Tensor& running_mean, const Tensor& running_var,
+                        const std::optional<Tensor>& batches, double momentum, double eps, bool relu) {
+    const c10::cuda::CUDAGuard guard(x.device());
+    const int64_t c = x.size(1), rows = x.numel() / c;
+    Tensor y = at::empty_like(x);
+    Tensor mask = at::empty({relu ? rows * c / 8 : 0}, x.options().dtype(at::kByte));
+    Tensor stats = at::empty({2, c}, weight.options());
+    Tensor ws = workspace(x, c);
+    float* at = stats.data_ptr<float>();
+    TORCH_CHECK(al_bn_forward(type_code(x), x.data_ptr(), residual ? residual->data_ptr() : nullptr, y.data_ptr(),
+                              relu ? mask.data_ptr<uint8_t>() : nullptr, weight.data_ptr<float>(), bias.data_ptr<float>(),
+                              running_mean.data_ptr<float>(), running_var.data_ptr<float>(),
+                              batches ? (long long*)batches->data_ptr<int64_t>() : nullptr, at, at + c, ws.data_ptr(), (size_t)ws.numel(),
+                              (size_t)rows, (int)c, (float)momentum, (float)eps, c10::cuda::getCurrentCUDAStream().stream()) == 0,
+                al_last_error());
+    running_mean.unsafeGetTensorImpl()->bump_version();
+    running_var.unsafeGetTensorImpl()->bump_version();
+    if (batches) batches->unsafeGetTensorImpl()->bump_version();
+    ctx->save_for_backward({x, weight, stats, mask});
+    ctx->saved_data["relu"] = relu;
+    ctx->saved_data["eps"] = eps;
+    ctx->saved_data["residual"] = residual.has_value() && residual->requires_grad();
+    ctx->set_materialize_grads(false);
+    return y;
+  }
+
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    variable_list out(kArgs);
+    if (!grads[0].defined()) return out;
+    const variable_list saved = ctx->get_saved_variables();
+    const Tensor &x = saved[0], &weight = saved[1], &stats = saved[2], &mask = saved[3];
+    const bool relu = ctx->saved_data["relu"].toBool(), want_res = ctx->saved_data["residual"].toBool();
+    const c10::cuda::CUDAGuard guard(x.device());
+    const int64_t c = x.size(1), rows = x.numel() / c;
+    Tensor dy = grads[0];
+    if (at::GradMode::is_enabled() || dy.scalar_type() != x.scalar_type()) {
+      // a graph of the backward is wanted: operations that have a derivative themselves
+      if (relu) {
+        const Tensor bits = mask.view({x.size(0), x.size(2), x.size(3), c / 8, 1}).bitwise_right_shift(at::arange(8, mask.options())).bitwise_and(1);
+        dy = dy * bits.view({x.size(0), x.size(2), x.size(3), c}).permute({0, 3, 1, 2}).to(dy.scalar_type());
+      }
+      auto g = at::native_batch_norm_backward(dy, x, weight, {}, {}, stats[0], stats[1], true, ctx->saved_data["eps"].toDouble(), {true, true, true});
+      out[0] = std::get<0>(g);
+      out[1] = std::get<1>(g);
+      out[2] = std::get<2>(g);
+      if (want_res) out[3] = dy;
+      return out;
+    }
+    if (!dy.is_contiguous(at::MemoryFormat::ChannelsLast) || (uintptr_t)dy.data_ptr() % 16) dy = dy.clone(at::MemoryFormat::ChannelsLast);
+    Tensor dx = at::empty_like(x), dres, gw = at::empty_like(weight), gb = at::empty_like(weight);
+    if (want_res) dres = at::empty_like(x);
+    Tensor ws = workspace(x, c);
+    float* at = stats.data_ptr<float>();
+    TORCH_CHECK(al_bn_backward(type_code(x), x.data_ptr(), dy.data_ptr(), relu ? mask.data_ptr<uint8_t>() : nullptr, dx.data_ptr(),
+                               want_res ? dres.data_ptr() : nullptr, weight.data_ptr<float>(), at, at + c, gw.data_ptr<float>(),
+                               gb.data_ptr<float>(), ws.data_ptr(), (size_t)ws.numel(), (size_t)rows, (int)c,
+                               c10::cuda::getCurrentCUDAStream().stream()) == 0,
+                al_last_error());
+    out[0] = dx;
+    out[1] = gw;
+    out[2] = gb;
+    out[3] = dres;
+    return out;
+  }
+};
+
+Tensor batch_norm_act(const Tensor& x, const Tensor& weight, const Tensor& bias, const std::optional<Tensor>& residual,
+                      const Tensor& running_mean, const Tensor& running_var, const std::optional<Tensor>& batches, double momentum,
+                      double eps, bool relu) {
+  return BatchNormAct::apply(x, weight, bias, residual, running_mean, running_var, batches, momentum, eps, relu);
+}
+
+}  // namespace
+
+TORCH_LIBRARY(aluminum_b200, m) {
+  m.def("batch_norm_act(Tensor x, Tensor weight, Tensor bias, Tensor? residual, Tensor(a!) running_mean, Tensor(b!) running_var, "
+        "Tensor(c!)? batches, float momentum, float eps, bool relu) -> Tensor",
+        batch_norm_act);
+}

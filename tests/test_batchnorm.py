@@ -1,0 +1,115 @@
+"""Fused training batch norm (+ residual, + ReLU) against the same operation in 64 bits, and the calls that must still
+go through the modules."""
+import copy
+
+import pytest
+import torch
+from torch import nn
+
+from aluminum_b200.ops import batch_norm_act
+
+
+def reference(bn, x, residual, relu, dy):
+    """Outputs, gradients and running statistics in 64 bits."""
+    bn = copy.deepcopy(bn).double()
+    x = x.detach().double().requires_grad_()
+    res = residual.detach().double().requires_grad_() if residual is not None else None
+    y = bn(x)
+    if res is not None:
+        y = y + res
+    if relu:
+        y = y.relu()
+    y.backward(dy.double())
+    return y, x.grad, res.grad if res is not None else None, bn.weight.grad, bn.bias.grad, bn.running_mean, bn.running_var
+
+
+def rel(a, b):
+    return ((a.double() - b).norm() / b.norm().clamp_min(1e-30)).item()
+
+
+# channels: one column, a part of a warp's columns, whole warps and a ragged tile; rows around a thread's, a CTA's and the grid's share
+SHAPES = [(2, 8, 1, 1), (3, 24, 5, 7), (2, 64, 33, 31), (1, 264, 9, 9), (5, 2048, 7, 7), (24, 256, 56, 56), (9, 64, 112, 112)]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("shape", SHAPES)
+@pytest.mark.parametrize("relu,res", [(True, False), (True, True), (False, False), (False, True)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_against_64_bits(shape, relu, res, dtype):
+    torch.manual_seed(sum(shape))
+    cl = dict(memory_format=torch.channels_last)
+    n, c, h, w = shape
+    bn = nn.BatchNorm2d(c).cuda()
+    nn.init.uniform_(bn.weight, 0.5, 1.5)
+    nn.init.uniform_(bn.bias, -1, 1)
+    offset = torch.linspace(-20, 20, c, device="cuda").view(1, c, 1, 1)   # means well away from 0: deviations, not squares, are summed
+    make = lambda: torch.randn(shape, device="cuda")
+    x = (make() + offset).to(dtype).contiguous(**cl).requires_grad_()
+    residual = make().to(dtype).contiguous(**cl).requires_grad_() if res else None
+    dy = make().to(dtype).contiguous(**cl)
+    want = reference(bn, x, residual, relu, dy)
+    y = batch_norm_act(bn, x, nn.ReLU(inplace=True) if relu else None, residual)
+    assert "BatchNormAct" in y.grad_fn.name()
+    y.backward(dy)
+    # One rounding to 16 bits on the way out.  Gradients behind a ReLU: inputs reach 25, so sums in 32 bits are off by
+    # up to 25 * 1.5 * 2^-23 = 4.5e-6 in front of the ReLU; with a density of 0.4 around 0 that is 3.6e-6 of the
+    # elements whose gradient may pass or stop, and the square root of it in the norm.
+    flips = 1.9e-3 if relu else 0.0
+    eps = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11
+    small = n * h * w < 64        # few rows: the gradient of x is a difference of nearly equal terms
+    assert rel(y, want[0]) < eps
+    assert rel(x.grad, want[1]) < (0.5 if small else 4 * eps + flips)
+    if res:
+        assert rel(residual.grad, want[2]) < eps + flips
+    assert rel(bn.weight.grad, want[3]) < (1e-2 if small else 4 * eps)
+    assert rel(bn.bias.grad, want[4]) < 4 * eps
+    assert rel(bn.running_mean, want[5]) < 1e-6
+    assert rel(bn.running_var, want[6]) < 1e-5
+    assert int(bn.num_batches_tracked) == 1
+
+
+@pytest.mark.gpu
+def test_nan_infinity_and_second_derivative():
+    cl = dict(memory_format=torch.channels_last)
+    bn = nn.BatchNorm2d(16).cuda()
+    x = torch.randn(2, 16, 4, 4, device="cuda").bfloat16().contiguous(**cl)
+    x[0, 3, 1, 1] = float("nan")
+    x[1, 5, 0, 0] = float("inf")
+    y = batch_norm_act(bn, x, nn.ReLU())
+    want = torch.relu(copy.deepcopy(bn)(x))
+    assert torch.equal(torch.isnan(y), torch.isnan(want))
+    x = torch.randn(2, 16, 4, 4, device="cuda").bfloat16().contiguous(**cl).requires_grad_()
+    got = []
+    for f in (lambda: batch_norm_act(bn, x, nn.ReLU()), lambda: torch.relu(bn(x))):
+        g, = torch.autograd.grad(f().float().square().sum(), x, create_graph=True)
+        got.append(torch.autograd.grad(g.float().square().sum(), x)[0].double())
+    assert rel(got[0], got[1]) < 5e-2   # a chain of 16-bit operations, in another order
+
+
+@pytest.mark.gpu
+def test_calls_that_stay_with_the_modules():
+    cl = dict(memory_format=torch.channels_last)
+    x = torch.randn(2, 16, 4, 4, device="cuda").bfloat16().contiguous(**cl)
+    relu = nn.ReLU()
+    seen = []
+    hooked = nn.BatchNorm2d(16).cuda()
+    hooked.register_forward_hook(lambda *a: seen.append(1))
+    batch_norm_act(hooked, x, relu)
+    assert seen
+    bn = nn.BatchNorm2d(16).cuda()
+    for bad in (x.float(), x.contiguous(), x[:, :, ::2]):
+        got = batch_norm_act(copy.deepcopy(bn), bad, relu)
+        assert torch.equal(got, relu(copy.deepcopy(bn)(bad)))
+    assert torch.equal(batch_norm_act(copy.deepcopy(bn).eval(), x, relu), relu(copy.deepcopy(bn).eval()(x)))
+    with pytest.raises(ValueError):
+        batch_norm_act(bn, x[:1, :, :1, :1].contiguous(**cl), relu)
+
+
+def test_cpu_and_scripted_block():
+    from aluminum_b200.models.resnet import Bottleneck
+    bn, x = nn.BatchNorm2d(8), torch.randn(2, 8, 3, 3)
+    assert torch.equal(batch_norm_act(copy.deepcopy(bn), x, nn.ReLU(), x), torch.relu(bn(x) + x))
+    block = Bottleneck(16, 4)
+    scripted = torch.jit.script(copy.deepcopy(block))
+    x = torch.randn(2, 16, 5, 5)
+    assert torch.allclose(block(x), scripted(x), atol=1e-6)
