@@ -7,6 +7,7 @@ missing or broken native library can never be mistaken for a working fallback.
 from __future__ import annotations
 
 import ctypes as C
+import functools
 import os
 import threading
 from pathlib import Path
@@ -80,6 +81,7 @@ def _declare(lib) -> None:
         "al_rma_sync": (i, [vp, i]),
         "al_halo_exchange": (i, [vp, vpp, sz, sz, sz, sz, i, i, vp]),
         "al_halo_pack": (i, [vp, vp, sz, sz, sz, sz, sz, i, vp]),
+        "al_route_rows": (i, [i, vpp, szp, i, vpp, vp, vp]),
         "al_scale_cast": (i, [vp, i, vp, i, sz, d, vp]),
         "al_sgd_momentum": (i, [vp, vp, vp, sz, C.c_float, C.c_float, C.c_float, C.c_float, i, i, vp]),
         "al_fill_u32": (i, [vp, sz, C.c_uint32, vp]),
@@ -137,8 +139,18 @@ def check_ptr(p):
     return p
 
 
-def size_array(values):
+@functools.lru_cache(maxsize=64)
+def _size_type(n: int):
+    return C.c_size_t * n
+
+
+def size_array(values, times: int = 1):
     if values is None:
         return None
-    arr = (C.c_size_t * len(values))(*[int(v) for v in values])
-    return arr
+    n = len(values)
+    for v in values:
+        if type(v) is not int:
+            values = [int(v) for v in values]
+            break
+    arr = _size_type(n)(*values)
+    return arr if times == 1 else _size_type(n * times).from_buffer_copy(bytes(arr) * times)

@@ -248,7 +248,9 @@ class DeviceComm:
 
         def table(t):
             rows = [t] if (self.nlocal == 1 and t and not isinstance(t[0], (list, tuple))) else t
-            flat = [int(v) for row in rows for v in row]
+            if len(rows) == self.nlocal > 1 and len(rows[0]) == self.size and all(row is rows[0] for row in rows):
+                return size_array(rows[0], self.nlocal)   # every rank's row is the same
+            flat = [v for row in rows for v in row]
             if len(flat) != self.nlocal * self.size:
                 raise AlError(f"exchange_rows: tables need {self.nlocal} row(s) of {self.size} entries")
             return size_array(flat)

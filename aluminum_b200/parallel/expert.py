@@ -8,8 +8,12 @@ the receive buffer have to be known on the host to allocate it).
 """
 from __future__ import annotations
 
+import ctypes as C
+
 import torch
 
+from .. import _lib
+from .._lib import check
 from ._util import call, unwrap, wrap
 
 
@@ -21,6 +25,22 @@ def _prefix(counts):
     return out
 
 
+def _route(comm, dests):
+    """Stable order of every local rank's tokens by destination, and a (2, local ranks, ranks) buffer whose first half
+    holds the tokens per destination (one launch for all local ranks)."""
+    n, p = len(dests), comm.size
+    for d in dests:
+        if d.dim() != 1 or d.is_floating_point() or d.is_complex():
+            raise ValueError("dest_rank: a one-dimensional integer tensor per rank")
+    dests = [d.to(torch.int64).contiguous() for d in dests]
+    order = [torch.empty_like(d) for d in dests]
+    both = torch.empty((2, n, p), device=dests[0].device, dtype=torch.int64)
+    check(_lib.load().al_route_rows(n, (C.c_void_p * n)(*[d.data_ptr() for d in dests]), (C.c_size_t * n)(*[d.numel() for d in dests]), p,
+                                    (C.c_void_p * n)(*[o.data_ptr() for o in order]), both.data_ptr(),
+                                    torch.cuda.current_stream().cuda_stream))
+    return order, both
+
+
 def dispatch(comm, tokens, dest_rank):
     """Send every token (row of ``tokens``) to ``dest_rank[i]``.
 
@@ -28,13 +48,11 @@ def dispatch(comm, tokens, dest_rank):
     p = comm.size
     toks = [t.contiguous() for t in wrap(comm, tokens)]
     dests = wrap(comm, dest_rank)
-    order = [torch.argsort(d, stable=True).contiguous() for d in dests]   # int64: token i of the sorted order
-    send_counts = [torch.bincount(d, minlength=p).to(torch.int64) for d in dests]
-    recv_counts = [torch.empty(p, device=c.device, dtype=torch.int64) for c in send_counts]
-    call(comm, comm.alltoall, send_counts, recv_counts)
-    both = torch.stack([torch.stack(send_counts), torch.stack(recv_counts)]).cpu()   # the one host read
-    sc = [[int(v) for v in row] for row in both[0].tolist()]
-    rc = [[int(v) for v in row] for row in both[1].tolist()]
+    order, both = _route(comm, dests)
+    call(comm, comm.alltoall, list(both[0].unbind()), list(both[1].unbind()))
+    sc, rc = both.tolist()   # the one host read
+    if any(c < 0 for row in sc + rc for c in row):
+        raise ValueError(f"dest_rank: every destination must be a rank from 0 to {p - 1}")
     width = toks[0].shape[1]
     rb = width * toks[0].element_size()
     outs = [torch.empty((sum(r), width), device=toks[0].device, dtype=toks[0].dtype) for r in rc]

@@ -180,6 +180,9 @@ int al_halo_exchange(void* comm, float* const* tensors, size_t nc, size_t d_loca
 int al_halo_pack(float* packed, const float* tensor, size_t nc, size_t d_total, size_t plane, size_t d_first,
                  size_t depth, int unpack, void* stream);
 
+/* Stable order of n[r] tokens by destination rank and counts[r * p + d], for nlocal ranks; counts are -1 where a destination is none of the p ranks. */
+int al_route_rows(int nlocal, const long long* const* dest, const size_t* n, int p, long long* const* order, long long* counts, void* stream);
+
 /* ---- element-wise kernels ---- */
 int al_scale_cast(void* out, int out_dt, const void* in, int in_dt, size_t n, double scale, void* stream);
 int al_sgd_momentum(float* param, float* momentum, float* grad, size_t n, float lr, float mu, float weight_decay,

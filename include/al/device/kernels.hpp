@@ -36,6 +36,9 @@ bool collective_supported(DType in, DType wire, DType out, ReductionOperator op)
 bool bulk_staged_supported(DevColl kind, DType dt, ReductionOperator op);
 void launch_bulk_staged(const CollParams& P, DType dt, int ctas, int local_ranks, cudaStream_t stream);
 
+// ---- order of tokens by destination rank (kernels/route.cu) ----
+void launch_route(const RouteParams& P, int local_ranks, cudaStream_t stream);
+
 // ---- bulk-copy pipeline (kernels/bulk_pipeline.cu) ------------------------------
 /**
  * Large uniform allgather / alltoall (dt = u8, counts in bytes) and sum

@@ -265,6 +265,15 @@ struct RowsParams {
   int rank0;
 };
 
+/** Arguments of one routing launch (kernels/route.cu): one block per local rank. */
+struct RouteParams {
+  const long long* dest[kMaxRanks];  ///< destination rank of every token
+  size_t n[kMaxRanks];               ///< tokens
+  long long* order[kMaxRanks];       ///< tokens by destination, in order among those of one destination
+  long long* counts;                 ///< [local rank][p]: tokens per destination; all -1 if a destination is none of the p ranks
+  int p;
+};
+
 /** Arguments of one point-to-point launch (any mix of sends and receives). */
 struct P2PParams {
   static constexpr int kMaxItems = 16;

@@ -608,6 +608,21 @@ int al_halo_pack(float* packed, const float* tensor, size_t nc, size_t d_total, 
   });
 }
 
+int al_route_rows(int nlocal, const long long* const* dest, const size_t* n, int p, long long* const* order, long long* counts, void* stream) {
+  return guard([&] {
+    if (nlocal < 1 || nlocal > device::kMaxRanks || p < 1 || p > device::kMaxRanks) throw_al_exception("route: 1 to ", device::kMaxRanks, " ranks");
+    device::RouteParams P{};
+    for (int r = 0; r < nlocal; ++r) {
+      P.dest[r] = dest[r];
+      P.n[r] = n[r];
+      P.order[r] = order[r];
+    }
+    P.counts = counts;
+    P.p = p;
+    device::launch_route(P, nlocal, (cudaStream_t)stream);
+  });
+}
+
 // --------------------------------------------------------------- element-wise
 int al_scale_cast(void* out, int out_dt, const void* in, int in_dt, size_t n, double scale, void* stream) {
   return guard([&] { device::launch_scale_cast(out, (DType)out_dt, in, (DType)in_dt, n, scale, (cudaStream_t)stream); });

@@ -195,7 +195,13 @@ bool own_may_skip_staging(DevColl kind, const RankArgs& a, const CountTable& T, 
   }
 }
 
-/** Smallest vector (or whole message) that the bulk copy engine moves when all ranks are on one GPU. */
+/**
+ * Smallest vector (or whole message) that the bulk copy engine moves when all ranks are on one GPU.  Loops against bulk
+ * copies in us, at 1 and 4 MiB: allreduce of 4 ranks 26.6 / 25.2 and 39.8 / 31.3, of 8 ranks 42 / 31 and 66 / 47;
+ * reduce_scatter of 8 ranks 28.6 / 29.1 and 41 / 29; allgather of 4 ranks 17.5 / 18.1 and 23.4 / 21.7.  Below 1 MiB both
+ * wait for the host.  With two ranks the loops move data faster up to 8 MiB (allgather 17.8 / 20.6; 16 MiB 25.7 / 23.4).
+ */
+constexpr size_t kBulkStagedMinMoveTwo = size_t{16} << 20;
 constexpr size_t kBulkStagedMinBytes = size_t{1} << 20;
 
 void require_device() {
@@ -618,7 +624,7 @@ void DeviceCommunicator::collective(const CollDesc& d, const std::vector<RankArg
   // All ranks on this GPU: large operations are moved by the bulk copy engine, chunked by what staging holds.
   bool bulk_staged = I.nlocal > 1 && !use_window && !d.vector && d.ctas <= 0 && !tn.bulk_pipeline && in == wire && wire == out &&
                      bulk_staged_supported(d.kind, wire, d.op) && (d.kind == DevColl::allreduce || P.count * esz % 16 == 0) &&
-                     P.count * esz * (d.kind == DevColl::allreduce ? 1 : (size_t)p) >= kBulkStagedMinBytes;
+                     P.count * esz * (d.kind == DevColl::allreduce ? 1 : (size_t)p) >= (p == 2 && !reduces ? kBulkStagedMinMoveTwo : kBulkStagedMinBytes);
   for (int r = 0; bulk_staged && r < p; ++r)
     bulk_staged = P.own_direct[r] && (uintptr_t)P.send[r] % 16 == 0 && (uintptr_t)P.recv[r] % 16 == 0;
 

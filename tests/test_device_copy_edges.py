@@ -146,3 +146,41 @@ def test_large_operations_in_bulk_copies(al, p, stage):
         comm.allgather(both, algo="staged")
         assert all(torch.equal(b, torch.cat([full[r][r * n:(r + 1) * n] for r in range(p)])) for b in both)
     comm.close()
+
+
+@pytest.mark.parametrize("p", [2, 4, 8])
+@pytest.mark.parametrize("width,rows", [(16, 1), (16, 1000), (80, 333), (1024, 67), (4096, 5), (4112, 31), (12000, 9), (24, 77), (7, 50)])
+def test_rows_of_any_length(al, p, width, rows):
+    """Rows of `width` bytes: several to a warp's round, one, more than one round, and lengths that are no whole words."""
+    comm = al.DeviceComm(emulate=p)
+    table = lambda v: [v] * p
+    x = [small_ints(p * rows * width, torch.uint8, r).view(rows, p, width) for r in range(p)]
+    order = [torch.randperm(rows, generator=torch.Generator().manual_seed(r)).cuda() for r in range(p)]
+    out = [torch.zeros(p, rows, width, device="cuda", dtype=torch.uint8) for _ in range(p)]
+    comm.exchange_rows(x, out, width, p * width, width, table([rows] * p), table([0] * p), table([d * width for d in range(p)]),
+                       table([rows] * p), table([s * rows for s in range(p)]), table([0] * p), send_idx=order)
+    for r in range(p):
+        for s in range(p):
+            assert torch.equal(out[r][s], x[s][order[s], r])
+    comm.close()
+
+
+@pytest.mark.parametrize("p", [2, 3, 8])
+@pytest.mark.parametrize("tokens", [0, 1, 31, 32, 33, 1024, 1025, 40000])
+def test_routing_order_and_counts(al, p, tokens):
+    from aluminum_b200.parallel import expert
+    comm = al.DeviceComm(emulate=p)
+    g = torch.Generator(device="cuda").manual_seed(tokens)
+    dests = [torch.randint(0, p, (tokens,), generator=g, device="cuda") // (1 + r % 2) for r in range(p)]
+    order, both = expert._route(comm, dests)
+    for r in range(p):
+        assert torch.equal(order[r], torch.argsort(dests[r], stable=True))
+        assert torch.equal(both[0][r], torch.bincount(dests[r], minlength=p))
+    if tokens:
+        toks = [torch.zeros(tokens, 8, device="cuda") for _ in range(p)]
+        for wrong in (-1, p):
+            bad = [d.clone() for d in dests]
+            bad[0][-1] = wrong
+            with pytest.raises(ValueError):
+                expert.dispatch(comm, toks, bad)
+    comm.close()
