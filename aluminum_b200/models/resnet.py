@@ -11,7 +11,7 @@ from __future__ import annotations
 import torch
 from torch import nn
 
-from ..ops.batchnorm import batch_norm_act
+from ..ops.activations import batch_norm_act, max_pool
 
 
 class Bottleneck(nn.Module):
@@ -91,10 +91,9 @@ class ResNet(nn.Module):
 
     def forward(self, x):
         if torch.jit.is_scripting():
-            x = self.relu(self.bn1(self.conv1(x)))
+            x = self.maxpool(self.relu(self.bn1(self.conv1(x))))
         else:
-            x = batch_norm_act(self.bn1, self.conv1(x), self.relu)
-        x = self.maxpool(x)
+            x = max_pool(self.maxpool, batch_norm_act(self.bn1, self.conv1(x), self.relu))
         x = self.layer4(self.layer3(self.layer2(self.layer1(x))))
         return self.fc(torch.flatten(self.avgpool(x), 1))
 

@@ -1,7 +1,7 @@
 """Training batch norm of channels-last activations with the residual addition and the ReLU behind it fused in
-(``kernels/batchnorm.cu``, autograd in ``src/torch/batchnorm_autograd.cpp``).
+(``kernels/batchnorm.cu``), and max pooling (``kernels/maxpool.cu``); autograd in ``src/torch/activations_autograd.cpp``.
 
-:func:`batch_norm_act` takes the modules that a network holds (``nn.BatchNorm2d``, ``nn.ReLU``) and runs the fused kernels
+The functions take the modules that a network holds (``nn.BatchNorm2d``, ``nn.ReLU``, ``nn.MaxPool2d``) and run the kernels
 where they do exactly what the modules would: 16-bit channels-last CUDA activations in training, plain modules without
 hooks, ordinary reverse-mode autograd.  Everything else - evaluation, other types and layouts, hooks, tracing,
 functorch transforms, forward-mode AD - calls the modules.
@@ -59,3 +59,20 @@ def batch_norm_act(bn: nn.Module, x: torch.Tensor, relu: nn.Module | None = None
     if residual is not None:
         y = y + residual
     return y if relu is None else relu(y)
+
+
+def _one(v) -> int:
+    """The value of an int or of a pair of equal ints, else 0."""
+    if isinstance(v, (tuple, list)):
+        return v[0] if len(v) == 2 and v[0] == v[1] and type(v[0]) is int else 0
+    return v if type(v) is int else 0
+
+
+def max_pool(pool: nn.Module, x: torch.Tensor) -> torch.Tensor:
+    """``pool(x)``."""
+    if type(pool) is nn.MaxPool2d and _activation_ok(x) and x.get_device() == torch.cuda.current_device() and _bare(pool) and _modes_off():
+        k, stride, pad = _one(pool.kernel_size), _one(pool.stride), pool.padding if pool.padding == 0 else _one(pool.padding)
+        if (0 < k <= 15 and stride > 0 and _one(pool.dilation) == 1 and not pool.ceil_mode and not pool.return_indices
+                and (pad > 0 or pool.padding == 0) and 2 * pad <= k and min(x.shape[2:]) + 2 * pad >= k):
+            return _lib.torch_ops().max_pool.default(x, k, stride, pad)
+    return pool(x)

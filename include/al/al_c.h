@@ -195,6 +195,9 @@ int al_bn_forward(int dt, const void* x, const void* residual, void* y, unsigned
 int al_bn_backward(int dt, const void* x, const void* dy, const unsigned char* mask, void* dx, void* dres, const float* weight,
                    const float* save_mean, const float* save_invstd, float* grad_weight, float* grad_bias, void* workspace,
                    size_t workspace_bytes, size_t rows, int channels, void* stream);
+/* Max pooling, channels-last; shape: n, h, w, c, out h, out w, window, stride, padding.  place: one byte per output element. */
+int al_maxpool_forward(int dt, const void* x, void* y, unsigned char* place, const int* shape, void* stream);
+int al_maxpool_backward(int dt, const void* dy, const unsigned char* place, void* dx, const int* shape, void* stream);
 
 #ifdef __cplusplus
 }

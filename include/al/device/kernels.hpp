@@ -182,6 +182,12 @@ struct BnBackward {
 };
 void launch_bn_forward(const BnForward& a, DType dt, cudaStream_t stream);
 void launch_bn_backward(const BnBackward& a, DType dt, cudaStream_t stream);
+/** Max pooling of channels-last activations (bf16 or f16; kernels/maxpool.cu); place: the winner's k * row + column, a byte per output. */
+struct PoolShape {
+  int n, h, w, c, oh, ow, k, stride, pad;
+};
+void launch_maxpool_forward(const void* x, void* y, unsigned char* place, const PoolShape& s, DType dt, cudaStream_t stream);
+void launch_maxpool_backward(const void* dy, const unsigned char* place, void* dx, const PoolShape& s, DType dt, cudaStream_t stream);
 /** Fill with a 32-bit pattern (used by tests and benchmarks to flush L2). */
 void launch_fill_u32(uint32_t* out, size_t n, uint32_t value, cudaStream_t stream);
 

@@ -654,4 +654,12 @@ int al_bn_backward(int dt, const void* x, const void* dy, const unsigned char* m
   });
 }
 
+static device::PoolShape pool_shape(const int* s) { return {s[0], s[1], s[2], s[3], s[4], s[5], s[6], s[7], s[8]}; }
+int al_maxpool_forward(int dt, const void* x, void* y, unsigned char* place, const int* shape, void* stream) {
+  return guard([&] { device::launch_maxpool_forward(x, y, place, pool_shape(shape), (DType)dt, (cudaStream_t)stream); });
+}
+int al_maxpool_backward(int dt, const void* dy, const unsigned char* place, void* dx, const int* shape, void* stream) {
+  return guard([&] { device::launch_maxpool_backward(dy, place, dx, pool_shape(shape), (DType)dt, (cudaStream_t)stream); });
+}
+
 }  // extern "C"

@@ -1,6 +1,6 @@
-// Autograd of the fused batch norm (kernels/batchnorm.cu) for PyTorch, in native code: a small network's step is bound by
+// Autograd of the fused batch norm (kernels/batchnorm.cu) and of max pooling (kernels/maxpool.cu) for PyTorch, in native code: a small network's step is bound by
 // the host, and 53 layers of a Python autograd function cost it 2 ms more than the three framework operations each
-// replaces.  Registered as torch.ops.aluminum_b200.batch_norm_act; aluminum_b200/ops/batchnorm.py decides when it is called.
+// replaces.  Registered under torch.ops.aluminum_b200; aluminum_b200/ops/activations.py decides when they are called.
 #include <ATen/ATen.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
@@ -97,10 +97,64 @@ Tensor batch_norm_act(const Tensor& x, const Tensor& weight, const Tensor& bias,
   return BatchNormAct::apply(x, weight, bias, residual, running_mean, running_var, batches, momentum, eps, relu);
 }
 
+struct MaxPool : public torch::autograd::Function<MaxPool> {
+  static std::array<int, 9> shape(const Tensor& x, int64_t k, int64_t stride, int64_t pad) {
+    const int64_t h = x.size(2), w = x.size(3);
+    return {(int)x.size(0), (int)h, (int)w, (int)x.size(1), (int)((h + 2 * pad - k) / stride + 1), (int)((w + 2 * pad - k) / stride + 1),
+            (int)k, (int)stride, (int)pad};
+  }
+
+  static Tensor forward(AutogradContext* ctx, const Tensor& x, int64_t k, int64_t stride, int64_t pad) {
+    const c10::cuda::CUDAGuard guard(x.device());
+    const auto s = shape(x, k, stride, pad);
+    Tensor y = at::empty({s[0], s[3], s[4], s[5]}, x.options(), at::MemoryFormat::ChannelsLast);
+    Tensor place = at::empty({s[0], s[4], s[5], s[3]}, x.options().dtype(at::kByte));
+    TORCH_CHECK(al_maxpool_forward(type_code(x), x.data_ptr(), y.data_ptr(), place.data_ptr<uint8_t>(), s.data(),
+                                   c10::cuda::getCurrentCUDAStream().stream()) == 0,
+                al_last_error());
+    ctx->save_for_backward({x, place});
+    ctx->saved_data["k"] = k;
+    ctx->saved_data["stride"] = stride;
+    ctx->saved_data["pad"] = pad;
+    ctx->set_materialize_grads(false);
+    return y;
+  }
+
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    variable_list out(4);
+    if (!grads[0].defined()) return out;
+    const variable_list saved = ctx->get_saved_variables();
+    const Tensor &x = saved[0], &place = saved[1];
+    const int64_t k = ctx->saved_data["k"].toInt(), stride = ctx->saved_data["stride"].toInt(), pad = ctx->saved_data["pad"].toInt();
+    const c10::cuda::CUDAGuard guard(x.device());
+    const auto s = shape(x, k, stride, pad);
+    Tensor dy = grads[0];
+    if (at::GradMode::is_enabled() || dy.scalar_type() != x.scalar_type()) {
+      // a graph of the backward is wanted: the framework's own backward, with the places as its indices
+      const auto wide = place.options().dtype(at::kLong);
+      const Tensor p = place.to(at::kLong);
+      const Tensor h = at::arange(s[4], wide).mul(stride).sub(pad).view({1, s[4], 1, 1}) + at::floor_divide(p, k);
+      const Tensor w = at::arange(s[5], wide).mul(stride).sub(pad).view({1, 1, s[5], 1}) + at::remainder(p, k);
+      out[0] = at::max_pool2d_with_indices_backward(dy, x, {k, k}, {stride, stride}, {pad, pad}, {1, 1}, false, (h * s[2] + w).permute({0, 3, 1, 2}));
+      return out;
+    }
+    if (!dy.is_contiguous(at::MemoryFormat::ChannelsLast) || (uintptr_t)dy.data_ptr() % 16) dy = dy.clone(at::MemoryFormat::ChannelsLast);
+    Tensor dx = at::empty_like(x);
+    TORCH_CHECK(al_maxpool_backward(type_code(x), dy.data_ptr(), place.data_ptr<uint8_t>(), dx.data_ptr(), s.data(),
+                                    c10::cuda::getCurrentCUDAStream().stream()) == 0,
+                al_last_error());
+    out[0] = dx;
+    return out;
+  }
+};
+
+Tensor max_pool(const Tensor& x, int64_t k, int64_t stride, int64_t pad) { return MaxPool::apply(x, k, stride, pad); }
+
 }  // namespace
 
 TORCH_LIBRARY(aluminum_b200, m) {
   m.def("batch_norm_act(Tensor x, Tensor weight, Tensor bias, Tensor? residual, Tensor(a!) running_mean, Tensor(b!) running_var, "
         "Tensor(c!)? batches, float momentum, float eps, bool relu) -> Tensor",
         batch_norm_act);
+  m.def("max_pool(Tensor x, int k, int stride, int pad) -> Tensor", max_pool);
 }

@@ -6,7 +6,7 @@ import pytest
 import torch
 from torch import nn
 
-from aluminum_b200.ops import batch_norm_act
+from aluminum_b200.ops import batch_norm_act, max_pool
 
 
 def reference(bn, x, residual, relu, dy):
@@ -113,3 +113,40 @@ def test_cpu_and_scripted_block():
     scripted = torch.jit.script(copy.deepcopy(block))
     x = torch.randn(2, 16, 5, 5)
     assert torch.allclose(block(x), scripted(x), atol=1e-6)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("k,stride,pad", [(3, 2, 1), (2, 2, 0), (3, 1, 1), (5, 3, 2), (1, 1, 0), (2, 3, 1)])
+@pytest.mark.parametrize("shape", [(2, 8, 5, 5), (3, 24, 13, 7), (2, 64, 112, 112)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_max_pool(k, stride, pad, shape, dtype):
+    torch.manual_seed(k)
+    cl = dict(memory_format=torch.channels_last)
+    pool = nn.MaxPool2d(k, stride, pad)
+    x = torch.randint(-9, 9, shape, device="cuda").to(dtype).contiguous(**cl).requires_grad_()   # many equal values
+    y = max_pool(pool, x)
+    assert "MaxPool" in y.grad_fn.name() and "MaxPool2D" not in y.grad_fn.name()
+    xr = x.detach().double().contiguous().requires_grad_()
+    want = pool(xr)
+    assert torch.equal(y.double(), want)
+    dy = torch.randint(-3, 4, want.shape, device="cuda").to(dtype)   # sums of a few small integers are exact
+    y.backward(dy)
+    want.backward(dy.double())
+    assert torch.equal(x.grad.double(), xr.grad)
+    g, = torch.autograd.grad((max_pool(pool, x).float() ** 2).sum(), x, create_graph=True)
+    assert torch.equal(torch.autograd.grad(g.float().sum(), x)[0].double() != 0, torch.autograd.grad((pool(xr) ** 2).sum(), xr)[0] * 0 +
+                       torch.autograd.grad(torch.autograd.grad((pool(xr) ** 2).sum(), xr, create_graph=True)[0].sum(), xr)[0] != 0)
+
+
+@pytest.mark.gpu
+def test_max_pool_nan_and_module_calls():
+    cl = dict(memory_format=torch.channels_last)
+    x = torch.randn(2, 8, 6, 6, device="cuda").bfloat16().contiguous(**cl)
+    x[0, 1, 2, 3] = float("nan")
+    pool = nn.MaxPool2d(3, 2, 1)
+    assert torch.equal(torch.isnan(max_pool(pool, x)), torch.isnan(pool(x)))
+    for other in (nn.MaxPool2d(3, 2, 1, ceil_mode=True), nn.MaxPool2d((3, 2), 2), nn.MaxPool2d(2, dilation=2)):
+        assert torch.equal(max_pool(other, x.nan_to_num()), other(x.nan_to_num()))
+    assert torch.equal(max_pool(pool, x.float().nan_to_num()), pool(x.float().nan_to_num()))
+    with pytest.raises(RuntimeError):
+        max_pool(nn.MaxPool2d(3, 1, 2), x)
