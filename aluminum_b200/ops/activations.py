@@ -73,6 +73,7 @@ def max_pool(pool: nn.Module, x: torch.Tensor) -> torch.Tensor:
     if type(pool) is nn.MaxPool2d and _activation_ok(x) and x.get_device() == torch.cuda.current_device() and _bare(pool) and _modes_off():
         k, stride, pad = _one(pool.kernel_size), _one(pool.stride), pool.padding if pool.padding == 0 else _one(pool.padding)
         if (0 < k <= 15 and stride > 0 and _one(pool.dilation) == 1 and not pool.ceil_mode and not pool.return_indices
-                and (pad > 0 or pool.padding == 0) and 2 * pad <= k and min(x.shape[2:]) + 2 * pad >= k):
+                and (pad > 0 or pool.padding == 0) and 2 * pad <= k and min(x.shape[2:]) + 2 * pad >= k
+                and x.numel() * (1 + pad) ** 2 < 1 << 34):   # (the kernels count threads of 8 elements in 32 bits)
             return _lib.torch_ops().max_pool.default(x, k, stride, pad)
     return pool(x)

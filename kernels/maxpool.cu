@@ -28,16 +28,15 @@ union Bytes8 {
 
 template <typename T>
 __global__ void __launch_bounds__(kThreads) maxpool_forward_kernel(const T* __restrict__ x, T* __restrict__ y, unsigned char* __restrict__ place,
-                                                                   const PoolShape s, size_t total) {
-  const size_t i = (size_t)blockIdx.x * kThreads + threadIdx.x;
+                                                                   const PoolShape s, unsigned total) {
+  const unsigned i = blockIdx.x * kThreads + threadIdx.x;
   if (i >= total) return;
   const unsigned cols = (unsigned)s.c / 8;
-  const size_t pixel = i / cols;
-  const unsigned col = (unsigned)(i - pixel * cols);
-  const size_t row = pixel / (unsigned)s.ow;
+  const unsigned pixel = i / cols, col = i - pixel * cols;
+  const unsigned row = pixel / (unsigned)s.ow;
   const int ow = (int)(pixel - row * (unsigned)s.ow);
   const size_t n = row / (unsigned)s.oh;
-  const int oh = (int)(row - n * (unsigned)s.oh);
+  const int oh = (int)(row % (unsigned)s.oh);
   const int h0 = oh * s.stride - s.pad, w0 = ow * s.stride - s.pad;
   Pack8<T> best;
   Bytes8 at;
@@ -68,16 +67,15 @@ __global__ void __launch_bounds__(kThreads) maxpool_forward_kernel(const T* __re
 
 template <typename T>
 __global__ void __launch_bounds__(kThreads) maxpool_backward_kernel(const T* __restrict__ dy, const unsigned char* __restrict__ place,
-                                                                    T* __restrict__ dx, const PoolShape s, size_t total) {
-  const size_t i = (size_t)blockIdx.x * kThreads + threadIdx.x;
+                                                                    T* __restrict__ dx, const PoolShape s, unsigned total) {
+  const unsigned i = blockIdx.x * kThreads + threadIdx.x;
   if (i >= total) return;
   const unsigned cols = (unsigned)s.c / 8;
-  const size_t pixel = i / cols;
-  const unsigned col = (unsigned)(i - pixel * cols);
-  const size_t row = pixel / (unsigned)s.w;
+  const unsigned pixel = i / cols, col = i - pixel * cols;
+  const unsigned row = pixel / (unsigned)s.w;
   const int w = (int)(pixel - row * (unsigned)s.w) + s.pad;
   const size_t n = row / (unsigned)s.h;
-  const int h = (int)(row - n * (unsigned)s.h) + s.pad;
+  const int h = (int)(row % (unsigned)s.h) + s.pad;
   // windows [lo, hi] start at most k - 1 before this pixel and not behind it
   const int h_hi = min(h / s.stride, s.oh - 1), h_lo = h < s.k ? 0 : (h - s.k) / s.stride + 1;
   const int w_hi = min(w / s.stride, s.ow - 1), w_lo = w < s.k ? 0 : (w - s.k) / s.stride + 1;
@@ -108,17 +106,22 @@ void check_shape(const PoolShape& s) {
     throw_al_exception("max pooling: unsupported shape");
 }
 
-unsigned blocks_of(size_t total) { return (unsigned)((total + kThreads - 1) / kThreads); }
+/** Threads of a launch; the kernels count them in 32 bits (64-bit divisions doubled their time). */
+unsigned threads_of(size_t total) {
+  if (total > 0xffffff00u) throw_al_exception("max pooling: more than 2^35 elements");
+  return (unsigned)total;
+}
+unsigned blocks_of(unsigned total) { return (total + kThreads - 1) / kThreads; }
 
 template <typename T>
 void forward(const void* x, void* y, unsigned char* place, const PoolShape& s, cudaStream_t stream) {
-  const size_t total = (size_t)s.n * s.oh * s.ow * (s.c / 8);
+  const unsigned total = threads_of((size_t)s.n * s.oh * s.ow * (s.c / 8));
   maxpool_forward_kernel<T><<<blocks_of(total), kThreads, 0, stream>>>((const T*)x, (T*)y, place, s, total);
   AL_CHECK_CUDA(cudaGetLastError());
 }
 template <typename T>
 void backward(const void* dy, const unsigned char* place, void* dx, const PoolShape& s, cudaStream_t stream) {
-  const size_t total = (size_t)s.n * s.h * s.w * (s.c / 8);
+  const unsigned total = threads_of((size_t)s.n * s.h * s.w * (s.c / 8));
   maxpool_backward_kernel<T><<<blocks_of(total), kThreads, 0, stream>>>((const T*)dy, place, (T*)dx, s, total);
   AL_CHECK_CUDA(cudaGetLastError());
 }
