@@ -32,9 +32,10 @@ void launch_collective(const CollParams& P, DType in, DType wire, DType out, int
 bool collective_supported(DType in, DType wire, DType out, ReductionOperator op);
 
 // ---- staged operations with all ranks on this GPU, moved by the bulk copy engine (kernels/bulk_staged.cu) ----
-/** Element type and operator; the kernel also wants 16-byte aligned buffers (and slices) and P.own_direct on every rank. */
-bool bulk_staged_supported(DevColl kind, DType dt, ReductionOperator op);
-void launch_bulk_staged(const CollParams& P, DType dt, int ctas, int local_ranks, cudaStream_t stream);
+/** Element types of the buffers and of staging, and operator; the kernel also wants 16-byte aligned buffers (and slices) and,
+ *  with one type throughout, P.own_direct on every rank. */
+bool bulk_staged_supported(DevColl kind, DType user, DType wire, ReductionOperator op);
+void launch_bulk_staged(const CollParams& P, DType user, DType wire, int ctas, int local_ranks, cudaStream_t stream);
 
 // ---- order of tokens by destination rank (kernels/route.cu) ----
 void launch_route(const RouteParams& P, int local_ranks, cudaStream_t stream);

@@ -7,7 +7,8 @@
 // thread per CTA keeps up to 160 KB of loads under way per SM, across destinations and sources without a gap, and needs no
 // registers for them; reductions are folded out of shared memory while the next tiles arrive.  Loops -> bulk copies:
 // bucket of 4 x 26 MB 136 -> 103 us (525 MB through HBM, 5.1 TB/s), sequence-parallel pair of 4 ranks, 16384 x 8192 bf16,
-// 1668 -> 1036 us (5.4 GB, 5.2 TB/s), of 8 ranks, 2048 x 4096, 203 -> 163 us.
+// 1668 -> 1036 us (5.4 GB, 5.2 TB/s), of 8 ranks, 2048 x 4096, 203 -> 163 us; bucket of 8 x 12 MB with a bf16 wire, converted
+// between the tiles and staging by all threads, 116 -> 98 us.
 // (Between GPUs the engine's stores to peers were slower than SM stores - 4 GPUs, 1 GiB allgather 1534 us against
 // 1291 us - so ranks on GPUs of their own keep coll_kernel.)
 //
@@ -28,8 +29,10 @@ constexpr int kTile = 32768;
 constexpr size_t kSmem = (size_t)kBufs * kTile + 128;  // tiles + barriers
 constexpr int kThreads = 512;
 
-template <typename T, typename Red>
+/** T: element type in staging; U: element type of the user's buffers (another one for an allreduce with a narrower wire type). */
+template <typename T, typename U, typename Red>
 __global__ void __launch_bounds__(kThreads, 1) bulk_staged_kernel(const __grid_constant__ CollParams P, Red red) {
+  constexpr bool kMixed = !std::is_same<T, U>::value;
   extern __shared__ __align__(128) unsigned char dyn_smem[];
   const Workspace& ws = P.ws;
   const int p = ws.p;
@@ -140,8 +143,107 @@ __global__ void __launch_bounds__(kThreads, 1) bulk_staged_kernel(const __grid_c
     return bad == 0;
   };
 
+  uint32_t parity = 0;   // every thread's view of the ring's parities (thread 0 hands them over)
+  __shared__ uint32_t s_parity;
+  /** The same with conversion: jobs[0..n) whose `bytes` counts elements of In, converted to Out.  All threads convert out of
+   *  the tiles; eight elements are one or two 16-byte words on either side. */
+  auto convert_jobs = [&](int n, auto in_type, auto out_type) {
+    using In = decltype(in_type);
+    using Out = decltype(out_type);
+    constexpr uint32_t kElems = kTile / sizeof(In);
+    __syncthreads();
+    size_t total = 0;
+    for (int j = 0; j < n; ++j) total += (jobs[j].bytes / 8 * 8 + kElems - 1) / kElems;
+    struct Cursor { int j; size_t off; };
+    auto seek = [&](Cursor& at) {   // to the next tile that exists; called only while there is one
+      for (;;) {
+        if (at.j == n) { at.j = 0; at.off += kElems; }
+        if (at.off < jobs[at.j].bytes / 8 * 8) return;
+        ++at.j;
+      }
+    };
+    auto len = [&](const Cursor& at) {
+      const size_t left = jobs[at.j].bytes / 8 * 8 - at.off;
+      return (uint32_t)(left < kElems ? left : kElems);
+    };
+    Cursor in{0, 0}, out{0, 0};
+    auto load = [&](size_t t) {
+      const int s = (int)(t % kBufs);
+      seek(in);
+      const uint32_t bytes = len(in) * (uint32_t)sizeof(In);
+      bulk::mbar_expect_tx(ring.bar(s), bytes);
+      bulk::g2s(ring.tile(s), jobs[in.j].src + in.off * sizeof(In), bytes, ring.bar(s));
+      ++in.j;
+    };
+    if (threadIdx.x == 0) {
+      s_parity = ring.parity;
+      bulk::fence_proxy_async();
+      for (size_t t = 0; t < total && t < kBufs; ++t) load(t);
+    }
+    __syncthreads();
+    parity = s_parity;
+    struct alignas(8 * sizeof(In) < 16 ? 8 * sizeof(In) : 16) Ins { In e[8]; };
+    union Outs { Out e[8]; uint4 u[8 * sizeof(Out) / 16]; };
+    bool good = true;
+    for (size_t t = 0; t < total; ++t) {
+      const int s = (int)(t % kBufs);
+      const bool ok = bulk::mbar_wait(bars + 8 * s, (parity >> s) & 1u, P.timeout_ns);
+      parity ^= 1u << s;
+      seek(out);
+      const Job& job = jobs[out.j];
+      const uint32_t groups = len(out) / 8;
+      if (ok)
+        for (uint32_t g = threadIdx.x; g < groups; g += kThreads) {
+          const Ins v = ((const Ins*)(dyn_smem + (size_t)s * kTile))[g];
+          Outs o;
+#pragma unroll
+          for (int k = 0; k < 8; ++k) o.e[k] = Elem<Out>::down(Elem<In>::up(v.e[k]));
+          for (int i = 0; i < job.ndst; ++i) {
+            uint4* d = (uint4*)(job.dst[i] + (out.off + 8 * (size_t)g) * sizeof(Out));
+#pragma unroll
+            for (int q = 0; q < (int)(8 * sizeof(Out) / 16); ++q) d[q] = o.u[q];
+          }
+        }
+      ++out.j;
+      if (__syncthreads_or(!ok)) {   // also: everyone has read the tile
+        good = false;
+        if (threadIdx.x == 0)        // the copies in flight end before the block does (or it gives up on them)
+          for (size_t u = t; u < total && u < t + kBufs; ++u)
+            (void)bulk::mbar_wait(bars + 8 * (u % kBufs), (parity >> (u % kBufs) ^ (u == t)) & 1u, P.timeout_ns);
+        break;
+      }
+      if (threadIdx.x == 0 && t + kBufs < total) load(t + kBufs);
+    }
+    if (threadIdx.x == 0) ring.parity = parity;
+    for (int j = 0; j < n; ++j) {    // the elements behind the last eight
+      const size_t e = jobs[j].bytes / 8 * 8 + threadIdx.x;
+      if (e < jobs[j].bytes) {
+        const Out o = Elem<Out>::down(Elem<In>::up(__ldcg((const In*)jobs[j].src + e)));
+        for (int i = 0; i < jobs[j].ndst; ++i) ((Out*)jobs[j].dst[i])[e] = o;
+      }
+    }
+    bulk::fence_proxy_async();       // plain stores above, engine loads behind the next flag
+    __syncthreads();                 // the list may be filled again
+    if (!good && threadIdx.x == 0) report_timeout(ws, rank, rank, 6, make_epoch(P.seq, 1), 0);
+    return good;
+  };
+
   auto publish = [&](uint64_t c) {
     const size_t half_off = (size_t)((P.seq + c) & 1) * half;
+    if constexpr (kMixed) {   // allreduce; the own slice is rounded to the wire type like the others and goes through staging
+      const int n = two_phase ? p : 1;
+      if ((int)threadIdx.x < n) {
+        Job& job = jobs[threadIdx.x];
+        const int d = (rank + 1 + (int)threadIdx.x) % p;
+        const Part q = part_of(c, d);
+        job.src = send + (q.base + q.lo) * sizeof(U);
+        job.bytes = q.hi - q.lo;
+        job.ndst = 0;
+        for (int i = 0; i < (two_phase ? 1 : p); ++i)
+          job.dst[job.ndst++] = ws.stage[two_phase ? d : (rank + 1 + i) % p] + half_off + (size_t)rank * slot_b + q.lo * sizeof(T);
+      }
+      return convert_jobs(n, U(), T());
+    }
     if (kind == DevColl::allgather || (kind == DevColl::allreduce && !two_phase)) {  // one read, a store per rank
       if (threadIdx.x == 0) {
         Job& job = jobs[0];
@@ -175,8 +277,6 @@ __global__ void __launch_bounds__(kThreads, 1) bulk_staged_kernel(const __grid_c
   };
 
   /** Fold the p contributions of the own slice; the result goes to the receive buffer and, in two phases, to every peer. */
-  uint32_t parity = 0;   // every thread's view of the ring's parities (thread 0 hands them over)
-  __shared__ uint32_t s_parity;
   auto fold = [&](uint64_t c) {
     const size_t half_off = (size_t)((P.seq + c) & 1) * half;
     const Part q = part_of(c, rank);
@@ -184,9 +284,9 @@ __global__ void __launch_bounds__(kThreads, 1) bulk_staged_kernel(const __grid_c
     const size_t pitch = kind == DevColl::reduce_scatter ? (size_t)rank * count : 0;
     const char* own = send + (pitch + q.base + q.lo) * sizeof(T);
     const char* slots = ws.stage[rank] + half_off + q.lo * sizeof(T);
-    auto src = [&](int r) { return r == rank ? own : slots + (size_t)r * slot_b; };
+    auto src = [&](int r) { return !kMixed && r == rank ? own : slots + (size_t)r * slot_b; };
     auto dst = [&](int d) {
-      return d == rank ? recv + (q.base + q.lo) * sizeof(T) : ws.stage[d] + half_off + area_b + (size_t)rank * cap2_b + q.lo * sizeof(T);
+      return d == rank && !(kMixed && two_phase) ? recv + (q.base + q.lo) * sizeof(U) : ws.stage[d] + half_off + area_b + (size_t)rank * cap2_b + q.lo * sizeof(T);
     };
     const uint32_t sub = (uint32_t)(kTile / p) / 256 * 256;   // bytes of one rank's part of a tile
     const size_t n = (whole + sub - 1) / sub;
@@ -228,6 +328,15 @@ __global__ void __launch_bounds__(kThreads, 1) bulk_staged_kernel(const __grid_c
                 acc[k] = r == 0 ? a : red(acc[k], a);
               }
             }
+          if (kMixed && !two_phase) {
+            union { U e[VEC]; uint4 u[(VEC * sizeof(U) + 15) / 16]; } o;
+#pragma unroll
+            for (int k = 0; k < (int)VEC; ++k) o.e[k] = Elem<U>::down(finish_acc(acc[k], P.scale, P.int_div));
+            uint4* d = (uint4*)(dst(rank) + (off / sizeof(T) + VEC * (size_t)w) * sizeof(U));
+#pragma unroll
+            for (int q4 = 0; q4 < (int)(VEC * sizeof(U) / 16); ++q4) d[q4] = o.u[q4];
+            continue;
+          }
           Pack o;
 #pragma unroll
           for (int k = 0; k < (int)VEC; ++k) o.e[k] = Elem<T>::down(finish_acc(acc[k], P.scale, P.int_div));
@@ -257,9 +366,12 @@ __global__ void __launch_bounds__(kThreads, 1) bulk_staged_kernel(const __grid_c
         const A a = Elem<T>::up(__ldcg((const T*)src(r) + e));
         acc = r == 0 ? a : red(acc, a);
       }
-      const T o = Elem<T>::down(finish_acc(acc, P.scale, P.int_div));
-      for (int d = 0; d < p; ++d)
-        if (two_phase || d == rank) ((T*)dst(d))[e] = o;
+      const A v = finish_acc(acc, P.scale, P.int_div);
+      if (two_phase) {
+        for (int d = 0; d < p; ++d) ((T*)dst(d))[e] = Elem<T>::down(v);
+      } else {
+        ((U*)dst(rank))[e] = Elem<U>::down(v);
+      }
     }
     bulk::fence_proxy_async();   // plain stores above, engine loads of the peers behind the next flag
     if (!good && threadIdx.x == 0) report_timeout(ws, rank, rank, 6, make_epoch(P.seq, 1), 0);
@@ -269,16 +381,18 @@ __global__ void __launch_bounds__(kThreads, 1) bulk_staged_kernel(const __grid_c
   auto copy_out = [&](uint64_t c) {
     const char* mystage = ws.stage[rank] + (size_t)((P.seq + c) & 1) * half + (two_phase ? area_b : 0);
     const size_t pitch = two_phase ? 0 : count;
-    if ((int)threadIdx.x < p - 1) {
+    const int n = kMixed ? p : p - 1;   // the own slice is in place unless it still has to be converted
+    if ((int)threadIdx.x < n) {
       Job& job = jobs[threadIdx.x];
       const int r = (rank + 1 + (int)threadIdx.x) % p;
       const Part q = part_of(c, r);
       job.src = mystage + (size_t)r * slot_b + q.lo * sizeof(T);
-      job.bytes = (q.hi - q.lo) * sizeof(T);
+      job.bytes = (q.hi - q.lo) * (kMixed ? 1 : sizeof(T));
       job.ndst = 1;
-      job.dst[0] = recv + ((size_t)r * pitch + q.base + q.lo) * sizeof(T);
+      job.dst[0] = recv + ((size_t)r * pitch + q.base + q.lo) * sizeof(U);
     }
-    return copy_jobs(p - 1);
+    if constexpr (kMixed) return convert_jobs(n, T(), U());
+    return copy_jobs(n);
   };
 
   const uint64_t G = P.local_chunks[rank];
@@ -307,9 +421,9 @@ __global__ void __launch_bounds__(kThreads, 1) bulk_staged_kernel(const __grid_c
   }
 }
 
-template <typename T, typename Red>
+template <typename T, typename U = T, typename Red>
 void launch_one(const CollParams& P, Red red, int ctas, int local_ranks, cudaStream_t stream) {
-  auto k = bulk_staged_kernel<T, Red>;
+  auto k = bulk_staged_kernel<T, U, Red>;
   AL_CHECK_CUDA(cudaFuncSetAttribute((const void*)k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem));
   void* args[] = {(void*)&P, (void*)&red};
   AL_CHECK_CUDA(cudaLaunchCooperativeKernel((const void*)k, dim3((unsigned)ctas, (unsigned)local_ranks, 1), dim3(kThreads), args, kSmem, stream));
@@ -317,20 +431,23 @@ void launch_one(const CollParams& P, Red red, int ctas, int local_ranks, cudaStr
 
 }  // namespace
 
-bool bulk_staged_supported(DevColl kind, DType dt, ReductionOperator op) {
-  if (kind == DevColl::allgather || kind == DevColl::alltoall) return dt == DType::u8;
-  return (kind == DevColl::allreduce || kind == DevColl::reduce_scatter) && (op == ReductionOperator::sum || op == ReductionOperator::avg) &&
-         (dt == DType::f32 || dt == DType::bf16 || dt == DType::f16);
+bool bulk_staged_supported(DevColl kind, DType user, DType wire, ReductionOperator op) {
+  if (kind == DevColl::allgather || kind == DevColl::alltoall) return user == DType::u8 && wire == DType::u8;
+  if ((kind != DevColl::allreduce && kind != DevColl::reduce_scatter) || (op != ReductionOperator::sum && op != ReductionOperator::avg)) return false;
+  if (user == wire) return user == DType::f32 || user == DType::bf16 || user == DType::f16;
+  return kind == DevColl::allreduce && user == DType::f32 && (wire == DType::bf16 || wire == DType::f16);
 }
 
-void launch_bulk_staged(const CollParams& P, DType dt, int ctas, int local_ranks, cudaStream_t stream) {
+void launch_bulk_staged(const CollParams& P, DType user, DType wire, int ctas, int local_ranks, cudaStream_t stream) {
   const DevColl kind = (DevColl)P.kind;
-  if (!bulk_staged_supported(kind, dt, (ReductionOperator)P.op) || P.pipelined || P.slot_elems)
+  if (!bulk_staged_supported(kind, user, wire, (ReductionOperator)P.op) || P.pipelined || P.slot_elems)
     throw_al_exception("bulk staged kernel: unsupported operation");
-  switch (dt) {
+  const bool mixed = user != wire;
+  switch (wire) {
     case DType::f32: return launch_one<float>(P, RedSum(), ctas, local_ranks, stream);
-    case DType::bf16: return launch_one<__nv_bfloat16>(P, RedSum(), ctas, local_ranks, stream);
-    case DType::f16: return launch_one<__half>(P, RedSum(), ctas, local_ranks, stream);
+    case DType::bf16:
+      return mixed ? launch_one<__nv_bfloat16, float>(P, RedSum(), ctas, local_ranks, stream) : launch_one<__nv_bfloat16>(P, RedSum(), ctas, local_ranks, stream);
+    case DType::f16: return mixed ? launch_one<__half, float>(P, RedSum(), ctas, local_ranks, stream) : launch_one<__half>(P, RedSum(), ctas, local_ranks, stream);
     default: return launch_one<unsigned char>(P, RedNone(), ctas, local_ranks, stream);
   }
 }

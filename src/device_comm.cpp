@@ -622,11 +622,11 @@ void DeviceCommunicator::collective(const CollDesc& d, const std::vector<RankArg
   }
 
   // All ranks on this GPU: large operations are moved by the bulk copy engine, chunked by what staging holds.
-  bool bulk_staged = I.nlocal > 1 && !use_window && !d.vector && d.ctas <= 0 && !tn.bulk_pipeline && in == wire && wire == out &&
-                     bulk_staged_supported(d.kind, wire, d.op) && (d.kind == DevColl::allreduce || P.count * esz % 16 == 0) &&
+  bool bulk_staged = I.nlocal > 1 && !use_window && !d.vector && d.ctas <= 0 && !tn.bulk_pipeline && in == out &&
+                     bulk_staged_supported(d.kind, in, wire, d.op) && (d.kind == DevColl::allreduce || P.count * esz % 16 == 0) &&
                      P.count * esz * (d.kind == DevColl::allreduce ? 1 : (size_t)p) >= (p == 2 && !reduces ? kBulkStagedMinMoveTwo : kBulkStagedMinBytes);
   for (int r = 0; bulk_staged && r < p; ++r)
-    bulk_staged = P.own_direct[r] && (uintptr_t)P.send[r] % 16 == 0 && (uintptr_t)P.recv[r] % 16 == 0;
+    bulk_staged = (P.own_direct[r] || in != wire) && P.send[r] && P.recv[r] && (uintptr_t)P.send[r] % 16 == 0 && (uintptr_t)P.recv[r] % 16 == 0;
 
   // Large uniform reduce_scatter / allgather / alltoall run pipelined: smaller chunks, half of the
   // grid publishing while the other half consumes.
@@ -773,7 +773,7 @@ void DeviceCommunicator::collective(const CollDesc& d, const std::vector<RankArg
       return;
     }
   }
-  if (bulk_staged) return launch_bulk_staged(P, wire, I.sm_count / I.nlocal, I.nlocal, stream);
+  if (bulk_staged) return launch_bulk_staged(P, in, wire, I.sm_count / I.nlocal, I.nlocal, stream);
   launch_collective(P, in, wire, out, ctas, threads, I.nlocal, stream);
 }
 

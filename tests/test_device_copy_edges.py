@@ -124,6 +124,14 @@ def test_large_operations_in_bulk_copies(al, p, stage):
         assert all(torch.equal(o, want) for o in outs)
         comm.allreduce(xs, algo="two_shot" if p > 2 else "one_shot")
         assert all(torch.equal(x, want) for x in xs)
+    for wire, n in ((torch.bfloat16, 524288), (torch.float16, 1310727), (torch.bfloat16, 3000003)):
+        xs = [small_ints(n, torch.float32, r) for r in range(p)]
+        want = sum(xs)
+        outs = [torch.empty_like(x) for x in xs]
+        comm.allreduce(xs, outs, wire_dtype=wire)
+        assert all(torch.equal(o, want) for o in outs)
+        comm.allreduce(xs, wire_dtype=wire)
+        assert all(torch.equal(x, want) for x in xs)
     for dtype, n in ((torch.bfloat16, 262144), (torch.float32, 131072 * 3 + 4), (torch.float32, 655360 + 12)):
         full = [small_ints(p * n, dtype, 50 + r) for r in range(p)]
         want = sum(f.float() for f in full).to(dtype)
