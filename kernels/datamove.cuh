@@ -159,6 +159,7 @@ __device__ __forceinline__ void batched_units(size_t units, unsigned lane, unsig
 }
 
 /** Copy `nbytes` with `nlanes` cooperating threads (this thread is `lane`), whatever the two alignments. */
+template <int U = kUnroll>
 __device__ __forceinline__ void group_copy(char* dst, const char* src, size_t nbytes, bool src_is_staging,
                                            unsigned lane, unsigned nlanes) {
   if (nbytes == 0) return;
@@ -170,17 +171,18 @@ __device__ __forceinline__ void group_copy(char* dst, const char* src, size_t nb
   const WordSource s(src + head, src_is_staging);
   auto store = [&](size_t i, const uint4& v) { d[i] = v; };
   if (s.sh == 0) {
-    if (src_is_staging) batched_units<kUnroll>(nv, lane, nlanes, [&](size_t i) { return __ldcg(s.base + i); }, store);
-    else batched_units<kUnroll>(nv, lane, nlanes, [&](size_t i) { return s.base[i]; }, store);
+    if (src_is_staging) batched_units<U>(nv, lane, nlanes, [&](size_t i) { return __ldcg(s.base + i); }, store);
+    else batched_units<U>(nv, lane, nlanes, [&](size_t i) { return s.base[i]; }, store);
   } else {
-    batched_units<kUnroll / 4>(nv, lane, nlanes, [&](size_t i) { return s.shifted(i); }, store);
+    batched_units<U / 4>(nv, lane, nlanes, [&](size_t i) { return s.shifted(i); }, store);
   }
   for (size_t k = done + lane; k < nbytes; k += nlanes) dst[k] = src_is_staging ? __ldcg(src + k) : src[k];
 }
 
-/** Copy with all threads of the CTA. */
+/** Copy with all threads of the CTA.  (Kernels that are held to 64 registers and spill with eight loads pass U = 4.) */
+template <int U = kUnroll>
 __device__ __forceinline__ void cta_copy(char* dst, const char* src, size_t nbytes, bool src_is_staging) {
-  group_copy(dst, src, nbytes, src_is_staging, threadIdx.x, blockDim.x);
+  group_copy<U>(dst, src, nbytes, src_is_staging, threadIdx.x, blockDim.x);
 }
 
 // ---------------------------------------------------------------------------

@@ -94,7 +94,7 @@ __global__ void __launch_bounds__(512, 2) nvls_allreduce_kernel(const __grid_con
     const size_t base = c * full_e, len = clamp_len(P.count, base, full_e);
     size_t lo, hi;
     split_range(len, blockIdx.x, gridDim.x, 16 / sizeof(T), lo, hi);
-    if (hi > lo) cta_copy(mystage + lo * sizeof(T), (const char*)(send + base + lo), (hi - lo) * sizeof(T), false);
+    if (hi > lo) cta_copy<4>(mystage + lo * sizeof(T), (const char*)(send + base + lo), (hi - lo) * sizeof(T), false);
 
     const uint64_t e = make_epoch(P.seq, c + 1);
     arrive_and_post(ws, rank, FlagLayout::off_A, 0, gridDim.x, e, c == 0, (int)(P.seq & 1), G, my_proto);
@@ -109,7 +109,7 @@ __global__ void __launch_bounds__(512, 2) nvls_allreduce_kernel(const __grid_con
     arrive_and_post(ws, rank, FlagLayout::off_B, 1, gridDim.x, e, false, 0, 0);
     if (!wait_all(ws, rank, FlagLayout::off_B, 1, e, P.timeout_ns)) return;
 
-    if (hi > lo) cta_copy((char*)(recv + base + lo), mystage + lo * sizeof(T), (hi - lo) * sizeof(T), true);
+    if (hi > lo) cta_copy<4>((char*)(recv + base + lo), mystage + lo * sizeof(T), (hi - lo) * sizeof(T), true);
   }
   if (G > 1) {
     const uint64_t e = make_epoch(P.seq, 1);
@@ -166,7 +166,7 @@ __global__ void __launch_bounds__(512, 2) nvls_allreduce_pipelined_kernel(const 
       const size_t base = c * chunk_e, len = clamp_len(P.count, base, chunk_e);
       size_t lo, hi;
       split_range(len, b, n_in, 16 / sizeof(T), lo, hi);
-      if (hi > lo) cta_copy(mystage + lo * sizeof(T), (const char*)(send + base + lo), (hi - lo) * sizeof(T), false);
+      if (hi > lo) cta_copy<4>(mystage + lo * sizeof(T), (const char*)(send + base + lo), (hi - lo) * sizeof(T), false);
       arrive_and_post_ring(ws, rank, FlagLayout::off_A, 0, c, D, n_in, make_epoch(P.seq, c + 1), c == 0, (int)(P.seq & 1), G, my_proto);
     }
   } else if (b < n_in + n_red) {
@@ -196,7 +196,7 @@ __global__ void __launch_bounds__(512, 2) nvls_allreduce_pipelined_kernel(const 
       const size_t base = c * chunk_e, len = clamp_len(P.count, base, chunk_e);
       size_t lo, hi;
       split_range(len, b - n_in - n_red, n_out, 16 / sizeof(T), lo, hi);
-      if (hi > lo) cta_copy((char*)(recv + base + lo), mystage + lo * sizeof(T), (hi - lo) * sizeof(T), true);
+      if (hi > lo) cta_copy<4>((char*)(recv + base + lo), mystage + lo * sizeof(T), (hi - lo) * sizeof(T), true);
       arrive_and_post_ring(ws, rank, FlagLayout::off_C, 2, c, D, n_out, make_epoch(P.seq, c + 1), false, 0, 0);
     }
   }
@@ -245,7 +245,7 @@ __global__ void __launch_bounds__(512, 2) nvls_reduce_scatter_kernel(const __gri
       if (hi > lo)
         for (int i = 0; i < p; ++i) {
           const int d = (rank + i) % p;
-          cta_copy(mystage + (size_t)d * cap_b + lo * sizeof(T), (const char*)(send + (size_t)d * P.count + base + lo),
+          cta_copy<4>(mystage + (size_t)d * cap_b + lo * sizeof(T), (const char*)(send + (size_t)d * P.count + base + lo),
                    (hi - lo) * sizeof(T), false);
         }
       arrive_and_post(ws, rank, FlagLayout::off_A, 0, n_in, make_epoch(P.seq, c + 1), c == 0, (int)(P.seq & 1), G, my_proto);

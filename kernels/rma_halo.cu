@@ -143,8 +143,8 @@ __global__ void __launch_bounds__(512, 2) halo_pack_kernel(float* packed, const 
     if (len > hi - lo) len = hi - lo;
     const float* t = tensor + (c * d_total + d_first) * plane + within;
     float* pk = packed + lo;
-    if (unpack) cta_copy((char*)t, (const char*)pk, len * sizeof(float), false);
-    else cta_copy((char*)pk, (const char*)t, len * sizeof(float), false);
+    if (unpack) cta_copy<4>((char*)t, (const char*)pk, len * sizeof(float), false);
+    else cta_copy<4>((char*)pk, (const char*)t, len * sizeof(float), false);
     lo += len;
   }
 }
