@@ -122,7 +122,8 @@ def torch_ops():
         load()
         path = _LIB_PATH.with_name("libal_torch.so")
         if not path.exists():
-            raise AlError(f"native library missing: {path}")
+            from . import _build
+            _build.build(tools=False)
         torch.ops.load_library(str(path))
         _torch_ops = torch.ops.aluminum_b200
     return _torch_ops

@@ -32,8 +32,8 @@ void launch_collective(const CollParams& P, DType in, DType wire, DType out, int
 bool collective_supported(DType in, DType wire, DType out, ReductionOperator op);
 
 // ---- staged operations with all ranks on this GPU, moved by the bulk copy engine (kernels/bulk_staged.cu) ----
-/** Element types of the buffers and of staging, and operator; the kernel also wants 16-byte aligned buffers (and slices) and,
- *  with one type throughout, P.own_direct on every rank. */
+/** Element types of the buffers and of staging, and operator; the kernel also wants 16-byte aligned buffers and,
+ *  with one type throughout and unless a reduce_scatter's slices are no whole words, P.own_direct on every rank. */
 bool bulk_staged_supported(DevColl kind, DType user, DType wire, ReductionOperator op);
 void launch_bulk_staged(const CollParams& P, DType user, DType wire, int ctas, int local_ranks, cudaStream_t stream);
 

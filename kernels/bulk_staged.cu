@@ -8,7 +8,8 @@
 // registers for them; reductions are folded out of shared memory while the next tiles arrive.  Loops -> bulk copies:
 // bucket of 4 x 26 MB 136 -> 103 us (525 MB through HBM, 5.1 TB/s), sequence-parallel pair of 4 ranks, 16384 x 8192 bf16,
 // 1668 -> 1036 us (5.4 GB, 5.2 TB/s), of 8 ranks, 2048 x 4096, 203 -> 163 us; bucket of 8 x 12 MB with a bf16 wire, converted
-// between the tiles and staging by all threads, 116 -> 98 us.
+// between the tiles and staging by all threads, 116 -> 98 us.  Slices that begin anywhere (pair of 8 ranks, 16344 x 990 bf16)
+// are shifted into the destination's words out of the tiles: 417 -> 330 us.
 // (Between GPUs the engine's stores to peers were slower than SM stores - 4 GPUs, 1 GiB allgather 1534 us against
 // 1291 us - so ranks on GPUs of their own keep coll_kernel.)
 //
@@ -29,8 +30,9 @@ constexpr int kTile = 32768;
 constexpr size_t kSmem = (size_t)kBufs * kTile + 128;  // tiles + barriers
 constexpr int kThreads = 512;
 
-/** T: element type in staging; U: element type of the user's buffers (another one for an allreduce with a narrower wire type). */
-template <typename T, typename U, typename Red>
+/** T: element type in staging; U: element type of the user's buffers (another one for an allreduce with a narrower wire type);
+ *  RAGGED: slices do not begin on 16-byte boundaries of the user's buffers (as a run-time choice it cost the others 4 %). */
+template <typename T, typename U, bool RAGGED, typename Red>
 __global__ void __launch_bounds__(kThreads, 1) bulk_staged_kernel(const __grid_constant__ CollParams P, Red red) {
   constexpr bool kMixed = !std::is_same<T, U>::value;
   extern __shared__ __align__(128) unsigned char dyn_smem[];
@@ -53,6 +55,7 @@ __global__ void __launch_bounds__(kThreads, 1) bulk_staged_kernel(const __grid_c
   const size_t slot_b = two_phase ? cap2_b : cap_b;
   const size_t unit = two_phase ? (size_t)p * (cap2_b / sizeof(T)) : cap_b / sizeof(T);  // elements per chunk (of a slice)
   const size_t count = P.count;                                                          // vector, or one rank's slice
+  constexpr bool ragged = RAGGED;
   const char* send = (const char*)P.send[rank];
   char* recv = (char*)P.recv[rank];
   const unsigned cta = blockIdx.x, nct = gridDim.x;
@@ -145,6 +148,85 @@ __global__ void __launch_bounds__(kThreads, 1) bulk_staged_kernel(const __grid_c
 
   uint32_t parity = 0;   // every thread's view of the ring's parities (thread 0 hands them over)
   __shared__ uint32_t s_parity;
+  /** The same for jobs of one destination where source and destination lie differently in their 16-byte words: tiles of aligned
+   *  words arrive by the engine, all threads shift them into the destination's words. */
+  auto shift_jobs = [&](int n) {
+    constexpr uint32_t kWords = kTile / 16 - 1;   // of the destination; an unaligned source takes one more
+    __syncthreads();
+    auto words_of = [&](int j) {
+      const size_t head = (0 - (uintptr_t)jobs[j].dst[0]) & 15;
+      return jobs[j].bytes > head ? (jobs[j].bytes - head) / 16 : (size_t)0;
+    };
+    size_t total = 0;
+    for (int j = 0; j < n; ++j) total += (words_of(j) + kWords - 1) / kWords;
+    struct Cursor { int j; size_t off; };
+    auto seek = [&](Cursor& at) {   // to the next tile that exists; called only while there is one
+      for (;;) {
+        if (at.j == n) { at.j = 0; at.off += kWords; }
+        if (at.off < words_of(at.j)) return;
+        ++at.j;
+      }
+    };
+    auto len = [&](const Cursor& at) {
+      const size_t left = words_of(at.j) - at.off;
+      return (uint32_t)(left < kWords ? left : kWords);
+    };
+    Cursor in{0, 0}, out{0, 0};
+    auto load = [&](size_t t) {
+      const int s = (int)(t % kBufs);
+      seek(in);
+      const char* src = jobs[in.j].src + ((0 - (uintptr_t)jobs[in.j].dst[0]) & 15) + 16 * in.off;
+      const unsigned sh = (unsigned)((uintptr_t)src & 15);
+      const uint32_t bytes = 16 * (len(in) + (sh ? 1u : 0u));
+      bulk::mbar_expect_tx(ring.bar(s), bytes);
+      bulk::g2s(ring.tile(s), src - sh, bytes, ring.bar(s));
+      ++in.j;
+    };
+    if (threadIdx.x == 0) {
+      s_parity = ring.parity;
+      bulk::fence_proxy_async();
+      for (size_t t = 0; t < total && t < kBufs; ++t) load(t);
+    }
+    __syncthreads();
+    parity = s_parity;
+    bool good = true;
+    for (size_t t = 0; t < total; ++t) {
+      const int s = (int)(t % kBufs);
+      const bool ok = bulk::mbar_wait(bars + 8 * s, (parity >> s) & 1u, P.timeout_ns);
+      parity ^= 1u << s;
+      seek(out);
+      const size_t head = (0 - (uintptr_t)jobs[out.j].dst[0]) & 15;
+      const uint32_t words = len(out);
+      WordSource from((const char*)dyn_smem + (size_t)s * kTile, false);
+      from.sh = (unsigned)((uintptr_t)(jobs[out.j].src + head) & 15);
+      uint4* d = (uint4*)(jobs[out.j].dst[0] + head) + out.off;
+      if (ok) {
+        if (from.sh)
+          for (uint32_t w = threadIdx.x; w < words; w += kThreads) d[w] = from.shifted(w);
+        else
+          for (uint32_t w = threadIdx.x; w < words; w += kThreads) d[w] = from.base[w];
+      }
+      ++out.j;
+      if (__syncthreads_or(!ok)) {   // also: everyone has read the tile
+        good = false;
+        if (threadIdx.x == 0)        // the copies in flight end before the block does (or it gives up on them)
+          for (size_t u = t; u < total && u < t + kBufs; ++u)
+            (void)bulk::mbar_wait(bars + 8 * (u % kBufs), (parity >> (u % kBufs) ^ (u == t)) & 1u, P.timeout_ns);
+        break;
+      }
+      if (threadIdx.x == 0 && t + kBufs < total) load(t + kBufs);
+    }
+    if (threadIdx.x == 0) ring.parity = parity;
+    for (int j = 0; j < n; ++j) {    // bytes in front of the first word and behind the last
+      const size_t head = (0 - (uintptr_t)jobs[j].dst[0]) & 15, behind = head + 16 * words_of(j) + (threadIdx.x - 16);
+      if (threadIdx.x < 16 && threadIdx.x < head && threadIdx.x < jobs[j].bytes) jobs[j].dst[0][threadIdx.x] = __ldcg(jobs[j].src + threadIdx.x);
+      if (threadIdx.x >= 16 && threadIdx.x < 32 && behind < jobs[j].bytes) jobs[j].dst[0][behind] = __ldcg(jobs[j].src + behind);
+    }
+    bulk::fence_proxy_async();       // plain stores above, engine loads behind the next flag
+    __syncthreads();                 // the list may be filled again
+    if (!good && threadIdx.x == 0) report_timeout(ws, rank, rank, 6, make_epoch(P.seq, 1), 0);
+    return good;
+  };
   /** The same with conversion: jobs[0..n) whose `bytes` counts elements of In, converted to Out.  All threads convert out of
    *  the tiles; eight elements are one or two 16-byte words on either side. */
   auto convert_jobs = [&](int n, auto in_type, auto out_type) {
@@ -252,16 +334,29 @@ __global__ void __launch_bounds__(kThreads, 1) bulk_staged_kernel(const __grid_c
         job.bytes = (q.hi - q.lo) * sizeof(T);
         job.ndst = 0;
         for (int i = 1; i < p; ++i) job.dst[job.ndst++] = ws.stage[(rank + i) % p] + half_off + (size_t)rank * slot_b + q.lo * sizeof(T);
+        char* mine = recv + ((size_t)rank * count + q.base + q.lo) * sizeof(T);
         if (kind == DevColl::allgather) {
-          char* mine = recv + ((size_t)rank * count + q.base + q.lo) * sizeof(T);
-          if (mine != job.src) job.dst[job.ndst++] = mine;
+          if (ragged) {   // the own part does not lie on word boundaries of the receive buffer
+            jobs[1] = job;
+            jobs[1].dst[0] = mine;
+            jobs[1].ndst = 1;
+            if (mine == job.src) jobs[1].bytes = 0;
+          } else if (mine != job.src) {
+            job.dst[job.ndst++] = mine;
+          }
         }
       }
-      return copy_jobs(1);
+      const bool done = copy_jobs(1);
+      if constexpr (ragged) {
+        if (!done) return false;
+        if (threadIdx.x == 0) jobs[0] = jobs[1];
+        return shift_jobs(1);
+      }
+      return done;
     }
     // slice d goes to rank d; the own one stays (reductions) or is copied to its place
     const size_t pitch = two_phase ? 0 : count;
-    const bool keep = reduces || send == recv;
+    const bool keep = two_phase || (reduces && !ragged) || (!reduces && send == recv);   // a ragged own slice is folded out of staging
     const int n = keep ? p - 1 : p;
     if ((int)threadIdx.x < n) {
       Job& job = jobs[threadIdx.x];
@@ -270,10 +365,11 @@ __global__ void __launch_bounds__(kThreads, 1) bulk_staged_kernel(const __grid_c
       job.src = send + ((size_t)d * pitch + q.base + q.lo) * sizeof(T);
       job.bytes = (q.hi - q.lo) * sizeof(T);
       job.ndst = 1;
-      job.dst[0] = d == rank ? recv + ((size_t)rank * count + q.base + q.lo) * sizeof(T)
+      job.dst[0] = d == rank && !reduces ? recv + ((size_t)rank * count + q.base + q.lo) * sizeof(T)
                              : ws.stage[d] + half_off + (size_t)rank * slot_b + q.lo * sizeof(T);
     }
-    return copy_jobs(n);
+    if constexpr (ragged) return shift_jobs(n);
+    else return copy_jobs(n);
   };
 
   /** Fold the p contributions of the own slice; the result goes to the receive buffer and, in two phases, to every peer. */
@@ -284,7 +380,7 @@ __global__ void __launch_bounds__(kThreads, 1) bulk_staged_kernel(const __grid_c
     const size_t pitch = kind == DevColl::reduce_scatter ? (size_t)rank * count : 0;
     const char* own = send + (pitch + q.base + q.lo) * sizeof(T);
     const char* slots = ws.stage[rank] + half_off + q.lo * sizeof(T);
-    auto src = [&](int r) { return !kMixed && r == rank ? own : slots + (size_t)r * slot_b; };
+    auto src = [&](int r) { return !kMixed && !ragged && r == rank ? own : slots + (size_t)r * slot_b; };
     auto dst = [&](int d) {
       return d == rank && !(kMixed && two_phase) ? recv + (q.base + q.lo) * sizeof(U) : ws.stage[d] + half_off + area_b + (size_t)rank * cap2_b + q.lo * sizeof(T);
     };
@@ -392,6 +488,7 @@ __global__ void __launch_bounds__(kThreads, 1) bulk_staged_kernel(const __grid_c
       job.dst[0] = recv + ((size_t)r * pitch + q.base + q.lo) * sizeof(U);
     }
     if constexpr (kMixed) return convert_jobs(n, T(), U());
+    if constexpr (ragged) return shift_jobs(n);
     return copy_jobs(n);
   };
 
@@ -423,7 +520,8 @@ __global__ void __launch_bounds__(kThreads, 1) bulk_staged_kernel(const __grid_c
 
 template <typename T, typename U = T, typename Red>
 void launch_one(const CollParams& P, Red red, int ctas, int local_ranks, cudaStream_t stream) {
-  auto k = bulk_staged_kernel<T, U, Red>;
+  auto k = bulk_staged_kernel<T, U, false, Red>;
+  if ((DevColl)P.kind != DevColl::allreduce && P.count * sizeof(T) % 16 != 0) k = bulk_staged_kernel<T, T, true, Red>;
   AL_CHECK_CUDA(cudaFuncSetAttribute((const void*)k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem));
   void* args[] = {(void*)&P, (void*)&red};
   AL_CHECK_CUDA(cudaLaunchCooperativeKernel((const void*)k, dim3((unsigned)ctas, (unsigned)local_ranks, 1), dim3(kThreads), args, kSmem, stream));

@@ -623,10 +623,10 @@ void DeviceCommunicator::collective(const CollDesc& d, const std::vector<RankArg
 
   // All ranks on this GPU: large operations are moved by the bulk copy engine, chunked by what staging holds.
   bool bulk_staged = I.nlocal > 1 && !use_window && !d.vector && d.ctas <= 0 && !tn.bulk_pipeline && in == out &&
-                     bulk_staged_supported(d.kind, in, wire, d.op) && (d.kind == DevColl::allreduce || P.count * esz % 16 == 0) &&
+                     bulk_staged_supported(d.kind, in, wire, d.op) &&
                      P.count * esz * (d.kind == DevColl::allreduce ? 1 : (size_t)p) >= (p == 2 && !reduces ? kBulkStagedMinMoveTwo : kBulkStagedMinBytes);
   for (int r = 0; bulk_staged && r < p; ++r)
-    bulk_staged = (P.own_direct[r] || in != wire) && P.send[r] && P.recv[r] && (uintptr_t)P.send[r] % 16 == 0 && (uintptr_t)P.recv[r] % 16 == 0;
+    bulk_staged = (P.own_direct[r] || in != wire || (d.kind == DevColl::reduce_scatter && P.count * esz % 16 != 0)) && P.send[r] && P.recv[r] && (uintptr_t)P.send[r] % 16 == 0 && (uintptr_t)P.recv[r] % 16 == 0;
 
   // Large uniform reduce_scatter / allgather / alltoall run pipelined: smaller chunks, half of the
   // grid publishing while the other half consumes.
@@ -747,7 +747,7 @@ void DeviceCommunicator::collective(const CollDesc& d, const std::vector<RankArg
     Wp.allow_multimem = tn.window_multimem ? (1 | (p >= tn.window_multimem_ag_ranks ? 2 : 0)) : 0;
     const size_t moved = P.count * esz * (d.kind == DevColl::alltoall ? (size_t)p : 1);
     int wctas = d.ctas > 0 ? d.ctas : (int)std::max<size_t>(1, std::min<size_t>(ceil_div(moved, (size_t)32768), (size_t)tn.window_ctas));
-    if (I.nlocal > 1) wctas = std::max(1, std::min(wctas, I.sm_count / I.nlocal));
+    wctas = std::max(1, std::min(wctas, I.sm_count / I.nlocal));   // one CTA per SM: they wait for each other
     I.stats.window++;
     launch_window(Wp, wire, d.op, wctas, threads, I.nlocal, stream);
     return;

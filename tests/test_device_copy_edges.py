@@ -132,7 +132,8 @@ def test_large_operations_in_bulk_copies(al, p, stage):
         assert all(torch.equal(o, want) for o in outs)
         comm.allreduce(xs, wire_dtype=wire)
         assert all(torch.equal(x, want) for x in xs)
-    for dtype, n in ((torch.bfloat16, 262144), (torch.float32, 131072 * 3 + 4), (torch.float32, 655360 + 12)):
+    for dtype, n in ((torch.bfloat16, 262144), (torch.float32, 131072 * 3 + 4), (torch.float32, 655360 + 12),
+                     (torch.bfloat16, 524288 + 1), (torch.float32, 262144 + 3), (torch.bfloat16, 1310720 + 13)):
         full = [small_ints(p * n, dtype, 50 + r) for r in range(p)]
         want = sum(f.float() for f in full).to(dtype)
         outs = [torch.empty(n, device="cuda", dtype=dtype) for _ in range(p)]
