@@ -63,6 +63,7 @@ def _declare(lib) -> None:
         "al_host_comm_create_group": (vp, [C.POINTER(C.c_int), i]),
         "al_dev_comm_split": (vp, [vp, i, i, vp]), "al_dev_comm_destroy": (None, [vp]),
         "al_dev_comm_rank": (i, [vp]), "al_dev_comm_size": (i, [vp]), "al_dev_comm_nlocal": (i, [vp]),
+        "al_dev_comm_device": (i, [vp]),
         "al_dev_comm_has_multicast": (i, [vp]), "al_dev_comm_backing": (C.c_char_p, [vp]),
         "al_dev_comm_set_timeout_ms": (i, [vp, d]), "al_dev_comm_stats": (i, [vp, u64p]),
         "al_dev_comm_status": (i, [vp, u64p]),
@@ -81,7 +82,7 @@ def _declare(lib) -> None:
         "al_rma_sync": (i, [vp, i]),
         "al_halo_exchange": (i, [vp, vpp, sz, sz, sz, sz, i, i, vp]),
         "al_halo_pack": (i, [vp, vp, sz, sz, sz, sz, sz, i, vp]),
-        "al_route_rows": (i, [i, vpp, szp, i, vpp, vp, vp]),
+        "al_route_rows": (i, [vp, i, vpp, szp, vpp, vp, vp]),
         "al_scale_cast": (i, [vp, i, vp, i, sz, d, vp]),
         "al_sgd_momentum": (i, [vp, vp, vp, sz, C.c_float, C.c_float, C.c_float, C.c_float, i, i, vp]),
         "al_fill_u32": (i, [vp, sz, C.c_uint32, vp]),

@@ -54,6 +54,7 @@ class DeviceComm:
         self.rank = lib.al_dev_comm_rank(self._h)
         self.size = lib.al_dev_comm_size(self._h)
         self.nlocal = lib.al_dev_comm_nlocal(self._h)
+        self.device_index = lib.al_dev_comm_device(self._h)
         self.emulated = self.nlocal > 1 or bool(emulate)
         self._symm = {}
 

@@ -13,7 +13,7 @@ import ctypes as C
 import torch
 
 from .. import _lib
-from .._lib import check
+from .._lib import AlError, check
 from ._util import call, unwrap, wrap
 
 
@@ -25,19 +25,34 @@ def _prefix(counts):
     return out
 
 
+_INTS = (torch.int64, torch.int32, torch.int16, torch.int8, torch.uint8)
+
+
+def _on_device(comm, what, tensors):
+    """Kernels get plain addresses: one tensor per local rank, all on the communicator's GPU."""
+    if len(tensors) != comm.nlocal:
+        raise AlError(f"{what}: expected {comm.nlocal} tensor(s), one per local rank, got {len(tensors)}")
+    for t in tensors:
+        if t.get_device() != comm.device_index:   # (-1 for host memory)
+            raise AlError(f"{what}: must be on the communicator's GPU (cuda:{comm.device_index}), not on {t.device}")
+
+
 def _route(comm, dests):
     """Stable order of every local rank's tokens by destination, and a (2, local ranks, ranks) buffer whose first half
     holds the tokens per destination (one launch for all local ranks)."""
     n, p = len(dests), comm.size
-    for d in dests:
-        if d.dim() != 1 or d.is_floating_point() or d.is_complex():
+    dests = list(dests)
+    _on_device(comm, "dest_rank", dests)
+    for r, d in enumerate(dests):
+        if d.dim() != 1 or d.dtype not in _INTS:
             raise ValueError("dest_rank: a one-dimensional integer tensor per rank")
-    dests = [d.to(torch.int64).contiguous() for d in dests]
-    order = [torch.empty_like(d) for d in dests]
+        if d.dtype != torch.int64 or not d.is_contiguous():
+            dests[r] = d.to(torch.int64).contiguous()
+    sizes = [d.numel() for d in dests]
     both = torch.empty((2, n, p), device=dests[0].device, dtype=torch.int64)
-    check(_lib.load().al_route_rows(n, (C.c_void_p * n)(*[d.data_ptr() for d in dests]), (C.c_size_t * n)(*[d.numel() for d in dests]), p,
-                                    (C.c_void_p * n)(*[o.data_ptr() for o in order]), both.data_ptr(),
-                                    torch.cuda.current_stream().cuda_stream))
+    order = [torch.empty_like(d) for d in dests]
+    check(_lib.load().al_route_rows(comm._h, n, (C.c_void_p * n)(*[d.data_ptr() for d in dests]), (C.c_size_t * n)(*sizes),
+                                    (C.c_void_p * n)(*[o.data_ptr() for o in order]), both.data_ptr(), comm._stream()))
     return order, both
 
 
@@ -48,6 +63,10 @@ def dispatch(comm, tokens, dest_rank):
     p = comm.size
     toks = [t.contiguous() for t in wrap(comm, tokens)]
     dests = wrap(comm, dest_rank)
+    _on_device(comm, "tokens", toks)
+    for t, d in zip(toks, dests):
+        if d.numel() > t.shape[0]:
+            raise ValueError("dispatch: dest_rank has more entries than there are tokens")
     order, both = _route(comm, dests)
     call(comm, comm.alltoall, list(both[0].unbind()), list(both[1].unbind()))
     sc, rc = both.tolist()   # the one host read

@@ -89,6 +89,7 @@ void al_dev_comm_destroy(void* comm);
 int al_dev_comm_rank(void* comm);
 int al_dev_comm_size(void* comm);
 int al_dev_comm_nlocal(void* comm);
+int al_dev_comm_device(void* comm);
 int al_dev_comm_has_multicast(void* comm);
 const char* al_dev_comm_backing(void* comm);
 int al_dev_comm_set_timeout_ms(void* comm, double ms);
@@ -180,8 +181,9 @@ int al_halo_exchange(void* comm, float* const* tensors, size_t nc, size_t d_loca
 int al_halo_pack(float* packed, const float* tensor, size_t nc, size_t d_total, size_t plane, size_t d_first,
                  size_t depth, int unpack, void* stream);
 
-/* Stable order of n[r] tokens by destination rank and counts[r * p + d], for nlocal ranks; counts are -1 where a destination is none of the p ranks. */
-int al_route_rows(int nlocal, const long long* const* dest, const size_t* n, int p, long long* const* order, long long* counts, void* stream);
+/* Stable order of n[r] tokens by destination rank and counts[r * size + d], for the communicator's nlocal local ranks; counts are -1 where a
+   destination is no rank of the communicator.  dest, order and counts are memory of the communicator's GPU. */
+int al_route_rows(void* comm, int nlocal, const long long* const* dest, const size_t* n, long long* const* order, long long* counts, void* stream);
 
 /* ---- element-wise kernels ---- */
 int al_scale_cast(void* out, int out_dt, const void* in, int in_dt, size_t n, double scale, void* stream);

@@ -295,6 +295,7 @@ int al_dev_comm_nlocal(void* comm) {
   auto* c = (DeviceCommunicator*)comm;
   return c->is_emulated() ? c->size() : 1;
 }
+int al_dev_comm_device(void* comm) { return ((DeviceCommunicator*)comm)->device(); }
 int al_dev_comm_has_multicast(void* comm) { return ((DeviceCommunicator*)comm)->has_multicast() ? 1 : 0; }
 const char* al_dev_comm_backing(void* comm) { return ((DeviceCommunicator*)comm)->memory_backing(); }
 int al_dev_comm_set_timeout_ms(void* comm, double ms) {
@@ -608,9 +609,12 @@ int al_halo_pack(float* packed, const float* tensor, size_t nc, size_t d_total, 
   });
 }
 
-int al_route_rows(int nlocal, const long long* const* dest, const size_t* n, int p, long long* const* order, long long* counts, void* stream) {
+int al_route_rows(void* comm, int nlocal, const long long* const* dest, const size_t* n, long long* const* order, long long* counts, void* stream) {
   return guard([&] {
-    if (nlocal < 1 || nlocal > device::kMaxRanks || p < 1 || p > device::kMaxRanks) throw_al_exception("route: 1 to ", device::kMaxRanks, " ranks");
+    DeviceCommunicator& c = *(DeviceCommunicator*)comm;
+    ScopedDevice on_device(c.device());
+    const int expect = c.is_emulated() ? c.size() : 1;
+    if (nlocal != expect) throw_al_exception("expected ", expect, " local rank(s), got ", nlocal);
     device::RouteParams P{};
     for (int r = 0; r < nlocal; ++r) {
       P.dest[r] = dest[r];
@@ -618,8 +622,8 @@ int al_route_rows(int nlocal, const long long* const* dest, const size_t* n, int
       P.order[r] = order[r];
     }
     P.counts = counts;
-    P.p = p;
-    device::launch_route(P, nlocal, (cudaStream_t)stream);
+    P.p = c.size();
+    device::launch_route(P, nlocal, pick_stream(&c, stream));
   });
 }
 

@@ -1,0 +1,43 @@
+"""Which inputs a token dispatch refuses, before anything is launched."""
+from types import SimpleNamespace
+
+import pytest
+import torch
+
+from aluminum_b200 import _lib
+from aluminum_b200.parallel import expert
+
+
+def test_host_memory_never_reaches_the_kernel(monkeypatch):
+    """The routing kernel reads and writes plain addresses: destinations that are not on the communicator's GPU, or not one
+    tensor per rank, raise before the library is called."""
+    called = []
+    monkeypatch.setattr(_lib, "load", lambda: called.append(1) or pytest.fail("the library was called"))
+    comm = SimpleNamespace(size=2, nlocal=2, device_index=0, _h=None, _stream=lambda: None)
+    dest = torch.tensor([0, 1, 1])
+    for dests in ([dest, dest], [dest], [dest] * 3):
+        with pytest.raises(_lib.AlError):
+            expert._route(comm, dests)
+        with pytest.raises(_lib.AlError):
+            expert.dispatch(comm, [torch.zeros(3, 4)] * len(dests), dests)
+    assert not called
+
+
+@pytest.mark.gpu
+def test_refused_inputs_leave_the_communicator_usable():
+    import aluminum_b200 as al
+    al.init()
+    comm = al.DeviceComm(emulate=2)
+    toks = [torch.arange(12., device="cuda").view(3, 4) + r for r in range(2)]
+    dest = torch.tensor([1, 0, 1], device="cuda")
+    for bad_toks, bad, error in ((toks, [dest, dest.cpu()], _lib.AlError), (toks, [dest.cpu(), dest.cpu()], _lib.AlError),
+                                 (toks, [dest], _lib.AlError), ([toks[0], toks[1].cpu()], [dest, dest], _lib.AlError),
+                                 (toks, [dest, dest.repeat(2)], ValueError), (toks, [dest, dest.bool()], ValueError),
+                                 (toks, [dest, dest.float()], ValueError), (toks, [dest, dest.view(3, 1)], ValueError)):
+        with pytest.raises(error):
+            expert.dispatch(comm, bad_toks, bad)
+    got, state = expert.dispatch(comm, toks, [dest, dest.to(torch.uint8)])
+    assert torch.equal(got[0], torch.stack([toks[0][1], toks[1][1]]))
+    back = expert.combine(comm, got, state)
+    assert all(torch.equal(b, t) for b, t in zip(back, toks))
+    comm.close()
