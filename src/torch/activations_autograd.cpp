@@ -23,6 +23,17 @@ int type_code(const Tensor& t) { return (int)(t.scalar_type() == at::kBFloat16 ?
 /** Partial sums of at most 148 x 3 CTAs of 256 channels (8 bytes each) and 16 bytes per channel. */
 Tensor workspace(const Tensor& x, int64_t channels) { return at::empty({148 * 3 * 256 * 8 + 16 * channels}, x.options().dtype(at::kByte)); }
 
+/**
+ * A saved tensor as the kernels read it.  Saved-tensor hooks give back the values but not always the layout (a copy to pinned
+ * host memory and back drops channels-last); what has lost its layout or alignment is laid out again, anything else that
+ * changed is an error before a kernel gets its address.
+ */
+Tensor restored(const Tensor& t, at::IntArrayRef sizes, at::ScalarType type, const Tensor& like, at::MemoryFormat format) {
+  TORCH_CHECK(t.device() == like.device() && t.scalar_type() == type && t.sizes() == sizes,
+              "a saved tensor came back with another device, type or shape");
+  return t.is_contiguous(format) && (uintptr_t)t.data_ptr() % 16 == 0 ? t : t.clone(format);
+}
+
 struct BatchNormAct : public torch::autograd::Function<BatchNormAct> {
   static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& weight, const Tensor& bias,
                         const std::optional<Tensor>& residual, const Tensor& running_mean, const Tensor& running_var,
@@ -55,11 +66,11 @@ struct BatchNormAct : public torch::autograd::Function<BatchNormAct> {
     variable_list out(kArgs);
     if (!grads[0].defined()) return out;
     const variable_list saved = ctx->get_saved_variables();
-    const Tensor &x = saved[0], &weight = saved[1], &stats = saved[2], &mask = saved[3];
+    Tensor x = saved[0], weight = saved[1], stats = saved[2], mask = saved[3];
     const bool relu = ctx->saved_data["relu"].toBool(), want_res = ctx->saved_data["residual"].toBool();
-    const c10::cuda::CUDAGuard guard(x.device());
-    const int64_t c = x.size(1), rows = x.numel() / c;
     Tensor dy = grads[0];
+    const c10::cuda::CUDAGuard guard(dy.device());
+    const int64_t c = x.size(1), rows = x.numel() / c;
     if (at::GradMode::is_enabled() || dy.scalar_type() != x.scalar_type()) {
       // a graph of the backward is wanted: operations that have a derivative themselves
       if (relu) {
@@ -74,6 +85,10 @@ struct BatchNormAct : public torch::autograd::Function<BatchNormAct> {
       return out;
     }
     if (!dy.is_contiguous(at::MemoryFormat::ChannelsLast) || (uintptr_t)dy.data_ptr() % 16) dy = dy.clone(at::MemoryFormat::ChannelsLast);
+    x = restored(x, dy.sizes(), dy.scalar_type(), dy, at::MemoryFormat::ChannelsLast);
+    weight = restored(weight, {c}, at::kFloat, dy, at::MemoryFormat::Contiguous);
+    stats = restored(stats, {2, c}, at::kFloat, dy, at::MemoryFormat::Contiguous);
+    mask = restored(mask, {relu ? rows * c / 8 : 0}, at::kByte, dy, at::MemoryFormat::Contiguous);
     Tensor dx = at::empty_like(x), dres, gw = at::empty_like(weight), gb = at::empty_like(weight);
     if (want_res) dres = at::empty_like(x);
     Tensor ws = workspace(x, c);
@@ -124,11 +139,11 @@ struct MaxPool : public torch::autograd::Function<MaxPool> {
     variable_list out(4);
     if (!grads[0].defined()) return out;
     const variable_list saved = ctx->get_saved_variables();
-    const Tensor &x = saved[0], &place = saved[1];
+    const Tensor& x = saved[0];   // (only its shape matters here)
+    Tensor place = saved[1], dy = grads[0];
     const int64_t k = ctx->saved_data["k"].toInt(), stride = ctx->saved_data["stride"].toInt(), pad = ctx->saved_data["pad"].toInt();
-    const c10::cuda::CUDAGuard guard(x.device());
+    const c10::cuda::CUDAGuard guard(dy.device());
     const auto s = shape(x, k, stride, pad);
-    Tensor dy = grads[0];
     if (at::GradMode::is_enabled() || dy.scalar_type() != x.scalar_type()) {
       // a graph of the backward is wanted: the framework's own backward, with the places as its indices
       const auto wide = place.options().dtype(at::kLong);
@@ -139,7 +154,8 @@ struct MaxPool : public torch::autograd::Function<MaxPool> {
       return out;
     }
     if (!dy.is_contiguous(at::MemoryFormat::ChannelsLast) || (uintptr_t)dy.data_ptr() % 16) dy = dy.clone(at::MemoryFormat::ChannelsLast);
-    Tensor dx = at::empty_like(x);
+    place = restored(place, {s[0], s[4], s[5], s[3]}, at::kByte, dy, at::MemoryFormat::Contiguous);
+    Tensor dx = at::empty(x.sizes(), dy.options(), at::MemoryFormat::ChannelsLast);
     TORCH_CHECK(al_maxpool_backward(type_code(x), dy.data_ptr(), place.data_ptr<uint8_t>(), dx.data_ptr(), s.data(),
                                     c10::cuda::getCurrentCUDAStream().stream()) == 0,
                 al_last_error());

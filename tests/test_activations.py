@@ -150,3 +150,32 @@ def test_max_pool_nan_and_module_calls():
     assert torch.equal(max_pool(pool, x.float().nan_to_num()), pool(x.float().nan_to_num()))
     with pytest.raises(RuntimeError):
         max_pool(nn.MaxPool2d(3, 1, 2), x)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("hooks", ["pinned", "permuted", "unaligned"])
+def test_saved_tensors_in_another_layout(hooks):
+    """Saved-tensor hooks give back the values, not always the layout: gradients are those without hooks, bit for bit."""
+    def unaligned(t):
+        flat = torch.empty(t.numel() + 1, device=t.device, dtype=t.dtype)[1:]
+        return torch.as_strided(flat, t.shape, t.stride()).copy_(t)
+    context = {"pinned": lambda: torch.autograd.graph.save_on_cpu(pin_memory=True),   # comes back contiguous, not channels-last
+               "permuted": lambda: torch.autograd.graph.saved_tensors_hooks(lambda t: t, lambda t: t.contiguous().clone()),
+               "unaligned": lambda: torch.autograd.graph.saved_tensors_hooks(lambda t: t, unaligned)}[hooks]
+    torch.manual_seed(3)
+    cl = dict(memory_format=torch.channels_last)
+    bn, pool = nn.BatchNorm2d(24).cuda(), nn.MaxPool2d(3, 2, 1)
+    x0, r0 = (torch.randn(3, 24, 9, 7, device="cuda").bfloat16().contiguous(**cl) for _ in range(2))
+    got = []
+    for hooked in (False, True):
+        b = copy.deepcopy(bn)
+        x, r = x0.clone().requires_grad_(), r0.clone().requires_grad_()
+        if hooked:
+            with context():
+                y = max_pool(pool, batch_norm_act(b, x, nn.ReLU(), r))
+        else:
+            y = max_pool(pool, batch_norm_act(b, x, nn.ReLU(), r))
+        assert "MaxPool" in y.grad_fn.name() and "MaxPool2D" not in y.grad_fn.name()
+        y.backward(torch.linspace(-1, 1, y.numel(), device="cuda").view(y.shape).bfloat16().contiguous(**cl))
+        got.append([x.grad, r.grad, b.weight.grad, b.bias.grad])
+    assert all(torch.equal(u, v) for u, v in zip(*got))
