@@ -41,11 +41,11 @@ def _modes_off() -> bool:
 
 
 def _fusable(bn: nn.Module, x) -> bool:
-    return (type(bn) is nn.BatchNorm2d and bn.training and bn.track_running_stats and bn.momentum is not None and _activation_ok(x)
+    # (_modes_off() first: a compiler that traces this function sees a constant there and nothing of what follows)
+    return (_modes_off() and type(bn) is nn.BatchNorm2d and bn.training and bn.track_running_stats and bn.momentum is not None and _activation_ok(x)
             and x.shape[1] == bn.num_features and x.get_device() == torch.cuda.current_device() and _bare(bn)
             and _parameter_ok(bn.weight, x) and _parameter_ok(bn.bias, x) and _parameter_ok(bn.running_mean, x)
-            and _parameter_ok(bn.running_var, x) and (bn.num_batches_tracked is None or bn.num_batches_tracked.get_device() == x.get_device())
-            and _modes_off())
+            and _parameter_ok(bn.running_var, x) and (bn.num_batches_tracked is None or bn.num_batches_tracked.get_device() == x.get_device()))
 
 
 def batch_norm_act(bn: nn.Module, x: torch.Tensor, relu: nn.Module | None = None, residual: torch.Tensor | None = None) -> torch.Tensor:
@@ -70,7 +70,7 @@ def _one(v) -> int:
 
 def max_pool(pool: nn.Module, x: torch.Tensor) -> torch.Tensor:
     """``pool(x)``."""
-    if type(pool) is nn.MaxPool2d and _activation_ok(x) and x.get_device() == torch.cuda.current_device() and _bare(pool) and _modes_off():
+    if _modes_off() and type(pool) is nn.MaxPool2d and _activation_ok(x) and x.get_device() == torch.cuda.current_device() and _bare(pool):
         k, stride, pad = _one(pool.kernel_size), _one(pool.stride), pool.padding if pool.padding == 0 else _one(pool.padding)
         if (0 < k <= 15 and stride > 0 and _one(pool.dilation) == 1 and not pool.ceil_mode and not pool.return_indices
                 and (pad > 0 or pool.padding == 0) and 2 * pad <= k and min(x.shape[2:]) + 2 * pad >= k

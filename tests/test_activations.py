@@ -179,3 +179,14 @@ def test_saved_tensors_in_another_layout(hooks):
         y.backward(torch.linspace(-1, 1, y.numel(), device="cuda").view(y.shape).bfloat16().contiguous(**cl))
         got.append([x.grad, r.grad, b.weight.grad, b.bias.grad])
     assert all(torch.equal(u, v) for u, v in zip(*got))
+
+
+@pytest.mark.parametrize("training", [True, False])
+def test_compiled_model_stays_one_graph(training):
+    from aluminum_b200.models.resnet import ResNet
+    torch.manual_seed(0)
+    model, x = ResNet((1, 1, 1, 1), num_classes=10).train(training), torch.randn(2, 3, 32, 32)
+    want = copy.deepcopy(model)(x)
+    torch._dynamo.reset()
+    got = torch.compile(copy.deepcopy(model), fullgraph=True, backend="eager")(x)   # raises at a graph break
+    assert torch.allclose(got, want, atol=1e-5)
