@@ -14,6 +14,7 @@ from torch.autograd import forward_ad
 
 from .. import _lib
 
+_PLAIN = (torch.Tensor, nn.Parameter)
 _TYPES = (torch.bfloat16, torch.float16)
 
 
@@ -29,7 +30,13 @@ def _activation_ok(x) -> bool:
 
 
 def _parameter_ok(t, x) -> bool:
-    return t is not None and not t.is_inference() and t.dtype == torch.float32 and t.is_contiguous() and t.get_device() == x.get_device() and t.data_ptr() % 16 == 0
+    """A plain tensor with one fp32 value per channel (of another length the module raises; a subclass may have no memory of its own)."""
+    return (type(t) in _PLAIN and not t.is_inference() and t.dtype == torch.float32 and t.numel() == x.shape[1] and t.is_contiguous()
+            and t.get_device() == x.get_device() and t.data_ptr() % 16 == 0)
+
+
+def _count_ok(t, x) -> bool:
+    return t is None or (type(t) in _PLAIN and t.dtype == torch.int64 and t.numel() == 1 and t.get_device() == x.get_device() and not t.is_inference())
 
 
 def _modes_off() -> bool:
@@ -45,7 +52,7 @@ def _fusable(bn: nn.Module, x) -> bool:
     return (_modes_off() and type(bn) is nn.BatchNorm2d and bn.training and bn.track_running_stats and bn.momentum is not None and _activation_ok(x)
             and x.shape[1] == bn.num_features and x.get_device() == torch.cuda.current_device() and _bare(bn)
             and _parameter_ok(bn.weight, x) and _parameter_ok(bn.bias, x) and _parameter_ok(bn.running_mean, x)
-            and _parameter_ok(bn.running_var, x) and (bn.num_batches_tracked is None or bn.num_batches_tracked.get_device() == x.get_device()))
+            and _parameter_ok(bn.running_var, x) and _count_ok(bn.num_batches_tracked, x))
 
 
 def batch_norm_act(bn: nn.Module, x: torch.Tensor, relu: nn.Module | None = None, residual: torch.Tensor | None = None) -> torch.Tensor:

@@ -190,3 +190,14 @@ def test_compiled_model_stays_one_graph(training):
     torch._dynamo.reset()
     got = torch.compile(copy.deepcopy(model), fullgraph=True, backend="eager")(x)   # raises at a graph break
     assert torch.allclose(got, want, atol=1e-5)
+
+
+def test_parameters_of_another_length_or_kind_go_to_the_module():
+    from aluminum_b200.ops import activations
+
+    class Wrapped(torch.Tensor):
+        pass
+    x = torch.zeros(1, 8, 2, 2)
+    assert activations._parameter_ok(torch.zeros(8), x) and activations._parameter_ok(nn.Parameter(torch.zeros(8)), x)
+    for other in (torch.zeros(7), torch.zeros(16), torch.zeros(8).double(), torch.zeros(8).as_subclass(Wrapped), None):
+        assert not activations._parameter_ok(other, x)
