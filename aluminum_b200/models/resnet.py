@@ -52,6 +52,8 @@ class Shortcut(nn.Sequential):
                 x = m(x)
             return x
         else:
+            if len(self) != 2:   # something was added or taken out
+                return super().forward(x)
             return batch_norm_act(self[1], self[0](x))
 
 

@@ -19,8 +19,8 @@ _TYPES = (torch.bfloat16, torch.float16)
 
 
 def _bare(m: nn.Module) -> bool:
-    """No hook would be missed by not calling the module."""
-    return not (m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks)
+    """Neither a hook nor a forward of the instance's own would be missed by not calling the module."""
+    return not ("forward" in m.__dict__ or m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks)
 
 
 def _activation_ok(x) -> bool:

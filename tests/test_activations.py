@@ -201,3 +201,16 @@ def test_parameters_of_another_length_or_kind_go_to_the_module():
     assert activations._parameter_ok(torch.zeros(8), x) and activations._parameter_ok(nn.Parameter(torch.zeros(8)), x)
     for other in (torch.zeros(7), torch.zeros(16), torch.zeros(8).double(), torch.zeros(8).as_subclass(Wrapped), None):
         assert not activations._parameter_ok(other, x)
+
+
+def test_forward_of_the_instances_own():
+    from aluminum_b200.models.resnet import Shortcut
+    from aluminum_b200.ops import activations
+    for m in (nn.BatchNorm2d(8), nn.ReLU(), nn.MaxPool2d(2)):
+        assert activations._bare(m)
+        m.forward = m.forward
+        assert not activations._bare(m)
+    x = torch.randn(2, 4, 3, 3)
+    parts = [nn.Conv2d(4, 8, 1), nn.BatchNorm2d(8), nn.ReLU()]
+    for n in (1, 2, 3):
+        assert torch.equal(Shortcut(*copy.deepcopy(parts[:n]))(x), nn.Sequential(*copy.deepcopy(parts[:n]))(x))
