@@ -74,8 +74,9 @@ struct BatchNormAct : public torch::autograd::Function<BatchNormAct> {
     if (at::GradMode::is_enabled() || dy.scalar_type() != x.scalar_type()) {
       // a graph of the backward is wanted: operations that have a derivative themselves
       if (relu) {
-        const Tensor bits = mask.view({x.size(0), x.size(2), x.size(3), c / 8, 1}).bitwise_right_shift(at::arange(8, mask.options())).bitwise_and(1);
-        dy = dy * bits.view({x.size(0), x.size(2), x.size(3), c}).permute({0, 3, 1, 2}).to(dy.scalar_type());
+        const Tensor bits = mask.reshape({x.size(0), x.size(2), x.size(3), c / 8, 1}).bitwise_right_shift(at::arange(8, mask.options())).bitwise_and(1);
+        const Tensor passes = bits.reshape({x.size(0), x.size(2), x.size(3), c}).permute({0, 3, 1, 2}).to(at::kBool);
+        dy = at::where(passes, dy, at::zeros({}, dy.options()));   // (not a product: an infinite gradient that the ReLU stops is 0)
       }
       auto g = at::native_batch_norm_backward(dy, x, weight, {}, {}, stats[0], stats[1], true, ctx->saved_data["eps"].toDouble(), {true, true, true});
       out[0] = std::get<0>(g);

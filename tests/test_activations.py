@@ -214,3 +214,16 @@ def test_forward_of_the_instances_own():
     parts = [nn.Conv2d(4, 8, 1), nn.BatchNorm2d(8), nn.ReLU()]
     for n in (1, 2, 3):
         assert torch.equal(Shortcut(*copy.deepcopy(parts[:n]))(x), nn.Sequential(*copy.deepcopy(parts[:n]))(x))
+
+
+@pytest.mark.gpu
+def test_stopped_infinite_gradient_in_a_graph_of_the_backward():
+    cl = dict(memory_format=torch.channels_last)
+    torch.manual_seed(5)
+    bn = nn.BatchNorm2d(16).cuda()
+    x = torch.randn(2, 16, 6, 6, device="cuda").bfloat16().contiguous(**cl).requires_grad_()
+    y = batch_norm_act(bn, x, nn.ReLU())
+    dy = torch.where(y > 0, torch.randn_like(y), float("inf")).detach()
+    g, = torch.autograd.grad(y, x, dy, retain_graph=True)
+    h, = torch.autograd.grad(y, x, dy, create_graph=True)
+    assert torch.isfinite(g).all() and rel(h.detach(), g.double()) < 1e-2
