@@ -153,46 +153,64 @@ int slots_cfg() { return std::max(2, std::min(16, tuning().dev_mailbox_slots)); 
 /** Packet slot of the point-to-point path: twice the largest payload (every 8 bytes carry 4 of payload). */
 size_t p2p_ll_slot_cfg() { return 2 * round_up(std::min(tuning().p2p_ll_max_bytes, kP2PLLMaxPayloadBytes), (size_t)4096); }
 
-/**
- * May rank r's contribution to its own result skip its staging slot?  Staging makes any overlap of the two buffers safe
- * (everything is read before anything is written), so the direct route is taken only where the bytes that are
- * written cannot be bytes that another thread still has to read: where the own slice lies on the place it would be
- * copied or reduced to (in place), or where the ranges do not meet.  A reduction reads the own slice together with
- * staged ones in 16-byte vectors and wants it aligned.
- */
-bool own_may_skip_staging(DevColl kind, const RankArgs& a, const CountTable& T, size_t count, int p, int r, int root,
-                          bool two_phase, size_t esz, size_t esz_out) {
-  if (!a.send || !a.recv) return false;
-  const char* send = (const char*)a.send;
-  const char* recv = (const char*)a.recv;
-  auto apart = [](const char* x, size_t nx, const char* y, size_t ny) { return x + nx <= y || y + ny <= x; };
+/** The memory of the caller that a rank reads or writes in an operation. */
+struct Span {
+  const char* at = nullptr;
+  size_t n = 0;
+  bool meets(const Span& o) const { return at < o.at + o.n && o.at < at + n; }
+};
+
+/** What local rank r reads (`sent`) or has written to it. */
+Span span_of(DevColl kind, const RankArgs& a, const CountTable& T, size_t count, int p, int r, int root, bool sent, size_t esz) {
   auto extent = [&](const size_t* counts, const size_t* displs) {
     size_t m = 0;
     for (int i = 0; i < p; ++i)
       if (counts[i]) m = std::max(m, displs[i] + counts[i]);
-    return m * esz;
+    return m;
   };
+  const char* at = (const char*)(sent ? a.send : a.recv);
+  size_t n = count;
+  if (kind == DevColl::reduce && !sent && r != root) n = 0;
+  if (kind == DevColl::reduce_scatter) n = sent ? extent(T.recv_counts, T.send_displs) : T.recv_counts[r];
+  if (kind == DevColl::allgather && sent) n = T.send_counts[r];
+  else if (kind == DevColl::allgather || kind == DevColl::alltoall) n = sent ? extent(T.send_counts, T.send_displs) : extent(T.recv_counts, T.recv_displs);
+  return Span{at, at ? n * esz : 0};
+}
+
+/**
+ * May local rank r's contribution to its own result skip its staging slot?  Staging makes any overlap of buffers safe
+ * (everything is read before anything is written), so the direct route is taken only where the bytes that are
+ * written cannot be bytes that another thread still has to read: where the own slice lies on the place it would be
+ * copied or reduced to (in place), or where the ranges do not meet.  That holds for the buffers of the other ranks in this
+ * process too (one rank's receive buffer may be another's send buffer): a reduction reads the own slice when the others may
+ * have written their results, data movement writes the own place while the others still read.  A reduction reads the own
+ * slice together with staged ones in 16-byte vectors and wants it aligned.
+ */
+bool own_may_skip_staging(DevColl kind, const CountTable* tab, const Span* sent, const Span* received, int rank0, int nlocal, int r,
+                          int root, bool two_phase, size_t esz, size_t esz_out) {
+  const CountTable& T = tab[r];
+  const Span in = sent[r], out = received[r];
+  if (!in.at || !out.at) return false;
+  Span own = in, place = out;   // the own contribution, and where it goes
   switch (kind) {
-    case DevColl::allreduce:
     case DevColl::reduce:
-      if (kind == DevColl::reduce && r != root) return false;
-      if ((uintptr_t)send % 16 != 0 || (two_phase && (uintptr_t)recv % 16 != 0)) return false;
-      return (send == recv && esz == esz_out) || apart(send, count * esz, recv, count * esz_out);
-    case DevColl::reduce_scatter: {
-      const char* own = send + T.send_displs[r] * esz;
-      const size_t n = T.recv_counts[r] * esz;
-      return (uintptr_t)own % 16 == 0 && ((own == recv && esz == esz_out) || apart(own, n, recv, T.recv_counts[r] * esz_out));
-    }
+      if (r != root) return false;
+      break;
+    case DevColl::allreduce: break;
+    case DevColl::reduce_scatter: own = Span{in.at + T.send_displs[r] * esz, T.recv_counts[r] * esz}; break;
     case DevColl::allgather:
-    case DevColl::alltoall: {
-      const bool ag = kind == DevColl::allgather;
+    case DevColl::alltoall:
       if (T.send_counts[r] != T.recv_counts[r] || esz != esz_out) return false;
-      const char* own = send + (ag ? 0 : T.send_displs[r] * esz);
-      const size_t all = ag ? T.send_counts[r] * esz : extent(T.send_counts, T.send_displs);
-      return own == recv + T.recv_displs[r] * esz || apart(send, all, recv, extent(T.recv_counts, T.recv_displs));
-    }
+      if (kind == DevColl::alltoall) own = Span{in.at + T.send_displs[r] * esz, T.send_counts[r] * esz};
+      place = Span{out.at + T.recv_displs[r] * esz, T.recv_counts[r] * esz};
+      break;
     default: return false;
   }
+  const bool moves = kind == DevColl::allgather || kind == DevColl::alltoall;
+  if (!moves && ((uintptr_t)own.at % 16 != 0 || (two_phase && (uintptr_t)out.at % 16 != 0))) return false;
+  for (int s = rank0; s < rank0 + nlocal; ++s)
+    if (s != r && (own.meets(received[s]) || (moves && place.meets(sent[s])))) return false;
+  return (own.at == place.at && esz == esz_out) || !(moves ? in : own).meets(out);
 }
 
 /**
@@ -593,6 +611,7 @@ void DeviceCommunicator::collective(const CollDesc& d, const std::vector<RankArg
     throw_al_exception("the nvls path serves reduce_scatter (for allreduce use AllreduceAlgo::nvls)");
   }
 
+  Span sent[kMaxRanks], received[kMaxRanks];
   for (int lr = 0; lr < I.nlocal; ++lr) {
     const int r = I.rank0 + lr;
     const RankArgs& a = ranks[(size_t)lr];
@@ -615,11 +634,14 @@ void DeviceCommunicator::collective(const CollDesc& d, const std::vector<RankArg
         T.send_displs[i] = T.recv_displs[i] = (size_t)i * d.count * unit;
       }
     }
-    P.own_direct[r] = p > 1 && in == wire && (wire == out || !P.two_phase) && algo != AllreduceAlgo::nvls &&
-                              own_may_skip_staging(d.kind, a, T, P.count, p, r, d.root, P.two_phase != 0, dtype_size(in), dtype_size(out))
+    sent[r] = span_of(d.kind, a, T, P.count, p, r, d.root, true, dtype_size(in));
+    received[r] = span_of(d.kind, a, T, P.count, p, r, d.root, false, dtype_size(out));
+  }
+  for (int r = I.rank0; p > 1 && in == wire && (wire == out || !P.two_phase) && algo != AllreduceAlgo::nvls && r < I.rank0 + I.nlocal; ++r)
+    P.own_direct[r] = own_may_skip_staging(d.kind, P.tab, sent, received, I.rank0, I.nlocal, r, d.root, P.two_phase != 0, dtype_size(in),
+                                           dtype_size(out))
                           ? 1
                           : 0;
-  }
 
   // All ranks on this GPU: large operations are moved by the bulk copy engine, chunked by what staging holds.
   bool bulk_staged = I.nlocal > 1 && !use_window && !d.vector && d.ctas <= 0 && !tn.bulk_pipeline && in == out &&

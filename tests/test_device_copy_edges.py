@@ -193,3 +193,32 @@ def test_routing_order_and_counts(al, p, tokens):
             with pytest.raises(ValueError):
                 expert.dispatch(comm, toks, bad)
     comm.close()
+
+
+@pytest.mark.parametrize("n", [4099, 262144])   # (262144 fp32: where the bulk copy engine takes over; one chunk)
+def test_receive_buffers_that_are_other_ranks_send_buffers(comm, n):
+    """With all ranks in one process a rank's result may land on what another rank still has to send: everything is read first."""
+    p = comm.size
+    fresh = lambda m: [small_ints(m, torch.float32, r) for r in range(p)]
+    turn = lambda bufs: bufs[1:] + bufs[:1]      # rank r receives where rank r + 1 sends from
+    for algo in ("one_shot", "two_shot"):
+        xs = fresh(n)
+        want = sum(xs)
+        comm.allreduce(xs, turn(xs), algo=algo)
+        assert all(torch.equal(x, want) for x in xs)
+    full = fresh(p * n)
+    want = [f.clone() for f in full]
+    comm.alltoall(full, turn(full), algo="staged")
+    for r, got in enumerate(turn(full)):
+        assert torch.equal(got, torch.cat([f[r * n:(r + 1) * n] for f in want]))
+    full = fresh(p * n)
+    want = sum(full)
+    place = lambda r: slice((r + 1) % p * n, ((r + 1) % p + 1) * n)   # the slice that rank r + 1 contributes to its own result
+    comm.reduce_scatter(full, [f[place(r)] for r, f in enumerate(turn(full))], algo="staged")
+    for r, f in enumerate(turn(full)):
+        assert torch.equal(f[place(r)], want[r * n:(r + 1) * n])
+    full = fresh(p * n)
+    shards = [f[:n] for f in full]
+    want = torch.cat([s.clone() for s in shards])
+    comm.allgather(shards, turn(full), algo="staged")
+    assert all(torch.equal(f, want) for f in full)
