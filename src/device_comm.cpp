@@ -222,6 +222,9 @@ bool own_may_skip_staging(DevColl kind, const CountTable* tab, const Span* sent,
 constexpr size_t kBulkStagedMinMoveTwo = size_t{16} << 20;
 constexpr size_t kBulkStagedMinBytes = size_t{1} << 20;
 
+/** Threads of a CTA: whole warps (the loops of datamove.cuh deal in rounds of a warp), whatever the tuning was set to. */
+int cta_threads() { return std::max(32, std::min(512, tuning().threads_per_cta) / 32 * 32); }
+
 void require_device() {
   if (!cuda::device_usable()) throw_al_exception("the device backend needs a CUDA device, none is usable in this process");
 }
@@ -604,7 +607,7 @@ void DeviceCommunicator::collective(const CollDesc& d, const std::vector<RankArg
       I.stats.bytes += P.count * esz * (size_t)p;
       I.stats.kernels++;
       I.stats.rs_nvls++;
-      launch_nvls_reduce_scatter(N, wire, d.op, nctas, std::min(512, tn.threads_per_cta), stream);
+      launch_nvls_reduce_scatter(N, wire, d.op, nctas, cta_threads(), stream);
       return;
     }
   } else if (d.path == CollPath::nvls) {
@@ -701,7 +704,7 @@ void DeviceCommunicator::collective(const CollDesc& d, const std::vector<RankArg
   }
 
   // ---- grid ------------------------------------------------------------------------
-  int threads = std::min(512, tn.threads_per_cta);
+  int threads = cta_threads();
   int ctas = d.ctas > 0 ? d.ctas : (int)std::max<size_t>(1, ceil_div(max_work_bytes, (size_t)32768));
   int cap = tn.max_ctas;
   if (d.kind == DevColl::allreduce && algo == AllreduceAlgo::nvls) cap = zero_copy ? tn.max_ctas_zero_copy : tn.max_ctas_nvls;

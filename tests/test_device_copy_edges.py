@@ -222,3 +222,24 @@ def test_receive_buffers_that_are_other_ranks_send_buffers(comm, n):
     want = torch.cat([s.clone() for s in shards])
     comm.allgather(shards, turn(full), algo="staged")
     assert all(torch.equal(f, want) for f in full)
+
+
+@pytest.mark.parametrize("threads", [16, 100, 333, 511])
+def test_threads_that_are_no_whole_warps(al, comm, threads):
+    """The loops deal in rounds of a warp; a tuning that is no multiple of one is rounded, not half obeyed."""
+    p, old = comm.size, al.get_tuning("threads_per_cta")
+    al.set_tuning("threads_per_cta", threads)
+    try:
+        for n in (4099, 300001):
+            for dtype, algo in ((torch.float32, "one_shot"), (torch.float32, "two_shot"), (torch.int32, "one_shot")):
+                xs = [small_ints(n, dtype, r) for r in range(p)]
+                want = sum(xs)
+                outs = [torch.zeros_like(x) for x in xs]
+                comm.allreduce(xs, outs, algo=algo)
+                assert all(torch.equal(o, want) for o in outs)
+            xs = [small_ints(n, torch.uint8, r) for r in range(p)]
+            outs = [torch.zeros(p * n, device="cuda", dtype=torch.uint8) for _ in range(p)]
+            comm.allgather(xs, outs, algo="staged")
+            assert all(torch.equal(o, torch.cat(xs)) for o in outs)
+    finally:
+        al.set_tuning("threads_per_cta", old)
