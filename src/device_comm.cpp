@@ -647,7 +647,8 @@ void DeviceCommunicator::collective(const CollDesc& d, const std::vector<RankArg
                           : 0;
 
   // All ranks on this GPU: large operations are moved by the bulk copy engine, chunked by what staging holds.
-  bool bulk_staged = I.nlocal > 1 && !use_window && !d.vector && d.ctas <= 0 && !tn.bulk_pipeline && in == out &&
+  // (Its CTAs take a whole SM each, so a caller who asked for smaller CTAs gets the loops.)
+  bool bulk_staged = I.nlocal > 1 && !use_window && !d.vector && d.ctas <= 0 && cta_threads() == 512 && !tn.bulk_pipeline && in == out &&
                      bulk_staged_supported(d.kind, in, wire, d.op) &&
                      P.count * esz * (d.kind == DevColl::allreduce ? 1 : (size_t)p) >= (p == 2 && !reduces ? kBulkStagedMinMoveTwo : kBulkStagedMinBytes);
   for (int r = 0; bulk_staged && r < p; ++r)
@@ -663,8 +664,9 @@ void DeviceCommunicator::collective(const CollDesc& d, const std::vector<RankArg
   // (Real ranks also pipeline as soon as a slice does not fit one staging slot: the alternative would be
   // several chunks one after the other, each with its handshakes exposed.)
   const bool slice_exceeds_slot = !I.emulated && P.count > cap_e;
-  if (!bulk_staged && (((d.kind == DevColl::reduce_scatter || d.kind == DevColl::allgather || d.kind == DevColl::alltoall) && !d.vector &&
-       p > 1 && !use_window && (P.count * esz >= X.pipeline_min_bytes || slice_exceeds_slot)) || ar_pipelined)) {
+  const bool pipelines = ((d.kind == DevColl::reduce_scatter || d.kind == DevColl::allgather || d.kind == DevColl::alltoall) && !d.vector &&
+       p > 1 && !use_window && (P.count * esz >= X.pipeline_min_bytes || slice_exceeds_slot)) || ar_pipelined;
+  if (pipelines && !bulk_staged) {
     size_t chunk_b = std::max<size_t>(P.count * esz / 8, size_t{4} << 20);
     chunk_b = std::min(chunk_b / 256 * 256, cap_e * esz);
     if (chunk_b >= 256 && chunk_b < P.count * esz) {
@@ -798,7 +800,10 @@ void DeviceCommunicator::collective(const CollDesc& d, const std::vector<RankArg
       return;
     }
   }
-  if (bulk_staged) return launch_bulk_staged(P, in, wire, I.sm_count / I.nlocal, I.nlocal, stream);
+  if (bulk_staged) {   // one CTA per SM, within the budget of the loops that it stands in for
+    const int budget = std::max(1, pipelines ? tn.max_ctas_pipelined : tn.max_ctas);
+    return launch_bulk_staged(P, in, wire, std::min(budget, I.sm_count / I.nlocal), I.nlocal, stream);
+  }
   launch_collective(P, in, wire, out, ctas, threads, I.nlocal, stream);
 }
 

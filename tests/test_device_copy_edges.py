@@ -243,3 +243,32 @@ def test_threads_that_are_no_whole_warps(al, comm, threads):
             assert all(torch.equal(o, torch.cat(xs)) for o in outs)
     finally:
         al.set_tuning("threads_per_cta", old)
+
+
+@pytest.mark.parametrize("limits", [dict(max_ctas=1, max_ctas_pipelined=2), dict(max_ctas=5, max_ctas_pipelined=3), dict(threads_per_cta=256)])
+def test_bulk_copies_within_the_callers_limits(al, comm, limits):
+    """Grid sizes down to one CTA per rank (many rounds of tiles each), and smaller CTAs, for which the loops stand in."""
+    p, old = comm.size, {k: al.get_tuning(k) for k in limits}
+    for k, v in limits.items():
+        al.set_tuning(k, v)
+    try:
+        for n in (524288 + 9, 3000003):
+            xs = [small_ints(n, torch.float32, r) for r in range(p)]
+            want = sum(xs)
+            outs = [torch.empty_like(x) for x in xs]
+            comm.allreduce(xs, outs, algo="two_shot")
+            assert all(torch.equal(o, want) for o in outs)
+            comm.allreduce(xs, wire_dtype=torch.bfloat16)
+            assert all(torch.equal(x, want) for x in xs)
+        n = 2097152 + 5
+        full = [small_ints(p * n, torch.float32, r) for r in range(p)]
+        want = sum(full)
+        outs = [torch.empty(n, device="cuda") for _ in range(p)]
+        comm.reduce_scatter(full, outs, algo="staged")
+        assert all(torch.equal(outs[r], want[r * n:(r + 1) * n]) for r in range(p))
+        both = [torch.empty_like(f) for f in full]
+        comm.allgather(outs, both, algo="staged")
+        assert all(torch.equal(b, want) for b in both)
+    finally:
+        for k, v in old.items():
+            al.set_tuning(k, v)
