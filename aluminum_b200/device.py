@@ -88,7 +88,9 @@ class DeviceComm:
         check(self._lib.al_dev_comm_stats(self._h, out))
         names = ["ops", "bytes", "kernels", "timeouts", "one_shot", "two_shot", "nvls", "nvls_zero_copy", "bulk_pipeline",
                  "window", "ll", "rows", "rs_nvls"]
-        return dict(zip(names, [int(v) for v in out]))
+        stats = dict(zip(names, [int(v) for v in out]))
+        stats["bulk_staged"] = int(self._lib.al_dev_comm_bulk_staged_ops(self._h))
+        return stats
 
     def status(self) -> dict:
         out = (C.c_uint64 * 6)()

@@ -312,6 +312,7 @@ int al_dev_comm_stats(void* comm, uint64_t* out) {
     out[8] = s.bulk_pipeline; out[9] = s.window; out[10] = s.ll; out[11] = s.rows; out[12] = s.rs_nvls;
   });
 }
+uint64_t al_dev_comm_bulk_staged_ops(void* comm) { return ((DeviceCommunicator*)comm)->stats().bulk_staged; }
 int al_dev_comm_status(void* comm, uint64_t* out) {
   device::DeviceStatus s = ((DeviceCommunicator*)comm)->status();
   out[0] = s.code; out[1] = s.rank; out[2] = s.peer; out[3] = s.where; out[4] = s.epoch; out[5] = s.seen;

@@ -801,6 +801,7 @@ void DeviceCommunicator::collective(const CollDesc& d, const std::vector<RankArg
     }
   }
   if (bulk_staged) {   // one CTA per SM, within the budget of the loops that it stands in for
+    I.stats.bulk_staged++;
     const int budget = std::max(1, pipelines ? tn.max_ctas_pipelined : tn.max_ctas);
     return launch_bulk_staged(P, in, wire, std::min(budget, I.sm_count / I.nlocal), I.nlocal, stream);
   }

@@ -272,3 +272,84 @@ def test_bulk_copies_within_the_callers_limits(al, comm, limits):
     finally:
         for k, v in old.items():
             al.set_tuning(k, v)
+
+
+def test_which_operations_the_bulk_copies_take(al, comm):
+    p = comm.size
+
+    def taken(call):
+        before = comm.stats()["bulk_staged"]
+        call()
+        return comm.stats()["bulk_staged"] - before
+    n = 524288 + 12
+    xs = [small_ints(n, torch.float32, r) for r in range(p)]
+    want = sum(xs)
+    outs = [torch.empty_like(x) for x in xs]
+    for algo in ("one_shot", "two_shot"):
+        assert taken(lambda: comm.allreduce(xs, outs, algo=algo)) == 1
+        assert all(torch.equal(o, want) for o in outs)
+    assert taken(lambda: comm.allreduce(xs, outs, wire_dtype=torch.bfloat16, algo="one_shot")) == 1
+    assert all(torch.equal(o, want) for o in outs)
+    # not: below 1 MiB, operators other than sums, a grid size of the caller's own, smaller CTAs, unaligned buffers
+    assert taken(lambda: comm.allreduce([x[:262140] for x in xs], [o[:262140] for o in outs], algo="one_shot")) == 0
+    assert taken(lambda: comm.allreduce(xs, outs, "max", algo="one_shot")) == 0
+    assert taken(lambda: comm.allreduce(xs, outs, algo="one_shot", ctas=4)) == 0
+    shifted = [small_ints(n, torch.float32, r, 1) for r in range(p)]
+    assert taken(lambda: comm.allreduce(shifted, outs, algo="one_shot")) == 0
+    assert all(torch.equal(o, sum(shifted)) for o in outs)
+    old = al.get_tuning("threads_per_cta")
+    al.set_tuning("threads_per_cta", 256)
+    assert taken(lambda: comm.allreduce(xs, outs, algo="one_shot")) == 0
+    al.set_tuning("threads_per_cta", old)
+
+
+@pytest.mark.parametrize("n", [(8 << 20) // 4, (8 << 20) // 4 + 3])   # 16 MiB in all on two ranks: where their bulk copies begin
+def test_large_moves(al, comm, n):
+    p = comm.size
+    full = [small_ints(p * n, torch.int32, r) for r in range(p)]
+    outs = [torch.empty_like(f) for f in full]
+    before = comm.stats()["bulk_staged"]
+    comm.alltoall(full, outs, algo="staged")
+    assert all(torch.equal(outs[r], torch.cat([f[r * n:(r + 1) * n] for f in full])) for r in range(p))
+    shards = [f[:n] for f in full]
+    comm.allgather(shards, outs, algo="staged")
+    assert all(torch.equal(o, torch.cat(shards)) for o in outs)
+    assert comm.stats()["bulk_staged"] == before + 2
+    if p == 2:
+        small = [f[:2 * n - 16] for f in full]
+        comm.alltoall(small, [o[:2 * n - 16] for o in outs], algo="staged")
+        assert comm.stats()["bulk_staged"] == before + 2
+
+
+@pytest.mark.parametrize("shift", [64, 4096 + 4])
+def test_large_partly_overlapping_buffers(al, comm, shift):
+    """Beyond 1 MiB: only forms that send everything through staging may use bulk copies then (one chunk each here)."""
+    p, n = comm.size, 524288 + 4
+
+    def buffers(m):
+        base = [small_ints(m + shift, torch.float32, r) for r in range(p)]
+        return [b[:m] for b in base], [b[shift:] for b in base]
+    before = comm.stats()["bulk_staged"]
+    for algo in ("one_shot", "two_shot"):
+        xs, outs = buffers(n)
+        want = sum(xs)
+        comm.allreduce(xs, outs, algo=algo)
+        assert all(torch.equal(o, want) for o in outs)
+    full, outs = buffers(p * n)
+    want = [torch.cat([f[r * n:(r + 1) * n] for f in full]) for r in range(p)]
+    comm.alltoall(full, outs, algo="staged")
+    assert all(torch.equal(o, w) for o, w in zip(outs, want))
+    assert comm.stats()["bulk_staged"] == before
+    for algo in ("one_shot", "two_shot"):
+        xs, outs = buffers(n)
+        want = sum(xs)
+        comm.allreduce(xs, outs, wire_dtype=torch.bfloat16, algo=algo)
+        assert all(torch.equal(o, want) for o in outs)
+    m = n + 1   # slices that are no whole 16-byte words
+    full, _ = buffers(p * m)
+    want = sum(full)
+    outs = [f[shift + r * m // 4 * 4:][:m] for r, f in enumerate(full)]
+    comm.reduce_scatter(full, [o if o.numel() == m else f[:m] for o, f in zip(outs, full)], algo="staged")
+    for r, (o, f) in enumerate(zip(outs, full)):
+        assert torch.equal(o if o.numel() == m else f[:m], want[r * m:(r + 1) * m])
+    assert comm.stats()["bulk_staged"] == before + 3
