@@ -124,7 +124,7 @@ __global__ void __launch_bounds__(512) bulk_pipeline_kernel(const __grid_constan
 #pragma unroll
           for (int r = 0; r < kMaxRanks; ++r) slot[r] = mystage + (size_t)r * cap_b;
           T* out = (T*)recv + base + lo;
-          cta_reduce<T, T, Red>(out, slot, lo * sizeof(T), p, hi - lo, red, P.scale, P.int_div);
+          cta_reduce<T, T>(out, slot, lo * sizeof(T), p, hi - lo, red, P.scale, P.int_div);
         }
       } else {
         const plan::Share sh = plan::share_of(slice_b, slot_b, c, part, n_con, kBulkTile);

@@ -35,6 +35,8 @@ inline bool family_serves(int fam, DevColl kind) {
 template <typename Ti, typename Tw, typename To, typename Red, int FAM = kFamAll>
 __global__ void __launch_bounds__(512, 1) coll_kernel(const __grid_constant__ CollParams P, Red red) {
   constexpr bool kReduces = FAM != kFamMove, kMoves = FAM != kFamReduce;
+  constexpr int kCopyUnroll = FAM == kFamMove ? kUnroll : kUnroll / 2;   // next to the folding loops eight loads per copying thread spill
+  constexpr int kPair = FAM == kFamAll ? 1 : 2;   // conversions beside the fold leave registers for one vector of up to four ranks
   const Workspace& ws = P.ws;
   const int p = ws.p;
   const int rank = P.rank0 + (int)blockIdx.y;
@@ -141,7 +143,7 @@ __global__ void __launch_bounds__(512, 1) coll_kernel(const __grid_constant__ Co
         dst = (char*)(recv + T.recv_displs[rank] + base + lo);
         if (dst == (const char*)src) continue;
       }
-      group_publish<Ti, Tw>(dst, src, hi - lo, lane, lanes);
+      group_publish<Ti, Tw, kCopyUnroll>(dst, src, hi - lo, lane, lanes);
     }
   };
 
@@ -166,12 +168,12 @@ __global__ void __launch_bounds__(512, 1) coll_kernel(const __grid_constant__ Co
       To* out = recv + base + s_lo + lo;
       auto area = [&](int d) { return ws.stage[d] + half_off + area_b + (size_t)rank * cap2_b + lo * sizeof(Tw); };
       if constexpr (kSame) {
-        reduce_to<Tw, To>(two_phase ? (1u << p) - 1 : 1u << rank, [&](int d) { return !two_phase || (own && d == rank) ? out : (To*)area(d); },
+        reduce_to<Tw, To, kPair>(two_phase ? (1u << p) - 1 : 1u << rank, [&](int d) { return !two_phase || (own && d == rank) ? out : (To*)area(d); },
                           src, p, hi - lo, red, P.scale, P.int_div);
       } else if (two_phase) {
-        reduce_to<Tw, Tw>((1u << p) - 1, [&](int d) { return (Tw*)area(d); }, src, p, hi - lo, red, P.scale, P.int_div);
+        reduce_to<Tw, Tw, kPair>((1u << p) - 1, [&](int d) { return (Tw*)area(d); }, src, p, hi - lo, red, P.scale, P.int_div);
       } else {
-        reduce_to<Tw, To>(1u << rank, [&](int) { return out; }, src, p, hi - lo, red, P.scale, P.int_div);
+        reduce_to<Tw, To, kPair>(1u << rank, [&](int) { return out; }, src, p, hi - lo, red, P.scale, P.int_div);
       }
     }
   };
@@ -209,7 +211,7 @@ __global__ void __launch_bounds__(512, 1) coll_kernel(const __grid_constant__ Co
       split_range(len, part, nparts, VEC, lo, hi);
       if (hi <= lo) continue;
       if constexpr (std::is_same<Tw, To>::value)
-        group_copy((char*)(recv + to + lo), src + lo * sizeof(Tw), (hi - lo) * sizeof(Tw), true, lane, lanes);
+        group_copy<kCopyUnroll, Rest::spread>((char*)(recv + to + lo), src + lo * sizeof(Tw), (hi - lo) * sizeof(Tw), true, lane, lanes);
       else if (two_phase)
         cta_expand<Tw, To>(recv + to + lo, (const Tw*)src + lo, hi - lo);
     }

@@ -96,13 +96,16 @@ __device__ __forceinline__ size_t clamp_len(size_t count, size_t lo, size_t cap)
 // ---------------------------------------------------------------------------
 // What bounds the loops below is the number of bytes in flight: the staged kernel runs 512 threads per SM (its
 // register count allows one CTA), so with 4 x 16 bytes per thread 148 SMs keep 4.8 MB under way where HBM3e at
-// about 0.8 us of latency wants 6 MB.  Eight loads per thread and an end that is one more round of independent
-// (predicated) loads instead of up to three dependent ones cover that (halo exchange of 8 MiB planes on one GPU
-// 31.4 -> 27.6 us, ring pass of 4 x 25 MB 103.5 -> 90.5 us; conversions, one element at a time before, allreduce of
-// 8 x 3,000,009 fp32 with a bf16 wire 240 -> 116 us).  Loops that are not inlined, or two CTAs of 64 registers, spill
-// inside the loop and were slower (bucket of 4 x 26 MB: 166 and 195 us against 136 us).  Buffers whose addresses differ modulo 16 (rows
-// or slices of an odd number of elements) are read as aligned 16-byte words and shifted into place, so that they
-// move in 16-byte stores too instead of in units of the common alignment.
+// about 0.8 us of latency wants 6 MB.  Eight loads per thread cover that in kernels that only copy (halo exchange of
+// 8 MiB planes on one GPU 31.4 -> 27.6 us, ring pass of 4 x 25 MB 103.5 -> 90.5 us).  In an instantiation with folding loops the
+// copies keep four: with eight, and an end of a round under predicates, they spilled 0.5 to 1.4 KB per thread, and what no
+// other kernel takes over got slower.  Four loads before that / eight / now, us, all ranks on one GPU: allreduce max of 4 x 8 MiB
+// fp32 87 / 105 / 66, sum of 4 x 64 MiB 589 / 705 / 439, of 8 x 8 MiB int32 426 / 371 / 228, of 8 x 8 MiB int8 1737 / 463 / 242,
+// reduce max of 8 x 8 MiB 163 / 224 / 95, bcast of 4 x 64 MiB 224 / 260 / 216.  (Conversions were done one element at a time before:
+// allreduce of 8 x 8 MiB fp32 with an fp16 wire 267 / 173 / 148 us.)  Loops that are not inlined, or two CTAs of 64 registers, spill
+// inside the loop and were slower.  Buffers whose addresses differ modulo 16 (rows or slices of an odd number of
+// elements) are read as aligned 16-byte words and shifted into place, so that they move in 16-byte stores too instead
+// of in units of the common alignment.
 constexpr int kUnroll = 8;
 
 /** 16-byte source words at any byte address: word i is bytes [16 i, 16 i + 16) of `src`.  An unaligned word is put
@@ -132,34 +135,73 @@ struct WordSource {
   }
 };
 
-/** For every i in [0, units): store(i, load(i)), U independent loads per thread before the first store.  A warp takes U
- *  rows of 32 consecutive units, so that its accesses differ by constants and share one address register. */
-template <int U, typename Load, typename Store>
+/** What batched_units() does with the units that are less than a round. */
+enum class Rest {
+  spread,    ///< over all warps: half of U loads at once, half of that, then singly (fewest registers)
+  together,  ///< a warp's rows like before, all at once under predicates (least latency; kernels with many such loops spill over it)
+  row        ///< together, for a group that is one warp
+};
+
+/** For every i in [0, units): store(i, load(i)), U independent loads per thread before the first store.  In a full round a
+ *  warp takes U rows of 32 consecutive units, so that its accesses differ by constants and share one address register. */
+template <int U, Rest REST = Rest::spread, typename Load, typename Store>
 __device__ __forceinline__ void batched_units(size_t units, unsigned lane, unsigned nlanes, Load load, Store store) {
   const unsigned warps = nlanes >> 5;   // (of a group that is no multiple of 32 threads the last few stay idle)
   if ((lane >> 5) >= warps) return;
-  const size_t step = (size_t)warps * (32 * U);
+  const size_t step = (size_t)warps * 32;
   uint4 v[U];
-  for (size_t i = (size_t)(lane >> 5) * (32 * U) + (lane & 31); i < units; i += step) {
-    if (i + 32 * (U - 1) < units) {
+  auto batch = [&](size_t i, size_t apart, auto n) __attribute__((always_inline)) {
 #pragma unroll
-      for (int k = 0; k < U; ++k) v[k] = load(i + 32 * k);
+    for (int k = 0; k < decltype(n)::value; ++k) v[k] = load(i + k * apart);
 #pragma unroll
-      for (int k = 0; k < U; ++k) store(i + 32 * k, v[k]);
-    } else {
-      const unsigned left = (unsigned)((units - i + 31) >> 5);
+    for (int k = 0; k < decltype(n)::value; ++k) store(i + k * apart, v[k]);
+  };
+  const size_t first = (size_t)(lane >> 5) * (32 * U) + (lane & 31);
+  if constexpr (REST == Rest::together) {
+    for (size_t i = first; i < units; i += U * step) {
+      if (i + 32 * (U - 1) < units) {
+        batch(i, 32, std::integral_constant<int, U>());
+      } else {
+        const unsigned left = (unsigned)((units - i + 31) >> 5);
 #pragma unroll
-      for (int k = 0; k < U; ++k)
-        if (k < left) v[k] = load(i + 32 * k);
+        for (int k = 0; k < U; ++k)
+          if (k < left) v[k] = load(i + 32 * k);
 #pragma unroll
-      for (int k = 0; k < U; ++k)
-        if (k < left) store(i + 32 * k, v[k]);
+        for (int k = 0; k < U; ++k)
+          if (k < left) store(i + 32 * k, v[k]);
+      }
     }
+  } else {
+    size_t done = 0;
+    for (; done + U * step <= units; done += U * step) batch(done + first, 32, std::integral_constant<int, U>());
+    size_t i = done + lane;
+    if constexpr (REST == Rest::row) {
+#pragma unroll
+      for (int k = 0; k < U; ++k)
+        if (i + k * step < units) v[k] = load(i + k * step);
+#pragma unroll
+      for (int k = 0; k < U; ++k)
+        if (i + k * step < units) store(i + k * step, v[k]);
+      return;
+    }
+    auto some = [&](auto n) __attribute__((always_inline)) {
+      constexpr int N = decltype(n)::value;
+      if constexpr (N >= 2) {
+        if (i + (N - 1) * step < units) {
+          batch(i, step, n);
+          i += N * step;
+        }
+      }
+    };
+    some(std::integral_constant<int, U / 2>());
+    some(std::integral_constant<int, U / 4>());
+#pragma unroll 1
+    for (; i < units; i += step) store(i, load(i));
   }
 }
 
 /** Copy `nbytes` with `nlanes` cooperating threads (this thread is `lane`), whatever the two alignments. */
-template <int U = kUnroll>
+template <int U = kUnroll, Rest REST = U == kUnroll ? Rest::together : Rest::spread>
 __device__ __forceinline__ void group_copy(char* dst, const char* src, size_t nbytes, bool src_is_staging,
                                            unsigned lane, unsigned nlanes) {
   if (nbytes == 0) return;
@@ -171,15 +213,16 @@ __device__ __forceinline__ void group_copy(char* dst, const char* src, size_t nb
   const WordSource s(src + head, src_is_staging);
   auto store = [&](size_t i, const uint4& v) { d[i] = v; };
   if (s.sh == 0) {
-    if (src_is_staging) batched_units<U>(nv, lane, nlanes, [&](size_t i) { return __ldcg(s.base + i); }, store);
-    else batched_units<U>(nv, lane, nlanes, [&](size_t i) { return s.base[i]; }, store);
+    if (src_is_staging) batched_units<U, REST>(nv, lane, nlanes, [&](size_t i) { return __ldcg(s.base + i); }, store);
+    else batched_units<U, REST>(nv, lane, nlanes, [&](size_t i) { return s.base[i]; }, store);
   } else {
-    batched_units<U / 4>(nv, lane, nlanes, [&](size_t i) { return s.shifted(i); }, store);
+    batched_units<U / 4, REST>(nv, lane, nlanes, [&](size_t i) { return s.shifted(i); }, store);
   }
   for (size_t k = done + lane; k < nbytes; k += nlanes) dst[k] = src_is_staging ? __ldcg(src + k) : src[k];
 }
 
-/** Copy with all threads of the CTA.  (Kernels that are held to 64 registers and spill with eight loads pass U = 4.) */
+/** Copy with all threads of the CTA.  (Kernels that are held to 64 registers and spill with eight loads pass U = 4; the three
+ *  NVLS kernels take 55 to 63 registers then and spill nothing.) */
 template <int U = kUnroll>
 __device__ __forceinline__ void cta_copy(char* dst, const char* src, size_t nbytes, bool src_is_staging) {
   group_copy<U>(dst, src, nbytes, src_is_staging, threadIdx.x, blockDim.x);
@@ -243,10 +286,10 @@ struct Converter {
 };
 
 /** Single destination (16-byte aligned), a subset of the CTA's threads: used to serve all peers of a small message at once. */
-template <typename Ti, typename Tw>
+template <typename Ti, typename Tw, int U = kUnroll>
 __device__ __forceinline__ void group_publish(char* dst, const Ti* src, size_t n, unsigned lane, unsigned nlanes) {
   if constexpr (std::is_same<Ti, Tw>::value) {
-    group_copy(dst, (const char*)src, n * sizeof(Ti), false, lane, nlanes);
+    group_copy<U, Rest::spread>(dst, (const char*)src, n * sizeof(Ti), false, lane, nlanes);
   } else {
     using C = Converter<Ti, Tw>;
     const size_t nv = C::aligned(src) ? n / C::VEC : 0;
@@ -305,9 +348,9 @@ __device__ __forceinline__ A finish_acc(A a, double scale, int int_div) {
  * the first Tw element of rank r's contribution, dst(d) the first To element of a destination; both are called with
  * compile-time ranks.  Contributions are folded in rank order so every rank computes
  * bit-identical results.  A destination may alias one of the sources.  Where an address is not 16-byte aligned
- * everything is read element by element.
+ * everything is read element by element.  PAIR: vectors that a thread reads at once of up to four ranks.
  */
-template <typename Tw, typename To, typename Red, typename Src, typename Dst>
+template <typename Tw, typename To, int PAIR = 2, typename Red, typename Src, typename Dst>
 __device__ __forceinline__ void reduce_to(unsigned ranks, Dst dst, Src src, int p, size_t n, Red red, double scale, int int_div) {
   using Aw = typename Elem<Tw>::Acc;
   using Ao = typename Elem<To>::Acc;
@@ -373,7 +416,7 @@ __device__ __forceinline__ void reduce_to(unsigned ranks, Dst dst, Src src, int 
       }
     }
   };
-  if (p <= kMaxRanks / 2) rounds(std::integral_constant<int, kMaxRanks / 2>(), std::integral_constant<int, 2>());
+  if (p <= kMaxRanks / 2) rounds(std::integral_constant<int, kMaxRanks / 2>(), std::integral_constant<int, PAIR>());
   else rounds(std::integral_constant<int, kMaxRanks>(), std::integral_constant<int, 1>());
   // scalar remainder (and the whole range when an address is not aligned for vector accesses)
   for (size_t i = nvec * VEC + threadIdx.x; i < n; i += stride) {
@@ -393,10 +436,10 @@ __device__ __forceinline__ void reduce_to(unsigned ranks, Dst dst, Src src, int 
 }
 
 /** One destination, contributions at bases[r] + byte_off. */
-template <typename Tw, typename To, typename Red>
+template <typename Tw, typename To, int PAIR = 2, typename Red>
 __device__ __forceinline__ void cta_reduce(To* out, char* const* bases, size_t byte_off, int p, size_t n, Red red, double scale,
                                            int int_div) {
-  reduce_to<Tw, To>(1u, [&](int) { return out; }, [&](int r) { return bases[r] + byte_off; }, p, n, red, scale, int_div);
+  reduce_to<Tw, To, PAIR>(1u, [&](int) { return out; }, [&](int r) { return bases[r] + byte_off; }, p, n, red, scale, int_div);
 }
 
 }  // namespace device
