@@ -353,3 +353,20 @@ def test_large_partly_overlapping_buffers(al, comm, shift):
     for r, (o, f) in enumerate(zip(outs, full)):
         assert torch.equal(o if o.numel() == m else f[:m], want[r * m:(r + 1) * m])
     assert comm.stats()["bulk_staged"] == before + 3
+
+
+@pytest.mark.parametrize("p,width,rows", [(2, 2064, 33), (4, 3072, 65), (3, 4080, 7), (8, 2050, 20), (2, 4095, 40), (2, 4112, 8200), (2, 4099, 8200)])
+def test_rows_in_rounds_of_four_and_eight(al, p, width, rows):
+    """Rows between 2 and 4 KiB (one round of eight loads), and longer ones in an exchange of more than 128 MiB (rounds of four)."""
+    comm = al.DeviceComm(emulate=p)
+    table = lambda v: [v] * p
+    x = [small_ints(p * rows * width, torch.uint8, r).view(p, rows, width) for r in range(p)]
+    order = [torch.randperm(rows, generator=torch.Generator().manual_seed(r)).cuda() for r in range(p)]
+    out = [torch.zeros(p, rows, width, device="cuda", dtype=torch.uint8) for _ in range(p)]
+    offsets = table([d * rows * width for d in range(p)])
+    comm.exchange_rows(x, out, width, width, width, table([rows] * p), table([0] * p), offsets, table([rows] * p), table([0] * p), offsets,
+                       send_idx=order)
+    for r in range(p):
+        for s in range(p):
+            assert torch.equal(out[r][s], x[s][r][order[s]])
+    comm.close()
