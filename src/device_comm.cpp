@@ -214,13 +214,17 @@ bool own_may_skip_staging(DevColl kind, const CountTable* tab, const Span* sent,
 }
 
 /**
- * Smallest vector (or whole message) that the bulk copy engine moves when all ranks are on one GPU.  Loops against bulk
- * copies in us, at 1 and 4 MiB: allreduce of 4 ranks 26.6 / 25.2 and 39.8 / 31.3, of 8 ranks 42 / 31 and 66 / 47;
- * reduce_scatter of 8 ranks 28.6 / 29.1 and 41 / 29; allgather of 4 ranks 17.5 / 18.1 and 23.4 / 21.7.  Below 1 MiB both
- * wait for the host.  With two ranks the loops move data faster up to 8 MiB (allgather 17.8 / 20.6; 16 MiB 25.7 / 23.4).
+ * Smallest vector (or whole message), in bytes of the caller's buffers, that the bulk copy engine moves when all ranks are
+ * on one GPU.  Loops / bulk copies in us: two ranks, allreduce of 2, 8, 16 MiB 13.7 / 15.3, 21.1 / 21.2, 39.3 / 31.1 and with a narrower
+ * wire 13.7 / 14.1, 21.3 / 21.0, 34.7 / 31.1; three, 2, 4, 8 MiB 21.0 / 23.7, 25.0 / 25.9, 34.6 / 33.8; four 24.4 / 25.6, 29.5 / 28.4,
+ * 43.7 / 40.5, but with a narrower wire 40.6 / 41.8 at 8 and 92.2 / 94.5 at 25 MiB, 225 / 217 at 64; eight, 1 and 4 MiB 31.6 / 28.2 and
+ * 59.1 / 44.4, narrower wire 33.7 / 32.8 at 2 MiB.  The moves and reduce_scatter lie between.
  */
-constexpr size_t kBulkStagedMinMoveTwo = size_t{16} << 20;
-constexpr size_t kBulkStagedMinBytes = size_t{1} << 20;
+size_t bulk_staged_min_bytes(int p, bool narrower_wire) {
+  if (p == 2) return size_t{16} << 20;
+  if (p <= 4) return size_t{narrower_wire ? 32 : 8} << 20;
+  return size_t{narrower_wire ? 2 : 1} << 20;
+}
 
 /** Threads of a CTA: whole warps (the loops of datamove.cuh deal in rounds of a warp), whatever the tuning was set to. */
 int cta_threads() { return std::max(32, std::min(512, tuning().threads_per_cta) / 32 * 32); }
@@ -650,7 +654,7 @@ void DeviceCommunicator::collective(const CollDesc& d, const std::vector<RankArg
   // (Its CTAs take a whole SM each, so a caller who asked for smaller CTAs gets the loops.)
   bool bulk_staged = I.nlocal > 1 && !use_window && !d.vector && d.ctas <= 0 && cta_threads() == 512 && !tn.bulk_pipeline && in == out &&
                      bulk_staged_supported(d.kind, in, wire, d.op) &&
-                     P.count * esz * (d.kind == DevColl::allreduce ? 1 : (size_t)p) >= (p == 2 && !reduces ? kBulkStagedMinMoveTwo : kBulkStagedMinBytes);
+                     P.count * dtype_size(in) * (d.kind == DevColl::allreduce ? 1 : (size_t)p) >= bulk_staged_min_bytes(p, in != wire);
   for (int r = 0; bulk_staged && r < p; ++r)
     bulk_staged = (P.own_direct[r] || in != wire || (d.kind == DevColl::reduce_scatter && P.count * esz % 16 != 0)) && P.send[r] && P.recv[r] && (uintptr_t)P.send[r] % 16 == 0 && (uintptr_t)P.recv[r] % 16 == 0;
 

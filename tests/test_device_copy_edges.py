@@ -245,6 +245,11 @@ def test_threads_that_are_no_whole_warps(al, comm, threads):
         al.set_tuning("threads_per_cta", old)
 
 
+def bulk_from(p, wire=False):
+    """Bytes of a vector from which the bulk copies take an operation of p ranks."""
+    return (16 if p == 2 else (32 if wire else 8) if p <= 4 else (2 if wire else 1)) << 20
+
+
 @pytest.mark.parametrize("limits", [dict(max_ctas=1, max_ctas_pipelined=2), dict(max_ctas=5, max_ctas_pipelined=3), dict(threads_per_cta=256)])
 def test_bulk_copies_within_the_callers_limits(al, comm, limits):
     """Grid sizes down to one CTA per rank (many rounds of tiles each), and smaller CTAs, for which the loops stand in."""
@@ -252,7 +257,7 @@ def test_bulk_copies_within_the_callers_limits(al, comm, limits):
     for k, v in limits.items():
         al.set_tuning(k, v)
     try:
-        for n in (524288 + 9, 3000003):
+        for n in (bulk_from(p) // 4 + 9, bulk_from(p, True) // 4 + 900003):
             xs = [small_ints(n, torch.float32, r) for r in range(p)]
             want = sum(xs)
             outs = [torch.empty_like(x) for x in xs]
@@ -281,17 +286,18 @@ def test_which_operations_the_bulk_copies_take(al, comm):
         before = comm.stats()["bulk_staged"]
         call()
         return comm.stats()["bulk_staged"] - before
-    n = 524288 + 12
+    n = bulk_from(p, True) // 4 + 12
     xs = [small_ints(n, torch.float32, r) for r in range(p)]
     want = sum(xs)
     outs = [torch.empty_like(x) for x in xs]
-    for algo in ("one_shot", "two_shot"):
-        assert taken(lambda: comm.allreduce(xs, outs, algo=algo)) == 1
-        assert all(torch.equal(o, want) for o in outs)
-    assert taken(lambda: comm.allreduce(xs, outs, wire_dtype=torch.bfloat16, algo="one_shot")) == 1
-    assert all(torch.equal(o, want) for o in outs)
-    # not: below 1 MiB, operators other than sums, a grid size of the caller's own, smaller CTAs, unaligned buffers
-    assert taken(lambda: comm.allreduce([x[:262140] for x in xs], [o[:262140] for o in outs], algo="one_shot")) == 0
+    for wire in (None, torch.bfloat16):
+        least = bulk_from(p, wire is not None) // 4
+        for algo in ("one_shot", "two_shot"):
+            for m in (least, least + 9, n):
+                assert taken(lambda: comm.allreduce([x[:m] for x in xs], [o[:m] for o in outs], wire_dtype=wire, algo=algo)) == 1
+                assert all(torch.equal(o[:m], want[:m]) for o in outs)
+            assert taken(lambda: comm.allreduce([x[:least - 4] for x in xs], [o[:least - 4] for o in outs], wire_dtype=wire, algo=algo)) == 0
+    # nor: operators other than sums, a grid size of the caller's own, smaller CTAs, unaligned buffers
     assert taken(lambda: comm.allreduce(xs, outs, "max", algo="one_shot")) == 0
     assert taken(lambda: comm.allreduce(xs, outs, algo="one_shot", ctas=4)) == 0
     shifted = [small_ints(n, torch.float32, r, 1) for r in range(p)]
@@ -301,6 +307,32 @@ def test_which_operations_the_bulk_copies_take(al, comm):
     al.set_tuning("threads_per_cta", 256)
     assert taken(lambda: comm.allreduce(xs, outs, algo="one_shot")) == 0
     al.set_tuning("threads_per_cta", old)
+
+
+@pytest.mark.parametrize("stage", [1 << 20, 64 << 20])
+@pytest.mark.parametrize("dtype,odd", [(torch.float32, 0), (torch.bfloat16, 7), (torch.float16, 8)])
+def test_bulk_copies_from_their_smallest_sizes_on(al, stage, dtype, odd):
+    """Reductions where the bulk copies begin, in one chunk and (small staging) in many."""
+    old = al.get_tuning("dev_stage_bytes")
+    al.set_tuning("dev_stage_bytes", stage)
+    for p in (2, 3, 4):
+        comm = al.DeviceComm(emulate=p)
+        n = bulk_from(p) // dtype.itemsize + odd
+        xs = [small_ints(n, dtype, r) for r in range(p)]
+        want = sum(x.float() for x in xs).to(dtype)
+        outs = [torch.empty_like(x) for x in xs]
+        for algo in ("one_shot", "two_shot"):
+            comm.allreduce(xs, outs, algo=algo)
+            assert all(torch.equal(o, want) for o in outs)
+        m = bulk_from(p) // dtype.itemsize // p // 8 * 8 + 8 + odd
+        full = [small_ints(p * m, dtype, 9 + r) for r in range(p)]
+        want = sum(f.float() for f in full).to(dtype)
+        outs = [torch.empty(m, device="cuda", dtype=dtype) for _ in range(p)]
+        comm.reduce_scatter(full, outs, algo="staged")
+        assert all(torch.equal(o, want[r * m:(r + 1) * m]) for r, o in enumerate(outs))
+        assert comm.stats()["bulk_staged"] == 3
+        comm.close()
+    al.set_tuning("dev_stage_bytes", old)
 
 
 @pytest.mark.parametrize("n", [(8 << 20) // 4, (8 << 20) // 4 + 3])   # 16 MiB in all on two ranks: where their bulk copies begin
@@ -323,8 +355,9 @@ def test_large_moves(al, comm, n):
 
 @pytest.mark.parametrize("shift", [64, 4096 + 4])
 def test_large_partly_overlapping_buffers(al, comm, shift):
-    """Beyond 1 MiB: only forms that send everything through staging may use bulk copies then (one chunk each here)."""
-    p, n = comm.size, 524288 + 4
+    """Where the bulk copies begin: only forms that send everything through staging may use bulk copies then (one chunk each here)."""
+    p = comm.size
+    n = bulk_from(p) // 4 + 4
 
     def buffers(m):
         base = [small_ints(m + shift, torch.float32, r) for r in range(p)]
@@ -335,17 +368,18 @@ def test_large_partly_overlapping_buffers(al, comm, shift):
         want = sum(xs)
         comm.allreduce(xs, outs, algo=algo)
         assert all(torch.equal(o, want) for o in outs)
-    full, outs = buffers(p * n)
-    want = [torch.cat([f[r * n:(r + 1) * n] for f in full]) for r in range(p)]
+    m = n // p // 4 * 4     # (one chunk)
+    full, outs = buffers(p * m)
+    want = [torch.cat([f[r * m:(r + 1) * m] for f in full]) for r in range(p)]
     comm.alltoall(full, outs, algo="staged")
     assert all(torch.equal(o, w) for o, w in zip(outs, want))
     assert comm.stats()["bulk_staged"] == before
     for algo in ("one_shot", "two_shot"):
-        xs, outs = buffers(n)
+        xs, outs = buffers(bulk_from(p, True) // 4)
         want = sum(xs)
         comm.allreduce(xs, outs, wire_dtype=torch.bfloat16, algo=algo)
         assert all(torch.equal(o, want) for o in outs)
-    m = n + 1   # slices that are no whole 16-byte words
+    m += 1   # slices that are no whole 16-byte words
     full, _ = buffers(p * m)
     want = sum(full)
     outs = [f[shift + r * m // 4 * 4:][:m] for r, f in enumerate(full)]
