@@ -41,3 +41,31 @@ def test_refused_inputs_leave_the_communicator_usable():
     back = expert.combine(comm, got, state)
     assert all(torch.equal(b, t) for b, t in zip(back, toks))
     comm.close()
+
+
+@pytest.mark.parametrize("p", [1, 2, 8])
+@pytest.mark.parametrize("n", [0, 1, 33, 5000])
+def test_order_and_counts_by_sorting(p, n):
+    d = torch.randint(0, p, (n,), generator=torch.Generator().manual_seed(n))
+    counts = torch.empty(p, dtype=torch.int64)
+    assert torch.equal(expert._sorted_route(d, p, counts), torch.argsort(d, stable=True))
+    assert torch.equal(counts, torch.bincount(d, minlength=p))
+    for wrong in (-1, p) if n else ():
+        bad = d.clone()
+        bad[n // 2] = wrong
+        expert._sorted_route(bad, p, counts)
+        assert (counts == -1).all()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [410_000, 410_001])
+def test_either_side_of_the_sorting_limit(n):
+    import aluminum_b200 as al
+    al.init()
+    comm = al.DeviceComm(emulate=2)
+    dests = [torch.randint(0, 2, (n,), device="cuda"), torch.randint(0, 2, (5,), device="cuda")]
+    order, both = expert._route(comm, dests)
+    for r in range(2):
+        assert torch.equal(order[r], torch.argsort(dests[r], stable=True))
+        assert torch.equal(both[0][r], torch.bincount(dests[r], minlength=2))
+    comm.close()
