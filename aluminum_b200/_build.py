@@ -9,6 +9,8 @@ Python package can build itself without CMake.
 """
 from __future__ import annotations
 
+import contextlib
+import fcntl
 import hashlib
 import os
 import shutil
@@ -69,10 +71,38 @@ def _headers_digest() -> str:
     return h.hexdigest()
 
 
-def _torch_dir() -> Path:
-    """PyTorch's folder, without importing it."""
+def _torch_dir() -> Path | None:
+    """PyTorch's folder, without importing it; None where PyTorch, its headers or its CUDA libraries are not installed (the
+    communication library and the tools do not need them)."""
     import importlib.util
-    return Path(next(iter(importlib.util.find_spec("torch").submodule_search_locations)))
+    spec = importlib.util.find_spec("torch")
+    for d in (spec.submodule_search_locations or ()) if spec else ():
+        if (Path(d) / "include" / "torch" / "library.h").exists() and (Path(d) / "lib" / "libtorch_cuda.so").exists():
+            return Path(d)
+    return None
+
+
+def _torch_stamp() -> str:
+    """Changes with the installed PyTorch, whose headers and binary interface the autograd operators are built for."""
+    d = _torch_dir()
+    version = d / "version.py" if d else None
+    return f"{d}:{hashlib.sha1(version.read_bytes()).hexdigest() if version and version.exists() else ''}"
+
+
+@contextlib.contextmanager
+def _locked():
+    """One build at a time: the ranks of a job may all find that the library is missing."""
+    OBJ.mkdir(parents=True, exist_ok=True)
+    with open(OBJ / ".lock", "w") as f:
+        fcntl.flock(f, fcntl.LOCK_EX)
+        yield
+
+
+def _link(out: Path, cmd: list[str]) -> None:
+    """Run cmd + the output's name; the file appears under `out` only when it is complete."""
+    part = out.with_name(f".{out.name}.{os.getpid()}.so")
+    _run(cmd + ["-o", str(part)])
+    os.replace(part, out)
 
 
 def _needs(obj: Path, src: Path, stamp: str) -> bool:
@@ -118,26 +148,32 @@ def build(tools: bool = True, jobs: int | None = None, verbose: bool = False) ->
     """Build the shared library (and the tools); returns the library path."""
     if shutil.which(NVCC) is None:
         raise RuntimeError(f"nvcc not found at {NVCC}")
-    OBJ.mkdir(parents=True, exist_ok=True)
+    with _locked():
+        return _build_locked(tools, jobs, verbose)
+
+
+def _build_locked(tools: bool, jobs: int | None, verbose: bool) -> Path:
     LIB.parent.mkdir(parents=True, exist_ok=True)
     BIN.mkdir(parents=True, exist_ok=True)
     stamp = _headers_digest() + hashlib.sha1(" ".join(CXXFLAGS + NVCCFLAGS).encode()).hexdigest()
     jobs = jobs or max(1, (os.cpu_count() or 4))
-    torch_srcs = sorted((ROOT / "src" / "torch").glob("*.cpp"))
+    torch_dir = _torch_dir()
+    torch_srcs = sorted((ROOT / "src" / "torch").glob("*.cpp")) if torch_dir else []
+    torch_stamp = stamp + _torch_stamp()
     srcs = library_sources()
     with ThreadPoolExecutor(jobs) as ex:
-        objs = list(ex.map(lambda s: _compile(s, stamp), torch_srcs + srcs))
-    torch_objs, objs = objs[:len(torch_srcs)], objs[len(torch_srcs):]
-    newest = max(o.stat().st_mtime_ns for o in objs)
-    if not LIB.exists() or LIB.stat().st_mtime_ns < newest:
-        _run([NVCC] + GENCODE + ["-shared", "-o", str(LIB)] + [str(o) for o in objs] +
-             ["-lpthread", "-ldl", "-lrt"])
-        if verbose:
-            print(f"linked {LIB}")
-    if not TORCH_LIB.exists() or TORCH_LIB.stat().st_mtime_ns < max(o.stat().st_mtime_ns for o in torch_objs + [LIB]):
-        _run([CXX, "-shared", "-o", str(TORCH_LIB)] + [str(o) for o in torch_objs] +
-             [f"-L{LIB.parent}", "-lal_b200", f"-L{_torch_dir() / 'lib'}", "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-lc10", "-lc10_cuda",
-              "-Wl,-rpath,$ORIGIN"])
+        torch_jobs = [ex.submit(_compile, s, torch_stamp) for s in torch_srcs]
+        objs = list(ex.map(lambda s: _compile(s, stamp), srcs))
+        newest = max(o.stat().st_mtime_ns for o in objs)
+        if not LIB.exists() or LIB.stat().st_mtime_ns < newest:
+            _link(LIB, [NVCC] + GENCODE + ["-shared"] + [str(o) for o in objs] + ["-lpthread", "-ldl", "-lrt"])
+            if verbose:
+                print(f"linked {LIB}")
+        torch_objs = [j.result() for j in torch_jobs]
+    if torch_objs and (not TORCH_LIB.exists() or TORCH_LIB.stat().st_mtime_ns < max(o.stat().st_mtime_ns for o in torch_objs + [LIB])):
+        _link(TORCH_LIB, [CXX, "-shared"] + [str(o) for o in torch_objs] +
+              [f"-L{LIB.parent}", "-lal_b200", f"-L{torch_dir / 'lib'}", "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-lc10", "-lc10_cuda",
+               "-Wl,-rpath,$ORIGIN"])
     if tools:
         todo = {n: [ROOT / s for s in ss] for n, ss in TOOLS.items() if all((ROOT / s).exists() for s in ss)}
 

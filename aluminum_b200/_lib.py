@@ -121,12 +121,13 @@ def torch_ops():
     if _torch_ops is None:
         import torch
         load()
-        path = _LIB_PATH.with_name("libal_torch.so")
-        if not path.exists():
-            from . import _build
-            _build.build(tools=False)
-        torch.ops.load_library(str(path))
-        _torch_ops = torch.ops.aluminum_b200
+        with _lock:
+            path = _LIB_PATH.with_name("libal_torch.so")
+            if not path.exists():
+                from . import _build
+                _build.build(tools=False)
+            torch.ops.load_library(str(path))
+            _torch_ops = torch.ops.aluminum_b200
     return _torch_ops
 
 
