@@ -86,8 +86,6 @@ def _declare(lib) -> None:
         "al_scale_cast": (i, [vp, i, vp, i, sz, d, vp]),
         "al_sgd_momentum": (i, [vp, vp, vp, sz, C.c_float, C.c_float, C.c_float, C.c_float, i, i, vp]),
         "al_fill_u32": (i, [vp, sz, C.c_uint32, vp]),
-        "al_bn_forward": (i, [i] + [vp] * 12 + [sz, sz, i, C.c_float, C.c_float, vp]),
-        "al_bn_backward": (i, [i] + [vp] * 11 + [sz, sz, i, vp]),
     }
     for name, (res, args) in sig.items():
         fn = getattr(lib, name)

@@ -193,6 +193,7 @@ int al_sgd_momentum(float* param, float* momentum, float* grad, size_t n, float 
                     float grad_scale, int first_step, int zero_grad, void* stream);
 int al_fill_u32(void* out, size_t n, uint32_t value, void* stream);
 /* Training batch norm + residual + ReLU over rows x channels (channels-last); residual, mask, running_*, batches may be NULL. */
+size_t al_bn_workspace_bytes(int channels);
 int al_bn_forward(int dt, const void* x, const void* residual, void* y, unsigned char* mask, const float* weight, const float* bias,
                   float* running_mean, float* running_var, long long* batches, float* save_mean, float* save_invstd,
                   void* workspace, size_t workspace_bytes, size_t rows, int channels, float momentum, float eps, void* stream);

@@ -181,6 +181,8 @@ struct BnBackward {
   size_t rows;
   int channels;
 };
+/** What either direction needs at most as workspace. */
+size_t bn_workspace_bytes(int channels);
 void launch_bn_forward(const BnForward& a, DType dt, cudaStream_t stream);
 void launch_bn_backward(const BnBackward& a, DType dt, cudaStream_t stream);
 /** Max pooling of channels-last activations (bf16 or f16; kernels/maxpool.cu); place: the winner's k * row + column, a byte per output. */

@@ -29,6 +29,7 @@ namespace device {
 namespace {
 
 constexpr int kBnThreads = 256;
+constexpr int kBnSms = 148;
 constexpr int kBnPerSm = 2;        // CTAs per SM (no spills at up to 128 registers): 2 x 256 threads x 8 x 16 bytes = 64 KB under way per SM
 constexpr int kBnStatRows = 8;     // rows a thread loads at once
 constexpr int kBnRows = 4;         // ... where it loads two or three arrays
@@ -55,7 +56,7 @@ BnGrid bn_grid(size_t rows, int channels, int rows_per_thread) {
   const size_t tile = (size_t)(kBnThreads >> g.lx) * (size_t)rows_per_thread;
   g.tiles = (unsigned)((rows + tile - 1) / tile);
   // one wave: every SM gets kBnPerSm CTAs, each of which walks its share of the tiles
-  g.nblk = std::max(1u, std::min(g.tiles, (unsigned)(148 * kBnPerSm) / g.ntile_y));
+  g.nblk = std::max(1u, std::min(g.tiles, (unsigned)(kBnSms * kBnPerSm) / g.ntile_y));
   g.each = g.tiles / g.nblk;
   g.more = g.tiles % g.nblk;
   g.tile_rows = (unsigned)tile;
@@ -448,6 +449,11 @@ void bn_backward(const BnBackward& a, cudaStream_t stream) {
 }
 
 }  // namespace
+
+size_t bn_workspace_bytes(int channels) {
+  // partial sums of one wave of CTAs, 256 channels each (or of one CTA per 256 channels), and the backward's coefficients
+  return (size_t)kBnSms * kBnPerSm * 256 * sizeof(float2) + 2 * sizeof(float2) * (size_t)channels;
+}
 
 void launch_bn_forward(const BnForward& a, DType dt, cudaStream_t stream) {
   if (dt == DType::bf16) return bn_forward<__nv_bfloat16>(a, stream);

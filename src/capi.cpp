@@ -642,6 +642,7 @@ int al_fill_u32(void* out, size_t n, uint32_t value, void* stream) {
   return guard([&] { device::launch_fill_u32((uint32_t*)out, n, value, (cudaStream_t)stream); });
 }
 
+size_t al_bn_workspace_bytes(int channels) { return device::bn_workspace_bytes(channels); }
 int al_bn_forward(int dt, const void* x, const void* residual, void* y, unsigned char* mask, const float* weight, const float* bias,
                   float* running_mean, float* running_var, long long* batches, float* save_mean, float* save_invstd,
                   void* workspace, size_t workspace_bytes, size_t rows, int channels, float momentum, float eps, void* stream) {

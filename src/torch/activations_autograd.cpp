@@ -20,8 +20,7 @@ constexpr int kArgs = 10;  // of forward()
 
 int type_code(const Tensor& t) { return (int)(t.scalar_type() == at::kBFloat16 ? Al::DType::bf16 : Al::DType::f16); }
 
-/** Partial sums of at most 148 x 3 CTAs of 256 channels (8 bytes each) and 16 bytes per channel. */
-Tensor workspace(const Tensor& x, int64_t channels) { return at::empty({148 * 3 * 256 * 8 + 16 * channels}, x.options().dtype(at::kByte)); }
+Tensor workspace(const Tensor& x, int64_t channels) { return at::empty({(int64_t)al_bn_workspace_bytes((int)channels)}, x.options().dtype(at::kByte)); }
 
 /**
  * A saved tensor as the kernels read it.  Saved-tensor hooks give back the values but not always the layout (a copy to pinned
