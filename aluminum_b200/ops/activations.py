@@ -29,14 +29,14 @@ def _activation_ok(x) -> bool:
             and x.numel() >= 2 * x.shape[1] > 0)
 
 
-def _parameter_ok(t, x) -> bool:
+def _parameter_ok(t, channels: int, device: int) -> bool:
     """A plain tensor with one fp32 value per channel (of another length the module raises; a subclass may have no memory of its own)."""
-    return (type(t) in _PLAIN and not t.is_inference() and t.dtype == torch.float32 and t.numel() == x.shape[1] and t.is_contiguous()
-            and t.get_device() == x.get_device() and t.data_ptr() % 16 == 0)
+    return (type(t) in _PLAIN and t.dtype == torch.float32 and t.numel() == channels and t.get_device() == device and t.is_contiguous()
+            and not t.is_inference() and t.data_ptr() % 16 == 0)
 
 
-def _count_ok(t, x) -> bool:
-    return t is None or (type(t) in _PLAIN and t.dtype == torch.int64 and t.numel() == 1 and t.get_device() == x.get_device() and not t.is_inference())
+def _count_ok(t, device: int) -> bool:
+    return t is None or (type(t) in _PLAIN and t.dtype == torch.int64 and t.numel() == 1 and t.get_device() == device and not t.is_inference())
 
 
 def _modes_off() -> bool:
@@ -47,21 +47,28 @@ def _modes_off() -> bool:
                 or g._global_forward_hooks or g._global_forward_pre_hooks or g._global_backward_hooks or g._global_backward_pre_hooks)
 
 
-def _fusable(bn: nn.Module, x) -> bool:
+def _tensors(bn: nn.Module, x):
+    """Weight, bias, running statistics and count of a batch norm that the kernels may run on x, else None."""
     # (_modes_off() first: a compiler that traces this function sees a constant there and nothing of what follows)
-    return (_modes_off() and type(bn) is nn.BatchNorm2d and bn.training and bn.track_running_stats and bn.momentum is not None and _activation_ok(x)
-            and x.shape[1] == bn.num_features and x.get_device() == torch.cuda.current_device() and _bare(bn)
-            and _parameter_ok(bn.weight, x) and _parameter_ok(bn.bias, x) and _parameter_ok(bn.running_mean, x)
-            and _parameter_ok(bn.running_var, x) and _count_ok(bn.num_batches_tracked, x))
+    if not (_modes_off() and type(bn) is nn.BatchNorm2d and bn.training and bn.track_running_stats and bn.momentum is not None
+            and _activation_ok(x) and _bare(bn)):
+        return None
+    c, device = bn.num_features, x.get_device()
+    found = weight, bias, mean, var, count = bn.weight, bn.bias, bn.running_mean, bn.running_var, bn.num_batches_tracked
+    if (x.shape[1] == c and device == torch.cuda.current_device() and _parameter_ok(weight, c, device) and _parameter_ok(bias, c, device)
+            and _parameter_ok(mean, c, device) and _parameter_ok(var, c, device) and _count_ok(count, device)):
+        return found
+    return None
 
 
 def batch_norm_act(bn: nn.Module, x: torch.Tensor, relu: nn.Module | None = None, residual: torch.Tensor | None = None) -> torch.Tensor:
     """``relu(bn(x) + residual)``; without ``relu`` or ``residual`` the same without that part."""
-    if (_fusable(bn, x) and (relu is None or (type(relu) is nn.ReLU and _bare(relu)))
+    found = _tensors(bn, x)
+    if (found is not None and (relu is None or (type(relu) is nn.ReLU and _bare(relu)))
             and (residual is None or (_activation_ok(residual) and residual.shape == x.shape and residual.dtype == x.dtype
                                       and residual.get_device() == x.get_device()))):
-        return _lib.torch_ops().batch_norm_act.default(x, bn.weight, bn.bias, residual, bn.running_mean, bn.running_var,
-                                                       bn.num_batches_tracked, bn.momentum, bn.eps, relu is not None)
+        weight, bias, mean, var, count = found
+        return _lib.torch_ops().batch_norm_act.default(x, weight, bias, residual, mean, var, count, bn.momentum, bn.eps, relu is not None)
     y = bn(x)
     if residual is not None:
         y = y + residual

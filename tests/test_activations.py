@@ -197,10 +197,9 @@ def test_parameters_of_another_length_or_kind_go_to_the_module():
 
     class Wrapped(torch.Tensor):
         pass
-    x = torch.zeros(1, 8, 2, 2)
-    assert activations._parameter_ok(torch.zeros(8), x) and activations._parameter_ok(nn.Parameter(torch.zeros(8)), x)
+    assert activations._parameter_ok(torch.zeros(8), 8, -1) and activations._parameter_ok(nn.Parameter(torch.zeros(8)), 8, -1)
     for other in (torch.zeros(7), torch.zeros(16), torch.zeros(8).double(), torch.zeros(8).as_subclass(Wrapped), None):
-        assert not activations._parameter_ok(other, x)
+        assert not activations._parameter_ok(other, 8, -1)
 
 
 def test_forward_of_the_instances_own():
