@@ -15,7 +15,7 @@
 // LeVeque, "Updating formulae and a pairwise algorithm for computing sample variances", 1979), in fp32 and in a fixed order.
 //
 // Measured, one B200, ResNet-50 training step in bf16: batch 256 53.7 -> 26.2 ms, batch 24 (bound by the host's launches:
-// 1013 -> 795 a step) 10.9 -> 9.0 ms.  Three CTAs per SM (80 registers, spills in the gradient kernels) took 27.8 ms.
+// 1013 -> 795 a step) 10.9 -> 9.0 ms (repeats differ by up to 8 %).  Three CTAs per SM (80 registers, spills in the gradient kernels) took 27.8 ms.
 #include <algorithm>
 
 #include "al/cuda/cuda.hpp"

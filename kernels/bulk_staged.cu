@@ -2,14 +2,14 @@
 // moved by the bulk copy engine (cp.async.bulk) through shared memory.
 //
 // Publish, handshake, consume, chunks, epochs and flags are those of the serial schedule of coll_kernel.cuh.  What differs is
-// what bounds it: with all ranks on one GPU the staging traffic is HBM traffic, and the load / store loops of that kernel
-// (16 warps per SM, load - wait - store) reach 3.2 TB/s of it, waiting for memory more than two thirds of the time.  Here one
-// thread per CTA keeps up to 160 KB of loads under way per SM, across destinations and sources without a gap, and needs no
-// registers for them; reductions are folded out of shared memory while the next tiles arrive.  Loops -> bulk copies:
-// bucket of 4 x 26 MB 136 -> 103 us (525 MB through HBM, 5.1 TB/s), sequence-parallel pair of 4 ranks, 16384 x 8192 bf16,
-// 1668 -> 1036 us (5.4 GB, 5.2 TB/s), of 8 ranks, 2048 x 4096, 203 -> 163 us; bucket of 8 x 12 MB with a bf16 wire, converted
-// between the tiles and staging by all threads, 116 -> 98 us.  Slices that begin anywhere (pair of 8 ranks, 16344 x 990 bf16)
-// are shifted into the destination's words out of the tiles: 417 -> 330 us.
+// what bounds it: with all ranks on one GPU the staging traffic is HBM traffic, and the load / store loops of that kernel keep
+// what 16 warps per SM hold in registers under way.  Here one thread per CTA keeps up to 160 KB of loads under way per SM,
+// across destinations and sources without a gap, and needs no registers for them; reductions are folded out of shared
+// memory while the next tiles arrive.  Loops / bulk copies, us: bucket of 4 x 26 MB 104 / 99 (525 MB of staged traffic, 5.3 TB/s),
+// bf16 allreduce of 2 x 128 MiB 303 / 240, reduce_scatter of 4 x 128 MiB 307 / 258, alltoall of 8 x 4 MiB 42.8 / 28.3, bucket of 8 x 12 MB
+// with a bf16 wire, converted between the tiles and staging by all threads, 103 / 90.  Slices that begin anywhere are shifted into
+// the destination's words out of the tiles, which is what gains most: reduce_scatter of 4 x 256 MiB 1127 / 604, of 8 x 128 MiB 843 / 655,
+// allgather of 2 x 128 MiB 209 / 157.  (Reduce_scatter of eight ranks in whole words is the other way round from 32 MiB on: 144 / 161.)
 // (Between GPUs the engine's stores to peers were slower than SM stores - 4 GPUs, 1 GiB allgather 1534 us against
 // 1291 us - so ranks on GPUs of their own keep coll_kernel.)
 //
