@@ -138,7 +138,7 @@ struct WordSource {
 /** What batched_units() does with the units that are less than a round. */
 enum class Rest {
   spread,    ///< over all warps: half of U loads at once, half of that, then singly (fewest registers)
-  together,  ///< a warp's rows like before, all at once under predicates (least latency; kernels with many such loops spill over it)
+  together,  ///< a warp's rows as in a full round, all at once under predicates (least latency; kernels with many such loops spill over it)
   row        ///< together, for a group that is one warp
 };
 
