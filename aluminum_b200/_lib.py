@@ -66,6 +66,7 @@ def _declare(lib) -> None:
         "al_dev_comm_device": (i, [vp]),
         "al_dev_comm_has_multicast": (i, [vp]), "al_dev_comm_backing": (C.c_char_p, [vp]),
         "al_dev_comm_set_timeout_ms": (i, [vp, d]), "al_dev_comm_stats": (i, [vp, u64p]), "al_dev_comm_bulk_staged_ops": (C.c_uint64, [vp]),
+        "al_dev_comm_local_ops": (C.c_uint64, [vp]),
         "al_dev_comm_status": (i, [vp, u64p]),
         "al_dev_collective": (i, [vp, i, i, vpp, vpp, sz, i, i, i, i, i, i, i, szp, szp, szp, szp, d, i, i, vp, vpp]),
         "al_dev_exchange_rows": (i, [vp, i, vpp, vpp, vpp, vpp, sz, sz, sz, szp, szp, szp, szp, szp, szp, vp, vpp]),

@@ -90,6 +90,7 @@ class DeviceComm:
                  "window", "ll", "rows", "rs_nvls"]
         stats = dict(zip(names, [int(v) for v in out]))
         stats["bulk_staged"] = int(self._lib.al_dev_comm_bulk_staged_ops(self._h))
+        stats["local"] = int(self._lib.al_dev_comm_local_ops(self._h))
         return stats
 
     def status(self) -> dict:

@@ -99,6 +99,8 @@ int al_dev_comm_abort(void* comm, const char* why);
 int al_dev_comm_stats(void* comm, uint64_t* out);
 /** Staged operations with all ranks on one GPU that the bulk copy engine moved. */
 uint64_t al_dev_comm_bulk_staged_ops(void* comm);
+/** Operations with all ranks on one GPU that ran straight between their buffers. */
+uint64_t al_dev_comm_local_ops(void* comm);
 /** Status record: out[0]=code, [1]=rank, [2]=peer, [3]=where, [4]=epoch, [5]=seen. Never fails. */
 int al_dev_comm_status(void* comm, uint64_t* out);
 /**

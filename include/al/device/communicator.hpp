@@ -99,6 +99,7 @@ struct CommStats {
   uint64_t ll = 0;              ///< operations that ran as low-latency packets
   uint64_t rows = 0;            ///< row exchanges (alltoall with fused pack / unpack)
   uint64_t bulk_staged = 0;     ///< staged operations with all ranks on this GPU that the bulk copy engine moved
+  uint64_t local = 0;           ///< operations with all ranks on this GPU that ran straight between their buffers
 };
 
 }  // namespace device

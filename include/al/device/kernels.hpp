@@ -37,6 +37,14 @@ bool collective_supported(DType in, DType wire, DType out, ReductionOperator op)
 bool bulk_staged_supported(DevColl kind, DType user, DType wire, ReductionOperator op);
 void launch_bulk_staged(const CollParams& P, DType user, DType wire, int ctas, int local_ranks, cudaStream_t stream);
 
+// ---- all ranks on this GPU: straight between their buffers (kernels/local_*.cu) ----
+/**
+ * At most max_ctas CTAs of `threads` (whole warps).  The caller has made sure that no byte is written that is read elsewhere.
+ * launch_local_reduce: false (nothing launched) without a kernel for these types and this operator.
+ */
+bool launch_local_reduce(const LocalReduceParams& P, DType user, DType wire, ReductionOperator op, int max_ctas, int threads, cudaStream_t stream);
+void launch_local_copy(LocalCopyParams& P, int max_ctas, int threads, cudaStream_t stream);
+
 // ---- order of tokens by destination rank (kernels/route.cu) ----
 void launch_route(const RouteParams& P, int local_ranks, cudaStream_t stream);
 

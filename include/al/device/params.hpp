@@ -265,6 +265,40 @@ struct RowsParams {
   int rank0;
 };
 
+/**
+ * Operations of ranks that all live on this GPU, straight between their buffers (kernels/local_*.cu).  Indexed by rank; `flags` are the
+ * ranks' flag areas, whose status words say whether an earlier operation failed.
+ */
+struct LocalReduceParams {
+  uint64_t* flags[kMaxRanks];
+  const void* src[kMaxRanks];    ///< the whole vector that a rank contributes
+  void* dst[kMaxRanks];          ///< where its result goes (the vector, or its slice); all on the same address modulo 16 unless scatter
+  size_t count;                  ///< elements of a result
+  double scale;
+  int int_div;
+  int p;
+  int scatter;                   ///< 1: rank r gets slice r
+  int round_result;              ///< a narrower type between GPUs: the result is rounded to it as well (two phases)
+};
+
+/** Copies: job j moves `rows` rows of bytes[j] bytes. */
+struct LocalCopyParams {
+  static constexpr int kMaxJobs = kMaxRanks * kMaxRanks;
+  uint64_t* flags[kMaxRanks];
+  int p;
+  int jobs;
+  int fans;                      ///< 1: every job has several destinations, fan[d] + dst[j] for every d in to[j] (all fan[] the same modulo 16)
+  unsigned rows;
+  size_t src_stride, dst_stride; ///< from row to row
+  const char* src[kMaxJobs];
+  char* dst[kMaxJobs];
+  size_t bytes[kMaxJobs];
+  char* fan[kMaxRanks];
+  unsigned char to[kMaxJobs];
+  unsigned tile;                 ///< filled by the launcher: bytes that a warp takes at a time
+  unsigned first[kMaxJobs + 1];  ///< ... and the first tile of every job
+};
+
 /** Arguments of one routing launch (kernels/route.cu): one block per local rank. */
 struct RouteParams {
   const long long* dest[kMaxRanks];  ///< destination rank of every token

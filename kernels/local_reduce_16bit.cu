@@ -1,0 +1,29 @@
+// 16-bit floating-point reductions between buffers on this GPU (folded in fp32).
+#include "local_reduce.cuh"
+
+namespace Al {
+namespace internal {
+namespace device {
+
+namespace {
+template <typename T>
+bool run(const LocalReduceParams& P, ReductionOperator op, int max_ctas, int threads, cudaStream_t stream) {
+  switch (op) {
+    case ReductionOperator::sum:
+    case ReductionOperator::avg: local_reduce_launch<T, T, true>(P, RedSum(), max_ctas, threads, stream); return true;
+    case ReductionOperator::max: local_reduce_launch<T, T, true>(P, RedMax(), max_ctas, threads, stream); return true;
+    case ReductionOperator::min: local_reduce_launch<T, T, true>(P, RedMin(), max_ctas, threads, stream); return true;
+    default: return false;
+  }
+}
+}  // namespace
+
+bool local_reduce_16bit(const LocalReduceParams& P, DType dt, ReductionOperator op, int max_ctas, int threads, cudaStream_t stream) {
+  if (dt == DType::bf16) return run<__nv_bfloat16>(P, op, max_ctas, threads, stream);
+  if (dt == DType::f16) return run<__half>(P, op, max_ctas, threads, stream);
+  return false;
+}
+
+}  // namespace device
+}  // namespace internal
+}  // namespace Al

@@ -100,7 +100,7 @@ int al_info(char* buf, size_t buflen) {
   X(dev_stage_bytes) X(dev_mailbox_bytes) X(dev_wait_timeout_ms) X(dev_enable_nvls)   \
   X(max_ctas) X(max_ctas_nvls) X(max_ctas_zero_copy) X(threads_per_cta) X(debug_checks) X(debug_guard) X(stream_pool_size)    \
   X(disable_background_streams) X(host_serialize) X(host_two_level) X(host_two_level_max_bytes) X(fault_rank) X(fault_op) X(fault_kind) X(fault_delay_ms) X(fault_jitter_us) \
-  X(p2p_max_ctas) X(bulk_pipeline) X(bulk_pub_ctas) X(bulk_con_ctas) X(ll_max_ctas) X(dev_mailbox_slots) X(p2p_rendezvous_bytes) X(p2p_ll_max_bytes) X(nvls_chunk_bytes) X(max_ctas_pipelined) X(window_enable) X(window_ctas) X(window_multimem) X(window_multimem_ag_ranks) X(window_rs_min_ranks) X(window_rs_min_bytes)
+  X(p2p_max_ctas) X(local_direct) X(bulk_pipeline) X(bulk_pub_ctas) X(bulk_con_ctas) X(ll_max_ctas) X(dev_mailbox_slots) X(p2p_rendezvous_bytes) X(p2p_ll_max_bytes) X(nvls_chunk_bytes) X(max_ctas_pipelined) X(window_enable) X(window_ctas) X(window_multimem) X(window_multimem_ag_ranks) X(window_rs_min_ranks) X(window_rs_min_bytes)
 
 namespace {
 /** "ll_max_bytes" or "ll_max_bytes@4" -> member pointer and row (-1 = all rows); nullptr if not a crossover. */
@@ -313,6 +313,7 @@ int al_dev_comm_stats(void* comm, uint64_t* out) {
   });
 }
 uint64_t al_dev_comm_bulk_staged_ops(void* comm) { return ((DeviceCommunicator*)comm)->stats().bulk_staged; }
+uint64_t al_dev_comm_local_ops(void* comm) { return ((DeviceCommunicator*)comm)->stats().local; }
 int al_dev_comm_status(void* comm, uint64_t* out) {
   device::DeviceStatus s = ((DeviceCommunicator*)comm)->status();
   out[0] = s.code; out[1] = s.rank; out[2] = s.peer; out[3] = s.where; out[4] = s.epoch; out[5] = s.seen;

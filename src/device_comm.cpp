@@ -134,6 +134,11 @@ struct DeviceCommunicator::Impl {
     push_table();
   }
 
+  void begin_local(uint64_t** flags, cudaStream_t stream);
+  void end_local();
+  bool local_reduce(const CollParams& P, DType user, DType wire, ReductionOperator op, cudaStream_t stream);
+  bool local_move(const CollParams& P, cudaStream_t stream);
+
   /** Make `stream` wait for the communicator's previous operation if that ran on another stream. */
   void order_after_previous(cudaStream_t stream) {
     if (have_last && last_stream != stream) {
@@ -211,6 +216,33 @@ bool own_may_skip_staging(DevColl kind, const CountTable* tab, const Span* sent,
   for (int s = rank0; s < rank0 + nlocal; ++s)
     if (s != r && (own.meets(received[s]) || (moves && place.meets(sent[s])))) return false;
   return (own.at == place.at && esz == esz_out) || !(moves ? in : own).meets(out);
+}
+
+/**
+ * May ranks that all live on this GPU run a uniform operation straight between their buffers?  One pass reads and writes at once there,
+ * so no byte may be written that another thread still has to read: receive buffers meet neither each other nor any send
+ * buffer, except where a rank's own contribution lies exactly where its result goes (in place): every thread reads the
+ * elements that it writes before it writes them.
+ */
+bool local_buffers_apart(DevColl kind, const CountTable* tab, const Span* sent, const Span* received, int p, size_t esz) {
+  for (int r = 0; r < p; ++r) {
+    if (!sent[r].at || !received[r].at) return false;
+    for (int s = 0; s < p; ++s) {
+      if (s != r && received[r].meets(received[s])) return false;
+      if (!received[r].meets(sent[s])) continue;
+      if (s != r || kind == DevColl::alltoall) return false;
+      const char *own = sent[r].at, *place = received[r].at;
+      if (kind == DevColl::reduce_scatter) own += tab[r].send_displs[r] * esz;
+      if (kind == DevColl::allgather) place += tab[r].recv_displs[r] * esz;
+      if (own != place) return false;
+    }
+  }
+  return true;
+}
+
+/** CTAs of an operation straight between buffers: the ranks' budget of `each` CTAs, within what the GPU holds at once. */
+int local_ctas(int each, int ranks, int threads, int sm_count) {
+  return std::max(1, std::min(std::max(1, each) * ranks, sm_count * (1024 / threads)));
 }
 
 /**
@@ -366,6 +398,83 @@ void DeviceCommunicator::check_status() const {
 }
 
 CommStats DeviceCommunicator::stats() const { return impl_->stats; }
+
+// ---------------------------------------------------------------------------
+// all ranks on this GPU: straight between their buffers
+// ---------------------------------------------------------------------------
+void DeviceCommunicator::Impl::begin_local(uint64_t** flags, cudaStream_t stream) {
+  for (int r = 0; r < p; ++r) flags[r] = ws.flags[r];
+  order_after_previous(stream);
+}
+
+void DeviceCommunicator::Impl::end_local() {
+  stats.ops++;
+  stats.kernels++;
+  stats.local++;
+}
+
+/** Reductions; false: there is no kernel for this operation or these addresses. */
+bool DeviceCommunicator::Impl::local_reduce(const CollParams& P, DType user, DType wire, ReductionOperator op, cudaStream_t stream) {
+  LocalReduceParams L{};
+  const size_t esz = dtype_size(user);
+  for (int r = 0; r < p; ++r) {
+    L.src[r] = P.send[r];
+    L.dst[r] = P.recv[r];
+    if ((uintptr_t)P.send[r] % esz || (uintptr_t)P.recv[r] % esz) return false;
+    if (P.kind == (int)DevColl::allreduce && ((uintptr_t)P.recv[r] ^ (uintptr_t)P.recv[0]) % 16) return false;
+  }
+  L.count = P.count;
+  L.scale = P.scale;
+  L.int_div = P.int_div;
+  L.p = p;
+  L.scatter = P.kind == (int)DevColl::reduce_scatter;
+  L.round_result = user != wire && P.two_phase;
+  begin_local(L.flags, stream);
+  const int threads = cta_threads();
+  if (!launch_local_reduce(L, user, wire, op, local_ctas(tuning().max_ctas, p, threads, sm_count), threads, stream)) return false;
+  end_local();
+  return true;
+}
+
+/** Allgather and alltoall (counts in bytes). */
+bool DeviceCommunicator::Impl::local_move(const CollParams& P, cudaStream_t stream) {
+  LocalCopyParams L{};
+  L.p = p;
+  L.rows = 1;
+  const bool gathers = P.kind == (int)DevColl::allgather;
+  L.fans = gathers;
+  for (int r = 0; r < p; ++r) {
+    L.fan[r] = (char*)P.recv[r];
+    L.fans = L.fans && ((uintptr_t)P.recv[r] ^ (uintptr_t)P.recv[0]) % 16 == 0;
+  }
+  for (int s = 0; s < p; ++s) {
+    const char* from = (const char*)P.send[s];
+    const size_t at = (size_t)s * P.count;   // of rank s's slice in a result
+    if (L.fans) {
+      const int j = L.jobs++;
+      L.src[j] = from;
+      L.dst[j] = (char*)at;
+      L.bytes[j] = P.count;
+      L.to[j] = (unsigned char)((1u << p) - 1);
+      if (from == L.fan[s] + at) L.to[j] &= (unsigned char)~(1u << s);   // in place
+      continue;
+    }
+    for (int i = 0; i < p; ++i) {
+      const int d = (s + i) % p;
+      const char* src = gathers ? from : from + (size_t)d * P.count;
+      if (src == L.fan[d] + at) continue;
+      const int j = L.jobs++;
+      L.src[j] = src;
+      L.dst[j] = L.fan[d] + at;
+      L.bytes[j] = P.count;
+    }
+  }
+  begin_local(L.flags, stream);
+  const int threads = cta_threads();
+  launch_local_copy(L, local_ctas(tuning().max_ctas, p, threads, sm_count), threads, stream);
+  end_local();
+  return true;
+}
 
 // ---------------------------------------------------------------------------
 // collectives
@@ -649,6 +758,17 @@ void DeviceCommunicator::collective(const CollDesc& d, const std::vector<RankArg
                                            dtype_size(out))
                           ? 1
                           : 0;
+
+  // All ranks on this GPU: straight between their buffers, where these allow it and the caller asked for nothing else.
+  const bool moves_uniform = d.kind == DevColl::allgather || d.kind == DevColl::alltoall;
+  if (I.emulated && p > 1 && tn.local_direct && !use_window && !tn.bulk_pipeline && !d.vector && d.ctas <= 0 && P.count > 0 && in == out &&
+      (d.kind == DevColl::allreduce ? d.algo == AllreduceAlgo::automatic : d.path == CollPath::automatic) &&
+      (d.kind == DevColl::allreduce || d.kind == DevColl::reduce_scatter || moves_uniform) &&
+      local_buffers_apart(d.kind, P.tab, sent, received, p, dtype_size(in)) &&
+      (moves_uniform ? I.local_move(P, stream) : I.local_reduce(P, in, wire, d.op, stream))) {
+    I.stats.bytes += bytes;
+    return;
+  }
 
   // All ranks on this GPU: large operations are moved by the bulk copy engine, chunked by what staging holds.
   // (Its CTAs take a whole SM each, so a caller who asked for smaller CTAs gets the loops.)

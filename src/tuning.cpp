@@ -38,6 +38,7 @@ void Tuning::load_from_env() {
   max_ctas_zero_copy = (int)env_long("AL_MAX_CTAS_ZERO_COPY", max_ctas_zero_copy);
   threads_per_cta = (int)env_long("AL_THREADS_PER_CTA", threads_per_cta);
   p2p_max_ctas = (int)env_long("AL_DEV_P2P_CTAS", p2p_max_ctas);
+  local_direct = env_long("AL_LOCAL_DIRECT", local_direct) != 0;
   bulk_pipeline = env_long("AL_DEV_BULK_PIPELINE", bulk_pipeline) != 0;
   bulk_pub_ctas = (int)env_long("AL_DEV_BULK_PUB_CTAS", bulk_pub_ctas);
   bulk_con_ctas = (int)env_long("AL_DEV_BULK_CON_CTAS", bulk_con_ctas);
@@ -131,6 +132,7 @@ std::string Tuning::describe() const {
      << "max_ctas_zero_copy = " << max_ctas_zero_copy << "\n"
      << "threads_per_cta = " << threads_per_cta << "\n"
      << "p2p_max_ctas = " << p2p_max_ctas << "\n"
+     << "local_direct = " << local_direct << "\n"
      << "bulk_pipeline = " << bulk_pipeline << "\n"
      << "bulk_pub_ctas = " << bulk_pub_ctas << "\n"
      << "bulk_con_ctas = " << bulk_con_ctas << "\n"

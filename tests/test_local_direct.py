@@ -1,0 +1,231 @@
+"""Operations of ranks that all live on one GPU, straight between their buffers (kernels/local_*.cu): every form that they
+accept gives bit for bit what the staging protocol gives, and what they must not take goes through staging.
+
+The kernels that ranks on GPUs of their own run are tested on one GPU in the other files where a call names its path; the tests
+there that leave it open are run again here with ``local_direct`` off.
+"""
+import random
+
+import pytest
+import torch
+
+import test_device_emulated
+import test_device_paths
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def al():
+    import aluminum_b200 as al
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    al.init()
+    return al
+
+
+@pytest.fixture
+def staged(al):
+    al.set_tuning("local_direct", 0)
+    yield
+    al.set_tuning("local_direct", 1)
+
+
+def values(n, dtype, seed, shift=0):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    if not dtype.is_floating_point:
+        return torch.randint(-1000, 1000, (n + shift,), generator=g, device="cuda").to(dtype)[shift:]
+    return (torch.rand(n + shift, generator=g, device="cuda", dtype=torch.float64) * 2 - 1).to(dtype)[shift:]
+
+
+def both(al, comm, call, taken=1):
+    """The results of call() straight between buffers and through staging; `taken`: how many operations the first way took."""
+    before = comm.stats()["local"]
+    direct = call()
+    assert comm.stats()["local"] - before == taken
+    al.set_tuning("local_direct", 0)
+    try:
+        old = call()
+    finally:
+        al.set_tuning("local_direct", 1)
+    assert comm.stats()["local"] - before == taken
+    torch.cuda.synchronize()
+    assert comm.status()["code"] == 0
+    return direct, old
+
+
+def same(direct, old):
+    for a, b in zip(direct, old):
+        assert torch.equal(a.view(torch.uint8) if a.dtype != torch.uint8 else a, b.view(torch.uint8) if b.dtype != torch.uint8 else b)
+
+
+# beyond what travels as packets (2 MiB per rank at most), around whole words and warps' shares
+LENGTHS = [3 << 20, (3 << 20) + 2, (3 << 20) + 18, (5 << 20) + 1034]
+
+
+@pytest.mark.parametrize("p", [2, 3, 4, 5, 8])
+@pytest.mark.parametrize("dtype,ops", [(torch.float32, ("sum", "avg", "min", "max")), (torch.bfloat16, ("sum", "max")), (torch.float16, ("avg", "min")),
+                                       (torch.float64, ("sum", "max")), (torch.int32, ("sum", "avg", "min")), (torch.int64, ("sum", "max"))])
+def test_allreduce_equals_staging(al, p, dtype, ops):
+    comm = al.DeviceComm(emulate=p)
+    for k, nbytes in enumerate(LENGTHS):
+        n = nbytes // dtype.itemsize
+        op = ops[k % len(ops)]
+        for shift, out_shift in ((0, 0), (1, 0), (0, 1), (1, 1)):
+            def out_of_place():
+                xs = [values(n, dtype, r, shift) for r in range(p)]
+                whole = [torch.zeros(n + out_shift + 3, dtype=dtype, device="cuda") for _ in range(p)]
+                comm.allreduce(xs, [w[out_shift:out_shift + n] for w in whole], op)
+                return whole                     # with what lies before and behind the result
+            same(*both(al, comm, out_of_place))
+
+            def in_place():
+                xs = [values(n, dtype, r, shift) for r in range(p)]
+                comm.allreduce(xs, op=op, scale=0.375 if dtype.is_floating_point else 1.0)
+                return xs
+            same(*both(al, comm, in_place))
+    comm.close()
+
+
+@pytest.mark.parametrize("p", [2, 3, 4, 8])
+@pytest.mark.parametrize("wire", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("n", [1, 5, 4097, 300001, 3000009])
+def test_narrower_type_between_ranks_rounds_as_staging_does(al, p, wire, n):
+    comm = al.DeviceComm(emulate=p)
+    for shift in (0, 1):
+        def call():
+            xs = [values(n, torch.float32, r, shift) for r in range(p)]
+            comm.allreduce(xs, scale=1.0 / p, wire_dtype=wire)
+            outs = [torch.zeros(n, device="cuda") for _ in range(p)]
+            comm.allreduce(xs, outs, wire_dtype=wire)
+            return xs + outs
+        same(*both(al, comm, call, 2))
+    comm.close()
+
+
+@pytest.mark.parametrize("p", [2, 3, 4, 8])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.int64])
+def test_reduce_scatter_allgather_alltoall_equal_staging(al, p, dtype):
+    comm = al.DeviceComm(emulate=p)
+    for nbytes in ((2 << 20) + 16, (2 << 20) + 8 + 2 * dtype.itemsize, (3 << 20) + 5 * dtype.itemsize):
+        n = nbytes // dtype.itemsize             # per slice: more than the packets carry, whole words and not
+        for shift in (0, 1):
+            def reduce_scatter():
+                xs = [values(p * n, dtype, r, shift) for r in range(p)]
+                whole = [torch.zeros(n + 3, dtype=dtype, device="cuda") for _ in range(p)]
+                comm.reduce_scatter(xs, [w[:n] for w in whole])
+                mine = [x[r * n:(r + 1) * n] for r, x in enumerate(xs)]   # each result on the own contribution
+                comm.reduce_scatter(xs, mine)
+                return whole + xs
+            same(*both(al, comm, reduce_scatter, 2))
+
+            def allgather():
+                whole = [torch.zeros(p * n + 5, dtype=dtype, device="cuda") for _ in range(p)]
+                comm.allgather([values(n, dtype, r, shift) for r in range(p)], [w[2 * shift:2 * shift + p * n] for w in whole])
+                own = [torch.zeros(p * n + 5, dtype=dtype, device="cuda") for _ in range(p)]
+                for r in range(p):
+                    own[r][shift + r * n:shift + (r + 1) * n] = values(n, dtype, r)
+                comm.allgather([w[shift:shift + p * n] for w in own])
+                uneven = [torch.zeros(p * n + 9, dtype=dtype, device="cuda") for _ in range(p)]   # receive buffers on different addresses modulo 16
+                comm.allgather([values(n, dtype, r) for r in range(p)], [w[r:r + p * n] for r, w in enumerate(uneven)])
+                return whole + own + uneven
+            same(*both(al, comm, allgather, 3))
+
+            def alltoall():
+                whole = [torch.zeros(p * n + 5, dtype=dtype, device="cuda") for _ in range(p)]
+                comm.alltoall([values(p * n, dtype, r, shift) for r in range(p)], [w[1:1 + p * n] for w in whole])
+                return whole
+            same(*both(al, comm, alltoall))
+    comm.close()
+
+
+@pytest.mark.parametrize("limits", [dict(max_ctas=1), dict(threads_per_cta=96), dict(threads_per_cta=512, max_ctas=3)])
+def test_within_the_callers_limits(al, limits):
+    p, n, old = 4, 1 << 20, {k: al.get_tuning(k) for k in limits}
+    comm = al.DeviceComm(emulate=p)
+    for k, v in limits.items():
+        al.set_tuning(k, v)
+    try:
+        xs = [values(n + 3, torch.float32, r) for r in range(p)]
+        outs = [torch.empty_like(x) for x in xs]
+        comm.allreduce(xs, outs, "max")
+        assert all(torch.equal(o, torch.stack(xs).amax(0)) for o in outs)
+        full = [torch.empty(p * (n + 3), device="cuda") for _ in range(p)]
+        comm.allgather(xs, full)
+        assert all(torch.equal(f, torch.cat(xs)) for f in full)
+        assert comm.stats()["local"] == 2
+    finally:
+        for k, v in old.items():
+            al.set_tuning(k, v)
+        comm.close()
+
+
+def test_what_goes_through_staging(al):
+    """Buffers that meet, in-place forms that are read elsewhere, and calls that name a path or a grid."""
+    p, n = 4, 1 << 20
+    comm = al.DeviceComm(emulate=p)
+    xs = [values(n, torch.float32, r) for r in range(p)]
+    want = torch.stack(xs).amax(0)
+    turned = xs[1:] + xs[:1]
+
+    def outs():
+        return [torch.empty_like(x) for x in xs]
+    for kw in (dict(algo="one_shot"), dict(algo="two_shot"), dict(ctas=4)):
+        o = outs()
+        comm.allreduce(xs, o, "max", **kw)
+        assert all(torch.equal(v, want) for v in o)
+    base = [values(n + 64, torch.float32, r) for r in range(p)]
+    w = torch.stack([b[:n] for b in base]).amax(0)
+    o = [b[64:] for b in base]                   # partly on the own contribution
+    comm.allreduce([b[:n] for b in base], o, "max")
+    assert all(torch.equal(v, w) for v in o)
+    saved = [x.clone() for x in xs]
+    comm.alltoall(xs, turned)                    # a receive buffer that is another rank's send buffer
+    m = n // p
+    assert all(torch.equal(turned[r], torch.cat([s[r * m:(r + 1) * m] for s in saved])) for r in range(p))
+    ys = [x.clone() for x in saved]
+    comm.alltoall(ys)
+    assert all(torch.equal(ys[r], torch.cat([s[r * m:(r + 1) * m] for s in saved])) for r in range(p))
+    ys = [x.clone() for x in saved]
+    comm.reduce_scatter(ys, op="max")            # results at the start of buffers that are still read
+    assert all(torch.equal(ys[r][:m], want[r * m:(r + 1) * m]) for r in range(p))
+    comm.allreduce(saved, outs(), "prod")        # no kernel for the operator
+    assert comm.stats()["local"] == 0
+    comm.close()
+
+
+@pytest.mark.parametrize("kind", ["allreduce", "reduce_scatter", "allgather", "alltoall"])
+def test_random_forms_equal_staging(al, kind):
+    rng = random.Random(kind)
+    for k in range(12):
+        p = rng.choice([2, 3, 4, 5, 6, 7, 8])
+        dtype = rng.choice([torch.float32, torch.bfloat16, torch.float16, torch.int32])
+        n = rng.randint(1_100_000, 1_900_000)   # beyond the packets in every type
+        shifts = [rng.choice([0, 0, 1, 2, 3, 4, 8]) for _ in range(2 * p)]
+        comm = al.DeviceComm(emulate=p)
+
+        def call():
+            send = n * (p if kind in ("reduce_scatter", "alltoall") else 1)
+            recv = n * (p if kind in ("allgather", "alltoall") else 1)
+            xs = [values(send, dtype, r, shifts[r]) for r in range(p)]
+            whole = [torch.zeros(recv + 12, dtype=dtype, device="cuda") for _ in range(p)]
+            outs = [w[shifts[p + r]:shifts[p + r] + recv] for r, w in enumerate(whole)]
+            getattr(comm, kind)(xs, outs)
+            return whole
+        phases = {s * dtype.itemsize % 16 for s in shifts[p:]}
+        same(*both(al, comm, call, 0 if kind == "allreduce" and len(phases) > 1 else 1))   # (results on different addresses modulo 16)
+        comm.close()
+
+
+@pytest.mark.parametrize("test", [test_device_emulated.test_pipelined_schedule, test_device_paths.test_two_rank_allreduce_is_pipelined_above_threshold])
+def test_staging_between_gpus(al, staged, test):
+    test(al)
+
+
+@pytest.mark.parametrize("p", [2, 8])
+def test_staging_between_gpus_of_large_operations(al, staged, p):
+    comm = al.DeviceComm(emulate=p)
+    test_device_emulated.test_reduce_scatter_allgather_alltoall(comm, 131072 * 8 + 3)
+    test_device_emulated.test_allreduce_f32(comm, 3000001, "auto")
+    assert comm.stats()["local"] == 0
+    comm.close()
