@@ -269,11 +269,17 @@ class DeviceComm:
                 arr[i] = t.data_ptr() if t is not None else None
             return arr
 
+        def room(tensors, lst):
+            """Bytes from each tensor on that rows may lie in, where indexes on the GPU say which."""
+            if lst is None or self.nlocal == 1:
+                return None
+            return size_array([t.untyped_storage().nbytes() - t.storage_offset() * t.element_size() for t in tensors])
+
         sp = (C.c_void_p * self.nlocal)(*[t.data_ptr() for t in sends])
         rp = (C.c_void_p * self.nlocal)(*[t.data_ptr() for t in recvs])
         req = C.c_void_p(None)
-        check(self._lib.al_dev_exchange_rows(
-            self._h, self.nlocal, sp, rp, idx_ptrs(sidx), idx_ptrs(ridx), int(row_bytes), int(send_row_stride),
+        check(self._lib.al_dev_exchange_rows_sized(
+            self._h, self.nlocal, sp, rp, room(sends, sidx), room(recvs, ridx), idx_ptrs(sidx), idx_ptrs(ridx), int(row_bytes), int(send_row_stride),
             int(recv_row_stride), table(send_rows), table(send_first), table(send_peer_off), table(recv_rows),
             table(recv_first), table(recv_peer_off), self._stream(stream), C.byref(req) if nonblocking else None))
         return Request(req, True, (sends, recvs, sidx, ridx)) if nonblocking else None

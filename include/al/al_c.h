@@ -125,6 +125,13 @@ int al_dev_exchange_rows(void* comm, int nlocal, const void* const* send, void* 
                          const size_t* send_rows, const size_t* send_first, const size_t* send_peer_off,
                          const size_t* recv_rows, const size_t* recv_first, const size_t* recv_peer_off, void* stream,
                          void** req_out);
+/** The same with the number of bytes from send[lr] / recv[lr] on that indexed rows may lie in (NULL: not known, and indexed rows of
+ *  ranks on one GPU then go through staging). */
+int al_dev_exchange_rows_sized(void* comm, int nlocal, const void* const* send, void* const* recv, const size_t* send_bytes,
+                               const size_t* recv_bytes, const long long* const* send_idx, const long long* const* recv_idx,
+                               size_t row_bytes, size_t send_row_stride, size_t recv_row_stride, const size_t* send_rows,
+                               const size_t* send_first, const size_t* send_peer_off, const size_t* recv_rows, const size_t* recv_first,
+                               const size_t* recv_peer_off, void* stream, void** req_out);
 /**
  * Where the time of a small collective goes.  Same loop as al_dev_time_collective, with the kernels'
  * %globaltimer stamps switched on.  out_us[0..5] = medians in microseconds of: the event-pair time, the host

@@ -78,6 +78,7 @@ struct RowArgs {
   const long long* send_idx = nullptr;   ///< device memory, or nullptr
   const long long* recv_idx = nullptr;
   std::vector<size_t> send_rows, send_first, send_peer_off, recv_rows, recv_first, recv_peer_off;  ///< one entry per rank
+  size_t send_bytes = 0, recv_bytes = 0; ///< memory from send / recv on that indexed rows may lie in; 0 = not known
 };
 
 struct P2PDesc {

@@ -44,6 +44,7 @@ void launch_bulk_staged(const CollParams& P, DType user, DType wire, int ctas, i
  */
 bool launch_local_reduce(const LocalReduceParams& P, DType user, DType wire, ReductionOperator op, int max_ctas, int threads, cudaStream_t stream);
 void launch_local_copy(LocalCopyParams& P, int max_ctas, int threads, cudaStream_t stream);
+void launch_local_rows(LocalRowsParams& P, int max_ctas, int threads, cudaStream_t stream);
 
 // ---- order of tokens by destination rank (kernels/route.cu) ----
 void launch_route(const RouteParams& P, int local_ranks, cudaStream_t stream);

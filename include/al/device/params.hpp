@@ -299,6 +299,20 @@ struct LocalCopyParams {
   unsigned first[kMaxJobs + 1];  ///< ... and the first tile of every job
 };
 
+/** Row exchange; send_rows of a pair of ranks are what counts. */
+struct LocalRowsParams {
+  uint64_t* flags[kMaxRanks];
+  const void* send[kMaxRanks];
+  void* recv[kMaxRanks];
+  const long long* send_idx[kMaxRanks];
+  const long long* recv_idx[kMaxRanks];
+  RowTable tab[kMaxRanks];
+  size_t row_bytes, send_row_stride, recv_row_stride;
+  int p;
+  unsigned group, per_row;       ///< filled by the launcher: rows that a warp takes at a time, or parts that a row is cut into
+  unsigned first[kMaxRanks * kMaxRanks + 1];  ///< ... and the first unit of every pair [source][destination]
+};
+
 /** Arguments of one routing launch (kernels/route.cu): one block per local rank. */
 struct RouteParams {
   const long long* dest[kMaxRanks];  ///< destination rank of every token

@@ -423,6 +423,15 @@ int al_dev_exchange_rows(void* comm, int nlocal, const void* const* send, void* 
                          const size_t* send_rows, const size_t* send_first, const size_t* send_peer_off,
                          const size_t* recv_rows, const size_t* recv_first, const size_t* recv_peer_off, void* stream,
                          void** req_out) {
+  return al_dev_exchange_rows_sized(comm, nlocal, send, recv, nullptr, nullptr, send_idx, recv_idx, row_bytes, send_row_stride, recv_row_stride,
+                                    send_rows, send_first, send_peer_off, recv_rows, recv_first, recv_peer_off, stream, req_out);
+}
+
+int al_dev_exchange_rows_sized(void* comm, int nlocal, const void* const* send, void* const* recv, const size_t* send_bytes,
+                               const size_t* recv_bytes, const long long* const* send_idx, const long long* const* recv_idx,
+                               size_t row_bytes, size_t send_row_stride, size_t recv_row_stride, const size_t* send_rows,
+                               const size_t* send_first, const size_t* send_peer_off, const size_t* recv_rows, const size_t* recv_first,
+                               const size_t* recv_peer_off, void* stream, void** req_out) {
   return guard([&] {
     DeviceCommunicator& c = *(DeviceCommunicator*)comm;
     ScopedDevice on_device(c.device());
@@ -434,6 +443,8 @@ int al_dev_exchange_rows(void* comm, int nlocal, const void* const* send, void* 
       a.recv = recv[lr];
       a.send_idx = send_idx ? send_idx[lr] : nullptr;
       a.recv_idx = recv_idx ? recv_idx[lr] : nullptr;
+      a.send_bytes = send_bytes ? send_bytes[lr] : 0;
+      a.recv_bytes = recv_bytes ? recv_bytes[lr] : 0;
       const size_t row = (size_t)lr * p;
       a.send_rows.assign(send_rows + row, send_rows + row + p);
       a.send_first.assign(send_first + row, send_first + row + p);

@@ -138,6 +138,7 @@ struct DeviceCommunicator::Impl {
   void end_local();
   bool local_reduce(const CollParams& P, DType user, DType wire, ReductionOperator op, cudaStream_t stream);
   bool local_move(const CollParams& P, cudaStream_t stream);
+  bool local_rows(const RowsParams& R, const std::vector<RowArgs>& ranks, size_t total_rows, cudaStream_t stream);
 
   /** Make `stream` wait for the communicator's previous operation if that ran on another stream. */
   void order_after_previous(cudaStream_t stream) {
@@ -473,6 +474,59 @@ bool DeviceCommunicator::Impl::local_move(const CollParams& P, cudaStream_t stre
   const int threads = cta_threads();
   launch_local_copy(L, local_ctas(tuning().max_ctas, p, threads, sm_count), threads, stream);
   end_local();
+  return true;
+}
+
+/**
+ * Row exchanges; false where rows that are written may meet others that are read or written by another rank (what index arrays
+ * select is not known here: anything in the memory that the caller has named), or the two ends count differently.
+ */
+bool DeviceCommunicator::Impl::local_rows(const RowsParams& R, const std::vector<RowArgs>& ranks, size_t total_rows, cudaStream_t stream) {
+  Span sent[kMaxRanks], received[kMaxRanks];
+  auto reach = [&](const size_t* rows, const size_t* first, const size_t* off, size_t stride) {
+    size_t n = 0;
+    for (int i = 0; i < p; ++i)
+      if (rows[i]) n = std::max(n, off[i] + (first[i] + rows[i] - 1) * stride + R.row_bytes);
+    return n;
+  };
+  for (int r = 0; r < p; ++r) {
+    const RowTable& T = R.tab[r];
+    const RowArgs& a = ranks[(size_t)r];
+    for (int d = 0; d < p; ++d)
+      if (T.send_rows[d] != R.tab[d].recv_rows[r]) return false;
+    sent[r] = Span{(const char*)a.send, reach(T.send_rows, T.send_first, T.send_peer_off, R.send_row_stride)};
+    received[r] = Span{(const char*)a.recv, reach(T.recv_rows, T.recv_first, T.recv_peer_off, R.recv_row_stride)};
+    if (a.send_idx && sent[r].n) {
+      if (!a.send_bytes) return false;
+      sent[r].n = a.send_bytes;
+    }
+    if (a.recv_idx && received[r].n) {
+      if (!a.recv_bytes) return false;
+      received[r].n = a.recv_bytes;
+    }
+  }
+  for (int r = 0; r < p; ++r)
+    for (int s = 0; s < p; ++s)
+      if (received[r].meets(sent[s]) || (s != r && received[r].meets(received[s]))) return false;
+  if (total_rows >= (size_t{1} << 31) || total_rows * (R.row_bytes / 512 + 1) >= (size_t{1} << 31)) return false;   // (32-bit counts of what a warp takes)
+  LocalRowsParams L{};
+  L.p = p;
+  L.row_bytes = R.row_bytes;
+  L.send_row_stride = R.send_row_stride;
+  L.recv_row_stride = R.recv_row_stride;
+  for (int r = 0; r < p; ++r) {
+    L.send[r] = R.send[r];
+    L.recv[r] = R.recv[r];
+    L.send_idx[r] = R.send_idx[r];
+    L.recv_idx[r] = R.recv_idx[r];
+    L.tab[r] = R.tab[r];
+  }
+  begin_local(L.flags, stream);
+  const int threads = cta_threads();
+  launch_local_rows(L, local_ctas(tuning().max_ctas, p, threads, sm_count), threads, stream);
+  end_local();
+  stats.rows++;
+  stats.bytes += total_rows * R.row_bytes;
   return true;
 }
 
@@ -952,7 +1006,6 @@ void DeviceCommunicator::exchange_rows(const std::vector<RowArgs>& ranks, size_t
   R.row_bytes = row_bytes;
   R.send_row_stride = send_row_stride;
   R.recv_row_stride = recv_row_stride;
-  R.seq = ++I.seq;
   R.timeout_ns = I.timeout_ns;
   R.rank0 = I.rank0;
   size_t most_rows = 0, total_rows = 0;
@@ -983,6 +1036,8 @@ void DeviceCommunicator::exchange_rows(const std::vector<RowArgs>& ranks, size_t
     R.local_chunks[r] = std::max<uint64_t>(1, ceil_div(mx, per_chunk));
     if (R.local_chunks[r] >= (1u << 24) - 2) throw_al_exception("exchange_rows: too many rows for the configured staging size");
   }
+  if (I.emulated && p > 1 && tuning().local_direct && I.local_rows(R, ranks, total_rows, stream)) return;
+  R.seq = ++I.seq;
   const size_t work = std::min(total_rows / (size_t)I.nlocal, per_chunk * (size_t)p) * row_bytes;
   int ctas = (int)std::max<size_t>(1, std::min<size_t>(ceil_div(work, (size_t)65536), (size_t)tuning().max_ctas));
   if (I.nlocal > 1) ctas = std::max(1, std::min(ctas, I.sm_count / I.nlocal));

@@ -9,6 +9,7 @@ import random
 import pytest
 import torch
 
+import test_device_copy_edges
 import test_device_emulated
 import test_device_paths
 
@@ -229,3 +230,64 @@ def test_staging_between_gpus_of_large_operations(al, staged, p):
     test_device_emulated.test_allreduce_f32(comm, 3000001, "auto")
     assert comm.stats()["local"] == 0
     comm.close()
+
+
+@pytest.mark.parametrize("p", [2, 3, 8])
+@pytest.mark.parametrize("width,most", [(16, 300), (48, 700), (496, 90), (512, 200), (528, 33), (2048, 40), (2064, 40), (4096, 300), (12304, 9), (24, 77), (7, 50), (4099, 30)])
+def test_rows_equal_staging(al, p, width, most):
+    """Uneven row counts (some none), strided on one side and indexed on the other, around what a warp takes at a time."""
+    comm = al.DeviceComm(emulate=p)
+    counts = [[(7 * s + 13 * d * s) % (most + 1) if (s + d) % 4 else 0 for d in range(p)] for s in range(p)]
+    counts[0][p - 1] = most
+    back = [[counts[s][d] for s in range(p)] for d in range(p)]
+    first = lambda rows: [[sum(r[:i]) for i in range(p)] for r in rows]
+    zero = [[0] * p for _ in range(p)]
+    for indexed in ("neither", "send", "recv"):
+        def call():
+            g = torch.Generator().manual_seed(3)
+            x = [values(max(1, sum(counts[r])) * width, torch.uint8, r).view(-1, width) for r in range(p)]
+            wide = width + (16 if width % 16 == 0 else 5)     # rows further apart than they are long
+            out = [torch.zeros(max(1, sum(back[r])) * wide, dtype=torch.uint8, device="cuda") for r in range(p)]
+            kw = {}
+            if indexed == "send":
+                kw["send_idx"] = [torch.randperm(sum(c), generator=g).cuda() for c in counts]
+            if indexed == "recv":
+                kw["recv_idx"] = [torch.randperm(sum(c), generator=g).cuda() for c in back]
+            comm.exchange_rows(x, out, width, width, wide, counts, first(counts), zero, back, first(back), zero, **kw)
+            return out
+        same(*both(al, comm, call))
+    comm.close()
+
+
+def test_rows_that_meet_go_through_staging(al):
+    p, n, w = 4, 64, 32
+    comm = al.DeviceComm(emulate=p)
+    rows = [[n // p] * p for _ in range(p)]
+    first = [[d * (n // p) for d in range(p)] for _ in range(p)]
+    zero = [[0] * p for _ in range(p)]
+    x = [values(n * w, torch.uint8, r).view(n, w) for r in range(p)]
+    want = [torch.cat([s[r * n // p:(r + 1) * n // p] for s in x]) for r in range(p)]
+    args = (w, w, w, rows, first, zero, rows, first, zero)
+    comm.exchange_rows(x, x, *args)                                   # in place
+    assert all(torch.equal(a, b) for a, b in zip(x, want))
+    whole = values(2 * p * n * w, torch.uint8, 9).view(2 * p, n, w)   # indexed rows may lie anywhere in a tensor's memory
+    sends, recvs = [whole[2 * r] for r in range(p)], [whole[2 * r + 1] for r in range(p)]
+    want = [torch.cat([s[r * n // p:(r + 1) * n // p] for s in sends]) for r in range(p)]
+    order = [torch.arange(n, device="cuda") for _ in range(p)]
+    before = comm.stats()["local"]
+    comm.exchange_rows(sends, recvs, *args, send_idx=order)
+    assert all(torch.equal(a, b) for a, b in zip(recvs, want))
+    assert comm.stats()["local"] == before == 0 and comm.stats()["rows"] == 2
+    comm.exchange_rows(sends, recvs, *args)                           # without indexes their places are known
+    assert all(torch.equal(a, b) for a, b in zip(recvs, want))
+    assert comm.stats()["local"] == 1
+    comm.close()
+
+
+@pytest.mark.parametrize("p", [2, 4, 8])
+def test_row_exchange_between_gpus(al, staged, p):
+    test_device_paths.test_row_exchange_strided_indexed_and_chunked(al, p)
+    for width, rows in ((16, 1000), (80, 333), (4112, 31), (7, 50)):
+        test_device_copy_edges.test_rows_of_any_length(al, p, width, rows)
+    for width, rows in ((2064, 33), (4080, 7), (4112, 4200)):
+        test_device_copy_edges.test_rows_in_rounds_of_four_and_eight(al, p, width, rows)
