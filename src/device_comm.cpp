@@ -138,6 +138,7 @@ struct DeviceCommunicator::Impl {
   void end_local();
   bool local_reduce(const CollParams& P, DType user, DType wire, ReductionOperator op, cudaStream_t stream);
   bool local_move(const CollParams& P, cudaStream_t stream);
+  size_t local_p2p(const std::vector<P2PDesc>& items, std::vector<char>& placed, cudaStream_t stream);
   bool local_rows(const RowsParams& R, const std::vector<RowArgs>& ranks, size_t total_rows, cudaStream_t stream);
 
   /** Make `stream` wait for the communicator's previous operation if that ran on another stream. */
@@ -528,6 +529,56 @@ bool DeviceCommunicator::Impl::local_rows(const RowsParams& R, const std::vector
   stats.rows++;
   stats.bytes += total_rows * R.row_bytes;
   return true;
+}
+
+/**
+ * Point-to-point transfers whose both ends are in this call: straight from buffer to buffer.  Marks them in `placed` and returns how many
+ * items that were.  The k-th send of an ordered pair of ranks meets its k-th receive; a pair on which messages of earlier calls are
+ * under way, or whose ends disagree about the length, keeps its order through the mailbox, and so does the whole call where a
+ * buffer that is written meets another one of the call.
+ */
+size_t DeviceCommunicator::Impl::local_p2p(const std::vector<P2PDesc>& items, std::vector<char>& placed, cudaStream_t stream) {
+  constexpr size_t kMostItems = 64;
+  const size_t n = items.size();
+  if (n > kMostItems) return 0;
+  for (const P2PDesc& it : items)
+    if (it.owner < 0 || it.owner >= p || it.peer < 0 || it.peer >= p) return 0;
+  auto span = [](const P2PDesc& it) { return Span{it.is_send ? (const char*)it.sbuf : (const char*)it.rbuf, it.bytes}; };
+  for (size_t i = 0; i < n; ++i)
+    for (size_t j = 0; !items[i].is_send && j < n; ++j)
+      if (i != j && span(items[i]).meets(span(items[j]))) return 0;
+  LocalCopyParams L{};
+  L.p = p;
+  L.rows = 1;
+  std::vector<char> stays(n, 0);   // receives that a send of their pair could not be matched with
+  size_t taken = 0, moved = 0;
+  for (size_t i = 0; i < n; ++i) {
+    const P2PDesc& s = items[i];
+    if (!s.is_send || p2p_sent[(size_t)s.owner * (size_t)p + (size_t)s.peer] != p2p_recvd[(size_t)s.peer * (size_t)p + (size_t)s.owner]) continue;
+    for (size_t j = 0; j < n; ++j) {
+      const P2PDesc& r = items[j];
+      if (r.is_send || placed[j] || r.owner != s.peer || r.peer != s.owner) continue;
+      if (stays[j] || r.bytes != s.bytes) {
+        stays[j] = 1;
+        break;
+      }
+      const int k = L.jobs++;
+      L.src[k] = (const char*)s.sbuf;
+      L.dst[k] = (char*)r.rbuf;
+      L.bytes[k] = s.bytes;
+      placed[i] = placed[j] = 1;
+      taken += 2;
+      moved += 2 * s.bytes;
+      break;
+    }
+  }
+  if (!taken) return 0;
+  begin_local(L.flags, stream);
+  const int threads = cta_threads();
+  launch_local_copy(L, local_ctas(tuning().p2p_max_ctas, (int)taken, threads, sm_count), threads, stream);
+  end_local();
+  stats.bytes += moved;
+  return taken;
 }
 
 // ---------------------------------------------------------------------------
@@ -1063,6 +1114,8 @@ void DeviceCommunicator::p2p(const std::vector<P2PDesc>& items_in, cudaStream_t 
   // their pieces are numbered consecutively and have to land in order.
   std::vector<char> placed(items_in.size(), 0);
   size_t remaining = items_in.size();
+  if (I.emulated && tuning().local_direct) remaining -= I.local_p2p(items_in, placed, stream);
+  if (!remaining) return;
   I.order_after_previous(stream);
   // A buffer that is both sent and received by the same rank (in-place SendRecv /
   // MultiSendRecv) is sent from a stream-ordered temporary copy, so that arriving

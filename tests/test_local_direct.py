@@ -291,3 +291,63 @@ def test_row_exchange_between_gpus(al, staged, p):
         test_device_copy_edges.test_rows_of_any_length(al, p, width, rows)
     for width, rows in ((2064, 33), (4080, 7), (4112, 4200)):
         test_device_copy_edges.test_rows_in_rounds_of_four_and_eight(al, p, width, rows)
+
+
+def ring(p, src, dst, step=1):
+    return [x for r in range(p) for x in ((True, (r + step) % p, src[r], r), (False, (r - step) % p, dst[r], r))]
+
+
+@pytest.mark.parametrize("p", [2, 3, 8])
+def test_p2p_with_both_ends_in_the_call(al, p):
+    comm = al.DeviceComm(emulate=p)
+    for k, n in enumerate((1, 15, 16, 511, 4097, 65536, 2_097_153, 9_000_001)):
+        src = [values(n, torch.uint8, r, r % 4) for r in range(p)]
+        whole = [torch.zeros(n + 9, dtype=torch.uint8, device="cuda") for _ in range(p)]
+        before = comm.stats()["local"]
+        comm.p2p(ring(p, src, [w[3:3 + n] for w in whole]))
+        assert comm.stats()["local"] == before + 1
+        for r, w in enumerate(whole):
+            assert torch.equal(w[3:3 + n], src[(r - 1) % p]) and not w[:3].any() and not w[3 + n:].any()
+    # several messages of one pair meet in order, an empty one among them; a rank may send to itself
+    msgs = [values(n, torch.float32, n) for n in (1000, 0, 70000, 3)]
+    got = [torch.zeros_like(m) for m in msgs]
+    comm.p2p([(True, 1, m, 0) for m in msgs[:3]] + [(True, 0, msgs[3], 0)] + [(False, 0, g, 1) for g in got[:3]] + [(False, 0, got[3], 0)])
+    assert all(torch.equal(g, m) for g, m in zip(got, msgs)) and comm.status()["code"] == 0
+    comm.close()
+
+
+def test_p2p_order_beside_the_mailbox(al):
+    """Messages of which one end came in an earlier call stay in order before those that have both ends in a call."""
+    comm = al.DeviceComm(emulate=2)
+    comm.set_timeout_ms(3000)
+    m = [torch.full((100,), float(i), device="cuda") for i in range(5)]
+    g = [torch.zeros(100, device="cuda") for _ in range(5)]
+    comm.p2p([(True, 1, m[0], 0)])                                        # under way in the packet ring
+    comm.p2p([(True, 1, m[1], 0), (False, 0, g[0], 1)])                   # receives the first
+    comm.p2p([(False, 0, g[1], 1)])
+    assert comm.stats()["local"] == 0
+    comm.p2p([(True, 1, m[2], 0), (False, 0, g[2], 1), (True, 1, m[3], 0)])   # the last one is received later
+    comm.p2p([(False, 0, g[3], 1)])
+    comm.p2p([(True, 1, m[4], 0), (False, 0, g[4], 1)])
+    assert comm.stats()["local"] == 2
+    torch.cuda.synchronize()
+    assert all(torch.equal(a, b) for a, b in zip(g, m)) and comm.status()["code"] == 0
+    a = [torch.full((50001,), float(r), device="cuda") for r in range(2)]
+    comm.p2p(ring(2, a, a))                                               # in place
+    both_ways = [torch.full((6,), float(r), device="cuda") for r in range(2)]
+    comm.p2p([(True, 1, both_ways[0][:4], 0), (False, 0, both_ways[0][2:], 1)])   # the receive buffer meets the send buffer
+    torch.cuda.synchronize()
+    assert torch.all(a[0] == 1) and torch.all(a[1] == 0)
+    assert comm.stats()["local"] == 2 and comm.status()["code"] == 0
+    comm.close()
+
+
+@pytest.mark.parametrize("p", [2, 4])
+def test_p2p_between_gpus(al, staged, p):
+    test_device_paths.test_p2p_ring_of_slots_and_rendezvous_into_registered_buffers(al, p)
+    test_device_paths.test_p2p_small_messages_travel_as_packets(al, min(p, 3))
+    comm = al.DeviceComm(emulate=p)
+    test_device_emulated.test_p2p_sendrecv_ring(comm)
+    test_device_emulated.test_p2p_in_place_exchange(comm)
+    assert comm.stats()["local"] == 0
+    comm.close()
