@@ -39,7 +39,7 @@ void launch_bulk_staged(const CollParams& P, DType user, DType wire, int ctas, i
 
 // ---- all ranks on this GPU: straight between their buffers (kernels/local_*.cu) ----
 /**
- * At most max_ctas CTAs of `threads` (whole warps).  The caller has made sure that no byte is written that is read elsewhere.
+ * At most max_ctas CTAs of `threads` (whole warps); 0: the whole GPU.  The caller has made sure that no byte is written that is read elsewhere.
  * launch_local_reduce: false (nothing launched) without a kernel for these types and this operator.
  */
 bool launch_local_reduce(const LocalReduceParams& P, DType user, DType wire, ReductionOperator op, int max_ctas, int threads, cudaStream_t stream);

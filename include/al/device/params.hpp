@@ -296,7 +296,6 @@ struct LocalCopyParams {
   char* fan[kMaxRanks];
   unsigned char to[kMaxJobs];
   unsigned tile;                 ///< filled by the launcher: bytes that a warp takes at a time
-  unsigned first[kMaxJobs + 1];  ///< ... and the first tile of every job
 };
 
 /** Row exchange; send_rows of a pair of ranks are what counts. */

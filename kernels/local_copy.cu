@@ -4,9 +4,12 @@
 // mailboxes move it twice and make CTAs wait for each other.  Nothing waits here, so the launches are ordinary ones; the host has
 // checked that no byte is written that another thread still has to read (src/device_comm.cpp).
 //
-// Layout: warps are independent workers that take tiles of up to 2 KiB (four 16-byte loads per thread under way before the first
-// store; 2 x 512 threads per SM keep 64 KB under way) from the list of jobs in turn, so that any mix of sizes fills the GPU.
-// Tiles begin on 16-byte boundaries of the destination; sources on other addresses modulo 16 are shifted into place.
+// Layout: a warp takes a tile of up to 2 KiB (four 16-byte loads per thread under way before the first store; two per thread where each
+// goes to several destinations) of the list of jobs, so that any mix of sizes fills the GPU.  Tiles begin on 16-byte
+// boundaries of the destination; sources on other addresses modulo 16 are shifted into place.  The grid has a warp for every tile
+// unless the caller's budget of CTAs is less than the GPU: CTAs that come and go keep to one stretch of each buffer at a time, those of
+// one wave that walk the tiles drift apart.  One wave of 2 CTAs per SM / a warp per tile, us: 4 x 25 MB from buffer to buffer 37.7 / 32.4,
+// allgather of 8 x 2 MiB 32.8 / 26.5, of 4 x 64 MiB 245 / 204 (6.6 TB/s).
 #include "al/cuda/cuda.hpp"
 #include "al/device/kernels.hpp"
 #include "local_reduce.cuh"
@@ -17,8 +20,7 @@ namespace device {
 
 namespace {
 
-constexpr int kLoads = 4;   // per thread, before the first store
-constexpr unsigned kTile = 32 * 16 * kLoads;
+constexpr int kLoads = 4, kFanLoads = 2;   // per thread, before the first store
 
 /** group_copy() of one warp to several destinations with the same address modulo 16: `at(d)` of every d in `to`. */
 template <typename At>
@@ -39,33 +41,57 @@ __device__ __forceinline__ void warp_fanout(unsigned to, unsigned phase, At at, 
     for (int d = 0; d < kMaxRanks; ++d)
       if (to >> d & 1) ((uint4*)(at(d) + head))[i] = v;
   };
-  if (s.sh == 0) batched_units<kLoads, Rest::row>(nv, lane, 32, [&](size_t i) { return s.base[i]; }, store);
-  else batched_units<kLoads / 2, Rest::spread>(nv, lane, 32, [&](size_t i) { return s.shifted(i); }, store);
+  if (s.sh == 0) batched_units<kFanLoads, Rest::row>(nv, lane, 32, [&](size_t i) { return s.base[i]; }, store);
+  else batched_units<kFanLoads, Rest::spread>(nv, lane, 32, [&](size_t i) { return s.shifted(i); }, store);
   if (lane < n - done) bytes(done + lane);
 }
 
-/** FAN: every job has the destinations fan[d] + its offset, else the one destination dst. */
-template <bool FAN>
+/**
+ * FAN: every job has the destinations fan[d] + its offset, else the one destination dst.  WORDS: everything but the lengths is a whole
+ * number of 16-byte words.  blockIdx.y is the job; its warps take one tile of one of its rows each.
+ */
+template <bool FAN, bool WORDS>
 __global__ void __launch_bounds__(kLocalThreads, 2) local_copy_kernel(const __grid_constant__ LocalCopyParams P) {
-  if (any_poisoned(P.flags, P.p)) return;
-  const unsigned lane = threadIdx.x & 31;
-  const unsigned nwarps = gridDim.x * (blockDim.x >> 5), total = P.first[P.jobs];
-  int j = 0;
+  constexpr int U = FAN ? kFanLoads : kLoads;
+  const uint64_t failed = status_word(P.flags, P.p);
+  const unsigned lane = threadIdx.x & 31, j = blockIdx.y;
+  const size_t bytes = P.bytes[j];
+  const unsigned per_row = (unsigned)((bytes + 15 + P.tile - 1) / P.tile), total = per_row * P.rows;
+  const unsigned nwarps = gridDim.x * (blockDim.x >> 5);
   for (unsigned t = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); t < total; t += nwarps) {
-    while (t >= P.first[j + 1]) ++j;
-    const unsigned per_row = (P.first[j + 1] - P.first[j]) / P.rows;
-    const unsigned row = (t - P.first[j]) / per_row, k = (t - P.first[j]) - row * per_row;
+    const unsigned row = P.rows == 1 ? 0 : t / per_row, k = t - row * per_row;
     const char* src = P.src[j] + row * P.src_stride;
     char* dst = P.dst[j] + row * P.dst_stride;   // (FAN: an offset)
-    const unsigned phase = (unsigned)(((uintptr_t)dst + (FAN ? (uintptr_t)P.fan[0] : 0)) & 15);
-    size_t lo = (size_t)k * P.tile, hi = lo + P.tile - phase;
-    if (k) lo -= phase;
-    if (hi > P.bytes[j]) hi = P.bytes[j];
-    if (lo >= hi) continue;
-    if constexpr (FAN) {
-      warp_fanout(P.to[j], k ? 0 : phase, [&](int d) { return P.fan[d] + ((size_t)dst + lo); }, src + lo, hi - lo, lane);
+    if constexpr (WORDS) {
+      // A tile is at most 32 * U words; the bytes behind the last whole word go with the last tile.
+      const size_t words = bytes / 16, end = min(words, (size_t)(k + 1) * (P.tile / 16)), w0 = (size_t)k * (P.tile / 16) + lane;
+      uint4 v[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        if (w0 + 32 * u < end) v[u] = load_now((const uint4*)src + w0 + 32 * u);
+      if (__any_sync(0xffffffffu, failed != 0)) return;
+      auto put = [&](char* to) {
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+          if (w0 + 32 * u < end) ((uint4*)to)[w0 + 32 * u] = v[u];
+        if (k == per_row - 1 && lane < bytes % 16) to[words * 16 + lane] = src[words * 16 + lane];
+      };
+      if constexpr (FAN) {
+#pragma unroll
+        for (int d = 0; d < kMaxRanks; ++d)
+          if (P.to[j] >> d & 1) put(P.fan[d] + (size_t)dst);
+      } else {
+        put(dst);
+      }
     } else {
-      group_copy<kLoads, Rest::row>(dst + lo, src + lo, hi - lo, false, lane, 32);
+      if (__any_sync(0xffffffffu, failed != 0)) return;
+      const unsigned phase = (unsigned)(((uintptr_t)dst + (FAN ? (uintptr_t)P.fan[0] : 0)) & 15);
+      size_t lo = (size_t)k * P.tile, hi = lo + P.tile - phase;
+      if (k) lo -= phase;
+      if (hi > bytes) hi = bytes;
+      if (lo >= hi) continue;
+      if constexpr (FAN) warp_fanout(P.to[j], k ? 0 : phase, [&](int d) { return P.fan[d] + ((size_t)dst + lo); }, src + lo, hi - lo, lane);
+      else group_copy<kLoads, Rest::row>(dst + lo, src + lo, hi - lo, false, lane, 32);
     }
   }
 }
@@ -73,24 +99,28 @@ __global__ void __launch_bounds__(kLocalThreads, 2) local_copy_kernel(const __gr
 }  // namespace
 
 void launch_local_copy(LocalCopyParams& P, int max_ctas, int threads, cudaStream_t stream) {
-  size_t total = 0;
-  for (int j = 0; j < P.jobs; ++j) total += P.bytes[j] * P.rows;
-  // Small exchanges are cut finer, so that every warp of the GPU gets some; rows of whole tiles keep the divisions above exact.
-  const size_t warps = (size_t)max_ctas * (size_t)(threads / 32);
-  P.tile = 512;
-  while (P.tile < kTile && total / P.tile > 2 * warps) P.tile *= 2;
-  while (total / P.tile > (size_t{1} << 30)) P.tile *= 2;
-  unsigned n = 0;
+  size_t total = 0, longest = 0;
+  bool words = P.src_stride % 16 == 0 && P.dst_stride % 16 == 0;
+  for (int r = 0; P.fans && r < P.p; ++r) words = words && (uintptr_t)P.fan[r] % 16 == 0;
   for (int j = 0; j < P.jobs; ++j) {
-    P.first[j] = n;
-    n += (unsigned)((P.bytes[j] + 15 + P.tile - 1) / P.tile) * P.rows;
+    total += P.bytes[j] * P.rows;
+    longest = std::max(longest, P.bytes[j]);
+    words = words && (uintptr_t)P.src[j] % 16 == 0 && (uintptr_t)P.dst[j] % 16 == 0;
   }
-  P.first[P.jobs] = n;
-  if (n == 0) return;
-  const unsigned per = (unsigned)threads / 32;
-  const unsigned ctas = std::max(1u, std::min((unsigned)max_ctas, (n + per - 1) / per));
-  if (P.fans) local_copy_kernel<true><<<ctas, (unsigned)threads, 0, stream>>>(P);
-  else local_copy_kernel<false><<<ctas, (unsigned)threads, 0, stream>>>(P);
+  if (longest == 0) return;
+  // As much to a warp as leaves 16 of them to an SM.
+  const size_t most = 32 * 16 * (P.fans ? kFanLoads : kLoads);
+  size_t tile = 512;
+  while (tile < most && total / (2 * tile) >= 148 * 16) tile *= 2;
+  while (!words && longest / tile * P.rows > (size_t{1} << 30)) tile *= 2;
+  const size_t most_tiles = (longest + 15 + tile - 1) / tile * P.rows;
+  if (most_tiles >= (size_t{1} << 32)) throw_al_exception("internal error: a copy of ", longest, " bytes in one piece");
+  P.tile = (unsigned)tile;
+  const dim3 grid(local_grid(most_tiles, max_ctas > 0 ? std::max(1, max_ctas / P.jobs) : 0, threads), (unsigned)P.jobs);
+  if (P.fans && words) local_copy_kernel<true, true><<<grid, (unsigned)threads, 0, stream>>>(P);
+  else if (P.fans) local_copy_kernel<true, false><<<grid, (unsigned)threads, 0, stream>>>(P);
+  else if (words) local_copy_kernel<false, true><<<grid, (unsigned)threads, 0, stream>>>(P);
+  else local_copy_kernel<false, false><<<grid, (unsigned)threads, 0, stream>>>(P);
   AL_CHECK_CUDA(cudaGetLastError());
 }
 

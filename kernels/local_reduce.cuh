@@ -12,9 +12,10 @@
 // lie on another address modulo 16 than the result (slices of an odd number of elements) are read as aligned words and
 // shifted into place; the second word of each comes out of L1.
 //
-// Measured, one B200, through staging (loops or bulk copies, whichever was faster) / now, us: gradient bucket of 4 x 26 MB fp32 102.9 / 43.5,
-// 8 x 12 MB fp32 with a bf16 type between ranks 97.7 / 41.9, reduce_scatter and allgather of 8 x 16 MiB bf16 162 / 61.6, of 4 x 256 MiB
-// 1033 / 457 (5.9 TB/s of 6.5 that a plain copy reaches).
+// Measured, one B200, device time through staging (loops or bulk copies, whichever was faster) / here, us: gradient bucket of 4 x 26 MB
+// fp32 103 / 34.3, 8 x 12 MB fp32 with a bf16 type between ranks 95.3 / 31.6, reduce_scatter of 8 x 16 MiB bf16 86.9 / 24.4, of 4 x 256 MiB
+// 506 / 187 (7.2 TB/s, nearly all reads).  With one wave of 2 CTAs per SM that walks the vector instead of a warp per piece: 38.2, 36.5,
+// 28.6, 206.
 #pragma once
 #include "al/cuda/cuda.hpp"
 #include "al/device/kernels.hpp"
@@ -24,13 +25,33 @@ namespace Al {
 namespace internal {
 namespace device {
 
-constexpr int kLocalThreads = 512;
+constexpr int kLocalThreads = 512;   // of a CTA at most
+constexpr size_t kLocalWarps = 148 * 2 * kLocalThreads / 32;   // on the GPU at once
 
-/** Has an earlier operation of the communicator failed?  (Uniform over the warp; all ranks' words, all at once.) */
-__device__ __forceinline__ bool any_poisoned(uint64_t* const* flags, int p) {
+/**
+ * Has an earlier operation of the communicator failed?  A lane's word of the ranks' status words, to be looked at with
+ * __any_sync() behind the first loads of data, which this one's latency then overlaps.  Earlier kernels wrote it, so it may come out of
+ * L1: every warp of the grid asks, and past L1 all of them meet in a few sectors of L2 (allgather of 4 x 64 MiB 222 us).
+ */
+__device__ __forceinline__ uint64_t status_word(uint64_t* const* flags, int p) {
   const unsigned lane = threadIdx.x & 31;
-  const bool bad = lane < (unsigned)p && ld_relaxed_sys(flag_slot(flags[lane], FlagLayout::off_status, 0)) != 0;
-  return __any_sync(0xffffffffu, bad);
+  uint64_t v = 0;
+  if (lane < (unsigned)p)
+    asm volatile("ld.global.ca.u64 %0, [%1];" : "=l"(v) : "l"(flag_slot(flags[lane], FlagLayout::off_status, 0)) : "memory");
+  return v;
+}
+
+/** A load that stays where it is written (past L1: nothing here is read twice). */
+__device__ __forceinline__ uint4 load_now(const uint4* p) {
+  uint4 v;
+  asm volatile("ld.global.cg.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
+  return v;
+}
+
+/** CTAs for `tiles` of one warp each: one warp per tile, or what the caller's budget allows where that is less than one CTA per SM. */
+inline unsigned local_grid(size_t tiles, int max_ctas, int threads) {
+  const size_t per = (size_t)threads / 32, want = std::max<size_t>(1, (tiles + per - 1) / per);
+  return (unsigned)std::min<size_t>(want, max_ctas > 0 ? (size_t)max_ctas : size_t{0x7fffffff});
 }
 
 /** T: the buffers' type, W: the type that crosses the links between GPUs (contributions, and in two phases the result, are rounded to it). */
@@ -39,8 +60,8 @@ __global__ void __launch_bounds__(kLocalThreads, 2) local_reduce_kernel(const __
   using A = typename Elem<T>::Acc;
   constexpr int VEC = 16 / (int)sizeof(T);
   constexpr bool kRounds = !std::is_same<T, W>::value;
-  if (any_poisoned(P.flags, P.p)) return;
   const int p = P.p;
+  const uint64_t failed = status_word(P.flags, p);
   const size_t job = blockIdx.y;   // reduce_scatter: the rank whose slice this is
   const size_t from = P.scatter ? job * P.count : 0;
   const unsigned outs = P.scatter ? 1u << job : (1u << p) - 1;
@@ -67,10 +88,11 @@ __global__ void __launch_bounds__(kLocalThreads, 2) local_reduce_kernel(const __
       const WordSource s((const char*)(src(r) + head), false);
       return s.sh == 0 ? s.base[v] : s.shifted(v);
     } else {
-      return __ldcg((const uint4*)(src(r) + head) + v);
+      return load_now((const uint4*)(src(r) + head) + v);
     }
   };
-  for (size_t v0 = warp * (32 * U) + lane; v0 < nvec; v0 += nwarps * (32 * U)) {
+  for (size_t first = warp * (32 * U); first < nvec; first += nwarps * (32 * U)) {
+    const size_t v0 = first + lane;
     Pack w[R][U];
 #pragma unroll
     for (int r = 0; r < R; ++r)
@@ -79,6 +101,7 @@ __global__ void __launch_bounds__(kLocalThreads, 2) local_reduce_kernel(const __
         for (int u = 0; u < U; ++u)
           if (v0 + 32 * u < nvec) w[r][u].u = load(r, v0 + 32 * u);
       }
+    if (__any_sync(0xffffffffu, failed != 0)) return;
 #pragma unroll
     for (int u = 0; u < U; ++u)
       if (v0 + 32 * u < nvec) {
@@ -97,7 +120,7 @@ __global__ void __launch_bounds__(kLocalThreads, 2) local_reduce_kernel(const __
       }
   }
   // the elements before the first and behind the last whole word
-  if (warp == nwarps - 1) {
+  if (warp == nwarps - 1 && !__any_sync(0xffffffffu, failed != 0)) {
     const size_t i = lane < head ? lane : done + (lane - head);
     if (i < P.count) {
       A acc = in(src(0)[i]);
@@ -116,8 +139,7 @@ template <typename T, typename W, typename Red, int R, int U, bool SHIFT>
 void local_reduce_run(const LocalReduceParams& P, Red red, int max_ctas, int threads, cudaStream_t stream) {
   const int jobs = P.scatter ? P.p : 1;
   const size_t words = P.count * sizeof(T) / 16 + 1;
-  const size_t want = (words + (size_t)threads * U - 1) / ((size_t)threads * U);
-  const dim3 grid((unsigned)std::max<size_t>(1, std::min<size_t>(want, (size_t)std::max(1, max_ctas / jobs))), (unsigned)jobs);
+  const dim3 grid(local_grid((words + 32 * U - 1) / (32 * U), max_ctas > 0 ? std::max(1, max_ctas / jobs) : 0, threads), (unsigned)jobs);
   local_reduce_kernel<T, W, Red, R, U, SHIFT><<<grid, (unsigned)threads, 0, stream>>>(P, red);
   AL_CHECK_CUDA(cudaGetLastError());
 }

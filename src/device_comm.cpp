@@ -242,9 +242,10 @@ bool local_buffers_apart(DevColl kind, const CountTable* tab, const Span* sent, 
   return true;
 }
 
-/** CTAs of an operation straight between buffers: the ranks' budget of `each` CTAs, within what the GPU holds at once. */
-int local_ctas(int each, int ranks, int threads, int sm_count) {
-  return std::max(1, std::min(std::max(1, each) * ranks, sm_count * (1024 / threads)));
+/** CTAs of an operation straight between buffers: the ranks' budget of `each` CTAs, 0 (no limit) where that is one per SM and more. */
+int local_ctas(int each, int ranks, int sm_count) {
+  const int budget = std::max(1, each) * ranks;
+  return budget >= sm_count ? 0 : budget;
 }
 
 /**
@@ -262,6 +263,7 @@ size_t bulk_staged_min_bytes(int p, bool narrower_wire) {
 
 /** Threads of a CTA: whole warps (the loops of datamove.cuh deal in rounds of a warp), whatever the tuning was set to. */
 int cta_threads() { return std::max(32, std::min(512, tuning().threads_per_cta) / 32 * 32); }
+int local_threads() { return std::min(256, cta_threads()); }
 
 void require_device() {
   if (!cuda::device_usable()) throw_al_exception("the device backend needs a CUDA device, none is usable in this process");
@@ -432,8 +434,8 @@ bool DeviceCommunicator::Impl::local_reduce(const CollParams& P, DType user, DTy
   L.scatter = P.kind == (int)DevColl::reduce_scatter;
   L.round_result = user != wire && P.two_phase;
   begin_local(L.flags, stream);
-  const int threads = cta_threads();
-  if (!launch_local_reduce(L, user, wire, op, local_ctas(tuning().max_ctas, p, threads, sm_count), threads, stream)) return false;
+  const int threads = local_threads();
+  if (!launch_local_reduce(L, user, wire, op, local_ctas(tuning().max_ctas, p, sm_count), threads, stream)) return false;
   end_local();
   return true;
 }
@@ -472,8 +474,8 @@ bool DeviceCommunicator::Impl::local_move(const CollParams& P, cudaStream_t stre
     }
   }
   begin_local(L.flags, stream);
-  const int threads = cta_threads();
-  launch_local_copy(L, local_ctas(tuning().max_ctas, p, threads, sm_count), threads, stream);
+  const int threads = local_threads();
+  launch_local_copy(L, local_ctas(tuning().max_ctas, p, sm_count), threads, stream);
   end_local();
   return true;
 }
@@ -523,8 +525,8 @@ bool DeviceCommunicator::Impl::local_rows(const RowsParams& R, const std::vector
     L.tab[r] = R.tab[r];
   }
   begin_local(L.flags, stream);
-  const int threads = cta_threads();
-  launch_local_rows(L, local_ctas(tuning().max_ctas, p, threads, sm_count), threads, stream);
+  const int threads = local_threads();
+  launch_local_rows(L, local_ctas(tuning().max_ctas, p, sm_count), threads, stream);
   end_local();
   stats.rows++;
   stats.bytes += total_rows * R.row_bytes;
@@ -574,8 +576,8 @@ size_t DeviceCommunicator::Impl::local_p2p(const std::vector<P2PDesc>& items, st
   }
   if (!taken) return 0;
   begin_local(L.flags, stream);
-  const int threads = cta_threads();
-  launch_local_copy(L, local_ctas(tuning().p2p_max_ctas, (int)taken, threads, sm_count), threads, stream);
+  const int threads = local_threads();
+  launch_local_copy(L, local_ctas(tuning().p2p_max_ctas, (int)taken, sm_count), threads, stream);
   end_local();
   stats.bytes += moved;
   return taken;
