@@ -31,6 +31,8 @@ namespace Al {
 namespace internal {
 namespace device {
 
+struct HaloParams;
+
 /** Algorithm selector of the device allreduce (the reference's `algo` argument, made real). */
 enum class AllreduceAlgo : int { automatic = 0, one_shot, two_shot, nvls, ll };
 
@@ -233,6 +235,8 @@ class DeviceCommunicator {
   /** Workspace description (used by RMA and halo code). */
   const internal::device::Workspace& workspace() const;
   uint64_t next_halo_epoch();
+  /** Halo exchange of ranks that all live on this GPU, straight between their tensors; false: not such a case (nothing enqueued). */
+  bool local_halo(const internal::device::HaloParams& P, cudaStream_t stream);
 
   struct Impl;
   Impl* impl() const { return impl_.get(); }

@@ -604,6 +604,7 @@ int al_halo_exchange(void* comm, float* const* tensors, size_t nc, size_t d_loca
       P.hi[r] = r + 1 < p ? r + 1 : (periodic && p > 1 ? 0 : -1);
     }
     P.nc = nc; P.d_local = d_local; P.plane = plane; P.depth = depth;
+    if (ctas <= 0 && c.local_halo(P, pick_stream(&c, stream))) return;
     P.epoch = c.next_halo_epoch();
     P.timeout_ns = c.wait_timeout_ns();
     const int nlocal = c.is_emulated() ? p : 1;

@@ -583,6 +583,35 @@ size_t DeviceCommunicator::Impl::local_p2p(const std::vector<P2PDesc>& items, st
   return taken;
 }
 
+bool DeviceCommunicator::local_halo(const HaloParams& H, cudaStream_t stream) {
+  Impl& I = *impl_;
+  // (interior planes are only read and halo planes only written, as long as no halo is wider than its neighbour's interior)
+  if (!I.emulated || !tuning().local_direct || H.depth > H.d_local || H.nc >= (size_t{1} << 24)) return false;
+  LocalCopyParams L{};
+  L.p = I.p;
+  L.rows = (unsigned)H.nc;
+  const size_t plane = H.plane * sizeof(float), depth = H.depth * plane;
+  L.src_stride = L.dst_stride = H.d_local * plane + 2 * depth;
+  auto job = [&](int from, int to, size_t src, size_t dst) {
+    if (to < 0) return;
+    const int j = L.jobs++;
+    L.src[j] = (const char*)H.tensor[from] + src;
+    L.dst[j] = (char*)H.tensor[to] + dst;
+    L.bytes[j] = depth;
+  };
+  for (int r = 0; r < I.p; ++r) {
+    if (!H.tensor[r]) return false;
+    L.flags[r] = I.ws.flags[r];
+    job(r, H.lo[r], depth, depth + H.d_local * plane);   // the first planes become the lower neighbour's upper halo
+    job(r, H.hi[r], H.d_local * plane, 0);
+  }
+  const int threads = local_threads();
+  std::lock_guard<std::mutex> lock(I.mu);
+  if (L.rows && L.jobs) launch_local_copy(L, local_ctas(tuning().max_ctas, I.p, I.sm_count), threads, stream);
+  I.stats.local++;
+  return true;
+}
+
 // ---------------------------------------------------------------------------
 // collectives
 // ---------------------------------------------------------------------------

@@ -351,3 +351,31 @@ def test_p2p_between_gpus(al, staged, p):
     test_device_emulated.test_p2p_in_place_exchange(comm)
     assert comm.stats()["local"] == 0
     comm.close()
+
+
+@pytest.mark.parametrize("shape", [(1, 1, 1, 1, 1), (2, 3, 2, 5, 7), (1, 32, 4, 17, 19), (1, 5, 3, 64, 48), (1, 2, 16, 256, 252), (3, 1, 2, 300, 299)])
+def test_halo_equals_flags(al, shape):
+    from aluminum_b200.ops import HaloExchange
+    n, c, d, h, w = shape
+    for p, depth, periodic in ((2, 1, False), (2, 1, True), (4, 1, False), (3, min(2, d), True), (8, d, True), (4, d + 1, False)):
+        comm = al.DeviceComm(emulate=p)
+        comm.set_timeout_ms(3000)
+        hx = HaloExchange(comm, n, c, d, h, w, depth, periodic)
+
+        def call():
+            for r, t in enumerate(hx.tensors):
+                t.copy_(values(t.numel(), torch.float32, r).view(t.shape))
+            hx.exchange()
+            return [t.clone() for t in hx.tensors]
+        if depth <= d:
+            same(*both(al, comm, call))
+        else:     # halos wider than the interior: the neighbour's planes are not all its own
+            before = comm.stats()["local"]
+            call()
+            assert comm.stats()["local"] == before
+        comm.close()
+
+
+def test_halo_between_gpus(al, staged):
+    from test_device_misc import test_halo_exchange_emulated
+    test_halo_exchange_emulated(al)
