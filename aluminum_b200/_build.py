@@ -16,6 +16,7 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 from concurrent.futures import ThreadPoolExecutor
 from pathlib import Path
 
@@ -23,7 +24,7 @@ ROOT = Path(__file__).resolve().parent.parent
 PKG = ROOT / "aluminum_b200"
 OBJ = ROOT / "build" / "obj"
 LIB = PKG / "lib" / "libal_b200.so"
-TORCH_LIB = PKG / "lib" / "libal_torch.so"  # autograd operators (src/torch), linked against PyTorch
+TORCH_LIB = PKG / "lib" / "libal_torch.so"  # autograd operators and calls on tensors (src/torch), linked against PyTorch
 BIN = PKG / "bin"
 
 CUDA_HOME = Path(os.environ.get("CUDA_HOME", "/usr/local/cuda"))
@@ -133,7 +134,8 @@ def _compile(src: Path, stamp: str) -> Path:
         elif src.parent.name == "torch":
             inc = _torch_dir() / "include"
             _run([CXX] + [f for f in CXXFLAGS if f not in ("-Wall", "-Wextra")] +
-                 [f"-isystem{inc}", f"-isystem{inc / 'torch' / 'csrc' / 'api' / 'include'}", "-c", str(src), "-o", str(obj)])
+                 [f"-isystem{inc}", f"-isystem{inc / 'torch' / 'csrc' / 'api' / 'include'}", f"-isystem{sysconfig.get_paths()['include']}",
+                  "-c", str(src), "-o", str(obj)])
         else:
             _run([CXX] + CXXFLAGS + ["-c", str(src), "-o", str(obj)])
         _mark(obj, src, stamp)
@@ -172,7 +174,7 @@ def _build_locked(tools: bool, jobs: int | None, verbose: bool) -> Path:
         torch_objs = [j.result() for j in torch_jobs]
     if torch_objs and (not TORCH_LIB.exists() or TORCH_LIB.stat().st_mtime_ns < max(o.stat().st_mtime_ns for o in torch_objs + [LIB])):
         _link(TORCH_LIB, [CXX, "-shared"] + [str(o) for o in torch_objs] +
-              [f"-L{LIB.parent}", "-lal_b200", f"-L{torch_dir / 'lib'}", "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-lc10", "-lc10_cuda",
+              [f"-L{LIB.parent}", "-lal_b200", f"-L{torch_dir / 'lib'}", "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-ltorch_python", "-lc10", "-lc10_cuda",
                "-Wl,-rpath,$ORIGIN"])
     if tools:
         todo = {n: [ROOT / s for s in ss] for n, ss in TOOLS.items() if all((ROOT / s).exists() for s in ss)}

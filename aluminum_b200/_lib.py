@@ -131,6 +131,28 @@ def torch_ops():
     return _torch_ops
 
 
+_calls = None
+
+
+def calls():
+    """The native calls on tensors (``src/torch/comm_calls.hpp``, a Python module inside the operators' library), or None where
+    that library is not there or was built without Python's headers."""
+    global _calls
+    if _calls is None:
+        import importlib.machinery
+        import importlib.util
+        try:
+            torch_ops()
+            path = str(_LIB_PATH.with_name("libal_torch.so"))
+            loader = importlib.machinery.ExtensionFileLoader("al_torch", path)
+            module = importlib.util.module_from_spec(importlib.util.spec_from_file_location("al_torch", path, loader=loader))
+            module.set_error(AlError)
+            _calls = module
+        except (ImportError, OSError, RuntimeError):   # (not built here, and cannot be; no Python headers when it was built)
+            _calls = False
+    return _calls or None
+
+
 def check(rc: int) -> None:
     if rc != 0:
         raise AlError(load().al_last_error().decode(errors="replace"))

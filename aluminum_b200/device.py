@@ -26,6 +26,11 @@ def _dtype_code(dtype) -> int:
     return DTYPES[str(dtype).replace("torch.", "")]
 
 
+def _kept(*buffers):
+    """What an operation under way holds on to, whatever the caller does with its lists."""
+    return [list(b) if isinstance(b, list) else b for b in buffers]
+
+
 class _CudaBlob:
     """Exposes a raw device allocation through ``__cuda_array_interface__``."""
 
@@ -57,6 +62,7 @@ class DeviceComm:
         self.device_index = lib.al_dev_comm_device(self._h)
         self.emulated = self.nlocal > 1 or bool(emulate)
         self._symm = {}
+        self._calls = _lib.calls()
 
     @classmethod
     def from_ranks(cls, world_ranks, stream=None) -> "DeviceComm":
@@ -117,6 +123,8 @@ class DeviceComm:
 
     # ---- helpers ---------------------------------------------------------------------------
     def _stream(self, stream=None) -> C.c_void_p:
+        if stream is None and self._calls is not None:
+            return C.c_void_p(self._calls.current_stream())
         s = stream if stream is not None else self._torch.cuda.current_stream()
         return C.c_void_p(s.cuda_stream)
 
@@ -160,6 +168,13 @@ class DeviceComm:
 
     def _coll(self, kind, send, recv, count, op="sum", root=0, inplace=False, nonblocking=False, tables=None,
               wire_dtype=None, scale=1.0, algo="auto", ctas=0, stream=None):
+        if tables is None and self._calls is not None:
+            req = self._calls.collective(
+                self._h.value, self.nlocal, KINDS[kind], send, recv, int(count), _dtype_code(wire_dtype) if wire_dtype is not None else -1,
+                OPS[op], int(root), bool(inplace), float(scale), ALGOS[algo] if kind == "allreduce" else PATHS[algo], int(ctas),
+                None if stream is None else stream.cuda_stream, bool(nonblocking))
+            if req is not NotImplemented:
+                return Request(C.c_void_p(req), True, _kept(send, recv)) if nonblocking else None
         sends, recvs = self._as_list(send), self._as_list(recv)
         first_in = next((t for t in (sends if not inplace else recvs) if t is not None), None)
         first_out = next((t for t in recvs if t is not None), None)
@@ -246,6 +261,12 @@ class DeviceComm:
         ``send`` with ``id = send_first[d] + k`` (or ``send_idx[send_first[d] + k]`` when an int64 index tensor is
         given); row ``k`` received from rank ``r`` is written at ``recv_peer_off[r] + id * recv_row_stride`` of
         ``recv`` likewise.  Tables have one entry per rank (one row of entries per local rank in emulation)."""
+        if self._calls is not None:
+            req = self._calls.exchange_rows(self._h.value, self.nlocal, self.size, send, recv, int(row_bytes), int(send_row_stride),
+                                            int(recv_row_stride), send_rows, send_first, send_peer_off, recv_rows, recv_first, recv_peer_off,
+                                            send_idx, recv_idx, None if stream is None else stream.cuda_stream, bool(nonblocking))
+            if req is not NotImplemented:
+                return Request(C.c_void_p(req), True, _kept(send, recv, send_idx, recv_idx)) if nonblocking else None
         sends, recvs = self._as_list(send), self._as_list(recv)
         sidx = self._as_list(send_idx) if send_idx is not None else None
         ridx = self._as_list(recv_idx) if recv_idx is not None else None
@@ -318,6 +339,10 @@ class DeviceComm:
     # ---- point-to-point -----------------------------------------------------------------------
     def p2p(self, items, nonblocking=False, stream=None):
         """items: (is_send, peer, tensor[, owner]) tuples progressing together as one operation."""
+        if self._calls is not None:
+            req = self._calls.p2p(self._h.value, self.rank, items, None if stream is None else stream.cuda_stream, bool(nonblocking))
+            if req is not NotImplemented:
+                return Request(C.c_void_p(req), True, [it[2] for it in items]) if nonblocking else None
         n = len(items)
         is_send = (C.c_int * n)(*[1 if it[0] else 0 for it in items])
         peer = (C.c_int * n)(*[int(it[1]) for it in items])

@@ -31,3 +31,14 @@ def call(comm, fn, *lists, **kw):
     if comm.nlocal > 1:
         return fn(*lists, **kw)
     return fn(*[(l[0] if (isinstance(l, list) and len(l) == 1 and torch.is_tensor(l[0])) else l) for l in lists], **kw)
+
+
+def empties(comm, like, shapes):
+    """New tensors like those of ``like``; ``shapes`` is one shape (a tuple) for all or a list of shapes."""
+    if comm._calls is not None:
+        made = comm._calls.empties(like, shapes)
+        if made is not NotImplemented:
+            return made
+    if isinstance(shapes, tuple):
+        shapes = [shapes] * len(like)
+    return [torch.empty(s, device=t.device, dtype=t.dtype) for s, t in zip(shapes, like)]

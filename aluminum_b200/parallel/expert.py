@@ -14,7 +14,7 @@ import torch
 
 from .. import _lib
 from .._lib import AlError, check
-from ._util import call, unwrap, wrap
+from ._util import call, empties, unwrap, wrap
 
 
 def _prefix(counts):
@@ -68,7 +68,7 @@ def _route(comm, dests):
     both = torch.empty((2, n, p), device=dests[0].device, dtype=torch.int64)
     if max(sizes) * (p + 2) > _SORT_FROM * n:
         return [_sorted_route(d, p, c) for d, c in zip(dests, both[0].unbind())], both
-    order = [torch.empty_like(d) for d in dests]
+    order = empties(comm, dests, [(s,) for s in sizes])
     check(_lib.load().al_route_rows(comm._h, n, (C.c_void_p * n)(*[d.data_ptr() for d in dests]), (C.c_size_t * n)(*sizes),
                                     (C.c_void_p * n)(*[o.data_ptr() for o in order]), both.data_ptr(), comm._stream()))
     return order, both
@@ -86,13 +86,17 @@ def dispatch(comm, tokens, dest_rank):
         if d.numel() > t.shape[0]:
             raise ValueError("dispatch: dest_rank has more entries than there are tokens")
     order, both = _route(comm, dests)
-    call(comm, comm.alltoall, list(both[0].unbind()), list(both[1].unbind()))
-    sc, rc = both.tolist()   # the one host read
+    if comm.nlocal == p:     # every rank's counts are here
+        sc = both[0].tolist()
+        rc = [list(col) for col in zip(*sc)]
+    else:
+        call(comm, comm.alltoall, list(both[0].unbind()), list(both[1].unbind()))
+        sc, rc = both.tolist()   # the one host read
     if any(c < 0 for row in sc + rc for c in row):
         raise ValueError(f"dest_rank: every destination must be a rank from 0 to {p - 1}")
     width = toks[0].shape[1]
     rb = width * toks[0].element_size()
-    outs = [torch.empty((sum(r), width), device=toks[0].device, dtype=toks[0].dtype) for r in rc]
+    outs = empties(comm, [toks[0]] * len(rc), [(sum(r), width) for r in rc])
     one = comm.nlocal == 1
     zeros = [[0] * p for _ in sc]
     sf = [_prefix(r) for r in sc]
@@ -113,7 +117,7 @@ def combine(comm, expert_out, state):
     one = comm.nlocal == 1
     # directions swap: what was received is sent back, and lands through the sort permutation
     sc, sf, rc, rf = state["rc"], state["rf"], state["sc"], state["sf"]
-    back = [torch.empty((sum(r), width), device=outs_in[0].device, dtype=outs_in[0].dtype) for r in rc]
+    back = empties(comm, [outs_in[0]] * len(rc), [(sum(r), width) for r in rc])
     zeros = [[0] * p for _ in sc]
     pick = (lambda t: t[0]) if one else (lambda t: t)
     comm.exchange_rows(pick(outs_in), pick(back), rb, rb, rb, pick(sc), pick(sf), pick(zeros), pick(rc), pick(rf),

@@ -9,9 +9,7 @@ per process: :func:`aluminum_b200.parallel.autograd.seq_to_head` / ``head_to_seq
 """
 from __future__ import annotations
 
-import torch
-
-from ._util import unwrap, wrap
+from ._util import empties, unwrap, wrap
 
 
 def _tables(comm, rows, first, off):
@@ -26,7 +24,7 @@ def seq_to_head(comm, x):
     s, h, d = xs[0].shape
     esz = xs[0].element_size()
     rb = (h // p) * d * esz
-    outs = [torch.empty((s * p, h // p, d), device=t.device, dtype=t.dtype) for t in xs]
+    outs = empties(comm, xs, (s * p, h // p, d))
     sr, sf, so = _tables(comm, [s] * p, [0] * p, [j * rb for j in range(p)])
     rr, rf, ro = _tables(comm, [s] * p, [j * s for j in range(p)], [0] * p)
     one = comm.nlocal == 1
@@ -41,7 +39,7 @@ def head_to_seq(comm, x):
     s, hl, d = xs[0].shape
     esz = xs[0].element_size()
     rb = hl * d * esz
-    outs = [torch.empty((s // p, hl * p, d), device=t.device, dtype=t.dtype) for t in xs]
+    outs = empties(comm, xs, (s // p, hl * p, d))
     sr, sf, so = _tables(comm, [s // p] * p, [j * (s // p) for j in range(p)], [0] * p)
     rr, rf, ro = _tables(comm, [s // p] * p, [0] * p, [j * rb for j in range(p)])
     one = comm.nlocal == 1

@@ -9,6 +9,7 @@
 
 #include "al/al_c.h"
 #include "al/base.hpp"
+#include "comm_calls.hpp"
 
 namespace {
 
