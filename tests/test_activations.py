@@ -226,3 +226,25 @@ def test_stopped_infinite_gradient_in_a_graph_of_the_backward():
     g, = torch.autograd.grad(y, x, dy, retain_graph=True)
     h, = torch.autograd.grad(y, x, dy, create_graph=True)
     assert torch.isfinite(g).all() and rel(h.detach(), g.double()) < 1e-2
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("h,w", [(1, 1), (1, 2), (2, 1), (3, 3), (2, 7), (8, 9), (15, 16)])
+def test_pooling_by_three_every_two(h, w, dtype):
+    """Windows cut by every border, with equal values, both zeros, infinities and NaN among them: value and place of the module's winner."""
+    cl = dict(memory_format=torch.channels_last)
+    pool = nn.MaxPool2d(3, 2, 1)
+    g = torch.Generator(device="cuda").manual_seed(h * 20 + w)
+    special = torch.tensor([0.0, -0.0, 1.0, -1.0, 2.0, float("inf"), -float("inf"), -float("inf"), float("nan"), -3.0], device="cuda")
+    for most in (5, 8, 10):   # without infinities and NaN, without NaN, with all
+        x = special[torch.randint(0, most, (3, 16, h, w), generator=g, device="cuda")].to(dtype).contiguous(**cl).requires_grad_()
+        y = max_pool(pool, x)
+        assert "MaxPool" in y.grad_fn.name() and "MaxPool2D" not in y.grad_fn.name()
+        xr = x.detach().float().contiguous().requires_grad_()
+        want = pool(xr)
+        assert torch.equal(y.float().nan_to_num(nan=99.0), want.nan_to_num(nan=99.0))
+        dy = torch.randint(-3, 4, want.shape, generator=g, device="cuda").to(dtype)
+        y.backward(dy)
+        want.backward(dy.float())
+        assert torch.equal(x.grad.float(), xr.grad)
