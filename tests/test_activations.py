@@ -229,6 +229,29 @@ def test_stopped_infinite_gradient_in_a_graph_of_the_backward():
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("rows,channels", [(2, 8), (3, 64), (33, 264), (129, 2048), (1025, 520), (592 * 128 + 5, 64), (592 * 128 - 1, 72)])
+@pytest.mark.parametrize("offset", [0.0, 64.0])
+def test_statistics_at_the_edges_of_tiles_and_partials(rows, channels, offset):
+    """One row more or less than threads, tiles and CTAs have; means far from 0.  With a momentum of 1 the running statistics are the batch's."""
+    from aluminum_b200.ops import batch_norm_act
+    torch.manual_seed(rows)
+    x = (torch.randn(1, channels, rows, 1, device="cuda") + offset).bfloat16().contiguous(memory_format=torch.channels_last)
+    x[0, :, 0] += 3   # where the sums begin
+    bn = nn.BatchNorm2d(channels, momentum=1.0).cuda()
+    x.requires_grad_()
+    y = batch_norm_act(bn, x, nn.ReLU())
+    assert "BatchNormAct" in y.grad_fn.name()
+    v = x.detach().double()[0, :, :, 0]
+    mean, var = v.mean(1), v.var(1)
+    # fp32 sums of deviations: a few roundings of the deviations' size, and one of the mean's
+    assert ((bn.running_mean - mean).abs() <= 2e-6 * (var.sqrt() + 1) + 1.2e-7 * mean.abs()).all()
+    assert ((bn.running_var - var).abs() <= 5e-6 * var + 1e-12).all()
+    y.backward(torch.ones_like(y))
+    passes = (y.detach() > 0).double()[0, :, :, 0]
+    assert ((bn.bias.grad - passes.sum(1)).abs() <= 1e-6 * rows).all()
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("h,w", [(1, 1), (1, 2), (2, 1), (3, 3), (2, 7), (8, 9), (15, 16)])
 def test_pooling_by_three_every_two(h, w, dtype):
