@@ -12,6 +12,7 @@ import torch
 from torch import nn
 
 from ..ops.activations import batch_norm_act, max_pool
+from ..ops.convolution import stem_conv
 
 
 class Bottleneck(nn.Module):
@@ -95,7 +96,7 @@ class ResNet(nn.Module):
         if torch.jit.is_scripting():
             x = self.maxpool(self.relu(self.bn1(self.conv1(x))))
         else:
-            x = max_pool(self.maxpool, batch_norm_act(self.bn1, self.conv1(x), self.relu))
+            x = max_pool(self.maxpool, batch_norm_act(self.bn1, stem_conv(self.conv1, x), self.relu))
         x = self.layer4(self.layer3(self.layer2(self.layer1(x))))
         return self.fc(torch.flatten(self.avgpool(x), 1))
 

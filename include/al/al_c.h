@@ -212,6 +212,12 @@ int al_bn_backward(int dt, const void* x, const void* dy, const unsigned char* m
 /* Max pooling, channels-last; shape: n, h, w, c, out h, out w, window, stride, padding.  place: one byte per output element. */
 int al_maxpool_forward(int dt, const void* x, void* y, unsigned char* place, const int* shape, void* stream);
 int al_maxpool_backward(int dt, const void* dy, const unsigned char* place, void* dx, const int* shape, void* stream);
+/* First convolution (7 x 7, stride 2, border 3, three channels): images and weight laid out as 64 channels over 4 x 1 taps, and the packed
+ * weight's gradient back.  shape: n, h, w, out h, out w, out channels; strides in elements: n, channel, row, column of the images, then out
+ * channel, channel, row, column of the weight. */
+int al_stem_gather(int in_dt, const void* x, int dt, void* out, const float* weight, void* packed, const int* shape, const long long* strides,
+                   void* stream);
+int al_stem_scatter(int dt, const void* packed, float* grad, const int* shape, const long long* strides, void* stream);
 
 #ifdef __cplusplus
 }

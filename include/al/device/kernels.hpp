@@ -200,6 +200,16 @@ struct PoolShape {
 };
 void launch_maxpool_forward(const void* x, void* y, unsigned char* place, const PoolShape& s, DType dt, cudaStream_t stream);
 void launch_maxpool_backward(const void* dy, const unsigned char* place, void* dx, const PoolShape& s, DType dt, cudaStream_t stream);
+/**
+ * First convolution of a network (7 x 7, stride 2, border 3, three channels; kernels/stem.cu): the images, any strides, as
+ * (n, oh + 3, ow, 64) pixels for a convolution of 64 channels over 4 x 1 taps, the weight as (oc, 4, 64), and its gradient back.
+ */
+struct StemShape {
+  int n, h, w, oh, ow, oc;
+  long long xs[4], ws[4];   // strides, in elements, of the images and of the weight (n or oc, channel, row, column)
+};
+void launch_stem_gather(const StemShape& s, const void* x, DType in, void* out, const float* weight, void* packed, DType dt, cudaStream_t stream);
+void launch_stem_scatter(const StemShape& s, const void* packed, float* grad, DType dt, cudaStream_t stream);
 /** Fill with a 32-bit pattern (used by tests and benchmarks to flush L2). */
 void launch_fill_u32(uint32_t* out, size_t n, uint32_t value, cudaStream_t stream);
 

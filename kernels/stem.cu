@@ -1,0 +1,113 @@
+// Input of a network's first convolution (7 x 7 every two pixels, border 3, three channels) laid out for tensor cores, and the weight's
+// gradient back in the weight's layout.
+//
+// The library convolves three channels on its legacy tensor path alone, with an input that it pads to four or eight
+// channels first: 256 x 3 x 224 x 224 bf16 takes 1600 us forward and 911 us for the weight's gradient, of which memory would be 75 and 65.
+// Here the pixels that a row of outputs sees are put side by side as channels: 8 columns x 3 channels of two input rows
+// (48 channels, and 16 of zeros) make one pixel, and the convolution becomes one of 64 channels over four rows, which takes 261 and
+// 168 us.  (48 channels 335 / 179, two by two pixels as 16 channels and 4 x 4 taps 516 / 588, the seven rows on their own 273 / 326.)
+//
+// What bounds the layout kernel is writing 128 bytes per pixel (422 MB in that case).  A CTA has two input rows: it reads each once,
+// converts them into shared memory with their borders, and its threads write 16 bytes of a pixel each, eight to a pixel.
+#include "al/cuda/cuda.hpp"
+#include "al/device/kernels.hpp"
+#include "datamove.cuh"
+
+namespace Al {
+namespace internal {
+namespace device {
+
+namespace {
+
+constexpr int kThreads = 256;
+constexpr int kSeen = 8, kIn = 3, kCh = 64;   // columns that an output sees (one more than it has taps), channels of an image, of a pixel here
+constexpr int kRow = kSeen * kIn;             // values of one input row
+
+template <typename Ti, typename To>
+__global__ void __launch_bounds__(kThreads) stem_gather_kernel(const __grid_constant__ StemShape s, const Ti* __restrict__ x, To* __restrict__ out,
+                                                               const float* __restrict__ weight, To* __restrict__ packed, unsigned rows) {
+  auto as = [](Ti v) { return Elem<To>::down((float)Elem<Ti>::up(v)); };
+  const To zero = Elem<To>::down(0.f);
+  if (blockIdx.x >= rows) {   // the weight: [output][row pair][channel], zero where there is no tap
+    const unsigned i = (blockIdx.x - rows) * kThreads + threadIdx.x;
+    if (i >= (unsigned)s.oc * 4 * kCh) return;
+    const int c = (int)(i % kCh), a = (int)(i / kCh) % 4, o = (int)(i / (4 * kCh));
+    const int u = 2 * a + c / kRow, v = c % kRow / kIn, ch = c % kIn;
+    packed[i] = c < 2 * kRow && u < 7 && v < 7 ? Elem<To>::down(weight[o * s.ws[0] + ch * s.ws[1] + u * s.ws[2] + v * s.ws[3]]) : zero;
+    return;
+  }
+  extern __shared__ uint32_t smem[];   // two rows of (columns + border) x 3 values
+  const int cols = 2 * s.ow + 6, n = (int)(blockIdx.x / (unsigned)(s.oh + 3)), r = (int)(blockIdx.x % (unsigned)(s.oh + 3));
+  To* rowbuf = (To*)smem;
+  const Ti* image = x + (ptrdiff_t)n * s.xs[0];
+  for (int by = 0; by < 2; ++by) {
+    const int h = 2 * r + by - 3;
+    const bool in = h >= 0 && h < s.h;
+    const Ti* line = image + (ptrdiff_t)h * s.xs[2];
+    for (int i = threadIdx.x; i < cols * kIn; i += kThreads) {
+      // neighbours in memory go to neighbouring threads, whichever way the image is laid out
+      const int ch = s.xs[1] == 1 ? i % kIn : i / cols, pc = s.xs[1] == 1 ? i / kIn : i % cols, w = pc - 3;
+      rowbuf[(by * cols + pc) * kIn + ch] = in && w >= 0 && w < s.w ? as(line[(ptrdiff_t)w * s.xs[3] + ch * s.xs[1]]) : zero;
+    }
+  }
+  __syncthreads();
+  // a pixel's 24 values of a row begin 6 values behind its neighbour's: on 4 bytes, not on 16
+  uint4* dst = (uint4*)out + (size_t)blockIdx.x * s.ow * (kCh / 8);
+  for (int i = threadIdx.x; i < s.ow * (kCh / 8); i += kThreads) {
+    const int j = i / (kCh / 8), k = i % (kCh / 8);
+    uint4 v = uint4{0, 0, 0, 0};
+    if (k < 6) {
+      const uint32_t* p = smem + (((k / 3) * cols + 2 * j) * kIn + (k % 3) * 8) / 2;
+      v = uint4{p[0], p[1], p[2], p[3]};
+    }
+    dst[i] = v;
+  }
+}
+
+/** grad[o][ch][u][v] out of the gradient of the packed weight. */
+template <typename T>
+__global__ void __launch_bounds__(kThreads) stem_scatter_kernel(const __grid_constant__ StemShape s, const T* __restrict__ packed, float* __restrict__ grad) {
+  const unsigned i = blockIdx.x * kThreads + threadIdx.x;
+  if (i >= (unsigned)s.oc * kIn * 49) return;
+  const int v = (int)(i % 7), u = (int)(i / 7) % 7, ch = (int)(i / 49) % kIn, o = (int)(i / (49 * kIn));
+  grad[o * s.ws[0] + ch * s.ws[1] + u * s.ws[2] + v * s.ws[3]] = (float)Elem<T>::up(packed[(o * 4 + u / 2) * kCh + u % 2 * kRow + v * kIn + ch]);
+}
+
+void check(const StemShape& s) {
+  if (s.n < 1 || s.h < 1 || s.w < 1 || s.oc < 1 || s.oh != (s.h - 1) / 2 + 1 || s.ow != (s.w - 1) / 2 + 1 || s.w > 4000 ||
+      (size_t)s.n * (size_t)(s.oh + 3) > 0x70000000u || s.oc > 1 << 16)
+    throw_al_exception("first convolution: unsupported shape");
+}
+
+template <typename Ti, typename To>
+void gather(const StemShape& s, const void* x, void* out, const float* weight, void* packed, cudaStream_t stream) {
+  const unsigned rows = (unsigned)(s.n * (s.oh + 3)), more = (unsigned)((s.oc * 4 * kCh + kThreads - 1) / kThreads);
+  const size_t smem = (size_t)2 * (2 * s.ow + 6) * kIn * sizeof(To);   // (a whole number of 4-byte words: a row is 6 (ow + 3) values)
+  stem_gather_kernel<Ti, To><<<rows + more, kThreads, smem, stream>>>(s, (const Ti*)x, (To*)out, weight, (To*)packed, rows);
+  AL_CHECK_CUDA(cudaGetLastError());
+}
+
+}  // namespace
+
+void launch_stem_gather(const StemShape& s, const void* x, DType in, void* out, const float* weight, void* packed, DType dt, cudaStream_t stream) {
+  using bf = __nv_bfloat16;
+  check(s);
+  if (in == DType::f32 && dt == DType::bf16) return gather<float, bf>(s, x, out, weight, packed, stream);
+  if (in == DType::f32 && dt == DType::f16) return gather<float, __half>(s, x, out, weight, packed, stream);
+  if (in == DType::bf16 && dt == DType::bf16) return gather<bf, bf>(s, x, out, weight, packed, stream);
+  if (in == DType::f16 && dt == DType::f16) return gather<__half, __half>(s, x, out, weight, packed, stream);
+  throw_al_exception("first convolution: unsupported datatypes ", dtype_name(in), ", ", dtype_name(dt));
+}
+
+void launch_stem_scatter(const StemShape& s, const void* packed, float* grad, DType dt, cudaStream_t stream) {
+  check(s);
+  const unsigned blocks = (unsigned)((s.oc * kIn * 49 + kThreads - 1) / kThreads);
+  if (dt == DType::bf16) stem_scatter_kernel<__nv_bfloat16><<<blocks, kThreads, 0, stream>>>(s, (const __nv_bfloat16*)packed, grad);
+  else if (dt == DType::f16) stem_scatter_kernel<__half><<<blocks, kThreads, 0, stream>>>(s, (const __half*)packed, grad);
+  else throw_al_exception("first convolution: unsupported datatype ", dtype_name(dt));
+  AL_CHECK_CUDA(cudaGetLastError());
+}
+
+}  // namespace device
+}  // namespace internal
+}  // namespace Al

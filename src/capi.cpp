@@ -681,4 +681,15 @@ int al_maxpool_backward(int dt, const void* dy, const unsigned char* place, void
   return guard([&] { device::launch_maxpool_backward(dy, place, dx, pool_shape(shape), (DType)dt, (cudaStream_t)stream); });
 }
 
+static device::StemShape stem_shape(const int* s, const long long* t) {
+  return {s[0], s[1], s[2], s[3], s[4], s[5], {t[0], t[1], t[2], t[3]}, {t[4], t[5], t[6], t[7]}};
+}
+int al_stem_gather(int in_dt, const void* x, int dt, void* out, const float* weight, void* packed, const int* shape, const long long* strides,
+                   void* stream) {
+  return guard([&] { device::launch_stem_gather(stem_shape(shape, strides), x, (DType)in_dt, out, weight, packed, (DType)dt, (cudaStream_t)stream); });
+}
+int al_stem_scatter(int dt, const void* packed, float* grad, const int* shape, const long long* strides, void* stream) {
+  return guard([&] { device::launch_stem_scatter(stem_shape(shape, strides), packed, grad, (DType)dt, (cudaStream_t)stream); });
+}
+
 }  // extern "C"

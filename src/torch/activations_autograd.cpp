@@ -1,4 +1,5 @@
-// Autograd of the fused batch norm (kernels/batchnorm.cu) and of max pooling (kernels/maxpool.cu) for PyTorch, in native code: a small network's step is bound by
+// Autograd of the fused batch norm (kernels/batchnorm.cu), of max pooling (kernels/maxpool.cu) and of a network's first convolution
+// (kernels/stem.cu) for PyTorch, in native code: a small network's step is bound by
 // the host, and 53 layers of a Python autograd function cost it 2 ms more than the three framework operations each
 // replaces.  Registered under torch.ops.aluminum_b200; aluminum_b200/ops/activations.py decides when they are called.
 #include <ATen/ATen.h>
@@ -167,11 +168,70 @@ struct MaxPool : public torch::autograd::Function<MaxPool> {
 
 Tensor max_pool(const Tensor& x, int64_t k, int64_t stride, int64_t pad) { return MaxPool::apply(x, k, stride, pad); }
 
+/**
+ * First convolution: images of three channels laid out as 64 channels (kernels/stem.cu) and convolved by the library over 4 x 1 taps.
+ * No gradient of the images (ops/convolution.py sends what wants one to the module).
+ */
+struct StemConv : public torch::autograd::Function<StemConv> {
+  struct Shape {
+    std::array<int, 6> sizes;
+    std::array<long long, 8> strides;
+    Shape(at::IntArrayRef x, at::IntArrayRef x_strides, const Tensor& weight)
+        : sizes{(int)x[0], (int)x[2], (int)x[3], (int)((x[2] - 1) / 2 + 1), (int)((x[3] - 1) / 2 + 1), (int)weight.size(0)} {
+      for (int i = 0; i < 4; ++i) {
+        strides[i] = x_strides[i];
+        strides[4 + i] = weight.stride(i);
+      }
+    }
+  };
+
+  static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& weight, at::ScalarType type) {
+    const c10::cuda::CUDAGuard guard(x.device());
+    const Shape s(x.sizes(), x.strides(), weight);
+    const int64_t oc = weight.size(0);
+    Tensor seen = at::empty({s.sizes[0], 64, s.sizes[3] + 3, s.sizes[4]}, x.options().dtype(type), at::MemoryFormat::ChannelsLast);
+    Tensor packed = at::empty({oc, 64, 4, 1}, seen.options(), at::MemoryFormat::ChannelsLast);
+    const int in = x.scalar_type() == at::kFloat ? (int)Al::DType::f32 : type_code(x);
+    TORCH_CHECK(al_stem_gather(in, x.data_ptr(), type_code(seen), seen.data_ptr(), weight.data_ptr<float>(), packed.data_ptr(), s.sizes.data(),
+                               s.strides.data(), c10::cuda::getCurrentCUDAStream().stream()) == 0,
+                al_last_error());
+    ctx->save_for_backward({seen, packed});
+    ctx->saved_data["strides"] = weight.strides().vec();
+    return at::conv2d(seen, packed);
+  }
+
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    variable_list out(3);
+    if (!grads[0].defined()) return out;
+    const variable_list saved = ctx->get_saved_variables();
+    const Tensor &seen = saved[0], &packed = saved[1], &dy = grads[0];
+    const c10::cuda::CUDAGuard guard(dy.device());
+    const int64_t oc = packed.size(0);
+    Tensor g = std::get<1>(at::convolution_backward(dy, seen, packed, at::OptionalIntArrayRef(), {1, 1}, {0, 0}, {1, 1}, false, {0, 0}, 1, {false, true, false}));
+    if (at::GradMode::is_enabled()) {   // a graph of the backward is wanted: channel = (row of the pair, column, image channel), zeros behind
+      g = g.squeeze(3).slice(1, 0, 48).reshape({oc, 2, 8, 3, 4}).permute({0, 3, 4, 1, 2}).reshape({oc, 3, 8, 8});
+      out[1] = g.slice(2, 0, 7).slice(3, 0, 7).to(at::kFloat);
+      return out;
+    }
+    g = restored(g, {oc, 64, 4, 1}, seen.scalar_type(), dy, at::MemoryFormat::ChannelsLast);
+    Tensor grad = at::empty_strided({oc, 3, 7, 7}, ctx->saved_data["strides"].toIntVector(), g.options().dtype(at::kFloat));
+    const Shape s({seen.size(0), 3, 2 * (seen.size(2) - 3), 2 * seen.size(3)}, {0, 0, 0, 0}, grad);
+    TORCH_CHECK(al_stem_scatter(type_code(g), g.data_ptr(), grad.data_ptr<float>(), s.sizes.data(), s.strides.data(),
+                                c10::cuda::getCurrentCUDAStream().stream()) == 0,
+                al_last_error());
+    out[1] = grad;
+    return out;
+  }
+};
+
+Tensor stem_conv(const Tensor& x, const Tensor& weight, at::ScalarType type) { return StemConv::apply(x, weight, type); }
+
 }  // namespace
 
 TORCH_LIBRARY(aluminum_b200, m) {
   m.def("batch_norm_act(Tensor x, Tensor weight, Tensor bias, Tensor? residual, Tensor(a!) running_mean, Tensor(b!) running_var, "
         "Tensor(c!)? batches, float momentum, float eps, bool relu) -> Tensor",
         batch_norm_act);
+  m.def("stem_conv(Tensor x, Tensor weight, ScalarType type) -> Tensor", stem_conv);
   m.def("max_pool(Tensor x, int k, int stride, int pad) -> Tensor", max_pool);
 }

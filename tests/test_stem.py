@@ -1,0 +1,100 @@
+"""First convolution laid out for tensor cores against the module, and the calls that must still go through it."""
+import copy
+
+import pytest
+import torch
+from torch import nn
+
+from aluminum_b200.ops import stem_conv
+
+
+def stem(out=64, **kw):
+    return nn.Conv2d(3, out, 7, stride=2, padding=3, bias=False, **kw)
+
+
+def test_on_the_cpu_it_is_the_module():
+    conv, x = stem(8), torch.randn(2, 3, 9, 12)
+    assert torch.equal(stem_conv(conv, x), conv(x))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("shape", [(1, 1, 1), (2, 2, 3), (1, 7, 7), (3, 9, 12), (2, 33, 30), (2, 64, 225), (4, 224, 224)])
+@pytest.mark.parametrize("layout", ["rows", "channels_last", "part", "halves"])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_against_64_bits(shape, layout, dtype):
+    n, h, w = shape
+    torch.manual_seed(h)
+    x = torch.randn(n, 3, h, w, device="cuda")
+    if layout == "channels_last":
+        x = x.contiguous(memory_format=torch.channels_last)
+    elif layout == "part":
+        x = torch.randn(n, 4, h + 2, 2 * w + 1, device="cuda")[:, 1:, 1:h + 1, 1::2]
+    elif layout == "halves":
+        x = x.to(dtype)
+    conv = stem(16 if h < 60 else 64).cuda()
+    if layout != "rows":
+        conv = conv.to(memory_format=torch.channels_last)
+    with torch.autocast("cuda", dtype=dtype):
+        y = stem_conv(conv, x)
+    assert "StemConv" in y.grad_fn.name() and y.dtype == dtype and y.is_contiguous(memory_format=torch.channels_last)
+    ref = copy.deepcopy(conv).double()
+    with torch.no_grad():
+        ref.weight.copy_(conv.weight.to(dtype).double())     # what either way multiplies
+    want = ref(x.to(dtype).double())
+    dy = torch.randn(want.shape, device="cuda").to(dtype)
+    y.backward(dy)
+    want.backward(dy.double())
+    # one rounding of the result to 8 (bf16) or 11 bits, and fp32 sums
+    eps = 2 ** -8 if dtype == torch.bfloat16 else 2 ** -11
+    for got, exact in ((y, want), (conv.weight.grad, ref.weight.grad)):
+        assert (got.double() - exact).norm() <= 0.6 * eps * exact.norm() + 1e-6 * exact.norm() and got.shape == exact.shape
+    assert conv.weight.grad.stride() == conv.weight.stride()
+
+
+@pytest.mark.gpu
+def test_second_derivative_and_a_weight_that_changes_before_the_backward():
+    x, conv = torch.randn(2, 3, 18, 20, device="cuda"), stem(8).cuda()
+    with torch.autocast("cuda", dtype=torch.bfloat16):
+        a, b = stem_conv(conv, x), conv(x)
+    ga, = torch.autograd.grad((a.float() ** 2).sum(), conv.weight, create_graph=True)
+    gb, = torch.autograd.grad((b.float() ** 2).sum(), conv.weight, create_graph=True)
+    assert torch.allclose(ga, gb, rtol=2e-2, atol=2e-2 * gb.abs().max().item())
+    sa, sb = (torch.autograd.grad(g.square().sum(), conv.weight)[0] for g in (ga, gb))
+    assert (sa - sb).norm() <= 3e-2 * sb.norm()
+    with torch.autocast("cuda", dtype=torch.bfloat16):
+        y = stem_conv(conv, x)
+    with torch.no_grad():
+        conv.weight.add_(1)
+    y.sum().backward()
+    assert conv.weight.grad.isfinite().all()
+
+
+@pytest.mark.gpu
+def test_calls_that_stay_with_the_module():
+    x, conv = torch.randn(2, 3, 20, 20, device="cuda"), stem(16).cuda()
+
+    def taken(conv, x, dtype=torch.bfloat16):
+        with torch.autocast("cuda", dtype=dtype):
+            y, want = stem_conv(conv, x), conv(x)
+        if y.grad_fn is not None and "StemConv" in y.grad_fn.name():
+            return True
+        assert torch.equal(y, want)
+        return False
+    assert taken(conv, x)
+    assert not taken(conv, x.clone().requires_grad_())
+    assert not taken(conv.eval(), x)
+    conv.train()
+    with torch.no_grad():
+        assert not taken(conv, x)
+    with torch.inference_mode():
+        assert not taken(conv, x)
+    assert torch.equal(stem_conv(conv, x), conv(x)) and "StemConv" not in stem_conv(conv, x).grad_fn.name()   # no autocast
+    assert not taken(conv, x.half())                                   # of another type than autocast's
+    for other in (nn.Conv2d(3, 16, 7, stride=2, padding=3), nn.Conv2d(3, 16, 7, stride=2, padding=2, bias=False), nn.Conv2d(3, 16, 5, stride=2, padding=3, bias=False),
+                  nn.Conv2d(3, 16, 7, padding=3, bias=False), stem(12), stem(16, padding_mode="circular"), stem(16).requires_grad_(False)):
+        assert not taken(other.cuda(), x)
+    hooked = stem(16).cuda()
+    hooked.register_forward_hook(lambda m, i, o: o * 2)
+    assert not taken(hooked, x)
+    compiled = torch.compile(lambda c, v: stem_conv(c, v), backend="eager", fullgraph=True)
+    assert compiled(conv, x).shape == (2, 16, 10, 10)
