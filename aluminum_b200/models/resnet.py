@@ -11,7 +11,7 @@ from __future__ import annotations
 import torch
 from torch import nn
 
-from ..ops.activations import batch_norm_act, max_pool
+from ..ops.activations import _bare, _modes_off, batch_norm_act, batch_norm_act_twice, max_pool
 from ..ops.convolution import stem_conv
 
 
@@ -42,6 +42,13 @@ class Bottleneck(nn.Module):
             out = batch_norm_act(self.bn1, self.conv1(x), self.relu)
             out = batch_norm_act(self.bn2, self.conv2(out), self.relu)
             return batch_norm_act(self.bn3, self.conv3(out), self.relu, identity)
+
+    def twice(self, x, same):
+        """forward(x) as two tensors, for the next block's first convolution and for its end; ``same`` is x, for the end of this one."""
+        identity = same if self.downsample is None else self.downsample(same)
+        out = batch_norm_act(self.bn1, self.conv1(x), self.relu)
+        out = batch_norm_act(self.bn2, self.conv2(out), self.relu)
+        return batch_norm_act_twice(self.bn3, self.conv3(out), self.relu, identity)
 
 
 class Shortcut(nn.Sequential):
@@ -92,12 +99,30 @@ class ResNet(nn.Module):
         mods += [Bottleneck(self.c, width) for _ in range(1, blocks)]
         return nn.Sequential(*mods)
 
+    @torch.jit.unused
+    def _blocks(self, x):
+        """The four stages; in training block by block, each handing its output to the next one twice, so that the two gradients are
+        added inside the batch norm's backward."""
+        stages = (self.layer1, self.layer2, self.layer3, self.layer4)
+        if _modes_off() and self.training and all(type(s) is nn.Sequential and _bare(s) and all(type(b) is Bottleneck and _bare(b) for b in s) for s in stages):
+            same = x
+            for stage in stages:
+                for block in stage:
+                    x, same = block.twice(x, same)
+            return x
+        for stage in stages:
+            x = stage(x)
+        return x
+
     def forward(self, x):
         if torch.jit.is_scripting():
             x = self.maxpool(self.relu(self.bn1(self.conv1(x))))
         else:
             x = max_pool(self.maxpool, batch_norm_act(self.bn1, stem_conv(self.conv1, x), self.relu))
-        x = self.layer4(self.layer3(self.layer2(self.layer1(x))))
+        if torch.jit.is_scripting():
+            x = self.layer4(self.layer3(self.layer2(self.layer1(x))))
+        else:
+            x = self._blocks(x)
         return self.fc(torch.flatten(self.avgpool(x), 1))
 
 

@@ -61,18 +61,36 @@ def _tensors(bn: nn.Module, x):
     return None
 
 
-def batch_norm_act(bn: nn.Module, x: torch.Tensor, relu: nn.Module | None = None, residual: torch.Tensor | None = None) -> torch.Tensor:
-    """``relu(bn(x) + residual)``; without ``relu`` or ``residual`` the same without that part."""
+def _fused(bn: nn.Module, x, relu, residual):
+    """The arguments of the fused operators, or None where the modules are called."""
     found = _tensors(bn, x)
     if (found is not None and (relu is None or (type(relu) is nn.ReLU and _bare(relu)))
             and (residual is None or (_activation_ok(residual) and residual.shape == x.shape and residual.dtype == x.dtype
                                       and residual.get_device() == x.get_device()))):
         weight, bias, mean, var, count = found
-        return _lib.torch_ops().batch_norm_act.default(x, weight, bias, residual, mean, var, count, bn.momentum, bn.eps, relu is not None)
+        return x, weight, bias, residual, mean, var, count, bn.momentum, bn.eps, relu is not None
+    return None
+
+
+def batch_norm_act(bn: nn.Module, x: torch.Tensor, relu: nn.Module | None = None, residual: torch.Tensor | None = None) -> torch.Tensor:
+    """``relu(bn(x) + residual)``; without ``relu`` or ``residual`` the same without that part."""
+    args = _fused(bn, x, relu, residual)
+    if args is not None:
+        return _lib.torch_ops().batch_norm_act.default(*args)
     y = bn(x)
     if residual is not None:
         y = y + residual
     return y if relu is None else relu(y)
+
+
+def batch_norm_act_twice(bn: nn.Module, x: torch.Tensor, relu: nn.Module | None = None, residual: torch.Tensor | None = None):
+    """:func:`batch_norm_act` for a result that is used in two places, as two tensors (on the same memory where the kernels run): the
+    backward then adds their two gradients where it reads them."""
+    args = _fused(bn, x, relu, residual)
+    if args is not None:
+        return _lib.torch_ops().batch_norm_act_twice.default(*args)
+    y = batch_norm_act(bn, x, relu, residual)
+    return y, y
 
 
 def _one(v) -> int:

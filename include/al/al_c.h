@@ -209,6 +209,10 @@ int al_bn_forward(int dt, const void* x, const void* residual, void* y, unsigned
 int al_bn_backward(int dt, const void* x, const void* dy, const unsigned char* mask, void* dx, void* dres, const float* weight,
                    const float* save_mean, const float* save_invstd, float* grad_weight, float* grad_bias, void* workspace,
                    size_t workspace_bytes, size_t rows, int channels, void* stream);
+/* The same for an output that was used twice: dy + dy2 is the gradient, and its part that passes the ReLU is left in sum (the residual's gradient). */
+int al_bn_backward_sum(int dt, const void* x, const void* dy, const void* dy2, const unsigned char* mask, void* dx, void* sum, const float* weight,
+                       const float* save_mean, const float* save_invstd, float* grad_weight, float* grad_bias, void* workspace,
+                       size_t workspace_bytes, size_t rows, int channels, void* stream);
 /* Max pooling, channels-last; shape: n, h, w, c, out h, out w, window, stride, padding.  place: one byte per output element. */
 int al_maxpool_forward(int dt, const void* x, void* y, unsigned char* place, const int* shape, void* stream);
 int al_maxpool_backward(int dt, const void* dy, const unsigned char* place, void* dx, const int* shape, void* stream);

@@ -180,7 +180,7 @@ struct BnForward {
   float momentum, eps;
 };
 struct BnBackward {
-  const void *x, *dy;
+  const void *x, *dy, *dy2;   ///< dy2 (or null): a second gradient to be added; dres is needed then and gets their sum behind the ReLU
   const unsigned char* mask;
   void *dx, *dres;
   const float *weight, *save_mean, *save_invstd;

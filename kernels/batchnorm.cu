@@ -344,11 +344,16 @@ __global__ void __launch_bounds__(kBnThreads, kBnPerSm)
 // ---------------------------------------------------------------------------
 // backward
 // ---------------------------------------------------------------------------
-/** part[b][c] = (sum of g, sum of g * (x - mean)) over the rows of CTA b, g the gradient behind the ReLU. */
-template <typename T, bool RELU>
+/**
+ * part[b][c] = (sum of g, sum of g * (x - mean)) over the rows of CTA b, g the gradient behind the ReLU.  SUM: the output was used
+ * twice (a block's input goes to its first convolution and to its end); the two gradients are added here, rounded as the
+ * framework's addition rounds them, and g is left in `sum`, which is the residual's gradient too: seven passes over the activation
+ * instead of the nine of an addition on its own, sums of it, and both gradients out of it.
+ */
+template <typename T, bool RELU, bool SUM>
 __global__ void __launch_bounds__(kBnThreads, kBnPerSm)
-    bn_grad_sums_kernel(const T* __restrict__ x, const T* __restrict__ dy, const unsigned char* __restrict__ mask,
-                        const float* __restrict__ save_mean, float2* __restrict__ part, const BnGrid g) {
+    bn_grad_sums_kernel(const T* __restrict__ x, const T* __restrict__ dy, const T* __restrict__ dy2, T* __restrict__ sum,
+                        const unsigned char* __restrict__ mask, const float* __restrict__ save_mean, float2* __restrict__ part, const BnGrid g) {
   constexpr int U = kBnRows;
   after_previous_kernel();
   const Place at(g);
@@ -361,15 +366,26 @@ __global__ void __launch_bounds__(kBnThreads, kBnPerSm)
     for (size_t t = blockIdx.x; t < g.tiles; t += g.nblk) {
       const size_t r0 = t * tile_rows + at.ty;
       const size_t i0 = r0 * g.cols + at.col;
-      Pack8<T> v[U], d[U];
+      Pack8<T> v[U], d[U], d2[SUM ? U : 1];
       unsigned bits[U];
 #pragma unroll
       for (int i = 0; i < U; ++i) {
         const bool in = r0 + (size_t)i * at.TY < g.rows;
         d[i].u = in ? ((const uint4*)dy)[i0 + i * step] : uint4{0, 0, 0, 0};
+        if constexpr (SUM)
+          if (in) d2[i].u = ((const uint4*)dy2)[i0 + i * step];
         if (in) v[i].u = ((const uint4*)x)[i0 + i * step];
         bits[i] = in ? 0xffu : 0u;
         if constexpr (RELU) bits[i] = in ? mask[i0 + i * step] : 0u;
+      }
+      if constexpr (SUM) {
+#pragma unroll
+        for (int i = 0; i < U; ++i)
+          if (r0 + (size_t)i * at.TY < g.rows) {
+#pragma unroll
+            for (int k = 0; k < 8; ++k) d[i].e[k] = Elem<T>::down(bits[i] >> k & 1 ? up(d[i].e[k]) + up(d2[i].e[k]) : 0.f);
+            ((uint4*)sum)[i0 + i * step] = d[i].u;
+          }
       }
 #pragma unroll
       for (int i = 0; i < U; ++i)
@@ -509,18 +525,22 @@ template <typename T>
 void bn_backward(const BnBackward& a, cudaStream_t stream) {
   const BnGrid g = bn_grid(a.rows, a.channels, kBnRows, kBnPerSm);
   bn_check(g, (size_t)a.channels * sizeof(float2), a.workspace_bytes);
+  if (a.dy2 && !a.dres) throw_al_exception("batch norm: the sum of two gradients needs a place");
   float2* coef = (float2*)a.workspace;
   float2* part = coef + a.channels;
   const dim3 grid(g.nblk, g.ntile_y);
-  launch_behind(a.mask ? bn_grad_sums_kernel<T, true> : bn_grad_sums_kernel<T, false>, grid, kBnThreads, stream, (const T*)a.x, (const T*)a.dy,
-                a.mask, a.save_mean, part, g);
+  const auto sums = a.dy2 ? (a.mask ? bn_grad_sums_kernel<T, true, true> : bn_grad_sums_kernel<T, false, true>)
+                          : (a.mask ? bn_grad_sums_kernel<T, true, false> : bn_grad_sums_kernel<T, false, false>);
+  launch_behind(sums, grid, kBnThreads, stream, (const T*)a.x, (const T*)a.dy, (const T*)a.dy2, (T*)a.dres, a.mask, a.save_mean, part, g);
   launch_behind(bn_grad_finish_kernel, (unsigned)a.channels / 8, dim3(8, kFinishRows), stream, part, a.save_invstd, a.grad_weight, a.grad_bias,
                 coef, g);
+  const void* dy = a.dy2 ? a.dres : a.dy;   // (the sum has passed the ReLU already)
   auto run = [&](auto kernel) {
-    launch_behind(kernel, grid, kBnThreads, stream, (const T*)a.x, (const T*)a.dy, a.mask, (T*)a.dx, (T*)a.dres, a.save_mean, a.save_invstd,
+    launch_behind(kernel, grid, kBnThreads, stream, (const T*)a.x, (const T*)dy, a.mask, (T*)a.dx, (T*)a.dres, a.save_mean, a.save_invstd,
                   a.weight, coef, g);
   };
-  if (a.dres && a.mask) run(bn_grad_apply_kernel<T, true, true>);
+  if (a.dy2) run(bn_grad_apply_kernel<T, false, false>);
+  else if (a.dres && a.mask) run(bn_grad_apply_kernel<T, true, true>);
   else if (a.dres) run(bn_grad_apply_kernel<T, true, false>);
   else if (a.mask) run(bn_grad_apply_kernel<T, false, true>);
   else run(bn_grad_apply_kernel<T, false, false>);

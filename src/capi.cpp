@@ -664,11 +664,19 @@ int al_bn_forward(int dt, const void* x, const void* residual, void* y, unsigned
                                workspace_bytes, rows, channels, momentum, eps}, (DType)dt, (cudaStream_t)stream);
   });
 }
+int al_bn_backward_sum(int dt, const void* x, const void* dy, const void* dy2, const unsigned char* mask, void* dx, void* sum, const float* weight,
+                       const float* save_mean, const float* save_invstd, float* grad_weight, float* grad_bias, void* workspace,
+                       size_t workspace_bytes, size_t rows, int channels, void* stream) {
+  return guard([&] {
+    device::launch_bn_backward({x, dy, dy2, mask, dx, sum, weight, save_mean, save_invstd, grad_weight, grad_bias, workspace, workspace_bytes,
+                                rows, channels}, (DType)dt, (cudaStream_t)stream);
+  });
+}
 int al_bn_backward(int dt, const void* x, const void* dy, const unsigned char* mask, void* dx, void* dres, const float* weight,
                    const float* save_mean, const float* save_invstd, float* grad_weight, float* grad_bias, void* workspace,
                    size_t workspace_bytes, size_t rows, int channels, void* stream) {
   return guard([&] {
-    device::launch_bn_backward({x, dy, mask, dx, dres, weight, save_mean, save_invstd, grad_weight, grad_bias, workspace, workspace_bytes,
+    device::launch_bn_backward({x, dy, nullptr, mask, dx, dres, weight, save_mean, save_invstd, grad_weight, grad_bias, workspace, workspace_bytes,
                                 rows, channels}, (DType)dt, (cudaStream_t)stream);
   });
 }

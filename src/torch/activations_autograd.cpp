@@ -18,7 +18,7 @@ using at::Tensor;
 using torch::autograd::AutogradContext;
 using torch::autograd::variable_list;
 
-constexpr int kArgs = 10;  // of forward()
+constexpr int kArgs = 11;  // of forward()
 
 int type_code(const Tensor& t) { return (int)(t.scalar_type() == at::kBFloat16 ? Al::DType::bf16 : Al::DType::f16); }
 
@@ -35,10 +35,11 @@ Tensor restored(const Tensor& t, at::IntArrayRef sizes, at::ScalarType type, con
   return t.is_contiguous(format) && (uintptr_t)t.data_ptr() % 16 == 0 ? t : t.clone(format);
 }
 
+/** `twice`: the output comes as two tensors on the same memory, whose gradients backward() adds where it reads them. */
 struct BatchNormAct : public torch::autograd::Function<BatchNormAct> {
-  static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& weight, const Tensor& bias,
-                        const std::optional<Tensor>& residual, const Tensor& running_mean, const Tensor& running_var,
-                        const std::optional<Tensor>& batches, double momentum, double eps, bool relu) {
+  static variable_list forward(AutogradContext* ctx, const Tensor& x, const Tensor& weight, const Tensor& bias,
+                               const std::optional<Tensor>& residual, const Tensor& running_mean, const Tensor& running_var,
+                               const std::optional<Tensor>& batches, double momentum, double eps, bool relu, bool twice) {
     const c10::cuda::CUDAGuard guard(x.device());
     const int64_t c = x.size(1), rows = x.numel() / c;
     Tensor y = at::empty_like(x);
@@ -60,18 +61,24 @@ struct BatchNormAct : public torch::autograd::Function<BatchNormAct> {
     ctx->saved_data["eps"] = eps;
     ctx->saved_data["residual"] = residual.has_value() && residual->requires_grad();
     ctx->set_materialize_grads(false);
-    return y;
+    if (twice) return {y, y.variable_data()};
+    return {y};
   }
 
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
     variable_list out(kArgs);
-    if (!grads[0].defined()) return out;
+    Tensor dy = grads[0], dy2 = grads.size() > 1 ? grads[1] : Tensor();
+    if (!dy.defined()) std::swap(dy, dy2);
+    if (!dy.defined()) return out;
     const variable_list saved = ctx->get_saved_variables();
     Tensor x = saved[0], weight = saved[1], stats = saved[2], mask = saved[3];
     const bool relu = ctx->saved_data["relu"].toBool(), want_res = ctx->saved_data["residual"].toBool();
-    Tensor dy = grads[0];
     const c10::cuda::CUDAGuard guard(dy.device());
     const int64_t c = x.size(1), rows = x.numel() / c;
+    if (dy2.defined() && (at::GradMode::is_enabled() || dy.scalar_type() != x.scalar_type() || dy2.scalar_type() != x.scalar_type())) {
+      dy = dy + dy2;
+      dy2.reset();
+    }
     if (at::GradMode::is_enabled() || dy.scalar_type() != x.scalar_type()) {
       // a graph of the backward is wanted: operations that have a derivative themselves
       if (relu) {
@@ -86,24 +93,33 @@ struct BatchNormAct : public torch::autograd::Function<BatchNormAct> {
       if (want_res) out[3] = dy;
       return out;
     }
-    if (!dy.is_contiguous(at::MemoryFormat::ChannelsLast) || (uintptr_t)dy.data_ptr() % 16) dy = dy.clone(at::MemoryFormat::ChannelsLast);
+    auto laid_out = [](const Tensor& t) {
+      return t.is_contiguous(at::MemoryFormat::ChannelsLast) && (uintptr_t)t.data_ptr() % 16 == 0 ? t : t.clone(at::MemoryFormat::ChannelsLast);
+    };
+    dy = laid_out(dy);
+    if (dy2.defined()) dy2 = laid_out(dy2);
     x = restored(x, dy.sizes(), dy.scalar_type(), dy, at::MemoryFormat::ChannelsLast);
     weight = restored(weight, {c}, at::kFloat, dy, at::MemoryFormat::Contiguous);
     stats = restored(stats, {2, c}, at::kFloat, dy, at::MemoryFormat::Contiguous);
     mask = restored(mask, {relu ? rows * c / 8 : 0}, at::kByte, dy, at::MemoryFormat::Contiguous);
     Tensor dx = at::empty_like(x), dres, gw = at::empty_like(weight), gb = at::empty_like(weight);
-    if (want_res) dres = at::empty_like(x);
+    if (want_res || dy2.defined()) dres = at::empty_like(x);
     Tensor ws = workspace(x, c);
     float* at = stats.data_ptr<float>();
-    TORCH_CHECK(al_bn_backward(type_code(x), x.data_ptr(), dy.data_ptr(), relu ? mask.data_ptr<uint8_t>() : nullptr, dx.data_ptr(),
-                               want_res ? dres.data_ptr() : nullptr, weight.data_ptr<float>(), at, at + c, gw.data_ptr<float>(),
-                               gb.data_ptr<float>(), ws.data_ptr(), (size_t)ws.numel(), (size_t)rows, (int)c,
-                               c10::cuda::getCurrentCUDAStream().stream()) == 0,
-                al_last_error());
+    void* const stream = c10::cuda::getCurrentCUDAStream().stream();
+    const unsigned char* passes = relu ? mask.data_ptr<uint8_t>() : nullptr;
+    const int rc = dy2.defined()
+                       ? al_bn_backward_sum(type_code(x), x.data_ptr(), dy.data_ptr(), dy2.data_ptr(), passes, dx.data_ptr(), dres.data_ptr(),
+                                            weight.data_ptr<float>(), at, at + c, gw.data_ptr<float>(), gb.data_ptr<float>(), ws.data_ptr(),
+                                            (size_t)ws.numel(), (size_t)rows, (int)c, stream)
+                       : al_bn_backward(type_code(x), x.data_ptr(), dy.data_ptr(), passes, dx.data_ptr(), want_res ? dres.data_ptr() : nullptr,
+                                        weight.data_ptr<float>(), at, at + c, gw.data_ptr<float>(), gb.data_ptr<float>(), ws.data_ptr(),
+                                        (size_t)ws.numel(), (size_t)rows, (int)c, stream);
+    TORCH_CHECK(rc == 0, al_last_error());
     out[0] = dx;
     out[1] = gw;
     out[2] = gb;
-    out[3] = dres;
+    if (want_res) out[3] = dres;
     return out;
   }
 };
@@ -111,7 +127,14 @@ struct BatchNormAct : public torch::autograd::Function<BatchNormAct> {
 Tensor batch_norm_act(const Tensor& x, const Tensor& weight, const Tensor& bias, const std::optional<Tensor>& residual,
                       const Tensor& running_mean, const Tensor& running_var, const std::optional<Tensor>& batches, double momentum,
                       double eps, bool relu) {
-  return BatchNormAct::apply(x, weight, bias, residual, running_mean, running_var, batches, momentum, eps, relu);
+  return BatchNormAct::apply(x, weight, bias, residual, running_mean, running_var, batches, momentum, eps, relu, false)[0];
+}
+
+std::tuple<Tensor, Tensor> batch_norm_act_twice(const Tensor& x, const Tensor& weight, const Tensor& bias, const std::optional<Tensor>& residual,
+                                                const Tensor& running_mean, const Tensor& running_var, const std::optional<Tensor>& batches,
+                                                double momentum, double eps, bool relu) {
+  const variable_list y = BatchNormAct::apply(x, weight, bias, residual, running_mean, running_var, batches, momentum, eps, relu, true);
+  return {y[0], y[1]};
 }
 
 struct MaxPool : public torch::autograd::Function<MaxPool> {
@@ -232,6 +255,9 @@ TORCH_LIBRARY(aluminum_b200, m) {
   m.def("batch_norm_act(Tensor x, Tensor weight, Tensor bias, Tensor? residual, Tensor(a!) running_mean, Tensor(b!) running_var, "
         "Tensor(c!)? batches, float momentum, float eps, bool relu) -> Tensor",
         batch_norm_act);
+  m.def("batch_norm_act_twice(Tensor x, Tensor weight, Tensor bias, Tensor? residual, Tensor(a!) running_mean, Tensor(b!) running_var, "
+        "Tensor(c!)? batches, float momentum, float eps, bool relu) -> (Tensor, Tensor)",
+        batch_norm_act_twice);
   m.def("stem_conv(Tensor x, Tensor weight, ScalarType type) -> Tensor", stem_conv);
   m.def("max_pool(Tensor x, int k, int stride, int pad) -> Tensor", max_pool);
 }

@@ -271,3 +271,72 @@ def test_pooling_by_three_every_two(h, w, dtype):
         y.backward(dy)
         want.backward(dy.float())
         assert torch.equal(x.grad.float(), xr.grad)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("shape", [(2, 8, 1, 1), (3, 24, 5, 7), (2, 264, 33, 31), (5, 2048, 7, 7), (24, 64, 56, 56)])
+@pytest.mark.parametrize("relu,res", [(True, True), (True, False), (False, True), (False, False)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_output_used_twice(shape, relu, res, dtype):
+    """The two gradients added by the kernel: bit for bit what the framework's addition of them gives."""
+    from aluminum_b200.ops import batch_norm_act_twice
+    torch.manual_seed(shape[1])
+    cl = dict(memory_format=torch.channels_last)
+    rand = lambda: torch.randn(shape, device="cuda").to(dtype).contiguous(**cl)
+    bn, x0, r0, a, b = nn.BatchNorm2d(shape[1]).cuda(), rand(), rand(), rand(), rand()
+    act = nn.ReLU() if relu else None
+
+    def run(use):
+        m, x, r = copy.deepcopy(bn), x0.clone().requires_grad_(), r0.clone().requires_grad_()
+        use(m, x, r if res else None)
+        return [x.grad, m.weight.grad, m.bias.grad, m.running_mean] + ([r.grad] if res else [])
+
+    def twice(m, x, r):
+        y, same = batch_norm_act_twice(m, x, act, r)
+        assert "BatchNormAct" in y.grad_fn.name() and same.data_ptr() == y.data_ptr() and same.grad_fn is y.grad_fn
+        torch.autograd.backward([y, same], [a, b])
+
+    def once(m, x, r):
+        batch_norm_act(m, x, act, r).backward(a + b)
+    assert all(torch.equal(u, v) for u, v in zip(run(twice), run(once)))
+    for used in (0, 1):   # only one of the two used
+        def single(m, x, r):
+            batch_norm_act_twice(m, x, act, r)[used].backward(a)
+        assert all(torch.equal(u, v) for u, v in zip(run(single), run(lambda m, x, r: batch_norm_act(m, x, act, r).backward(a))))
+
+    def graph(pair):
+        def use(m, x, r):
+            outputs, gradients = (batch_norm_act_twice(m, x, act, r), (a, b)) if pair else ((batch_norm_act(m, x, act, r),), (a + b,))
+            gx, = torch.autograd.grad(outputs, [x], gradients, create_graph=True)
+            (gx.float().square().mean() + outputs[0].float().mean()).backward()
+        return use
+    for u, v in zip(run(graph(True)), run(graph(False))):
+        assert torch.equal(u.nan_to_num(7.0), v.nan_to_num(7.0))
+
+
+@pytest.mark.gpu
+def test_network_block_by_block():
+    """The network's own loop over its blocks: the gradients of calling the stages, to what the order of one addition is worth;
+    hooks on a stage or a block are called."""
+    from aluminum_b200.models.resnet import ResNet
+    torch.manual_seed(0)
+    net = ResNet((2, 2, 1, 1), 10, width=16).cuda().to(memory_format=torch.channels_last)
+    for m in net.modules():
+        if isinstance(m, nn.BatchNorm2d):
+            nn.init.uniform_(m.weight, 0.5, 1.5)
+    x = torch.randn(4, 3, 64, 64, device="cuda")
+
+    def grads(net):
+        with torch.autocast("cuda", dtype=torch.bfloat16):
+            net(x).float().square().mean().backward()
+        return [p.grad for p in net.parameters()]
+    own, called, seen = copy.deepcopy(net), copy.deepcopy(net), []
+    for stage in (called.layer1, called.layer3):
+        stage.register_forward_hook(lambda *a: seen.append(1))
+    for u, v in zip(grads(own), grads(called)):
+        assert rel(u, v.double()) < 2e-2
+    assert len(seen) == 2
+    called = copy.deepcopy(net)
+    called.layer2[1].register_forward_pre_hook(lambda *a: seen.append(1))
+    grads(called)
+    assert len(seen) == 3
