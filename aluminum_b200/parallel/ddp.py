@@ -23,6 +23,7 @@ from typing import List, Optional
 import torch
 from torch import nn
 
+from .. import _lib
 from ..ops.elementwise import sgd_momentum_step
 
 
@@ -93,6 +94,7 @@ class DataParallel:
             b.pending = b.total
 
         # Re-point parameters and gradients at the flat buffers.
+        self._params, self._grad_views = order, []
         with torch.no_grad():
             for p, off in zip(order, offsets):
                 n = p.numel()
@@ -109,6 +111,7 @@ class DataParallel:
                     gview = self.flat_grad[off:off + n].view(p.shape)
                 p.data = view
                 p.grad = gview
+                self._grad_views.append(gview)
         if self.world > 1:
             for p in order:
                 p.register_post_accumulate_grad_hook(self._on_grad)
@@ -163,6 +166,26 @@ class DataParallel:
         self.finish_gradients()
         sgd_momentum_step(self.flat_param, self.flat_mom, self.flat_grad, self.lr, self.momentum, self.weight_decay,
                           1.0, first_step=(self.steps == 0), zero_grad=True)
+        self.launches += 1
+        self.steps += 1
+
+    def backward_and_step(self, loss: torch.Tensor) -> None:
+        """``loss.backward()`` and :meth:`step`.  With one rank nothing needs the gradients in the flat buffer: backward leaves
+        them as it made them and the optimizer reads them there, without a launch per tensor that adds them up first."""
+        own = (type(self).step is DataParallel.step and type(self).finish_gradients is DataParallel.finish_gradients
+               and not {"step", "finish_gradients"} & self.__dict__.keys())
+        calls = _lib.calls() if self.world == 1 and not self.timeline and own else None
+        if calls is None or not calls.lend_gradients(self._params, self._grad_views):
+            loss.backward()
+            self.step()
+            return
+        try:
+            loss.backward()
+        except BaseException:
+            calls.return_gradients(self._params, self._grad_views)
+            raise
+        calls.step_on_lent(self._params, self._grad_views, self.flat_param, self.flat_mom, self.flat_grad, float(self.lr), float(self.momentum),
+                           float(self.weight_decay), self.steps == 0)
         self.launches += 1
         self.steps += 1
 

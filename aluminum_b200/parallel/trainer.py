@@ -38,8 +38,11 @@ class Trainer:
         with torch.autocast("cuda", dtype=self.autocast_dtype, enabled=self.autocast_dtype is not None):
             out = self.dp(x)
             loss = self.loss_fn(out.float(), y)
-        loss.backward()
-        self.dp.step()
+        if isinstance(self.dp, DataParallel):
+            self.dp.backward_and_step(loss)
+        else:
+            loss.backward()
+            self.dp.step()
         return loss.detach()
 
     # ---- host -> device staging ---------------------------------------------------------------------

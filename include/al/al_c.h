@@ -200,6 +200,10 @@ int al_route_rows(void* comm, int nlocal, const long long* const* dest, const si
 int al_scale_cast(void* out, int out_dt, const void* in, int in_dt, size_t n, double scale, void* stream);
 int al_sgd_momentum(float* param, float* momentum, float* grad, size_t n, float lr, float mu, float weight_decay,
                     float grad_scale, int first_step, int zero_grad, void* stream);
+/** The same over n tensors (grad[k] of numel[k] elements belongs to elements at[k].. of the flat buffers; at[k] a multiple of 4, grad[k] 16-byte
+ *  aligned or NULL), whose gradients are added to what flat_grad holds; their part of flat_grad is zeroed. */
+int al_sgd_momentum_from(float* param, float* momentum, float* flat_grad, const float* const* grad, const size_t* at, const size_t* numel, int n,
+                         float lr, float mu, float weight_decay, float grad_scale, int first_step, void* stream);
 int al_fill_u32(void* out, size_t n, uint32_t value, void* stream);
 /* Training batch norm + residual + ReLU over rows x channels (channels-last); residual, mask, running_*, batches may be NULL. */
 size_t al_bn_workspace_bytes(int channels);

@@ -161,6 +161,13 @@ void launch_sgd_momentum(float* param, float* momentum, float* grad, size_t n, f
                          float weight_decay, float grad_scale, int first_step, int zero_grad,
                          cudaStream_t stream);
 /**
+ * The same for gradients that lie where backward left them, and are added to what the flat gradient holds (which is zeroed): the first
+ * `n` entries of grad / at / numel; elements of the flat buffers outside the tensors are not touched.
+ */
+void launch_sgd_momentum_from(float* param, float* momentum, float* flat_grad, const float* const* grad, const size_t* at,
+                              const size_t* numel, int n, float lr, float mu, float weight_decay, float grad_scale, int first_step,
+                              cudaStream_t stream);
+/**
  * Training batch norm of a channels-last activation (rows x channels, bf16 or f16; kernels/batchnorm.cu) with the
  * residual addition and the ReLU behind it.  residual and mask may be null (no addition, no ReLU); mask gets one byte per
  * 8 channels.  running_mean / running_var / batches (the count of batches) may be null.

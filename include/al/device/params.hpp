@@ -312,6 +312,16 @@ struct LocalRowsParams {
   unsigned first[kMaxRanks * kMaxRanks + 1];  ///< ... and the first unit of every pair [source][destination]
 };
 
+/** Tensors whose gradients an optimizer launch reads where backward left them (kernels/elementwise.cu). */
+struct GradTable {
+  static constexpr int kMax = 512;   ///< per launch: 12 KiB of arguments
+  const float* grad[kMax];           ///< 16-byte aligned; nullptr: nothing besides what the flat gradient holds
+  size_t at[kMax];                   ///< first element in the flat buffers, a multiple of 4
+  unsigned numel[kMax];
+  unsigned first[kMax + 1];          ///< first tile of every tensor
+  int n;
+};
+
 /** Arguments of one routing launch (kernels/route.cu): one block per local rank. */
 struct RouteParams {
   const long long* dest[kMaxRanks];  ///< destination rank of every token

@@ -651,6 +651,13 @@ int al_sgd_momentum(float* param, float* momentum, float* grad, size_t n, float 
     device::launch_sgd_momentum(param, momentum, grad, n, lr, mu, weight_decay, grad_scale, first_step, zero_grad, (cudaStream_t)stream);
   });
 }
+int al_sgd_momentum_from(float* param, float* momentum, float* flat_grad, const float* const* grad, const size_t* at, const size_t* numel, int n,
+                         float lr, float mu, float weight_decay, float grad_scale, int first_step, void* stream) {
+  return guard([&] {
+    device::launch_sgd_momentum_from(param, momentum, flat_grad, grad, at, numel, n, lr, mu, weight_decay, grad_scale, first_step,
+                                     (cudaStream_t)stream);
+  });
+}
 int al_fill_u32(void* out, size_t n, uint32_t value, void* stream) {
   return guard([&] { device::launch_fill_u32((uint32_t*)out, n, value, (cudaStream_t)stream); });
 }

@@ -6,6 +6,7 @@
 // the call itself), and raises the package's AlError otherwise.  The interpreter's lock is released around the library's call.
 #pragma once
 #if __has_include(<Python.h>)
+#include <c10/cuda/CUDACachingAllocator.h>
 #include <torch/csrc/autograd/python_variable.h>
 
 #include <vector>
@@ -307,6 +308,102 @@ PyObject* empties(PyObject*, PyObject* const* a, Py_ssize_t n) {
   });
 }
 
+/** Parameters, and the views of a flat buffer that hold their gradients. */
+struct Gradients {
+  Items params, views;
+  Gradients(PyObject* p, PyObject* v) : params(p), views(v) {
+    if (!params.list || !views.list || params.n != views.n) raise("internal error: as many views as parameters expected");
+    for (Py_ssize_t i = 0; i < params.n; ++i)
+      if (!THPVariable_Check(params[i]) || !THPVariable_Check(views[i])) raise("internal error: parameters and views are tensors");
+  }
+  const at::Tensor& param(Py_ssize_t i) const { return THPVariable_Unpack(params[i]); }
+  const at::Tensor& view(Py_ssize_t i) const { return THPVariable_Unpack(views[i]); }
+};
+
+/**
+ * (parameters, views): take the views off the parameters, so that backward leaves its gradients as they are instead of adding each to
+ * its view.  False, and nothing is changed, if a parameter's gradient is not its view.
+ */
+PyObject* lend_gradients(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  return guarded([&]() -> PyObject* {
+    need(n, 2);
+    const Gradients g(a[0], a[1]);
+    for (Py_ssize_t i = 0; i < g.params.n; ++i)
+      if (!g.param(i).grad().is_same(g.view(i))) Py_RETURN_FALSE;
+    for (Py_ssize_t i = 0; i < g.params.n; ++i) g.param(i).mutable_grad() = at::Tensor();
+    Py_RETURN_TRUE;
+  });
+}
+
+/** The same elements in the same order in memory (strides of dimensions of one element say nothing). */
+bool same_layout(const at::Tensor& a, const at::Tensor& b) {
+  if (a.sizes() != b.sizes()) return false;
+  for (int64_t d = 0; d < a.dim(); ++d)
+    if (a.size(d) > 1 && a.stride(d) != b.stride(d)) return false;
+  return true;
+}
+
+/** (parameters, views): give the views back, with what backward left added to them. */
+PyObject* return_gradients(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  return guarded([&]() -> PyObject* {
+    need(n, 2);
+    const Gradients g(a[0], a[1]);
+    const at::NoGradGuard no_grad;
+    for (Py_ssize_t i = 0; i < g.params.n; ++i) {
+      at::Tensor left = g.param(i).grad();
+      g.param(i).mutable_grad() = g.view(i);
+      if (left.defined() && !left.is_same(g.view(i))) g.view(i).add_(left);
+    }
+    Py_RETURN_NONE;
+  });
+}
+
+/**
+ * (parameters, views, flat parameters, flat momentum, flat gradients, lr, momentum, weight decay, first step): the optimizer step
+ * on the gradients that backward left, and the views back in their places, zeroed.
+ */
+PyObject* step_on_lent(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  return guarded([&]() -> PyObject* {
+    need(n, 9);
+    const Gradients g(a[0], a[1]);
+    for (int i = 2; i < 5; ++i)
+      if (!THPVariable_Check(a[i])) raise("internal error: flat buffers are tensors");
+    const at::Tensor &param = THPVariable_Unpack(a[2]), &momentum = THPVariable_Unpack(a[3]), &flat = THPVariable_Unpack(a[4]);
+    float value[3];
+    for (int i = 0; i < 3; ++i) value[i] = (float)PyFloat_AsDouble(a[5 + i]);
+    if (PyErr_Occurred()) throw Raised();
+    const at::NoGradGuard no_grad;
+    const c10::cuda::CUDAStream stream = c10::cuda::getCurrentCUDAStream();
+    const size_t count = (size_t)g.params.n;
+    std::vector<const float*> grad(count, nullptr);
+    std::vector<size_t> at(count), numel(count);
+    std::vector<at::Tensor> kept;
+    kept.reserve(count);
+    for (size_t i = 0; i < count; ++i) {
+      const at::Tensor& view = g.view((Py_ssize_t)i);
+      at::Tensor left = g.param((Py_ssize_t)i).grad();
+      g.param((Py_ssize_t)i).mutable_grad() = view;
+      at[i] = (size_t)(view.storage_offset() - flat.storage_offset());
+      numel[i] = (size_t)view.numel();
+      if (!left.defined()) continue;
+      if (left.scalar_type() == at::kFloat && left.layout() == at::kStrided && left.device() == view.device() && same_layout(left, view) &&
+          left.is_non_overlapping_and_dense() && (uintptr_t)left.data_ptr() % 16 == 0) {
+        grad[i] = left.data_ptr<float>();
+        // (backward may have made it on another stream: its memory stays until this one is past the optimizer)
+        c10::cuda::CUDACachingAllocator::recordStream(left.storage().data_ptr(), stream);
+        kept.push_back(std::move(left));
+      } else {
+        view.add_(left);
+      }
+    }
+    const int first = PyObject_IsTrue(a[8]);
+    return launch(false, [&](void**) {
+      return al_sgd_momentum_from(param.data_ptr<float>(), momentum.data_ptr<float>(), flat.data_ptr<float>(), grad.data(), at.data(), numel.data(),
+                                  (int)count, value[0], value[1], value[2], 1.f, first, (void*)stream.stream());
+    });
+  });
+}
+
 /** The handle of PyTorch's current stream. */
 PyObject* current_stream(PyObject*, PyObject*) {
   return guarded([&] { return PyLong_FromVoidPtr((void*)c10::cuda::getCurrentCUDAStream().stream()); });
@@ -319,7 +416,8 @@ PyObject* set_error(PyObject*, PyObject* type) {
 }
 
 #define AL_FAST(f) {#f, (PyCFunction)(void (*)(void))f, METH_FASTCALL, nullptr}
-PyMethodDef methods[] = {AL_FAST(collective), AL_FAST(exchange_rows), AL_FAST(p2p), AL_FAST(empties),
+PyMethodDef methods[] = {AL_FAST(collective), AL_FAST(exchange_rows), AL_FAST(p2p), AL_FAST(empties), AL_FAST(lend_gradients),
+                         AL_FAST(return_gradients), AL_FAST(step_on_lent),
                          {"current_stream", current_stream, METH_NOARGS, nullptr},
                          {"set_error", set_error, METH_O, nullptr},
                          {nullptr, nullptr, 0, nullptr}};
