@@ -12,7 +12,7 @@ import torch
 from torch import nn
 
 from ..ops.activations import _bare, _modes_off, batch_norm_act, batch_norm_act_twice, max_pool
-from ..ops.convolution import stem_conv
+from ..ops.convolution import cast_weights, convolve, stem_conv
 
 
 class Bottleneck(nn.Module):
@@ -45,10 +45,18 @@ class Bottleneck(nn.Module):
 
     def twice(self, x, same):
         """forward(x) as two tensors, for the next block's first convolution and for its end; ``same`` is x, for the end of this one."""
-        identity = same if self.downsample is None else self.downsample(same)
-        out = batch_norm_act(self.bn1, self.conv1(x), self.relu)
-        out = batch_norm_act(self.bn2, self.conv2(out), self.relu)
-        return batch_norm_act_twice(self.bn3, self.conv3(out), self.relu, identity)
+        convs, shortcut = [self.conv1, self.conv2, self.conv3], self.downsample
+        apart = shortcut is not None and type(shortcut) is Shortcut and len(shortcut) == 2 and _bare(shortcut)
+        if apart:
+            convs.append(shortcut[0])
+        w = cast_weights(convs, x) or [None] * len(convs)
+        if apart:
+            same = batch_norm_act(shortcut[1], convolve(shortcut[0], same, w[3]))
+        elif shortcut is not None:
+            same = shortcut(same)
+        out = batch_norm_act(self.bn1, convolve(self.conv1, x, w[0]), self.relu)
+        out = batch_norm_act(self.bn2, convolve(self.conv2, out, w[1]), self.relu)
+        return batch_norm_act_twice(self.bn3, convolve(self.conv3, out, w[2]), self.relu, same)
 
 
 class Shortcut(nn.Sequential):

@@ -198,6 +198,8 @@ int al_route_rows(void* comm, int nlocal, const long long* const* dest, const si
 
 /* ---- element-wise kernels ---- */
 int al_scale_cast(void* out, int out_dt, const void* in, int in_dt, size_t n, double scale, void* stream);
+/** Casts of `count` tensors (fp32 to f16 / bf16 or back, n[k] elements, all 16-byte aligned), one launch per 64 of them. */
+int al_cast_all(void* const* out, int out_dt, const void* const* in, int in_dt, const size_t* n, int count, void* stream);
 int al_sgd_momentum(float* param, float* momentum, float* grad, size_t n, float lr, float mu, float weight_decay,
                     float grad_scale, int first_step, int zero_grad, void* stream);
 /** The same over n tensors (grad[k] of numel[k] elements belongs to elements at[k].. of the flat buffers; at[k] a multiple of 4, grad[k] 16-byte

@@ -152,6 +152,8 @@ void launch_halo_unpack(float* tensor, const float* packed, size_t nc, size_t d_
 /** out[i] = (Tout)(in[i] * scale); in and out may alias when the types match. */
 void launch_scale_cast(void* out, DType out_dt, const void* in, DType in_dt, size_t n, double scale,
                        cudaStream_t stream);
+/** out[k][i] = (Tout)in[k][i] for i < n[k] of `count` tensors, fp32 to a 16-bit type or back; all 16-byte aligned.  One launch per 64 of them. */
+void launch_cast_all(void* const* out, DType out_dt, const void* const* in, DType in_dt, const size_t* n, int count, cudaStream_t stream);
 /**
  * Fused momentum-SGD over a flat fp32 parameter buffer:
  *   g = grad*grad_scale + wd*p;  m = mu*m + g (m = g on the first step);  p -= lr*m

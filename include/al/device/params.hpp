@@ -312,6 +312,16 @@ struct LocalRowsParams {
   unsigned first[kMaxRanks * kMaxRanks + 1];  ///< ... and the first unit of every pair [source][destination]
 };
 
+/** Tensors that one launch casts (kernels/elementwise.cu). */
+struct CastTable {
+  static constexpr int kMax = 64;
+  const void* in[kMax];              ///< in and out 16-byte aligned
+  void* out[kMax];
+  size_t n[kMax];
+  unsigned first[kMax + 1];          ///< first tile of every tensor
+  int count;
+};
+
 /** Tensors whose gradients an optimizer launch reads where backward left them (kernels/elementwise.cu). */
 struct GradTable {
   static constexpr int kMax = 512;   ///< per launch: 12 KiB of arguments

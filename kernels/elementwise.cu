@@ -59,6 +59,35 @@ __global__ void __launch_bounds__(kThreads) scale_f64_kernel(double* out, const 
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) out[i] = in[i] * scale;
 }
 
+/**
+ * Casts of several tensors: a CTA has 2048 elements of one of them, eight per thread.  A block's weights are small (4 K to 2.4 M elements), and a
+ * launch each way for every one of them costs more than moving them.
+ */
+constexpr unsigned kCastTile = kThreads * 8;
+
+template <typename Ti, typename To>
+__global__ void __launch_bounds__(kThreads) cast_all_kernel(const __grid_constant__ CastTable t) {
+  int k = 0;
+#pragma unroll
+  for (int s = CastTable::kMax / 2; s > 0; s >>= 1)
+    if (k + s < t.count && blockIdx.x >= t.first[k + s]) k += s;
+  const size_t i = (size_t)(blockIdx.x - t.first[k]) * kCastTile + (size_t)threadIdx.x * 8, n = t.n[k];
+  const Ti* in = (const Ti*)t.in[k] + i;
+  To* out = (To*)t.out[k] + i;
+  auto one = [](Ti v) { return Elem<To>::down((float)Elem<Ti>::up(v)); };
+  struct alignas(16) PI { Ti e[8]; };
+  struct alignas(16) PO { To e[8]; };
+  if (i + 8 <= n) {
+    const PI a = *(const PI*)in;
+    PO o;
+#pragma unroll
+    for (int e = 0; e < 8; ++e) o.e[e] = one(a.e[e]);
+    *(PO*)out = o;
+  } else {
+    for (int e = 0; e < 8 && i + e < n; ++e) out[e] = one(in[e]);
+  }
+}
+
 /** One element; the roundings are written out, so that every path to it gives the same bits. */
 __device__ __forceinline__ void sgd_update(float& p, float& m, float g, float lr, float mu, float wd, float gscale, int first) {
   const float ge = fmaf(wd, p, g * gscale);
@@ -179,6 +208,34 @@ void launch_scale_cast(void* out, DType out_dt, const void* in, DType in_dt, siz
     return;
   }
   throw_al_exception("scale_cast: unsupported type pair ", dtype_name(in_dt), " -> ", dtype_name(out_dt));
+}
+
+void launch_cast_all(void* const* out, DType out_dt, const void* const* in, DType in_dt, const size_t* n, int count, cudaStream_t stream) {
+  using bf = __nv_bfloat16;
+  void (*kernel)(const CastTable) = nullptr;
+  if (in_dt == DType::f32 && out_dt == DType::bf16) kernel = cast_all_kernel<float, bf>;
+  else if (in_dt == DType::f32 && out_dt == DType::f16) kernel = cast_all_kernel<float, __half>;
+  else if (in_dt == DType::bf16 && out_dt == DType::f32) kernel = cast_all_kernel<bf, float>;
+  else if (in_dt == DType::f16 && out_dt == DType::f32) kernel = cast_all_kernel<__half, float>;
+  else throw_al_exception("cast_all: unsupported type pair ", dtype_name(in_dt), " -> ", dtype_name(out_dt));
+  for (int from = 0; from < count; from += CastTable::kMax) {
+    CastTable t;
+    t.count = std::min(count - from, CastTable::kMax);
+    size_t tiles = 0;
+    for (int k = 0; k < t.count; ++k) {
+      t.in[k] = in[from + k];
+      t.out[k] = out[from + k];
+      t.n[k] = n[from + k];
+      if (((uintptr_t)t.in[k] | (uintptr_t)t.out[k]) % 16 != 0) throw_al_exception("cast_all: a tensor does not begin on 16 bytes");
+      t.first[k] = (unsigned)tiles;
+      tiles += (t.n[k] + kCastTile - 1) / kCastTile;
+      if (tiles > 0x7fffffff) throw_al_exception("cast_all: too many elements");
+    }
+    t.first[t.count] = (unsigned)tiles;
+    if (tiles == 0) continue;
+    kernel<<<(unsigned)tiles, kThreads, 0, stream>>>(t);
+    AL_CHECK_CUDA(cudaGetLastError());
+  }
 }
 
 void launch_sgd_momentum(float* param, float* momentum, float* grad, size_t n, float lr, float mu,

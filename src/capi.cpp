@@ -645,6 +645,9 @@ int al_route_rows(void* comm, int nlocal, const long long* const* dest, const si
 int al_scale_cast(void* out, int out_dt, const void* in, int in_dt, size_t n, double scale, void* stream) {
   return guard([&] { device::launch_scale_cast(out, (DType)out_dt, in, (DType)in_dt, n, scale, (cudaStream_t)stream); });
 }
+int al_cast_all(void* const* out, int out_dt, const void* const* in, int in_dt, const size_t* n, int count, void* stream) {
+  return guard([&] { device::launch_cast_all(out, (DType)out_dt, in, (DType)in_dt, n, count, (cudaStream_t)stream); });
+}
 int al_sgd_momentum(float* param, float* momentum, float* grad, size_t n, float lr, float mu, float weight_decay,
                     float grad_scale, int first_step, int zero_grad, void* stream) {
   return guard([&] {

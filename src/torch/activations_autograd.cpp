@@ -247,6 +247,53 @@ struct StemConv : public torch::autograd::Function<StemConv> {
   }
 };
 
+/** The weights of a block in a 16-bit type, and their gradients back in fp32, with one launch each way. */
+struct CastAll : public torch::autograd::Function<CastAll> {
+  /** Every tensor in `to`, dense and in the order of its memory. */
+  static std::vector<Tensor> cast(at::TensorList tensors, at::ScalarType from, at::ScalarType to) {
+    auto code = [](at::ScalarType t) { return (int)(t == at::kFloat ? Al::DType::f32 : t == at::kBFloat16 ? Al::DType::bf16 : Al::DType::f16); };
+    std::vector<Tensor> made;
+    std::vector<const void*> in;
+    std::vector<void*> out;
+    std::vector<size_t> n;
+    for (const Tensor& t : tensors) {
+      Tensor dense = t.is_non_overlapping_and_dense() && (uintptr_t)t.data_ptr() % 16 == 0 ? t : t.clone(at::MemoryFormat::Contiguous);
+      made.push_back(at::empty_strided(dense.sizes(), dense.strides(), dense.options().dtype(to)));
+      in.push_back(dense.data_ptr());
+      out.push_back(made.back().data_ptr());
+      n.push_back((size_t)dense.numel());
+    }
+    TORCH_CHECK(al_cast_all(out.data(), code(to), in.data(), code(from), n.data(), (int)n.size(), c10::cuda::getCurrentCUDAStream().stream()) == 0,
+                al_last_error());
+    return made;
+  }
+
+  static variable_list forward(AutogradContext* ctx, at::TensorList weights, at::ScalarType type) {
+    const c10::cuda::CUDAGuard guard(weights[0].device());
+    ctx->set_materialize_grads(false);
+    return cast(weights, at::kFloat, type);
+  }
+
+  static variable_list backward(AutogradContext*, variable_list grads) {
+    variable_list out(grads.size() + 1);
+    std::vector<Tensor> given;
+    for (const Tensor& g : grads)
+      if (g.defined()) given.push_back(g);
+    if (given.empty()) return out;
+    const c10::cuda::CUDAGuard guard(given[0].device());
+    const at::ScalarType type = given[0].scalar_type();
+    bool plain = !at::GradMode::is_enabled() && (type == at::kBFloat16 || type == at::kHalf);   // (no graph of the backward is wanted)
+    for (const Tensor& g : given) plain = plain && g.scalar_type() == type && g.layout() == at::kStrided && g.device() == given[0].device();
+    const std::vector<Tensor> made = plain ? cast(given, type, at::kFloat) : std::vector<Tensor>();
+    size_t next = 0;
+    for (size_t i = 0; i < grads.size(); ++i)
+      if (grads[i].defined()) out[i] = plain ? made[next++] : grads[i].to(at::kFloat);
+    return out;
+  }
+};
+
+std::vector<Tensor> cast_all(at::TensorList weights, at::ScalarType type) { return CastAll::apply(weights, type); }
+
 Tensor stem_conv(const Tensor& x, const Tensor& weight, at::ScalarType type) { return StemConv::apply(x, weight, type); }
 
 }  // namespace
@@ -258,6 +305,7 @@ TORCH_LIBRARY(aluminum_b200, m) {
   m.def("batch_norm_act_twice(Tensor x, Tensor weight, Tensor bias, Tensor? residual, Tensor(a!) running_mean, Tensor(b!) running_var, "
         "Tensor(c!)? batches, float momentum, float eps, bool relu) -> (Tensor, Tensor)",
         batch_norm_act_twice);
+  m.def("cast_all(Tensor[] weights, ScalarType type) -> Tensor[]", cast_all);
   m.def("stem_conv(Tensor x, Tensor weight, ScalarType type) -> Tensor", stem_conv);
   m.def("max_pool(Tensor x, int k, int stride, int pad) -> Tensor", max_pool);
 }

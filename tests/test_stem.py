@@ -98,3 +98,45 @@ def test_calls_that_stay_with_the_module():
     assert not taken(hooked, x)
     compiled = torch.compile(lambda c, v: stem_conv(c, v), backend="eager", fullgraph=True)
     assert compiled(conv, x).shape == (2, 16, 10, 10)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_weights_cast_together(dtype):
+    """Values, gradients and their layouts of autocast's casts one by one; sizes around a tile; a weight that goes unused."""
+    from aluminum_b200.ops.convolution import cast_weights, convolve
+    torch.manual_seed(0)
+    cl = dict(memory_format=torch.channels_last)
+    convs = [nn.Conv2d(16, 32, 3, padding=1, bias=False), nn.Conv2d(32, 128, 1, bias=False), nn.Conv2d(128, 7, 3, stride=2, bias=False),
+             nn.Conv2d(16, 1, 1, bias=False)]
+    convs = [c.cuda().to(**cl) for c in convs]
+    x = torch.randn(2, 16, 10, 10, device="cuda").to(dtype).contiguous(**cl)
+
+    def run(together):
+        net = [copy.deepcopy(c) for c in convs]
+        with torch.autocast("cuda", dtype=dtype):
+            w = cast_weights(net, x) if together else [None] * 4
+            y = x
+            for c, v in zip(net[:3], w):
+                assert not together or (v.dtype == dtype and torch.equal(v, c.weight.to(dtype)) and v.stride() == c.weight.stride())
+                y = convolve(c, y, v)
+            y.float().square().mean().backward()
+        return [y] + [c.weight.grad for c in net]
+    for a, b in zip(run(True), run(False)):
+        assert (a is None and b is None) or (torch.allclose(a, b, rtol=1e-2, atol=1e-4) and a.stride() == b.stride() and a.dtype == b.dtype)
+    with torch.autocast("cuda", dtype=dtype):
+        w = cast_weights(convs[:1], x)
+        g, = torch.autograd.grad(convolve(convs[0], x, w[0]).float().square().sum(), convs[0].weight, create_graph=True)
+        assert g.dtype == torch.float32
+        g.square().sum().backward()
+        assert convs[0].weight.grad.isfinite().any()
+        hooked, biased, frozen = (copy.deepcopy(convs[0]) for _ in range(3))
+        hooked.register_forward_pre_hook(lambda *a: None)
+        biased.bias = nn.Parameter(torch.zeros(32, device="cuda"))
+        frozen.weight.requires_grad_(False)
+        for other in (hooked, biased, frozen):
+            assert cast_weights([convs[0], other], x) is None
+        assert cast_weights(convs, x.float()) is None
+        with torch.no_grad():
+            assert cast_weights(convs, x) is None
+    assert cast_weights(convs, x) is None     # no autocast
