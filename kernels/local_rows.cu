@@ -1,12 +1,11 @@
 // Row exchanges of ranks that all live on this GPU: every row from tensor to tensor (the pack and the unpack of sequence <-> head
 // transpositions and of expert dispatch / combine included), where the staging protocol moves it through memory once more.
 //
-// What bounds them is HBM.  One wave of warps walks the exchange; each takes 2 KiB at a time: several rows where they are short, a part
+// What bounds them is HBM.  A warp takes 2 KiB at a time: several rows where they are short, a part
 // of one where it is long, four 16-byte loads per thread under way before the first store, whose row indexes were fetched together
 // just before.  An exchange that is too small to give every warp 2 KiB is dealt in pieces of 512 bytes.
-// Measured, one B200, device time through staging / here, us: transposition of 8 x 1024 x 32 x 128 bf16 (67 MB, 1 KiB rows) 69.7 / 24.4, dispatch of
-// 4 x 4099 tokens of 4 KiB 52.1 / 23.8 and combine 52.1 / 21.3 (20.5 at the copy rate), 2 x 16 rows of 512 bytes 13.9 / 2.3.  (A warp per piece
-// as in local_copy.cu: 57.6 for the first there and back, 27.8, 26.4: the tables of a pair of ranks are looked up once per piece.)
+// Measured, one B200, device time through staging / here, us: transposition of 8 x 1024 x 32 x 128 bf16 (67 MB, 1 KiB rows) 69.7 / 23.6, dispatch of
+// 4 x 4099 tokens of 4 KiB 52.1 / 23.8 and combine 52.1 / 21.3 (20.5 at the copy rate), 2 x 16 rows of 512 bytes 13.9 / 2.3.
 #include "al/cuda/cuda.hpp"
 #include "al/device/kernels.hpp"
 #include "local_reduce.cuh"
@@ -33,14 +32,14 @@ constexpr size_t kTile = 32 * 16 * kLoads;       // bytes that a warp takes at a
  * WORDS: everything lies on 16-byte boundaries; a warp then takes 32 * U words at a time, of several rows where they are short
  * (`group` rows; a row's `per_row` > 1 parts where it is long).  Else one row at a time.
  */
-template <bool WORDS, int U>
+template <bool WORDS, int U, bool EVEN>
 __global__ void __launch_bounds__(kLocalThreads, 2) local_rows_kernel(const __grid_constant__ LocalRowsParams P) {
-  if (__any_sync(0xffffffffu, status_word(P.flags, P.p) != 0)) return;
+  const uint64_t failed = status_word(P.flags, P.p);
   const unsigned lane = threadIdx.x & 31;
-  const unsigned nwarps = gridDim.x * (blockDim.x >> 5), total = P.first[P.p * P.p];
+  const unsigned nwarps = gridDim.x * (blockDim.x >> 5), end = EVEN ? P.first[blockIdx.y + 1] : P.first[P.p * P.p];
   const unsigned wpr = (unsigned)(P.row_bytes / 16);   // words per row
-  for (unsigned t = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); t < total; t += nwarps) {
-    const int q = place_of(P.first, P.p * P.p, t);
+  for (unsigned t = (EVEN ? P.first[blockIdx.y] : 0) + blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); t < end; t += nwarps) {
+    const int q = EVEN ? (int)blockIdx.y : place_of(P.first, P.p * P.p, t);
     const int s = q / P.p, d = q - s * P.p;
     const RowTable &S = P.tab[s], &D = P.tab[d];
     const char* src = (const char*)P.send[s] + S.send_peer_off[d];
@@ -64,13 +63,15 @@ __global__ void __launch_bounds__(kLocalThreads, 2) local_rows_kernel(const __gr
         if (w < words) {
           const unsigned r = P.per_row > 1 ? 0 : w / wpr, c = w - r * wpr;
           at[i] = (uint4*)to(k0 + r) + c;
-          v[i] = ((const uint4*)from(k0 + r))[c];
+          v[i] = load_now((const uint4*)from(k0 + r) + c);
         }
       }
+      if (__any_sync(0xffffffffu, failed != 0)) return;
 #pragma unroll
       for (int i = 0; i < U; ++i)
         if (w0 + 32 * i < words) *at[i] = v[i];
     } else {
+      if (__any_sync(0xffffffffu, failed != 0)) return;
       group_copy<kLoads, Rest::row>(to(unit), from(unit), P.row_bytes, false, lane, 32);
     }
   }
@@ -106,10 +107,24 @@ void launch_local_rows(LocalRowsParams& P, int max_ctas, int threads, cudaStream
     }
   P.first[p * p] = n;
   if (n == 0) return;
-  const unsigned ctas = local_grid(n, max_ctas > 0 ? max_ctas : 148 * (1024 / threads), threads);
-  if (!words) local_rows_kernel<false, 1><<<ctas, (unsigned)threads, 0, stream>>>(P);
-  else if (small) local_rows_kernel<true, 1><<<ctas, (unsigned)threads, 0, stream>>>(P);
-  else local_rows_kernel<true, kLoads><<<ctas, (unsigned)threads, 0, stream>>>(P);
+  // Pairs of about the same size: each has its part of the grid, and every warp one unit (transposition of 8 x 1024 x 32 x 128 there and back
+  // 47.2 us, 48.7 with one wave that walks them; dispatch and combine of uneven pairs 23.8 and 21.3 in one wave, 26.2 and 24.4 with a
+  // warp per unit that looks its pair up).
+  unsigned most = 0;
+  for (int q = 0; q < p * p; ++q) most = std::max(most, P.first[q + 1] - P.first[q]);
+  auto run = [&](auto kernel, dim3 grid) { kernel<<<grid, (unsigned)threads, 0, stream>>>(P); };
+  const int each = max_ctas > 0 ? std::max(1, max_ctas / (p * p)) : 0;
+  if ((size_t)most * (size_t)(p * p) <= (size_t)n + n / 4) {
+    const dim3 grid(local_grid(most, each, threads), (unsigned)(p * p));
+    if (!words) run(local_rows_kernel<false, 1, true>, grid);
+    else if (small) run(local_rows_kernel<true, 1, true>, grid);
+    else run(local_rows_kernel<true, kLoads, true>, grid);
+  } else {
+    const dim3 grid(local_grid(n, max_ctas > 0 ? max_ctas : 148 * (1024 / threads), threads));
+    if (!words) run(local_rows_kernel<false, 1, false>, grid);
+    else if (small) run(local_rows_kernel<true, 1, false>, grid);
+    else run(local_rows_kernel<true, kLoads, false>, grid);
+  }
   AL_CHECK_CUDA(cudaGetLastError());
 }
 
