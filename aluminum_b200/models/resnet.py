@@ -74,6 +74,8 @@ class Shortcut(nn.Sequential):
 
 
 class ResNet(nn.Module):
+    any_layout = True   # the first convolution takes images of any memory layout: the trainer need not lay them out
+
     def __init__(self, layers=(3, 4, 6, 3), num_classes: int = 1000, width: int = 64):
         super().__init__()
         self.c = width

@@ -59,7 +59,7 @@ def stem_conv(conv: nn.Module, x: torch.Tensor) -> torch.Tensor:
         weight, dtype = conv.weight, torch.get_autocast_dtype("cuda")
         if (dtype in _TYPES and type(x) is torch.Tensor and x.dim() == 4 and x.is_cuda and x.dtype in (torch.float32, dtype) and not x.requires_grad
                 and not x.is_inference() and x.shape[1] == 3 and 0 < x.shape[0] * (x.shape[2] + 8) < 1 << 30 and 0 < x.shape[2]
-                and 0 < x.shape[3] <= 4000 and x.get_device() == torch.cuda.current_device()
+                and 0 < x.shape[3] <= 700 and x.get_device() == torch.cuda.current_device()
                 and _weight_ok(weight, x.get_device()) and weight.shape[1:] == (3, 7, 7) and weight.shape[0] % 8 == 0 and 0 < weight.shape[0] <= 4096):
             return _lib.torch_ops().stem_conv.default(x, weight, dtype)
     return conv(x)

@@ -14,6 +14,7 @@ from typing import Iterable, Iterator, Tuple
 import torch
 from torch import nn
 
+from ..ops.activations import _bare
 from .ddp import DataParallel
 
 
@@ -33,7 +34,8 @@ class Trainer:
 
     # ---- one optimisation step on device-resident data -------------------------------------------
     def step_device(self, x: torch.Tensor, y: torch.Tensor) -> torch.Tensor:
-        if self.channels_last and x.dim() == 4:
+        m = getattr(self.dp, "module", None)
+        if self.channels_last and x.dim() == 4 and not (type(m).__dict__.get("any_layout", False) and _bare(m)):
             x = x.contiguous(memory_format=torch.channels_last)  # one device pass; the upload itself stays a plain copy
         with torch.autocast("cuda", dtype=self.autocast_dtype, enabled=self.autocast_dtype is not None):
             out = self.dp(x)

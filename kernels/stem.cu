@@ -7,8 +7,9 @@
 // (48 channels, and 16 of zeros) make one pixel, and the convolution becomes one of 64 channels over four rows, which takes 261 and
 // 168 us.  (48 channels 335 / 179, two by two pixels as 16 channels and 4 x 4 taps 516 / 588, the seven rows on their own 273 / 326.)
 //
-// What bounds the layout kernel is writing 128 bytes per pixel (422 MB in that case).  A CTA has two input rows: it reads each once,
-// converts them into shared memory with their borders, and its threads write 16 bytes of a pixel each, eight to a pixel.
+// What bounds the layout kernel is writing 128 bytes per pixel (422 MB in that case).  A CTA has eight input rows, a warp one of them: it
+// reads each once, converts it into shared memory with its border, and the threads write 16 bytes of a pixel each, eight to a
+// pixel.  (With two rows to a CTA the loads' latency was most of it: 141 us; now 93, 88 at the copy rate.)
 #include "al/cuda/cuda.hpp"
 #include "al/device/kernels.hpp"
 #include "datamove.cuh"
@@ -22,6 +23,8 @@ namespace {
 constexpr int kThreads = 256;
 constexpr int kSeen = 8, kIn = 3, kCh = 64;   // columns that an output sees (one more than it has taps), channels of an image, of a pixel here
 constexpr int kRow = kSeen * kIn;             // values of one input row
+constexpr int kPairs = 4;                     // row pairs of a CTA: as many rows as it has warps
+static_assert(2 * kPairs == kThreads / 32, "a warp has one row");
 
 template <typename Ti, typename To>
 __global__ void __launch_bounds__(kThreads) stem_gather_kernel(const __grid_constant__ StemShape s, const Ti* __restrict__ x, To* __restrict__ out,
@@ -36,31 +39,69 @@ __global__ void __launch_bounds__(kThreads) stem_gather_kernel(const __grid_cons
     packed[i] = c < 2 * kRow && u < 7 && v < 7 ? Elem<To>::down(weight[o * s.ws[0] + ch * s.ws[1] + u * s.ws[2] + v * s.ws[3]]) : zero;
     return;
   }
-  extern __shared__ uint32_t smem[];   // two rows of (columns + border) x 3 values
-  const int cols = 2 * s.ow + 6, n = (int)(blockIdx.x / (unsigned)(s.oh + 3)), r = (int)(blockIdx.x % (unsigned)(s.oh + 3));
-  To* rowbuf = (To*)smem;
-  const Ti* image = x + (ptrdiff_t)n * s.xs[0];
-  for (int by = 0; by < 2; ++by) {
-    const int h = 2 * r + by - 3;
-    const bool in = h >= 0 && h < s.h;
-    const Ti* line = image + (ptrdiff_t)h * s.xs[2];
-    for (int i = threadIdx.x; i < cols * kIn; i += kThreads) {
-      // neighbours in memory go to neighbouring threads, whichever way the image is laid out
-      const int ch = s.xs[1] == 1 ? i % kIn : i / cols, pc = s.xs[1] == 1 ? i / kIn : i % cols, w = pc - 3;
-      rowbuf[(by * cols + pc) * kIn + ch] = in && w >= 0 && w < s.w ? as(line[(ptrdiff_t)w * s.xs[3] + ch * s.xs[1]]) : zero;
+  extern __shared__ uint32_t smem[];   // 2 kPairs rows of (columns + border) x 3 values
+  const int cols = 2 * s.ow + 6, groups = (s.oh + 3 + kPairs - 1) / kPairs;
+  const int n = (int)(blockIdx.x / (unsigned)groups), r0 = (int)(blockIdx.x % (unsigned)groups) * kPairs;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  {
+    const int h = 2 * r0 + warp - 3;
+    To* buf = (To*)smem + warp * cols * kIn;
+    const Ti* line = x + (ptrdiff_t)n * s.xs[0] + (ptrdiff_t)h * s.xs[2];
+    if (h < 0 || h >= s.h) {
+      for (int i = lane; i < cols * kIn; i += 32) buf[i] = zero;
+    } else {
+      for (int i = lane; i < 3 * kIn; i += 32) buf[i] = zero;
+      for (int i = (s.w + 3) * kIn + lane; i < cols * kIn; i += 32) buf[i] = zero;
+      buf += 3 * kIn;
+      const int run = s.w * kIn;
+      if (s.xs[1] == 1 && s.xs[3] == kIn && sizeof(Ti) == 4 && (uintptr_t)line % 16 == 0) {   // channels-last: one run of values
+        for (int i0 = 0; i0 < run / 4; i0 += 4 * 32) {
+          float4 v[4];
+#pragma unroll
+          for (int k = 0; k < 4; ++k)
+            if (i0 + k * 32 + lane < run / 4) v[k] = ((const float4*)line)[i0 + k * 32 + lane];
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            const int i = i0 + k * 32 + lane;
+            if (i < run / 4) {
+              buf[4 * i] = Elem<To>::down(v[k].x);
+              buf[4 * i + 1] = Elem<To>::down(v[k].y);
+              buf[4 * i + 2] = Elem<To>::down(v[k].z);
+              buf[4 * i + 3] = Elem<To>::down(v[k].w);
+            }
+          }
+        }
+        for (int i = run / 4 * 4 + lane; i < run; i += 32) buf[i] = as(line[i]);
+      } else {
+        for (int w0 = 0; w0 < s.w; w0 += 4 * 32) {   // any strides: the channels of four pixels under way at once
+          Ti v[4][kIn];
+#pragma unroll
+          for (int k = 0; k < 4; ++k)
+#pragma unroll
+            for (int ch = 0; ch < kIn; ++ch)
+              if (w0 + k * 32 + lane < s.w) v[k][ch] = line[(ptrdiff_t)(w0 + k * 32 + lane) * s.xs[3] + ch * s.xs[1]];
+#pragma unroll
+          for (int k = 0; k < 4; ++k)
+#pragma unroll
+            for (int ch = 0; ch < kIn; ++ch)
+              if (w0 + k * 32 + lane < s.w) buf[(w0 + k * 32 + lane) * kIn + ch] = as(v[k][ch]);
+        }
+      }
     }
   }
   __syncthreads();
   // a pixel's 24 values of a row begin 6 values behind its neighbour's: on 4 bytes, not on 16
-  uint4* dst = (uint4*)out + (size_t)blockIdx.x * s.ow * (kCh / 8);
-  for (int i = threadIdx.x; i < s.ow * (kCh / 8); i += kThreads) {
-    const int j = i / (kCh / 8), k = i % (kCh / 8);
+  const int pixels = min(kPairs, s.oh + 3 - r0) * s.ow, k = threadIdx.x % (kCh / 8);
+  uint4* dst = (uint4*)out + ((size_t)n * (s.oh + 3) + r0) * s.ow * (kCh / 8);
+  int j = threadIdx.x / (kCh / 8) % s.ow, pair = threadIdx.x / (kCh / 8) / s.ow;
+  for (int i = threadIdx.x / (kCh / 8); i < pixels; i += kThreads / (kCh / 8)) {
     uint4 v = uint4{0, 0, 0, 0};
     if (k < 6) {
-      const uint32_t* p = smem + (((k / 3) * cols + 2 * j) * kIn + (k % 3) * 8) / 2;
+      const uint32_t* p = smem + (((2 * pair + k / 3) * cols + 2 * j) * kIn + (k % 3) * 8) / 2;
       v = uint4{p[0], p[1], p[2], p[3]};
     }
-    dst[i] = v;
+    dst[(size_t)i * (kCh / 8) + k] = v;
+    for (j += kThreads / (kCh / 8); j >= s.ow; j -= s.ow) ++pair;
   }
 }
 
@@ -74,15 +115,15 @@ __global__ void __launch_bounds__(kThreads) stem_scatter_kernel(const __grid_con
 }
 
 void check(const StemShape& s) {
-  if (s.n < 1 || s.h < 1 || s.w < 1 || s.oc < 1 || s.oh != (s.h - 1) / 2 + 1 || s.ow != (s.w - 1) / 2 + 1 || s.w > 4000 ||
-      (size_t)s.n * (size_t)(s.oh + 3) > 0x70000000u || s.oc > 1 << 16)
+  if (s.n < 1 || s.h < 1 || s.w < 1 || s.oc < 1 || s.oh != (s.h - 1) / 2 + 1 || s.ow != (s.w - 1) / 2 + 1 ||
+      (size_t)s.n * (size_t)(s.oh + 3) > 0x70000000u || s.w > 700 || s.oc > 1 << 16)
     throw_al_exception("first convolution: unsupported shape");
 }
 
 template <typename Ti, typename To>
 void gather(const StemShape& s, const void* x, void* out, const float* weight, void* packed, cudaStream_t stream) {
-  const unsigned rows = (unsigned)(s.n * (s.oh + 3)), more = (unsigned)((s.oc * 4 * kCh + kThreads - 1) / kThreads);
-  const size_t smem = (size_t)2 * (2 * s.ow + 6) * kIn * sizeof(To);   // (a whole number of 4-byte words: a row is 6 (ow + 3) values)
+  const unsigned rows = (unsigned)(s.n * ((s.oh + 3 + kPairs - 1) / kPairs)), more = (unsigned)((s.oc * 4 * kCh + kThreads - 1) / kThreads);
+  const size_t smem = (size_t)2 * kPairs * (2 * s.ow + 6) * kIn * sizeof(To);   // (a whole number of 4-byte words: a row is 6 (ow + 3) values)
   stem_gather_kernel<Ti, To><<<rows + more, kThreads, smem, stream>>>(s, (const Ti*)x, (To*)out, weight, (To*)packed, rows);
   AL_CHECK_CUDA(cudaGetLastError());
 }
