@@ -85,6 +85,7 @@ def _declare(lib) -> None:
         "al_halo_exchange": (i, [vp, vpp, sz, sz, sz, sz, i, i, vp]),
         "al_halo_pack": (i, [vp, vp, sz, sz, sz, sz, sz, i, vp]),
         "al_route_rows": (i, [vp, i, vpp, szp, vpp, vp, vp]),
+        "al_route_rows_read": (i, [vp, i, vpp, szp, vpp, vp, vp, vp]),
         "al_scale_cast": (i, [vp, i, vp, i, sz, d, vp]),
         "al_sgd_momentum": (i, [vp, vp, vp, sz, C.c_float, C.c_float, C.c_float, C.c_float, i, i, vp]),
         "al_fill_u32": (i, [vp, sz, C.c_uint32, vp]),

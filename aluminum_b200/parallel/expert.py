@@ -4,7 +4,8 @@ Both directions are one row exchange (kernels/rows.cu): dispatch reads the token
 permutation inside the kernel's publish step (no gather into a packed send buffer) and combine writes the
 returning tokens through the same permutation in its consume step (no scatter afterwards).  The per-peer
 token counts are exchanged with a small alltoall and read back with ONE device-to-host copy (the sizes of
-the receive buffer have to be known on the host to allocate it).
+the receive buffer have to be known on the host to allocate it); with all ranks in this process the routing kernel
+leaves them in pinned memory that the host polls.
 """
 from __future__ import annotations
 
@@ -37,11 +38,11 @@ def _on_device(comm, what, tensors):
             raise AlError(f"{what}: must be on the communicator's GPU (cuda:{comm.device_index}), not on {t.device}")
 
 
-# The routing kernel has one block per rank, all ranks at once: 30 us and (0.4 + 0.2 p) us per 1000 tokens.  A sort and a count take
-# 180 us a rank, one rank after the other, and little more for more tokens.  One rank, kernel / sort in us: p = 2, 131072 tokens
-# 137 / 185, 262144 tokens 245 / 216; p = 4, 65536 109 / 183, 131072 187 / 179; p = 8, 65536 167 / 182, 98304 229 / 187.
+# The routing kernel has one block per rank, all ranks at once: 25 us and (0.47 + 0.09 p) us per 1000 tokens.  A sort and a count take
+# 95 to 200 us a rank, one rank after the other, and little more for more tokens.  One rank, kernel / sort in us: p = 2, 131072 tokens
+# 106 / 155, 262144 tokens 186 / 158; p = 4, 131072 121 / 147, 262144 221 / 159; p = 8, 65536 102 / 143, 131072 176 / 143.
 # Sorted from tokens * (p + 2) > this, per local rank, on.
-_SORT_FROM = 820_000
+_SORT_FROM = 950_000
 
 
 def _sorted_route(d, p, counts):
@@ -53,9 +54,10 @@ def _sorted_route(d, p, counts):
     return order
 
 
-def _route(comm, dests):
+def _route(comm, dests, read=False):
     """Stable order of every local rank's tokens by destination, and a (2, local ranks, ranks) buffer whose first half
-    holds the tokens per destination (one launch for all local ranks)."""
+    holds the tokens per destination (one launch for all local ranks).  With ``read`` that half as lists instead, as soon as the
+    launch has them."""
     n, p = len(dests), comm.size
     dests = list(dests)
     _on_device(comm, "dest_rank", dests)
@@ -67,10 +69,16 @@ def _route(comm, dests):
     sizes = [d.numel() for d in dests]
     both = torch.empty((2, n, p), device=dests[0].device, dtype=torch.int64)
     if max(sizes) * (p + 2) > _SORT_FROM * n:
-        return [_sorted_route(d, p, c) for d, c in zip(dests, both[0].unbind())], both
+        order = [_sorted_route(d, p, c) for d, c in zip(dests, both[0].unbind())]
+        return order, both[0].tolist() if read else both
     order = empties(comm, dests, [(s,) for s in sizes])
-    check(_lib.load().al_route_rows(comm._h, n, (C.c_void_p * n)(*[d.data_ptr() for d in dests]), (C.c_size_t * n)(*sizes),
-                                    (C.c_void_p * n)(*[o.data_ptr() for o in order]), both.data_ptr(), comm._stream()))
+    args = (comm._h, n, (C.c_void_p * n)(*[d.data_ptr() for d in dests]), (C.c_size_t * n)(*sizes),
+            (C.c_void_p * n)(*[o.data_ptr() for o in order]), both.data_ptr())
+    if read:
+        counts = (C.c_longlong * (n * p))()
+        check(_lib.load().al_route_rows_read(*args, counts, comm._stream()))
+        return order, [counts[r * p:(r + 1) * p] for r in range(n)]
+    check(_lib.load().al_route_rows(*args, comm._stream()))
     return order, both
 
 
@@ -85,11 +93,11 @@ def dispatch(comm, tokens, dest_rank):
     for t, d in zip(toks, dests):
         if d.numel() > t.shape[0]:
             raise ValueError("dispatch: dest_rank has more entries than there are tokens")
-    order, both = _route(comm, dests)
     if comm.nlocal == p:     # every rank's counts are here
-        sc = both[0].tolist()
+        order, sc = _route(comm, dests, read=True)
         rc = [list(col) for col in zip(*sc)]
     else:
+        order, both = _route(comm, dests)
         call(comm, comm.alltoall, list(both[0].unbind()), list(both[1].unbind()))
         sc, rc = both.tolist()   # the one host read
     if any(c < 0 for row in sc + rc for c in row):

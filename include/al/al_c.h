@@ -195,6 +195,9 @@ int al_halo_pack(float* packed, const float* tensor, size_t nc, size_t d_total, 
 /* Stable order of n[r] tokens by destination rank and counts[r * size + d], for the communicator's nlocal local ranks; counts are -1 where a
    destination is no rank of the communicator.  dest, order and counts are memory of the communicator's GPU. */
 int al_route_rows(void* comm, int nlocal, const long long* const* dest, const size_t* n, long long* const* order, long long* counts, void* stream);
+/** The same for communicators whose ranks all live in this process: waits for the counts (not for the order) and leaves them in host[nlocal * size]. */
+int al_route_rows_read(void* comm, int nlocal, const long long* const* dest, const size_t* n, long long* const* order, long long* counts,
+                       long long* host, void* stream);
 
 /* ---- element-wise kernels ---- */
 int al_scale_cast(void* out, int out_dt, const void* in, int in_dt, size_t n, double scale, void* stream);

@@ -174,6 +174,12 @@ class DeviceCommunicator {
    */
   void exchange_rows(const std::vector<internal::device::RowArgs>& ranks, size_t row_bytes, size_t send_row_stride,
                      size_t recv_row_stride, cudaStream_t stream);
+  /**
+   * Order of every local rank's tokens by destination and their counts (device memory, [local rank][rank]); with `host` also the
+   * counts in host memory, for which the call then waits.
+   */
+  void route(int nlocal, const long long* const* dest, const size_t* n, long long* const* order, long long* counts, long long* host,
+             cudaStream_t stream);
   /** Enqueue point-to-point transfers that progress together. */
   void p2p(const std::vector<internal::device::P2PDesc>& items, cudaStream_t stream);
 

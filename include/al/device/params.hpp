@@ -338,6 +338,9 @@ struct RouteParams {
   size_t n[kMaxRanks];               ///< tokens
   long long* order[kMaxRanks];       ///< tokens by destination, in order among those of one destination
   long long* counts;                 ///< [local rank][p]: tokens per destination; all -1 if a destination is none of the p ranks
+  long long* host_counts;            ///< nullptr, or the same in pinned host memory, followed by ...
+  unsigned long long* host_flags;    ///< ... host_seq in word [local rank]
+  unsigned long long host_seq;
   int p;
 };
 

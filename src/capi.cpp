@@ -627,17 +627,16 @@ int al_route_rows(void* comm, int nlocal, const long long* const* dest, const si
   return guard([&] {
     DeviceCommunicator& c = *(DeviceCommunicator*)comm;
     ScopedDevice on_device(c.device());
-    const int expect = c.is_emulated() ? c.size() : 1;
-    if (nlocal != expect) throw_al_exception("expected ", expect, " local rank(s), got ", nlocal);
-    device::RouteParams P{};
-    for (int r = 0; r < nlocal; ++r) {
-      P.dest[r] = dest[r];
-      P.n[r] = n[r];
-      P.order[r] = order[r];
-    }
-    P.counts = counts;
-    P.p = c.size();
-    device::launch_route(P, nlocal, pick_stream(&c, stream));
+    c.route(nlocal, dest, n, order, counts, nullptr, pick_stream(&c, stream));
+  });
+}
+
+int al_route_rows_read(void* comm, int nlocal, const long long* const* dest, const size_t* n, long long* const* order, long long* counts,
+                       long long* host, void* stream) {
+  return guard([&] {
+    DeviceCommunicator& c = *(DeviceCommunicator*)comm;
+    ScopedDevice on_device(c.device());
+    c.route(nlocal, dest, n, order, counts, host, pick_stream(&c, stream));
   });
 }
 

@@ -59,6 +59,14 @@ struct DeviceCommunicator::Impl {
   size_t off_ll() const { return off_mbox() + (size_t)p * (size_t)ws.mbox_slots * ws.mbox_slot_bytes; }
   uint64_t p2p_launches = 0;
   uint64_t* stamps_dev = nullptr;
+  // What a routing launch writes for the host: one page per call under way, kept for the next call.
+  struct Mail {
+    long long counts[kMaxRanks * kMaxRanks];
+    unsigned long long flags[kMaxRanks];
+    unsigned long long seq;   // host only
+  };
+  std::vector<Mail*> mail_free, mail_all;
+  std::mutex mail_mu;
 
   void setup(std::unique_ptr<SymmBlock> b, int p_, int rank0_, int nlocal_) {
     p = p_; rank0 = rank0_; nlocal = nlocal_;
@@ -97,6 +105,7 @@ struct DeviceCommunicator::Impl {
     if (stamps_dev) AL_WARN_CUDA(cudaFree(stamps_dev));
     if (chain_event) AL_WARN_CUDA(cudaEventDestroy(chain_event));
     if (status_host) AL_WARN_CUDA(cudaFreeHost(status_host));
+    for (Mail* m : mail_all) AL_WARN_CUDA(cudaFreeHost(m));
   }
 
   static size_t block_bytes(int p, size_t half, size_t slot, int slots, size_t ll_slot) {
@@ -1130,6 +1139,68 @@ void DeviceCommunicator::exchange_rows(const std::vector<RowArgs>& ranks, size_t
   I.stats.kernels++;
   I.stats.rows++;
   launch_rows(R, ctas, threads, I.nlocal, stream);
+}
+
+// ---------------------------------------------------------------------------
+// order of tokens by destination
+// ---------------------------------------------------------------------------
+void DeviceCommunicator::route(int nlocal, const long long* const* dest, const size_t* n, long long* const* order, long long* counts,
+                               long long* host, cudaStream_t stream) {
+  Impl& I = *impl_;
+  if (nlocal != I.nlocal) throw_al_exception("expected ", I.nlocal, " local rank(s), got ", nlocal);
+  RouteParams P{};
+  for (int r = 0; r < nlocal; ++r) {
+    P.dest[r] = dest[r];
+    P.n[r] = n[r];
+    P.order[r] = order[r];
+  }
+  P.counts = counts;
+  P.p = I.p;
+  if (!host) return launch_route(P, nlocal, stream);
+  cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+  AL_CHECK_CUDA(cudaStreamIsCapturing(stream, &capturing));
+  if (capturing != cudaStreamCaptureStatusNone) throw_al_exception("the counts of a dispatch are read on the host: it cannot be captured");
+  Impl::Mail* m = nullptr;
+  {
+    std::lock_guard<std::mutex> lock(I.mail_mu);
+    if (I.mail_free.empty()) {
+      void* page = nullptr;
+      AL_CHECK_CUDA(cudaHostAlloc(&page, sizeof(Impl::Mail), cudaHostAllocMapped | cudaHostAllocPortable));
+      memset(page, 0, sizeof(Impl::Mail));
+      I.mail_all.push_back((Impl::Mail*)page);
+      I.mail_free.push_back((Impl::Mail*)page);
+    }
+    m = I.mail_free.back();
+    I.mail_free.pop_back();
+  }
+  void* dev = nullptr;
+  AL_CHECK_CUDA(cudaHostGetDevicePointer(&dev, m, 0));
+  P.host_counts = ((Impl::Mail*)dev)->counts;
+  P.host_flags = ((Impl::Mail*)dev)->flags;
+  P.host_seq = ++m->seq;
+  launch_route(P, nlocal, stream);
+  // Poll; the stream may hold other work of any length first, so the time limit begins when that is known to be over, and a stream
+  // that has failed ends the wait.  (On an error the page is not given back: the kernel may still write it.)
+  auto arrived = [&] {
+    for (int r = 0; r < nlocal; ++r)
+      if (__atomic_load_n(&m->flags[r], __ATOMIC_ACQUIRE) != m->seq) return false;
+    return true;
+  };
+  for (unsigned spin = 1; !arrived(); ++spin) {
+    if (spin % 4096) {
+#if defined(__x86_64__)
+      __builtin_ia32_pause();
+#endif
+      continue;
+    }
+    const cudaError_t e = cudaStreamQuery(stream);
+    if (e == cudaErrorNotReady) continue;
+    AL_CHECK_CUDA(e);
+    if (!arrived()) throw_al_exception("the counts of a dispatch did not arrive");   // (the stream has ended without an error)
+  }
+  std::copy(m->counts, m->counts + nlocal * I.p, host);
+  std::lock_guard<std::mutex> lock(I.mail_mu);
+  I.mail_free.push_back(m);
 }
 
 // ---------------------------------------------------------------------------

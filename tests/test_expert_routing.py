@@ -69,3 +69,47 @@ def test_either_side_of_the_sorting_limit(n):
         assert torch.equal(order[r], torch.argsort(dests[r], stable=True))
         assert torch.equal(both[0][r], torch.bincount(dests[r], minlength=2))
     comm.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("p", [2, 8])
+@pytest.mark.parametrize("tokens", [1, 31, 255, 256, 257, 8191, 8193, 30000])
+def test_counts_that_the_host_polls(p, tokens):
+    """Around what a warp keeps in registers (8 rows of 32 tokens, 32 warps); several calls, also from threads at once; refused under capture."""
+    import threading
+    import aluminum_b200 as al
+    al.init()
+    comm = al.DeviceComm(emulate=p)
+    g = torch.Generator(device="cuda").manual_seed(tokens)
+    dests = [[torch.randint(0, p, (max(0, tokens - r),), generator=g, device="cuda") for r in range(p)] for _ in range(6)]
+
+    def one(d):
+        order, counts = expert._route(comm, d, read=True)
+        for r in range(p):
+            assert counts[r] == torch.bincount(d[r], minlength=p).tolist()
+            assert torch.equal(order[r], torch.argsort(d[r], stable=True))
+    for d in dests:
+        one(d)
+    failed = []
+
+    def run(d):
+        try:
+            with torch.cuda.stream(torch.cuda.Stream()):
+                one(d)
+        except BaseException as e:
+            failed.append(e)
+    torch.cuda.synchronize()
+    threads = [threading.Thread(target=run, args=(d,)) for d in dests]
+    [t.start() for t in threads]
+    [t.join() for t in threads]
+    assert not failed, failed
+    bad = [d.clone() for d in dests[0]]
+    bad[0][-1] = p
+    assert expert._route(comm, bad, read=True)[1][0] == [-1] * p
+    s = torch.cuda.Stream()
+    graph = torch.cuda.CUDAGraph()
+    with pytest.raises(_lib.AlError, match="captured"):
+        with torch.cuda.graph(graph, stream=s):
+            expert._route(comm, dests[0], read=True)
+    one(dests[1])
+    comm.close()
