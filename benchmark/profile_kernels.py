@@ -33,6 +33,7 @@ def main():
         pass
     e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
     comm = None
+    al.set_tuning("local_direct", 0)   # the kernels that ranks on GPUs of their own run
     if a.case != "p2p":   # keep the emulated communicators' workspaces small: these cases do not use the mailboxes
         al.set_tuning("dev_mailbox_bytes", 1 << 20)
         al.set_tuning("p2p_ll_max_bytes", 65536)

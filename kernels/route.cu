@@ -7,8 +7,8 @@
 //
 // One block per rank: what bounds it is latency.  A warp has the destinations of eight rows under way at once and the segments' counts are
 // scanned by warps (one row after the other, and one thread for the scan: 8.3 us for 4 x 4099 tokens, now 7.1; 262144
-// tokens to two ranks 245, now 186).  With all ranks in this
-// process the counts go to pinned host memory, which the host polls, instead of through a copy that it waits for.
+// tokens to two ranks 245, now 186).  With all ranks in this process the counts go to pinned host memory, which the host polls, instead
+// of through a copy that it waits for: dispatch and combine of 4 x 4099 tokens 89.3 -> 77.7 us.
 #include "al/cuda/cuda.hpp"
 #include "al/device/kernels.hpp"
 #include "common.cuh"
