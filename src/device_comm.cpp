@@ -905,7 +905,7 @@ void DeviceCommunicator::collective(const CollDesc& d, const std::vector<RankArg
                           : 0;
 
   // All ranks on this GPU: straight between their buffers, where these allow it and the caller asked for nothing else.
-  const bool moves_uniform = d.kind == DevColl::allgather || d.kind == DevColl::alltoall;
+  const bool moves_uniform = (d.kind == DevColl::allgather || d.kind == DevColl::alltoall) && in == wire;   // (counts in bytes; conversions on the way are staged)
   if (I.emulated && p > 1 && tn.local_direct && !use_window && !tn.bulk_pipeline && !d.vector && d.ctas <= 0 && P.count > 0 && in == out &&
       (d.kind == DevColl::allreduce ? d.algo == AllreduceAlgo::automatic : d.path == CollPath::automatic) &&
       (d.kind == DevColl::allreduce || d.kind == DevColl::reduce_scatter || moves_uniform) &&

@@ -379,3 +379,19 @@ def test_halo_equals_flags(al, shape):
 def test_halo_between_gpus(al, staged):
     from test_device_misc import test_halo_exchange_emulated
     test_halo_exchange_emulated(al)
+
+
+@pytest.mark.parametrize("n", [3, 700_001])
+def test_movement_with_a_wire_type_is_not_taken(al, n):
+    """Its counts are elements, not bytes: it stays with the staged kernels."""
+    p = 4
+    comm = al.DeviceComm(emulate=p)
+
+    def call():
+        xs, full = ([values(m, torch.float32, r) for r in range(p)] for m in (n, p * n))
+        every, moved = ([torch.zeros(p * n, device="cuda") for _ in range(p)] for _ in range(2))
+        comm.allgather(xs, every, wire_dtype=torch.bfloat16)
+        comm.alltoall(full, moved, wire_dtype=torch.bfloat16)
+        return every + moved
+    same(*both(al, comm, call, 0))
+    comm.close()
