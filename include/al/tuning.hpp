@@ -38,6 +38,11 @@ struct Crossovers {
   size_t rs_nvls_min_bytes;        ///< AL_RS_NVLS_MIN: total message size from which reduce_scatter of private buffers reduces in the switch (staged NVLS; needs multicast and more than two ranks)
 };
 
+/** The sizes up to which operations travel as packets. */
+inline bool packet_limit(size_t Crossovers::*f) {
+  return f == &Crossovers::ll_max_bytes || f == &Crossovers::ar_ll_max_bytes || f == &Crossovers::ar_ll2_max_bytes;
+}
+
 struct Tuning {
   // ---- progress engine ------------------------------------------------------
   int pe_num_concurrent_ops = AL_PE_NUM_CONCURRENT_OPS_DEFAULT;  ///< AL_PE_NUM_CONCURRENT_OPS
@@ -71,6 +76,7 @@ struct Tuning {
   int threads_per_cta = 512;                   ///< AL_THREADS_PER_CTA
   int p2p_max_ctas = 64;                       ///< AL_DEV_P2P_CTAS: most CTAs one send or receive of a point-to-point launch gets (one per 64 KiB of a mailbox piece)
   bool local_direct = true;                    ///< AL_LOCAL_DIRECT: with all ranks of a communicator on one GPU, operations whose path the caller leaves open run straight between the ranks' buffers (0: through staging, packets and mailboxes, as between GPUs)
+  bool ll_limits_set = false;                  ///< a packet limit (ll_max_bytes, ar_ll_max_bytes, ar_ll2_max_bytes) was set by the environment or al_set_tuning: it is then obeyed with all ranks on one GPU too, where packets are otherwise left out
   bool bulk_pipeline = false;                  ///< AL_DEV_BULK_PIPELINE: pipelined reduce_scatter / allgather / alltoall move their data with the bulk copy engine (cp.async.bulk) when every buffer is 16-byte aligned
   int bulk_pub_ctas = 16;                      ///< AL_DEV_BULK_PUB_CTAS: publishing CTAs of that kernel (one issuing thread each)
   int bulk_con_ctas = 16;                      ///< AL_DEV_BULK_CON_CTAS: its consuming CTAs for allgather / alltoall (reduce_scatter reduces with SM loads and takes max_ctas/2)

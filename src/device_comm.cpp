@@ -145,8 +145,9 @@ struct DeviceCommunicator::Impl {
 
   void begin_local(uint64_t** flags, cudaStream_t stream);
   void end_local();
-  bool local_reduce(const CollParams& P, DType user, DType wire, ReductionOperator op, cudaStream_t stream);
-  bool local_move(const CollParams& P, cudaStream_t stream);
+  bool local_collective(const CollDesc& d, const std::vector<RankArgs>& ranks, DType user, DType wire, size_t count, double scale, int int_div,
+                        cudaStream_t stream);
+  void local_move(bool gathers, const std::vector<RankArgs>& ranks, size_t count, cudaStream_t stream);
   size_t local_p2p(const std::vector<P2PDesc>& items, std::vector<char>& placed, cudaStream_t stream);
   bool local_rows(const RowsParams& R, const std::vector<RowArgs>& ranks, size_t total_rows, cudaStream_t stream);
 
@@ -235,7 +236,7 @@ bool own_may_skip_staging(DevColl kind, const CountTable* tab, const Span* sent,
  * buffer, except where a rank's own contribution lies exactly where its result goes (in place): every thread reads the
  * elements that it writes before it writes them.
  */
-bool local_buffers_apart(DevColl kind, const CountTable* tab, const Span* sent, const Span* received, int p, size_t esz) {
+bool local_buffers_apart(DevColl kind, size_t slice, const Span* sent, const Span* received, int p) {
   for (int r = 0; r < p; ++r) {
     if (!sent[r].at || !received[r].at) return false;
     for (int s = 0; s < p; ++s) {
@@ -243,8 +244,8 @@ bool local_buffers_apart(DevColl kind, const CountTable* tab, const Span* sent, 
       if (!received[r].meets(sent[s])) continue;
       if (s != r || kind == DevColl::alltoall) return false;
       const char *own = sent[r].at, *place = received[r].at;
-      if (kind == DevColl::reduce_scatter) own += tab[r].send_displs[r] * esz;
-      if (kind == DevColl::allgather) place += tab[r].recv_displs[r] * esz;
+      if (kind == DevColl::reduce_scatter) own += (size_t)r * slice;
+      if (kind == DevColl::allgather) place += (size_t)r * slice;
       if (own != place) return false;
     }
   }
@@ -426,67 +427,79 @@ void DeviceCommunicator::Impl::end_local() {
   stats.local++;
 }
 
-/** Reductions; false: there is no kernel for this operation or these addresses. */
-bool DeviceCommunicator::Impl::local_reduce(const CollParams& P, DType user, DType wire, ReductionOperator op, cudaStream_t stream) {
-  LocalReduceParams L{};
-  const size_t esz = dtype_size(user);
+/** Uniform operations (`count` elements, or bytes of a movement, per vector or slice); false, and nothing enqueued: the buffers, types or operator do not allow it. */
+bool DeviceCommunicator::Impl::local_collective(const CollDesc& d, const std::vector<RankArgs>& ranks, DType user, DType wire, size_t count, double scale,
+                                                int int_div, cudaStream_t stream) {
+  const size_t esz = dtype_size(user), slice = count * esz, whole = slice * (size_t)p;
+  Span sent[kMaxRanks], received[kMaxRanks];
   for (int r = 0; r < p; ++r) {
-    L.src[r] = P.send[r];
-    L.dst[r] = P.recv[r];
-    if ((uintptr_t)P.send[r] % esz || (uintptr_t)P.recv[r] % esz) return false;
-    if (P.kind == (int)DevColl::allreduce && ((uintptr_t)P.recv[r] ^ (uintptr_t)P.recv[0]) % 16) return false;
+    const RankArgs& a = ranks[(size_t)r];
+    sent[r] = Span{(const char*)a.send, d.kind == DevColl::reduce_scatter || d.kind == DevColl::alltoall ? whole : slice};
+    received[r] = Span{(const char*)a.recv, d.kind == DevColl::allgather || d.kind == DevColl::alltoall ? whole : slice};
   }
-  L.count = P.count;
-  L.scale = P.scale;
-  L.int_div = P.int_div;
-  L.p = p;
-  L.scatter = P.kind == (int)DevColl::reduce_scatter;
-  L.round_result = user != wire && P.two_phase;
-  begin_local(L.flags, stream);
-  const int threads = local_threads();
-  if (!launch_local_reduce(L, user, wire, op, local_ctas(tuning().max_ctas, p, sm_count), threads, stream)) return false;
+  const bool moves = d.kind == DevColl::allgather || d.kind == DevColl::alltoall;
+  if (moves && user != wire) return false;   // (conversions on the way: the staged kernels)
+  if (!local_buffers_apart(d.kind, slice, sent, received, p)) return false;
+  if (moves) {
+    local_move(d.kind == DevColl::allgather, ranks, count, stream);
+  } else {
+    LocalReduceParams L{};
+    for (int r = 0; r < p; ++r) {
+      L.src[r] = ranks[(size_t)r].send;
+      L.dst[r] = ranks[(size_t)r].recv;
+      if ((uintptr_t)L.src[r] % esz || (uintptr_t)L.dst[r] % esz) return false;
+      if (d.kind == DevColl::allreduce && ((uintptr_t)L.dst[r] ^ (uintptr_t)L.dst[0]) % 16) return false;
+    }
+    L.count = count;
+    L.scale = scale;
+    L.int_div = int_div;
+    L.p = p;
+    L.scatter = d.kind == DevColl::reduce_scatter;
+    // (where the staged protocol would reduce in two phases, the result too crosses in the narrower type)
+    L.round_result = user != wire && p > 2 && d.kind == DevColl::allreduce && count * dtype_size(wire) > tuning().crossovers(p).ar_oneshot_max_bytes;
+    begin_local(L.flags, stream);
+    const int threads = local_threads();
+    if (!launch_local_reduce(L, user, wire, d.op, local_ctas(tuning().max_ctas, p, sm_count), threads, stream)) return false;
+  }
   end_local();
+  stats.bytes += count * dtype_size(wire);
   return true;
 }
 
-/** Allgather and alltoall (counts in bytes). */
-bool DeviceCommunicator::Impl::local_move(const CollParams& P, cudaStream_t stream) {
+/** Allgather or alltoall of `count` bytes per slice. */
+void DeviceCommunicator::Impl::local_move(bool gathers, const std::vector<RankArgs>& ranks, size_t count, cudaStream_t stream) {
   LocalCopyParams L{};
   L.p = p;
   L.rows = 1;
-  const bool gathers = P.kind == (int)DevColl::allgather;
   L.fans = gathers;
   for (int r = 0; r < p; ++r) {
-    L.fan[r] = (char*)P.recv[r];
-    L.fans = L.fans && ((uintptr_t)P.recv[r] ^ (uintptr_t)P.recv[0]) % 16 == 0;
+    L.fan[r] = (char*)ranks[(size_t)r].recv;
+    L.fans = L.fans && ((uintptr_t)L.fan[r] ^ (uintptr_t)L.fan[0]) % 16 == 0;
   }
   for (int s = 0; s < p; ++s) {
-    const char* from = (const char*)P.send[s];
-    const size_t at = (size_t)s * P.count;   // of rank s's slice in a result
+    const char* from = (const char*)ranks[(size_t)s].send;
+    const size_t at = (size_t)s * count;   // of rank s's slice in a result
     if (L.fans) {
       const int j = L.jobs++;
       L.src[j] = from;
       L.dst[j] = (char*)at;
-      L.bytes[j] = P.count;
+      L.bytes[j] = count;
       L.to[j] = (unsigned char)((1u << p) - 1);
       if (from == L.fan[s] + at) L.to[j] &= (unsigned char)~(1u << s);   // in place
       continue;
     }
     for (int i = 0; i < p; ++i) {
       const int d = (s + i) % p;
-      const char* src = gathers ? from : from + (size_t)d * P.count;
+      const char* src = gathers ? from : from + (size_t)d * count;
       if (src == L.fan[d] + at) continue;
       const int j = L.jobs++;
       L.src[j] = src;
       L.dst[j] = L.fan[d] + at;
-      L.bytes[j] = P.count;
+      L.bytes[j] = count;
     }
   }
   begin_local(L.flags, stream);
-  const int threads = local_threads();
-  launch_local_copy(L, local_ctas(tuning().max_ctas, p, sm_count), threads, stream);
-  end_local();
-  return true;
+  launch_local_copy(L, local_ctas(tuning().max_ctas, p, sm_count), local_threads(), stream);
 }
 
 /**
@@ -646,6 +659,26 @@ void DeviceCommunicator::collective(const CollDesc& d, const std::vector<RankArg
   if (!reduces && !(in == wire && wire == out) && !collective_supported(in, wire, out, ReductionOperator::sum))
     throw_al_exception("device backend: no kernel for this datatype conversion");
 
+  // All ranks on this GPU and nothing asked for but the operation: straight between the buffers, at every size unless the caller has set
+  // the packets' limits (device time of packets / between buffers, us: 8 x 1 KiB fp32 4.9 / 2.2, 4 x 600 KB bf16 8.7 / 2.8,
+  // 8 x 1 MiB fp32 23.5 / 3.6).
+  // Registered buffers, which the window kernels may want, are looked at first.
+  const Tuning& tn = tuning();
+  const bool local_open = I.emulated && p > 1 && tn.local_direct && !tn.bulk_pipeline && !d.vector && d.ctas <= 0 && d.count > 0 && in == out &&
+                          (d.kind == DevColl::allreduce ? d.algo == AllreduceAlgo::automatic : d.path == CollPath::automatic) &&
+                          (d.kind == DevColl::allreduce || d.kind == DevColl::reduce_scatter || d.kind == DevColl::allgather ||
+                           d.kind == DevColl::alltoall);
+  double scale = d.scale;
+  int int_div = 1;
+  if (d.op == ReductionOperator::avg) {
+    if (dtype_is_float(wire)) scale *= 1.0 / p;
+    else int_div = p;
+  }
+  if (local_open && !tn.ll_limits_set &&
+      (d.kind == DevColl::allreduce || d.count * unit * dtype_size(wire) * (size_t)p < tn.crossovers(p).window_min_bytes) &&
+      I.local_collective(d, ranks, in, wire, d.count * unit, scale, int_div, stream))
+    return;
+
   // Small uniform allreduce / reduce_scatter / allgather / alltoall travel as low-latency packets.  This
   // is decided first, before anything else is prepared: these calls are all about the time the host spends
   // here.  Eligibility depends on facts every rank shares (operation, count, type), so the ranks agree.
@@ -666,7 +699,6 @@ void DeviceCommunicator::collective(const CollDesc& d, const std::vector<RankArg
     if (forced && !fits && !fits2)
       throw_al_exception("the low-latency path was requested but the operation does not qualify (uniform allreduce / "
                          "reduce_scatter / allgather / alltoall of at most ", kLLPayloadBytes, " bytes per pair of ranks)");
-    const Tuning& tn = tuning();
     // One-phase packets cost an allreduce p-1 times the vector per rank: its limit is lower than that of the
     // other three operations (whose pair_bytes is one slice) and shrinks with the number of ranks.
     const size_t one_phase_max = d.kind == DevColl::allreduce
@@ -685,12 +717,8 @@ void DeviceCommunicator::collective(const CollDesc& d, const std::vector<RankArg
       L.count = d.count * unit;
       L.seq = ++I.seq;
       L.timeout_ns = I.timeout_ns;
-      L.scale = d.scale;
-      L.int_div = 1;
-      if (d.op == ReductionOperator::avg) {
-        if (dtype_is_float(wire)) L.scale *= 1.0 / p;
-        else L.int_div = p;
-      }
+      L.scale = scale;
+      L.int_div = int_div;
       L.kind = (int)d.kind;
       L.op = (int)d.op;
       L.rank0 = I.rank0;
@@ -717,12 +745,8 @@ void DeviceCommunicator::collective(const CollDesc& d, const std::vector<RankArg
   P.root = d.root;
   P.rank0 = I.rank0;
   P.count = d.count * unit;
-  P.scale = d.scale;
-  P.int_div = 1;
-  if (d.op == ReductionOperator::avg) {
-    if (dtype_is_float(wire)) P.scale *= 1.0 / p;
-    else P.int_div = p;
-  }
+  P.scale = scale;
+  P.int_div = int_div;
 
   const size_t esz = dtype_size(wire);
   const size_t half = I.ws.half_bytes;
@@ -732,7 +756,6 @@ void DeviceCommunicator::collective(const CollDesc& d, const std::vector<RankArg
   size_t max_work_bytes = 0;
 
   // ---- algorithm -----------------------------------------------------------------
-  const Tuning& tn = tuning();
   const Crossovers& X = tn.crossovers(p);
   const size_t bytes = P.count * esz;
   AllreduceAlgo algo = d.algo;
@@ -904,16 +927,7 @@ void DeviceCommunicator::collective(const CollDesc& d, const std::vector<RankArg
                           ? 1
                           : 0;
 
-  // All ranks on this GPU: straight between their buffers, where these allow it and the caller asked for nothing else.
-  const bool moves_uniform = (d.kind == DevColl::allgather || d.kind == DevColl::alltoall) && in == wire;   // (counts in bytes; conversions on the way are staged)
-  if (I.emulated && p > 1 && tn.local_direct && !use_window && !tn.bulk_pipeline && !d.vector && d.ctas <= 0 && P.count > 0 && in == out &&
-      (d.kind == DevColl::allreduce ? d.algo == AllreduceAlgo::automatic : d.path == CollPath::automatic) &&
-      (d.kind == DevColl::allreduce || d.kind == DevColl::reduce_scatter || moves_uniform) &&
-      local_buffers_apart(d.kind, P.tab, sent, received, p, dtype_size(in)) &&
-      (moves_uniform ? I.local_move(P, stream) : I.local_reduce(P, in, wire, d.op, stream))) {
-    I.stats.bytes += bytes;
-    return;
-  }
+  if (local_open && !use_window && I.local_collective(d, ranks, in, wire, P.count, P.scale, P.int_div, stream)) return;
 
   // All ranks on this GPU: large operations are moved by the bulk copy engine, chunked by what staging holds.
   // (Its CTAs take a whole SM each, so a caller who asked for smaller CTAs gets the loops.)

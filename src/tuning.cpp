@@ -61,7 +61,9 @@ void Tuning::load_from_env() {
       for (int row = 0; row < 3; ++row) {
         long v = env_long(e.env, -1);
         v = env_long((std::string(e.env) + suffix[row]).c_str(), v);
-        if (v >= 0) cross[row].*(e.field) = (size_t)v;
+        if (v < 0) continue;
+        cross[row].*(e.field) = (size_t)v;
+        ll_limits_set = ll_limits_set || packet_limit(e.field);
       }
   }
   window_enable = env_long("AL_WINDOW", window_enable) != 0;
