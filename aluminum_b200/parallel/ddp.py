@@ -171,11 +171,13 @@ class DataParallel:
 
     def backward_and_step(self, loss: torch.Tensor) -> None:
         """``loss.backward()`` and :meth:`step`.  With one rank nothing needs the gradients in the flat buffer: backward leaves
-        them as it made them and the optimizer reads them there, without a launch per tensor that adds them up first."""
+        them as it made them (all of them are then in memory beside the flat buffer until the step) and the optimizer reads them there,
+        without a launch per tensor that adds them up first.  A backward that runs hooks or functions written in Python, which may look at
+        ``flat_grad`` or at a parameter's ``grad``, finds the gradients there instead."""
         own = (type(self).step is DataParallel.step and type(self).finish_gradients is DataParallel.finish_gradients
                and not {"step", "finish_gradients"} & self.__dict__.keys())
         calls = _lib.calls() if self.world == 1 and not self.timeline and own else None
-        if calls is None or not calls.lend_gradients(self._params, self._grad_views):
+        if calls is None or not calls.lend_gradients(loss, self._params, self._grad_views):
             loss.backward()
             self.step()
             return

@@ -17,6 +17,11 @@ def al():
     return al
 
 
+@pytest.fixture(autouse=True)
+def repeatable(monkeypatch):
+    monkeypatch.setattr(torch.backends.cudnn, "deterministic", True)
+
+
 class Odd(torch.autograd.Function):
     """Identity on a parameter whose gradient comes expanded, transposed or off its 16 bytes."""
 
@@ -51,6 +56,14 @@ class Net(nn.Module):
         return x
 
 
+class Native(Net):
+    """The same without functions written in Python: gradients that are parts of one tensor, off their 16 bytes among them."""
+
+    def forward(self, x):
+        x = self.wide(self.bn(self.conv(x)).flatten(1))
+        return x + torch.cat([p.flatten() for p in self.odd]).square().sum()
+
+
 def pair(net, **kw):
     from aluminum_b200.parallel import DataParallel, Trainer
     made = []
@@ -61,10 +74,10 @@ def pair(net, **kw):
     return made
 
 
-def test_equals_the_step_on_the_flat_gradient(monkeypatch):
-    monkeypatch.setattr(torch.backends.cudnn, "deterministic", True)
+@pytest.mark.parametrize("net", [Net, Native])
+def test_equals_the_step_on_the_flat_gradient(net):
     torch.manual_seed(0)
-    (a, da), (b, db) = pair(Net())
+    (a, da), (b, db) = pair(net())
     x, y = torch.randn(6, 3, 8, 8, device="cuda"), torch.randint(0, 1029, (6,), device="cuda")
     for k in range(4):
         if k == 2:     # gradients that a backward of the caller's own has left
@@ -79,6 +92,99 @@ def test_equals_the_step_on_the_flat_gradient(monkeypatch):
             assert p.grad is view
     da.lr = db.lr = 0.5
     assert torch.equal(a.step_device(x, y), b.step_device(x, y)) and torch.equal(da.flat_param, db.flat_param)
+
+
+def lend(dp, x):
+    """A backward on lent gradients; False: they were not lent."""
+    from aluminum_b200 import _lib
+    loss = dp(x).square().mean()
+    if not _lib.calls().lend_gradients(loss, dp._params, dp._grad_views):
+        return False
+    assert all(p.grad is None for p in dp._params)
+    loss.backward()
+    return True
+
+
+def test_which_forms_reach_the_optimizer():
+    torch.manual_seed(0)
+    (_, da), (_, db) = pair(Native())
+    x = torch.randn(6, 3, 8, 8, device="cuda")
+    assert lend(da, x) and not lend(pair(Net())[0][1], x)
+    assert any(p.grad is not None and p.grad.data_ptr() % 16 for p in da._params) and any(p.grad is None for p in da._params)
+
+
+@pytest.mark.parametrize("kind", ["post_accumulate", "tensor", "module", "node", "activation"])
+def test_what_runs_in_the_backward_finds_the_gradients(kind):
+    """Clipping by way of the flat gradient or of a gradient held from before: lent gradients would be somewhere else."""
+    torch.manual_seed(0)
+    net = nn.Sequential(nn.Conv2d(3, 8, 3), nn.Flatten(), nn.Linear(8 * 36, 10))
+    (a, da), (b, db) = pair(net)
+    x, y, keep = torch.randn(6, 3, 8, 8, device="cuda"), torch.randint(0, 10, (6,), device="cuda"), []
+    for dp in (da, db):
+        held, (conv, _, linear) = [p.grad for p in dp._params], dp.module
+
+        def clip(*_, dp=dp, held=held):
+            dp.flat_grad.mul_(0.25)
+            held[-1].add_(0.125)
+        if kind == "post_accumulate":
+            linear.bias.register_post_accumulate_grad_hook(clip)
+        elif kind == "tensor":
+            conv.bias.register_hook(clip)
+        elif kind == "module":
+            linear.register_full_backward_hook(clip)
+        elif kind == "node":
+            keep.append(linear.bias.expand_as(linear.bias).grad_fn.next_functions[0][0])
+            keep[-1].register_hook(clip)
+        else:
+            conv.register_forward_hook(lambda m, i, o, clip=clip: o.register_hook(clip) and None)
+    for _ in range(2):
+        a.step_device(x, y)
+        b.step_device(x, y)
+    assert torch.equal(da.flat_param, db.flat_param) and torch.equal(da.flat_mom, db.flat_mom)
+
+
+def test_a_gradient_that_is_its_view_counts_once():
+    from aluminum_b200 import _lib
+    torch.manual_seed(0)
+    (_, da), (_, db) = pair(Native())
+    x = torch.randn(6, 3, 8, 8, device="cuda")
+    assert lend(da, x)
+    for k, (p, view) in enumerate(zip(da._params, da._grad_views)):
+        if k % 2 and p.grad is not None:
+            view.copy_(p.grad)
+            p.grad = view.detach() if k % 4 == 1 else view
+    _lib.calls().step_on_lent(da._params, da._grad_views, da.flat_param, da.flat_mom, da.flat_grad, 0.05, 0.9, 1e-3, True)
+    db(x).square().mean().backward()
+    db.step()
+    assert torch.equal(da.flat_param, db.flat_param) and torch.equal(da.flat_mom, db.flat_mom) and not da.flat_grad.any()
+    assert all(p.grad is v for p, v in zip(da._params, da._grad_views))
+
+
+def test_a_step_that_is_refused_keeps_the_gradients():
+    from aluminum_b200 import _lib
+    torch.manual_seed(0)
+    (_, da), (_, db) = pair(Native())
+    x, before = torch.randn(6, 3, 8, 8, device="cuda"), da.flat_param.clone()
+    assert lend(da, x)
+    with pytest.raises(_lib.AlError, match="not of the form"):     # views that do not begin on 16 bytes of the flat buffer
+        _lib.calls().step_on_lent(da._params, da._grad_views, da.flat_param, da.flat_mom, da.flat_grad[1:], 0.05, 0.9, 1e-3, True)
+    db(x).square().mean().backward()
+    assert torch.equal(da.flat_param, before) and torch.equal(da.flat_grad, db.flat_grad)
+    assert all(p.grad is v for p, v in zip(da._params, da._grad_views))
+
+
+def test_a_backward_on_lent_gradients_that_fails_keeps_what_it_has():
+    torch.manual_seed(0)
+    (_, da), _ = pair(Native())
+    net = da.module
+    s = net.conv(torch.randn(6, 3, 8, 8, device="cuda")).square()
+    s.sum().backward()
+    before = [v.clone() for v in da._grad_views]
+    with pytest.raises(RuntimeError, match="second time"):     # behind the last layers, whose gradients are there by then
+        da.backward_and_step(net.wide(net.bn(s).flatten(1)).square().mean())
+    assert da.steps == 0 and all(p.grad is v for p, v in zip(da._params, da._grad_views))
+    for p, was in zip(da._params, before):
+        assert torch.equal(p.grad, was) != (p is net.wide.weight or p is net.wide.bias or p is net.bn.weight or p is net.bn.bias)
 
 
 def test_a_backward_that_fails_keeps_what_it_has():

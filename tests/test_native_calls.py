@@ -117,3 +117,49 @@ def test_python_and_native_calls_agree(p):
     comm.close()
     with pytest.raises(al.AlError, match="closed"):
         comm.allreduce([torch.ones(4, device="cuda") for _ in range(p)])
+
+
+class Same(torch.autograd.Function):
+    @staticmethod
+    def forward(ctx, x):
+        return x.clone()
+
+    @staticmethod
+    def backward(ctx, g):
+        return g
+
+
+def test_gradients_are_lent_where_nothing_looks_at_them(calls):
+    nn, keep = torch.nn, []
+
+    def node_hook(net):
+        keep.append(net[0].weight.expand_as(net[0].weight).grad_fn.next_functions[0][0])
+        keep[-1].register_hook(lambda *a: None)
+
+    def lent(hook=None, use=lambda x: x, own=True):
+        net = nn.Sequential(nn.Linear(3, 4), nn.Linear(4, 2))
+        params = list(net.parameters())
+        for p in params:
+            p.grad = torch.zeros_like(p)
+        views = [p.grad for p in params]
+        if hook is not None:
+            hook(net)
+        if not own:
+            params[1].grad = None
+        was = [p.grad for p in params]
+        loss = use(net(torch.randn(5, 3))).sum()
+        if not calls.lend_gradients(loss, params, views):
+            assert all(p.grad is g for p, g in zip(params, was))
+            return False
+        assert all(p.grad is None for p in params)
+        loss.backward()
+        calls.return_gradients(params, views)
+        assert all(p.grad is v and v.any() for p, v in zip(params, views))
+        return True
+    assert lent() and lent(use=lambda x: x.relu().double()) and not lent(own=False)
+    for hook in (lambda n: n[0].weight.register_hook(lambda g: None), lambda n: n[0].weight.register_post_accumulate_grad_hook(lambda p: None),
+                 lambda n: n[1].register_full_backward_hook(lambda *a: None), lambda n: n[1].register_full_backward_pre_hook(lambda *a: None),
+                 lambda n: n[0].register_forward_hook(lambda m, i, o: o.register_hook(lambda g: None) and None), node_hook,
+                 lambda n: torch.autograd.graph.register_multi_grad_hook(list(n.parameters()), lambda *a: None)):
+        assert not lent(hook)
+    assert not lent(use=Same.apply) and not calls.lend_gradients(None, [], []) and not calls.lend_gradients(torch.zeros(1), [], [])
