@@ -11,7 +11,7 @@ mirrors the reference's ``include/Al.hpp:118-1911``.
 An *emulated* ``DeviceComm`` holds all ``p`` ranks in one process on one GPU;
 every argument then is a list with one tensor per rank and each call is one
 kernel launch: straight between the ranks' buffers where the call leaves the path
-open (and is too large for packets, where a limit of packets was set), else (and with the tuning ``local_direct`` at 0) a
+open (and is too large for packets, where a limit of packets is another than its default), else (and with the tuning ``local_direct`` at 0) a
 cooperative launch of the device protocol, which can so be tested on a single GPU.
 """
 from __future__ import annotations

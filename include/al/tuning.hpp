@@ -38,11 +38,6 @@ struct Crossovers {
   size_t rs_nvls_min_bytes;        ///< AL_RS_NVLS_MIN: total message size from which reduce_scatter of private buffers reduces in the switch (staged NVLS; needs multicast and more than two ranks)
 };
 
-/** The sizes up to which operations travel as packets. */
-inline bool packet_limit(size_t Crossovers::*f) {
-  return f == &Crossovers::ll_max_bytes || f == &Crossovers::ar_ll_max_bytes || f == &Crossovers::ar_ll2_max_bytes;
-}
-
 struct Tuning {
   // ---- progress engine ------------------------------------------------------
   int pe_num_concurrent_ops = AL_PE_NUM_CONCURRENT_OPS_DEFAULT;  ///< AL_PE_NUM_CONCURRENT_OPS
@@ -76,7 +71,6 @@ struct Tuning {
   int threads_per_cta = 512;                   ///< AL_THREADS_PER_CTA
   int p2p_max_ctas = 64;                       ///< AL_DEV_P2P_CTAS: most CTAs one send or receive of a point-to-point launch gets (one per 64 KiB of a mailbox piece)
   bool local_direct = true;                    ///< AL_LOCAL_DIRECT: with all ranks of a communicator on one GPU, operations whose path the caller leaves open run straight between the ranks' buffers (0: through staging, packets and mailboxes, as between GPUs)
-  bool ll_limits_set = false;                  ///< a packet limit (ll_max_bytes, ar_ll_max_bytes, ar_ll2_max_bytes) was set by the environment or al_set_tuning: it is then obeyed with all ranks on one GPU too, where packets are otherwise left out
   bool bulk_pipeline = false;                  ///< AL_DEV_BULK_PIPELINE: pipelined reduce_scatter / allgather / alltoall move their data with the bulk copy engine (cp.async.bulk) when every buffer is 16-byte aligned
   int bulk_pub_ctas = 16;                      ///< AL_DEV_BULK_PUB_CTAS: publishing CTAs of that kernel (one issuing thread each)
   int bulk_con_ctas = 16;                      ///< AL_DEV_BULK_CON_CTAS: its consuming CTAs for allgather / alltoall (reduce_scatter reduces with SM loads and takes max_ctas/2)
@@ -89,6 +83,11 @@ struct Tuning {
   };
   /** Row of the table for a communicator of `p` ranks. */
   const Crossovers& crossovers(int p) const { return cross[p <= 2 ? 0 : (p <= 4 ? 1 : 2)]; }
+  /**
+   * Is one of the packets' limits (ll_max_bytes, ar_ll_max_bytes, ar_ll2_max_bytes), in any row, another than its default?  They are then obeyed with
+   * all ranks on one GPU too, where packets are otherwise left out; with the defaults back in their places that ends.
+   */
+  bool packet_limits_set() const;
   bool window_enable = true;                   ///< AL_WINDOW: uniform reduce_scatter / allgather / alltoall / bcast on registered (or symm_alloc) buffers skip the staging area
   int window_ctas = 128;                       ///< AL_WINDOW_CTAS: CTA budget of a window kernel
   int window_multimem_ag_ranks = 16;          ///< AL_WINDOW_MULTIMEM_AG_RANKS: allgather uses multimem.st from this many ranks on (a multicast store returns to its sender too, which costs 1/(p-1) extra ingress)

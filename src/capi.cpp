@@ -135,7 +135,6 @@ int al_set_tuning(const char* name, double value) {
     if (auto f = crossover_field(n, &row)) {
       for (int r = 0; r < 3; ++r)
         if (row < 0 || row == r) t.cross[r].*f = (size_t)value;
-      t.ll_limits_set = t.ll_limits_set || packet_limit(f);
       return;
     }
 #define X(f) if (n == #f) { t.f = (decltype(t.f))value; return; }

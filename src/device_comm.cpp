@@ -659,8 +659,8 @@ void DeviceCommunicator::collective(const CollDesc& d, const std::vector<RankArg
   if (!reduces && !(in == wire && wire == out) && !collective_supported(in, wire, out, ReductionOperator::sum))
     throw_al_exception("device backend: no kernel for this datatype conversion");
 
-  // All ranks on this GPU and nothing asked for but the operation: straight between the buffers, at every size unless the caller has set
-  // the packets' limits (device time of packets / between buffers, us: 8 x 1 KiB fp32 4.9 / 2.2, 4 x 600 KB bf16 8.7 / 2.8,
+  // All ranks on this GPU and nothing asked for but the operation: straight between the buffers, at every size unless the packets'
+  // limits are set to others than their defaults (device time of packets / between buffers, us: 8 x 1 KiB fp32 4.9 / 2.2, 4 x 600 KB bf16 8.7 / 2.8,
   // 8 x 1 MiB fp32 23.5 / 3.6).
   // Registered buffers, which the window kernels may want, are looked at first.
   const Tuning& tn = tuning();
@@ -674,7 +674,7 @@ void DeviceCommunicator::collective(const CollDesc& d, const std::vector<RankArg
     if (dtype_is_float(wire)) scale *= 1.0 / p;
     else int_div = p;
   }
-  if (local_open && !tn.ll_limits_set &&
+  if (local_open && !tn.packet_limits_set() &&
       (d.kind == DevColl::allreduce || d.count * unit * dtype_size(wire) * (size_t)p < tn.crossovers(p).window_min_bytes) &&
       I.local_collective(d, ranks, in, wire, d.count * unit, scale, int_div, stream))
     return;

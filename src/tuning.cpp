@@ -61,9 +61,7 @@ void Tuning::load_from_env() {
       for (int row = 0; row < 3; ++row) {
         long v = env_long(e.env, -1);
         v = env_long((std::string(e.env) + suffix[row]).c_str(), v);
-        if (v < 0) continue;
-        cross[row].*(e.field) = (size_t)v;
-        ll_limits_set = ll_limits_set || packet_limit(e.field);
+        if (v >= 0) cross[row].*(e.field) = (size_t)v;
       }
   }
   window_enable = env_long("AL_WINDOW", window_enable) != 0;
@@ -105,6 +103,14 @@ void Tuning::load_from_env() {
   host_stage_bytes = host_stage_bytes / 4096 * 4096;
   if (host_stage_bytes < 4096) host_stage_bytes = 4096;
   if (host_mailbox_bytes < 256) host_mailbox_bytes = 256;
+}
+
+bool Tuning::packet_limits_set() const {
+  static const Tuning defaults;
+  for (int row = 0; row < 3; ++row)
+    for (auto f : {&Crossovers::ll_max_bytes, &Crossovers::ar_ll_max_bytes, &Crossovers::ar_ll2_max_bytes})
+      if (cross[row].*f != defaults.cross[row].*f) return true;
+  return false;
 }
 
 std::string Tuning::describe() const {
@@ -161,6 +167,7 @@ std::string Tuning::describe() const {
      << "  ar_ll_max_bytes         " << cross[0].ar_ll_max_bytes << "  " << cross[1].ar_ll_max_bytes << "  " << cross[2].ar_ll_max_bytes << "\n"
      << "  ar_ll2_max_bytes        " << cross[0].ar_ll2_max_bytes << "  " << cross[1].ar_ll2_max_bytes << "  " << cross[2].ar_ll2_max_bytes << "\n"
      << "  rs_nvls_min_bytes       " << cross[0].rs_nvls_min_bytes << "  " << cross[1].rs_nvls_min_bytes << "  " << cross[2].rs_nvls_min_bytes << "\n"
+     << "packet_limits_set = " << packet_limits_set() << "\n"
      << "trace = " << trace << "\n"
      << "debug_checks = " << debug_checks << "\n"
      << "debug_guard = " << debug_guard << "\n"

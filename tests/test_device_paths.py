@@ -19,10 +19,11 @@ def al():
     if not torch.cuda.is_available():
         pytest.skip("no CUDA device")
     al.init()
-    old = al.get_tuning("ll_max_bytes")
+    old = {row: al.get_tuning(f"ll_max_bytes@{row}") for row in (2, 4, 8)}
     al.set_tuning("ll_max_bytes", 1 << 20)  # the largest message the packet slots hold
     yield al
-    al.set_tuning("ll_max_bytes", old)
+    for row, v in old.items():
+        al.set_tuning(f"ll_max_bytes@{row}", v)
 
 
 def rand(n, dtype, seed):
@@ -88,7 +89,7 @@ def test_ll_allreduce_and_reduce_scatter(al, p, dtype):
 def test_ll_two_phase_allreduce(al, p, dtype):
     """Allreduce beyond the one-phase packet limit: reduce-scatter and allgather in packets inside one kernel.
     Odd lengths, unaligned views, in place and out of place, every rank bit-identical."""
-    old1, old2 = al.get_tuning("ll_max_bytes"), al.get_tuning("ar_ll2_max_bytes")
+    old = {f"{name}@{row}": al.get_tuning(f"{name}@{row}") for name in ("ll_max_bytes", "ar_ll2_max_bytes") for row in (2, 4, 8)}
     al.set_tuning("ll_max_bytes", 64)            # everything above 64 bytes takes the two-phase form
     al.set_tuning("ar_ll2_max_bytes", 4 << 20)
     comm = al.DeviceComm(emulate=p)
@@ -122,8 +123,8 @@ def test_ll_two_phase_allreduce(al, p, dtype):
             assert all(torch.equal(xs[0], x) for x in xs)
     finally:
         comm.close()
-        al.set_tuning("ll_max_bytes", old1)
-        al.set_tuning("ar_ll2_max_bytes", old2)
+        for name, v in old.items():
+            al.set_tuning(name, v)
 
 
 @pytest.mark.parametrize("p", [2, 4, 8])

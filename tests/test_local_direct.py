@@ -25,12 +25,6 @@ def al():
     return al
 
 
-@pytest.fixture(autouse=True)
-def packets_as_set(al):
-    """The limits of packets in force, as where a user has set them (sizes below them have their own test)."""
-    al.set_tuning("ar_ll2_max_bytes@4", al.get_tuning("ar_ll2_max_bytes@4"))
-
-
 @pytest.fixture
 def staged(al):
     al.set_tuning("local_direct", 0)
@@ -387,50 +381,52 @@ def test_halo_between_gpus(al, staged):
     test_halo_exchange_emulated(al)
 
 
-SMALL = """
-import sys
-sys.path.insert(0, "tests")
-import torch
-import aluminum_b200 as al
-from test_local_direct import both, same, values
-al.init()
-for p in (2, 3, 8):
-    comm = al.DeviceComm(emulate=p)
-    for dtype, op in ((torch.float32, "sum"), (torch.bfloat16, "avg"), (torch.float16, "max"), (torch.int32, "sum"), (torch.float64, "min")):
-        for n in (1, 2, 5, 64, 1023, 70001):
-            for shift in (0, 1):
-                def call():
-                    xs = [values(n, dtype, r, shift) for r in range(p)]
-                    outs = [torch.zeros(n + 2, dtype=dtype, device="cuda") for _ in range(p)]
-                    comm.allreduce(xs, [o[:n] for o in outs], op)
-                    comm.allreduce(xs, op=op)
-                    full = [values(p * n, dtype, r, shift) for r in range(p)]
-                    part = [torch.zeros(n + 2, dtype=dtype, device="cuda") for _ in range(p)]
-                    comm.reduce_scatter(full, [o[:n] for o in part], op)
-                    moved = [torch.zeros(p * n + 2, dtype=dtype, device="cuda") for _ in range(p)]
-                    comm.alltoall(full, [o[:p * n] for o in moved])
-                    every = [torch.zeros(p * n + 2, dtype=dtype, device="cuda") for _ in range(p)]
-                    comm.allgather(xs, [o[:p * n] for o in every])
-                    return outs + xs + part + moved + every
-                same(*both(al, comm, call, 5))
-    before = comm.stats()["ll"]
-    al.set_tuning("ll_max_bytes@%d" % p, al.get_tuning("ll_max_bytes@%d" % p))     # set: obeyed from here on
-    comm.allreduce([torch.ones(5, device="cuda") for _ in range(p)])
-    assert comm.stats()["ll"] == before + 1
-    comm.close()
-print("small ok")
-"""
-
-
 @pytest.mark.parametrize("p", [2, 3, 8])
-def test_small_operations_and_limits_that_are_set(p):
-    """At every size between buffers unless the packets' limits were set (a process of its own: setting them lasts)."""
-    import pathlib
-    import subprocess
-    import sys
-    root = pathlib.Path(__file__).resolve().parent.parent
-    r = subprocess.run([sys.executable, "-c", SMALL.replace("(2, 3, 8)", f"({p},)")], cwd=root, capture_output=True, text=True, timeout=300)
-    assert r.returncode == 0 and "small ok" in r.stdout, r.stdout + r.stderr
+@pytest.mark.parametrize("dtype,op", [(torch.float32, "sum"), (torch.bfloat16, "avg"), (torch.float16, "max"), (torch.int32, "sum"), (torch.float64, "min")])
+def test_small_operations(al, p, dtype, op):
+    """At every size between buffers unless the packets' limits were set."""
+    comm = al.DeviceComm(emulate=p)
+    for n in (1, 2, 5, 64, 1023, 70001):
+        for shift in (0, 1):
+            def call():
+                xs = [values(n, dtype, r, shift) for r in range(p)]
+                outs = [torch.zeros(n + 2, dtype=dtype, device="cuda") for _ in range(p)]
+                comm.allreduce(xs, [o[:n] for o in outs], op)
+                comm.allreduce(xs, op=op)
+                full = [values(p * n, dtype, r, shift) for r in range(p)]
+                part = [torch.zeros(n + 2, dtype=dtype, device="cuda") for _ in range(p)]
+                comm.reduce_scatter(full, [o[:n] for o in part], op)
+                moved = [torch.zeros(p * n + 2, dtype=dtype, device="cuda") for _ in range(p)]
+                comm.alltoall(full, [o[:p * n] for o in moved])
+                every = [torch.zeros(p * n + 2, dtype=dtype, device="cuda") for _ in range(p)]
+                comm.allgather(xs, [o[:p * n] for o in every])
+                return outs + xs + part + moved + every
+            same(*both(al, comm, call, 5))
+    comm.close()
+
+
+@pytest.mark.parametrize("name", ["ll_max_bytes", "ar_ll_max_bytes", "ar_ll2_max_bytes"])
+def test_packet_limits_that_are_set(al, name):
+    """Obeyed while one differs from its default; a value written back changes nothing, and defaults in their places end it."""
+    comm, keep = al.DeviceComm(emulate=4), {row: al.get_tuning(f"{name}@{row}") for row in (2, 4, 8)}
+    xs = [torch.ones(5, device="cuda") for _ in range(4)]
+
+    def route():
+        before = comm.stats()
+        comm.allreduce(xs)
+        return [k for k in ("ll", "local") if comm.stats()[k] > before[k]]
+    assert route() == ["local"] and "packet_limits_set = 0" in al.info()
+    for row, v in keep.items():
+        al.set_tuning(f"{name}@{row}", v)
+    assert route() == ["local"]
+    for row in (2, 4, 8):
+        try:
+            al.set_tuning(f"{name}@{row}", keep[row] + 4096)
+            assert route() == ["ll"] and "packet_limits_set = 1" in al.info()
+        finally:
+            al.set_tuning(f"{name}@{row}", keep[row])
+        assert route() == ["local"]
+    comm.close()
 
 
 @pytest.mark.parametrize("n", [3, 700_001])
