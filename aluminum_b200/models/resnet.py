@@ -43,17 +43,21 @@ class Bottleneck(nn.Module):
             out = batch_norm_act(self.bn2, self.conv2(out), self.relu)
             return batch_norm_act(self.bn3, self.conv3(out), self.relu, identity)
 
+    def plain(self) -> bool:
+        """Nothing but :meth:`forward`'s own steps happens to a block's input, and nothing in its place writes to it: :meth:`twice` may have it
+        as two tensors on the same memory."""
+        shortcut = self.downsample
+        first = [self.conv1] if shortcut is None else [self.conv1, shortcut[0]] if type(shortcut) is Shortcut and len(shortcut) == 2 else [None]
+        return _bare(self) and all(type(c) is nn.Conv2d and _bare(c) for c in first) and (shortcut is None or _bare(shortcut))
+
     def twice(self, x, same):
         """forward(x) as two tensors, for the next block's first convolution and for its end; ``same`` is x, for the end of this one."""
         convs, shortcut = [self.conv1, self.conv2, self.conv3], self.downsample
-        apart = shortcut is not None and type(shortcut) is Shortcut and len(shortcut) == 2 and _bare(shortcut)
-        if apart:
+        if shortcut is not None:
             convs.append(shortcut[0])
         w = cast_weights(convs, x) or [None] * len(convs)
-        if apart:
+        if shortcut is not None:
             same = batch_norm_act(shortcut[1], convolve(shortcut[0], same, w[3]))
-        elif shortcut is not None:
-            same = shortcut(same)
         out = batch_norm_act(self.bn1, convolve(self.conv1, x, w[0]), self.relu)
         out = batch_norm_act(self.bn2, convolve(self.conv2, out, w[1]), self.relu)
         return batch_norm_act_twice(self.bn3, convolve(self.conv3, out, w[2]), self.relu, same)
@@ -114,7 +118,7 @@ class ResNet(nn.Module):
         """The four stages; in training block by block, each handing its output to the next one twice, so that the two gradients are
         added inside the batch norm's backward."""
         stages = (self.layer1, self.layer2, self.layer3, self.layer4)
-        if _modes_off() and self.training and all(type(s) is nn.Sequential and _bare(s) and all(type(b) is Bottleneck and _bare(b) for b in s) for s in stages):
+        if _modes_off() and self.training and all(type(s) is nn.Sequential and _bare(s) and all(type(b) is Bottleneck and b.plain() for b in s) for s in stages):
             same = x
             for stage in stages:
                 for block in stage:

@@ -340,3 +340,40 @@ def test_network_block_by_block():
     called.layer2[1].register_forward_pre_hook(lambda *a: seen.append(1))
     grads(called)
     assert len(seen) == 3
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("where", ["conv1", "downsample", "shortcut", "convolution"])
+def test_modules_that_write_to_a_blocks_input(where):
+    """A module put in front of a block's first convolution or of its shortcut may work in place: both then see what it made."""
+    from aluminum_b200.models.resnet import ResNet, Shortcut
+    torch.manual_seed(0)
+    net = ResNet((2, 1, 1, 1), 10, width=16).cuda().to(memory_format=torch.channels_last)
+    for m in net.modules():
+        if isinstance(m, nn.BatchNorm2d):
+            nn.init.uniform_(m.weight, 0.5, 1.5)
+
+    class Gated(nn.Conv2d):
+        def forward(self, x):
+            return super().forward(x.mul_(0.5))
+    block = net.layer1[1]
+    if where == "conv1":
+        block.conv1 = nn.Sequential(nn.Hardswish(inplace=True), block.conv1)
+    elif where == "downsample":
+        block.downsample = nn.Hardswish(inplace=True)
+    elif where == "shortcut":
+        block = net.layer2[0]
+        block.downsample = Shortcut(nn.Sequential(nn.Hardswish(inplace=True), block.downsample[0]), block.downsample[1])
+    else:
+        block.conv1.__class__ = Gated
+    x = torch.randn(4, 3, 64, 64, device="cuda")
+
+    def grads(net):
+        with torch.autocast("cuda", dtype=torch.bfloat16):
+            net(x).float().square().mean().backward()
+        return [p.grad for p in net.parameters()]
+    own, called = copy.deepcopy(net), copy.deepcopy(net)
+    for stage in (called.layer1, called.layer2, called.layer3, called.layer4):
+        stage.register_forward_hook(lambda *a: None)     # the stages are called
+    for u, v in zip(grads(own), grads(called)):
+        assert rel(u, v.double()) < 2e-2
