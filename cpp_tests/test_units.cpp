@@ -20,6 +20,7 @@
 #include "al/util/resource_pool.hpp"
 #include "al/util/spsc_queue.hpp"
 #include "../kernels/bulk_tiles.cuh"
+#include "../kernels/local_grid.hpp"
 #include <cstring>
 #include <random>
 
@@ -39,6 +40,20 @@ static void test_meta() {
   std::vector<size_t> v{3, 0, 5};
   auto ps = excl_prefix_sum(v);
   CHECK(ps[0] == 0 && ps[1] == 3 && ps[2] == 3);
+}
+
+static void test_local_grid() {
+  // never more CTAs than the caller's budget, every job has a row of the grid or shares one, no idle rows of CTAs
+  for (int threads : {32, 96, 256, 512})
+    for (int jobs = 1; jobs <= 64; ++jobs)
+      for (int budget : {0, 1, 2, 7, 8, 56, 63, 64, 65, 127, 148})
+        for (size_t tiles : {size_t{0}, size_t{1}, size_t{15}, size_t{16}, size_t{17}, size_t{4099}, size_t{1} << 30}) {
+          const auto g = device::local_grid(tiles, jobs, budget, threads);
+          const size_t warps = (size_t)threads / 32, want = std::max<size_t>(1, (tiles + warps - 1) / warps);
+          CHECK(g.x >= 1 && g.y >= 1 && g.y <= (unsigned)jobs && g.x <= want);
+          if (budget) CHECK(g.x * g.y <= (unsigned)budget && (g.y == (unsigned)jobs || (g.y == (unsigned)budget && g.x == 1)));
+          else CHECK(g.y == (unsigned)jobs && g.x == want);
+        }
 }
 
 static void test_spsc() {
@@ -535,6 +550,7 @@ int main() {
   test_progress_thread_placement();
   test_arrival_counters();
   test_ring_pipeline_schedule();
+  test_local_grid();
   test_spsc();
   test_mpsc();
   test_allocator();

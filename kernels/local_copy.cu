@@ -116,12 +116,26 @@ void launch_local_copy(LocalCopyParams& P, int max_ctas, int threads, cudaStream
   const size_t most_tiles = (longest + 15 + tile - 1) / tile * P.rows;
   if (most_tiles >= (size_t{1} << 32)) throw_al_exception("internal error: a copy of ", longest, " bytes in one piece");
   P.tile = (unsigned)tile;
-  const dim3 grid(local_grid(most_tiles, max_ctas > 0 ? std::max(1, max_ctas / P.jobs) : 0, threads), (unsigned)P.jobs);
-  if (P.fans && words) local_copy_kernel<true, true><<<grid, (unsigned)threads, 0, stream>>>(P);
-  else if (P.fans) local_copy_kernel<true, false><<<grid, (unsigned)threads, 0, stream>>>(P);
-  else if (words) local_copy_kernel<false, true><<<grid, (unsigned)threads, 0, stream>>>(P);
-  else local_copy_kernel<false, false><<<grid, (unsigned)threads, 0, stream>>>(P);
-  AL_CHECK_CUDA(cudaGetLastError());
+  const LocalGrid g = local_grid(most_tiles, P.jobs, max_ctas, threads);
+  auto launch = [&](const LocalCopyParams& Q) {
+    const dim3 grid(g.x, (unsigned)Q.jobs);
+    if (Q.fans && words) local_copy_kernel<true, true><<<grid, (unsigned)threads, 0, stream>>>(Q);
+    else if (Q.fans) local_copy_kernel<true, false><<<grid, (unsigned)threads, 0, stream>>>(Q);
+    else if (words) local_copy_kernel<false, true><<<grid, (unsigned)threads, 0, stream>>>(Q);
+    else local_copy_kernel<false, false><<<grid, (unsigned)threads, 0, stream>>>(Q);
+    AL_CHECK_CUDA(cudaGetLastError());
+  };
+  if ((int)g.y == P.jobs) return launch(P);
+  // Fewer CTAs than jobs: some at a time.  (A loop over the jobs in the kernel costs all launches 8 registers, and with them a CTA per SM.)
+  for (int from = 0; from < P.jobs; from += (int)g.y) {
+    LocalCopyParams Q = P;
+    Q.jobs = std::min(P.jobs - from, (int)g.y);
+    std::copy_n(P.src + from, Q.jobs, Q.src);
+    std::copy_n(P.dst + from, Q.jobs, Q.dst);
+    std::copy_n(P.bytes + from, Q.jobs, Q.bytes);
+    std::copy_n(P.to + from, Q.jobs, Q.to);
+    launch(Q);
+  }
 }
 
 }  // namespace device

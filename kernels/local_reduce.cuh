@@ -20,6 +20,7 @@
 #include "al/cuda/cuda.hpp"
 #include "al/device/kernels.hpp"
 #include "datamove.cuh"
+#include "local_grid.hpp"
 
 namespace Al {
 namespace internal {
@@ -46,12 +47,6 @@ __device__ __forceinline__ uint4 load_now(const uint4* p) {
   uint4 v;
   asm volatile("ld.global.cg.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
   return v;
-}
-
-/** CTAs for `tiles` of one warp each: one warp per tile, or what the caller's budget allows where that is less than one CTA per SM. */
-inline unsigned local_grid(size_t tiles, int max_ctas, int threads) {
-  const size_t per = (size_t)threads / 32, want = std::max<size_t>(1, (tiles + per - 1) / per);
-  return (unsigned)std::min<size_t>(want, max_ctas > 0 ? (size_t)max_ctas : size_t{0x7fffffff});
 }
 
 /** T: the buffers' type, W: the type that crosses the links between GPUs (contributions, and in two phases the result, are rounded to it). */
@@ -139,8 +134,9 @@ template <typename T, typename W, typename Red, int R, int U, bool SHIFT>
 void local_reduce_run(const LocalReduceParams& P, Red red, int max_ctas, int threads, cudaStream_t stream) {
   const int jobs = P.scatter ? P.p : 1;
   const size_t words = P.count * sizeof(T) / 16 + 1;
-  const dim3 grid(local_grid((words + 32 * U - 1) / (32 * U), max_ctas > 0 ? std::max(1, max_ctas / jobs) : 0, threads), (unsigned)jobs);
-  local_reduce_kernel<T, W, Red, R, U, SHIFT><<<grid, (unsigned)threads, 0, stream>>>(P, red);
+  const LocalGrid grid = local_grid((words + 32 * U - 1) / (32 * U), jobs, max_ctas, threads);
+  if ((int)grid.y != jobs) throw_al_exception("internal error: fewer CTAs than ranks");   // (a budget is some CTAs for every rank)
+  local_reduce_kernel<T, W, Red, R, U, SHIFT><<<dim3(grid.x, grid.y), (unsigned)threads, 0, stream>>>(P, red);
   AL_CHECK_CUDA(cudaGetLastError());
 }
 

@@ -113,14 +113,14 @@ void launch_local_rows(LocalRowsParams& P, int max_ctas, int threads, cudaStream
   unsigned most = 0;
   for (int q = 0; q < p * p; ++q) most = std::max(most, P.first[q + 1] - P.first[q]);
   auto run = [&](auto kernel, dim3 grid) { kernel<<<grid, (unsigned)threads, 0, stream>>>(P); };
-  const int each = max_ctas > 0 ? std::max(1, max_ctas / (p * p)) : 0;
-  if ((size_t)most * (size_t)(p * p) <= (size_t)n + n / 4) {
-    const dim3 grid(local_grid(most, each, threads), (unsigned)(p * p));
+  const LocalGrid even = local_grid(most, p * p, max_ctas, threads);
+  if ((size_t)most * (size_t)(p * p) <= (size_t)n + n / 4 && even.y == (unsigned)(p * p)) {
+    const dim3 grid(even.x, even.y);
     if (!words) run(local_rows_kernel<false, 1, true>, grid);
     else if (small) run(local_rows_kernel<true, 1, true>, grid);
     else run(local_rows_kernel<true, kLoads, true>, grid);
   } else {
-    const dim3 grid(local_grid(n, max_ctas > 0 ? max_ctas : 148 * (1024 / threads), threads));
+    const dim3 grid(local_grid(n, 1, max_ctas > 0 ? max_ctas : 148 * (1024 / threads), threads).x);
     if (!words) run(local_rows_kernel<false, 1, false>, grid);
     else if (small) run(local_rows_kernel<true, 1, false>, grid);
     else run(local_rows_kernel<true, kLoads, false>, grid);

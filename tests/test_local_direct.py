@@ -161,6 +161,38 @@ def test_within_the_callers_limits(al, limits):
         comm.close()
 
 
+@pytest.mark.parametrize("p", [2, 3, 8])
+def test_fewer_ctas_than_parts(al, p):
+    """One CTA per rank, where there are p * (p - 1) copies, p * p pairs of row blocks or two planes per rank."""
+    from aluminum_b200.ops import HaloExchange
+    old, comm = al.get_tuning("max_ctas"), al.DeviceComm(emulate=p)
+    al.set_tuning("max_ctas", 1)
+    try:
+        for n in (5, 1024, 40_001):
+            def move():
+                xs = [values(p * n, torch.float32, r) for r in range(p)]
+                moved, every = ([torch.zeros(p * n + 4, device="cuda") for _ in range(p)] for _ in range(2))
+                comm.alltoall(xs, [m[:p * n] for m in moved])
+                comm.allgather([x[:n] for x in xs], [e[r % 4:r % 4 + p * n] for r, e in enumerate(every)])
+                rows = [torch.zeros(p * n, 8, device="cuda") for _ in range(p)]
+                first = [[d * n for d in range(p)] for _ in range(p)]
+                comm.exchange_rows([x.view(p * n, 1).expand(p * n, 8).contiguous() for x in xs], rows, 32, 32, 32, [[n] * p for _ in range(p)], first,
+                                   [[0] * p for _ in range(p)], [[n] * p for _ in range(p)], first, [[0] * p for _ in range(p)])
+                return moved + every + rows
+            same(*both(al, comm, move, 3))
+        hx = HaloExchange(comm, 2, 3, 4, 17, 19, 2, True)
+
+        def halo():
+            for r, t in enumerate(hx.tensors):
+                t.copy_(values(t.numel(), torch.float32, r).view(t.shape))
+            hx.exchange()
+            return [t.clone() for t in hx.tensors]
+        same(*both(al, comm, halo))
+    finally:
+        al.set_tuning("max_ctas", old)
+        comm.close()
+
+
 def test_what_goes_through_staging(al):
     """Buffers that meet, in-place forms that are read elsewhere, and calls that name a path or a grid."""
     p, n = 4, 1 << 20
