@@ -43,8 +43,8 @@ void launch_bulk_staged(const CollParams& P, DType user, DType wire, int ctas, i
  * launch_local_reduce: false (nothing launched) without a kernel for these types and this operator.
  */
 bool launch_local_reduce(const LocalReduceParams& P, DType user, DType wire, ReductionOperator op, int max_ctas, int threads, cudaStream_t stream);
-void launch_local_copy(LocalCopyParams& P, int max_ctas, int threads, cudaStream_t stream);
-void launch_local_rows(LocalRowsParams& P, int max_ctas, int threads, cudaStream_t stream);
+void launch_local_copy(LocalCopyParams& P, int max_ctas, int sm_count, int threads, cudaStream_t stream);
+void launch_local_rows(LocalRowsParams& P, int max_ctas, int sm_count, int threads, cudaStream_t stream);
 
 // ---- order of tokens by destination rank (kernels/route.cu) ----
 void launch_route(const RouteParams& P, int local_ranks, cudaStream_t stream);

@@ -98,7 +98,7 @@ __global__ void __launch_bounds__(kLocalThreads, 2) local_copy_kernel(const __gr
 
 }  // namespace
 
-void launch_local_copy(LocalCopyParams& P, int max_ctas, int threads, cudaStream_t stream) {
+void launch_local_copy(LocalCopyParams& P, int max_ctas, int sm_count, int threads, cudaStream_t stream) {
   size_t total = 0, longest = 0;
   bool words = P.src_stride % 16 == 0 && P.dst_stride % 16 == 0;
   for (int r = 0; P.fans && r < P.p; ++r) words = words && (uintptr_t)P.fan[r] % 16 == 0;
@@ -111,7 +111,7 @@ void launch_local_copy(LocalCopyParams& P, int max_ctas, int threads, cudaStream
   // As much to a warp as leaves 16 of them to an SM.
   const size_t most = 32 * 16 * (P.fans ? kFanLoads : kLoads);
   size_t tile = 512;
-  while (tile < most && total / (2 * tile) >= 148 * 16) tile *= 2;
+  while (tile < most && total / (2 * tile) >= (size_t)sm_count * 16) tile *= 2;
   while (!words && longest / tile * P.rows > (size_t{1} << 30)) tile *= 2;
   const size_t most_tiles = (longest + 15 + tile - 1) / tile * P.rows;
   if (most_tiles >= (size_t{1} << 32)) throw_al_exception("internal error: a copy of ", longest, " bytes in one piece");

@@ -27,7 +27,6 @@ namespace internal {
 namespace device {
 
 constexpr int kLocalThreads = 512;   // of a CTA at most
-constexpr size_t kLocalWarps = 148 * 2 * kLocalThreads / 32;   // on the GPU at once
 
 /**
  * Has an earlier operation of the communicator failed?  A lane's word of the ranks' status words, to be looked at with
@@ -140,21 +139,18 @@ void local_reduce_run(const LocalReduceParams& P, Red red, int max_ctas, int thr
   AL_CHECK_CUDA(cudaGetLastError());
 }
 
-/** SHIFTS: whether contributions on other addresses modulo 16 than the result are served (else the caller has checked that there are none). */
-template <typename T, typename W, bool SHIFTS, typename Red>
+/** SHIFT where a contribution lies on another address modulo 16 than the result. */
+template <typename T, typename W, typename Red>
 void local_reduce_launch(const LocalReduceParams& P, Red red, int max_ctas, int threads, cudaStream_t stream) {
   bool shifted = false;
   for (int job = 0; job < (P.scatter ? P.p : 1); ++job)
     for (int r = 0; r < P.p; ++r)
       shifted = shifted || (((uintptr_t)P.src[r] + (P.scatter ? (size_t)job * P.count * sizeof(T) : 0)) ^ (uintptr_t)P.dst[job]) % 16 != 0;
-  if constexpr (SHIFTS) {
-    if (shifted) {
-      if (P.p == 2) return local_reduce_run<T, W, Red, 2, 2, true>(P, red, max_ctas, threads, stream);
-      if (P.p <= 4) return local_reduce_run<T, W, Red, 4, 1, true>(P, red, max_ctas, threads, stream);
-      return local_reduce_run<T, W, Red, 8, 1, true>(P, red, max_ctas, threads, stream);
-    }
+  if (shifted) {
+    if (P.p == 2) return local_reduce_run<T, W, Red, 2, 2, true>(P, red, max_ctas, threads, stream);
+    if (P.p <= 4) return local_reduce_run<T, W, Red, 4, 1, true>(P, red, max_ctas, threads, stream);
+    return local_reduce_run<T, W, Red, 8, 1, true>(P, red, max_ctas, threads, stream);
   }
-  if (shifted) throw_al_exception("internal error: reduction between buffers on different addresses modulo 16");
   if (P.p == 2) return local_reduce_run<T, W, Red, 2, 4, false>(P, red, max_ctas, threads, stream);
   if (P.p <= 4) return local_reduce_run<T, W, Red, 4, 2, false>(P, red, max_ctas, threads, stream);
   return local_reduce_run<T, W, Red, 8, 1, false>(P, red, max_ctas, threads, stream);

@@ -10,9 +10,9 @@ template <typename T>
 bool run(const LocalReduceParams& P, ReductionOperator op, int max_ctas, int threads, cudaStream_t stream) {
   switch (op) {
     case ReductionOperator::sum:
-    case ReductionOperator::avg: local_reduce_launch<T, T, true>(P, RedSum(), max_ctas, threads, stream); return true;
-    case ReductionOperator::max: local_reduce_launch<T, T, true>(P, RedMax(), max_ctas, threads, stream); return true;
-    case ReductionOperator::min: local_reduce_launch<T, T, true>(P, RedMin(), max_ctas, threads, stream); return true;
+    case ReductionOperator::avg: local_reduce_launch<T, T>(P, RedSum(), max_ctas, threads, stream); return true;
+    case ReductionOperator::max: local_reduce_launch<T, T>(P, RedMax(), max_ctas, threads, stream); return true;
+    case ReductionOperator::min: local_reduce_launch<T, T>(P, RedMin(), max_ctas, threads, stream); return true;
     default: return false;
   }
 }

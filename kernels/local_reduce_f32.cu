@@ -7,11 +7,11 @@ namespace device {
 
 bool local_reduce_f32(const LocalReduceParams& P, DType wire, ReductionOperator op, int max_ctas, int threads, cudaStream_t stream) {
   const bool sum = op == ReductionOperator::sum || op == ReductionOperator::avg;
-  if (sum && wire == DType::bf16) local_reduce_launch<float, __nv_bfloat16, true>(P, RedSum(), max_ctas, threads, stream);
-  else if (sum && wire == DType::f16) local_reduce_launch<float, __half, true>(P, RedSum(), max_ctas, threads, stream);
-  else if (sum && wire == DType::f32) local_reduce_launch<float, float, true>(P, RedSum(), max_ctas, threads, stream);
-  else if (op == ReductionOperator::max && wire == DType::f32) local_reduce_launch<float, float, true>(P, RedMax(), max_ctas, threads, stream);
-  else if (op == ReductionOperator::min && wire == DType::f32) local_reduce_launch<float, float, true>(P, RedMin(), max_ctas, threads, stream);
+  if (sum && wire == DType::bf16) local_reduce_launch<float, __nv_bfloat16>(P, RedSum(), max_ctas, threads, stream);
+  else if (sum && wire == DType::f16) local_reduce_launch<float, __half>(P, RedSum(), max_ctas, threads, stream);
+  else if (sum && wire == DType::f32) local_reduce_launch<float, float>(P, RedSum(), max_ctas, threads, stream);
+  else if (op == ReductionOperator::max && wire == DType::f32) local_reduce_launch<float, float>(P, RedMax(), max_ctas, threads, stream);
+  else if (op == ReductionOperator::min && wire == DType::f32) local_reduce_launch<float, float>(P, RedMin(), max_ctas, threads, stream);
   else return false;
   return true;
 }

@@ -79,7 +79,7 @@ __global__ void __launch_bounds__(kLocalThreads, 2) local_rows_kernel(const __gr
 
 }  // namespace
 
-void launch_local_rows(LocalRowsParams& P, int max_ctas, int threads, cudaStream_t stream) {
+void launch_local_rows(LocalRowsParams& P, int max_ctas, int sm_count, int threads, cudaStream_t stream) {
   const int p = P.p;
   bool words = P.row_bytes % 16 == 0 && P.send_row_stride % 16 == 0 && P.recv_row_stride % 16 == 0;
   size_t rows = 0;
@@ -90,7 +90,7 @@ void launch_local_rows(LocalRowsParams& P, int max_ctas, int threads, cudaStream
       words = words && P.tab[s].send_peer_off[d] % 16 == 0 && P.tab[s].recv_peer_off[d] % 16 == 0;
     }
   }
-  const size_t warps = max_ctas > 0 ? (size_t)max_ctas * (size_t)(threads / 32) : kLocalWarps;
+  const size_t warps = max_ctas > 0 ? (size_t)max_ctas * (size_t)(threads / 32) : (size_t)sm_count * 2 * kLocalThreads / 32;
   const bool small = rows * P.row_bytes / kTile < warps;   // one load per thread then, so that more warps get some
   const unsigned unit = small ? 32 : 32 * kLoads;                 // words of 16 bytes
   P.group = P.per_row = 1;
@@ -120,7 +120,7 @@ void launch_local_rows(LocalRowsParams& P, int max_ctas, int threads, cudaStream
     else if (small) run(local_rows_kernel<true, 1, true>, grid);
     else run(local_rows_kernel<true, kLoads, true>, grid);
   } else {
-    const dim3 grid(local_grid(n, 1, max_ctas > 0 ? max_ctas : 148 * (1024 / threads), threads).x);
+    const dim3 grid(local_grid(n, 1, max_ctas > 0 ? max_ctas : sm_count * (1024 / threads), threads).x);
     if (!words) run(local_rows_kernel<false, 1, false>, grid);
     else if (small) run(local_rows_kernel<true, 1, false>, grid);
     else run(local_rows_kernel<true, kLoads, false>, grid);

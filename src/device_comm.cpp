@@ -499,7 +499,7 @@ void DeviceCommunicator::Impl::local_move(bool gathers, const std::vector<RankAr
     }
   }
   begin_local(L.flags, stream);
-  launch_local_copy(L, local_ctas(tuning().max_ctas, p, sm_count), local_threads(), stream);
+  launch_local_copy(L, local_ctas(tuning().max_ctas, p, sm_count), sm_count, local_threads(), stream);
 }
 
 /**
@@ -548,7 +548,7 @@ bool DeviceCommunicator::Impl::local_rows(const RowsParams& R, const std::vector
   }
   begin_local(L.flags, stream);
   const int threads = local_threads();
-  launch_local_rows(L, local_ctas(tuning().max_ctas, p, sm_count), threads, stream);
+  launch_local_rows(L, local_ctas(tuning().max_ctas, p, sm_count), sm_count, threads, stream);
   end_local();
   stats.rows++;
   stats.bytes += total_rows * R.row_bytes;
@@ -599,7 +599,7 @@ size_t DeviceCommunicator::Impl::local_p2p(const std::vector<P2PDesc>& items, st
   if (!taken) return 0;
   begin_local(L.flags, stream);
   const int threads = local_threads();
-  launch_local_copy(L, local_ctas(tuning().p2p_max_ctas, (int)taken, sm_count), threads, stream);
+  launch_local_copy(L, local_ctas(tuning().p2p_max_ctas, (int)taken, sm_count), sm_count, threads, stream);
   end_local();
   stats.bytes += moved;
   return taken;
@@ -629,7 +629,7 @@ bool DeviceCommunicator::local_halo(const HaloParams& H, cudaStream_t stream) {
   }
   const int threads = local_threads();
   std::lock_guard<std::mutex> lock(I.mu);
-  if (L.rows && L.jobs) launch_local_copy(L, local_ctas(tuning().max_ctas, I.p, I.sm_count), threads, stream);
+  if (L.rows && L.jobs) launch_local_copy(L, local_ctas(tuning().max_ctas, I.p, I.sm_count), I.sm_count, threads, stream);
   I.stats.local++;
   return true;
 }
@@ -1193,8 +1193,9 @@ void DeviceCommunicator::route(int nlocal, const long long* const* dest, const s
   P.host_flags = ((Impl::Mail*)dev)->flags;
   P.host_seq = ++m->seq;
   launch_route(P, nlocal, stream);
-  // Poll; the stream may hold other work of any length first, so the time limit begins when that is known to be over, and a stream
-  // that has failed ends the wait.  (On an error the page is not given back: the kernel may still write it.)
+  // Poll, on a core, as a read of the counts by way of the stream would wait too: the stream may hold other work of any length first.  There is no
+  // limit of time; what ends the wait are the counts, an error of the stream, and a stream that has ended without them.
+  // (On an error the page is not given back: the kernel may still write it.)
   auto arrived = [&] {
     for (int r = 0; r < nlocal; ++r)
       if (__atomic_load_n(&m->flags[r], __ATOMIC_ACQUIRE) != m->seq) return false;
