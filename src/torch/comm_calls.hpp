@@ -193,18 +193,29 @@ PyObject* collective(PyObject*, PyObject* const* a, Py_ssize_t n) {
   });
 }
 
-/** One table of a row exchange: a list of one list per local rank (or, for one rank, its list). */
-void table(PyObject* o, Py_ssize_t ranks, Py_ssize_t size, std::vector<size_t>& out) {
-  auto wrong = [&] { raise("exchange_rows: tables need " + std::to_string(ranks) + " row(s) of " + std::to_string(size) + " entries"); };
+/** One table of a row exchange: a list of one list per local rank (or, for one rank, its list).  False: rows or entries of another kind. */
+bool table(PyObject* o, Py_ssize_t ranks, Py_ssize_t size, std::vector<size_t>& out) {
   auto row = [&](const Items& r) {
-    for (Py_ssize_t i = 0; i < r.n; ++i) out.push_back((size_t)integer(r[i]));
+    for (Py_ssize_t i = 0; i < r.n; ++i) {
+      if (!PyLong_Check(r[i])) return false;
+      out.push_back((size_t)integer(r[i]));
+    }
+    return true;
   };
   out.clear();
   const Items rows(o);
-  if (ranks == 1 && (rows.n == 0 || !(PyList_Check(rows[0]) || PyTuple_Check(rows[0])))) row(rows);
-  else
-    for (Py_ssize_t r = 0; r < rows.n; ++r) row(Items(rows[r]));
-  if ((Py_ssize_t)out.size() != ranks * size) wrong();
+  if (!rows.list) return false;
+  if (ranks == 1 && (rows.n == 0 || !(PyList_Check(rows[0]) || PyTuple_Check(rows[0])))) {
+    if (!row(rows)) return false;
+  } else {
+    for (Py_ssize_t r = 0; r < rows.n; ++r) {
+      const Items one(rows[r]);
+      if (!one.list || !row(one)) return false;
+    }
+  }
+  if ((Py_ssize_t)out.size() != ranks * size)
+    raise("exchange_rows: tables need " + std::to_string(ranks) + " row(s) of " + std::to_string(size) + " entries");
+  return true;
 }
 
 /** (comm, local ranks, ranks, send, recv, row bytes, send stride, recv stride, six tables, send index, recv index, stream, request wanted) */
@@ -237,7 +248,7 @@ PyObject* exchange_rows(PyObject*, PyObject* const* a, Py_ssize_t n) {
     std::vector<size_t> t[6];
     for (int i = 0; i < 6; ++i) {
       t[i].reserve((size_t)(ranks * size));
-      table(a[8 + i], ranks, size, t[i]);
+      if (!table(a[8 + i], ranks, size, t[i])) return not_mine();
     }
     void *comm = handle(a[0]), *stream = stream_of(a[16]);
     const size_t bytes = (size_t)integer(a[5]), sstride = (size_t)integer(a[6]), rstride = (size_t)integer(a[7]);
@@ -265,6 +276,7 @@ PyObject* p2p(PyObject*, PyObject* const* a, Py_ssize_t n) {
       PyObject* it = items[(Py_ssize_t)i];
       if (!PyTuple_Check(it) || PyTuple_GET_SIZE(it) < 3 || !THPVariable_CheckExact(PyTuple_GET_ITEM(it, 2))) return not_mine();
       const at::Tensor& t = THPVariable_Unpack(PyTuple_GET_ITEM(it, 2));
+      if (PyFloat_Check(PyTuple_GET_ITEM(it, 1)) || (PyTuple_GET_SIZE(it) > 3 && PyFloat_Check(PyTuple_GET_ITEM(it, 3)))) return not_mine();
       const int sends = PyObject_IsTrue(PyTuple_GET_ITEM(it, 0));
       if (sends < 0) throw Raised();
       is_send[i] = sends;

@@ -42,6 +42,26 @@ def test_what_is_refused_and_what_is_left_to_python(calls):
     assert calls.p2p(0, 0, [(True, 1)], 0, False) is NotImplemented and calls.p2p(0, 0, iter(()), 0, False) is NotImplemented
 
 
+def test_tables_and_ranks_of_any_kind_are_left_to_python(calls):
+    """Ranges, arrays, tensors and other numbers than ints: Python converts them."""
+    import numpy as np
+    t, rows = torch.zeros(4), [[1, 1]] * 2
+
+    def call(ranks, table):
+        x = [t] * ranks if ranks > 1 else t
+        other = rows[:ranks]
+        return calls.exchange_rows(0, ranks, 2, x, x, 4, 4, 4, other, other, table, other, other, other, None, None, 0, False)
+    for table in ([range(0, 8, 4)] * 2, np.ones((2, 2), dtype=np.int64), torch.ones(2, 2, dtype=torch.int64), [np.ones(2, dtype=np.int64)] * 2,
+                  [[1.0, 1.0]] * 2, [[np.int64(1)] * 2] * 2, iter([[1, 1], [1, 1]])):
+        assert call(2, table) is NotImplemented
+    for table in (range(0, 8, 4), np.ones(2, dtype=np.int64), torch.ones(2, dtype=torch.int64), [range(2)], (1.0, 2.0)):
+        assert call(1, table) is NotImplemented
+    for table in ([1, 1], (1, 1), [[1, 1]], ((True, 1),)):
+        with pytest.raises(_lib.AlError, match="closed"):
+            call(1, table)
+    assert calls.p2p(0, 0, [(True, 1.0, t)], 0, False) is NotImplemented and calls.p2p(0, 0, [(True, 1, t, 0.0)], 0, False) is NotImplemented
+
+
 def test_new_tensors(calls):
     like = [torch.zeros(1), torch.zeros(1, dtype=torch.int16)]
     for shapes, want in (((3, 4), [(3, 4)] * 2), ([(0,), (2, 5)], [(0,), (2, 5)])):
