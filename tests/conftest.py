@@ -26,3 +26,13 @@ def built_lib():
 @pytest.fixture(scope="session")
 def bin_dir(built_lib):
     return ROOT / "aluminum_b200" / "bin"
+
+
+@pytest.fixture(scope="module", params=[1, 0], ids=["between_buffers", "flag_protocol"])
+def local_direct(request):
+    """Emulated ranks with calls that name no path straight between their buffers, and through the protocol of ranks on GPUs of their own."""
+    import aluminum_b200 as al
+    old = al.get_tuning("local_direct")
+    al.set_tuning("local_direct", request.param)
+    yield request.param
+    al.set_tuning("local_direct", old)

@@ -1,7 +1,6 @@
-"""Device collectives on ONE GPU: all ranks of a communicator are emulated in one
-process and every call is a single cooperative launch of the same kernels the
-multi-GPU path uses (flag protocol included).  Results are compared with plain
-PyTorch fp32 references of the same operation.
+"""Device collectives on ONE GPU: all ranks of a communicator are emulated in one process.  Every test runs twice: calls that
+name no path once straight between the ranks' buffers, and once as a single cooperative launch of the same kernels
+the multi-GPU path uses (flag protocol included).  Results are compared with plain PyTorch fp32 references of the same operation.
 """
 import pytest
 import torch
@@ -21,20 +20,22 @@ def al():
 
 
 @pytest.fixture(scope="module", params=[2, 4, 8])
-def comm(al, request):
+def comm(al, request, local_direct):
     c = al.DeviceComm(emulate=request.param)
     yield c
+    assert local_direct or c.stats()["local"] == 0
     c.close()
 
 
 @pytest.fixture(scope="module")
-def small_stage_comm(al):
+def small_stage_comm(al, local_direct):
     """Tiny staging halves force the multi-chunk paths (chunk loop + closing barrier)."""
     old = al.get_tuning("dev_stage_bytes")
     al.set_tuning("dev_stage_bytes", 65536)
     c = al.DeviceComm(emulate=4)
     al.set_tuning("dev_stage_bytes", old)
     yield c
+    assert local_direct or c.stats()["local"] == 0
     c.close()
 
 
@@ -285,6 +286,7 @@ def test_multichunk_paths(small_stage_comm):
             assert torch.equal(outs[d], torch.cat([a2a[r][d * 30011:(d + 1) * 30011] for r in range(p)]))
 
 
+@pytest.mark.usefixtures("local_direct")
 def test_pipelined_schedule(al):
     """Large uniform reduce_scatter / allgather / alltoall: publisher and consumer CTAs, many chunks."""
     old = al.get_tuning("pipeline_min_bytes")
@@ -317,16 +319,18 @@ def test_pipelined_schedule(al):
         al.set_tuning("pipeline_min_bytes", old)
 
 
-def test_barrier_nonblocking_and_stats(comm):
+def test_barrier_nonblocking_and_stats(comm, local_direct):
     p = comm.size
     comm.barrier()
     xs = [torch.full((1000,), float(r), device="cuda") for r in range(p)]
+    before = comm.stats()
     req = comm.allreduce(xs, nonblocking=True)
     req.wait()
     torch.cuda.synchronize()
     assert req.test()
     assert all(torch.all(x == sum(range(p))) for x in xs)
     st = comm.stats()
+    assert [k for k in ("local", "ll") if st[k] > before[k]] == ["local" if local_direct else "ll"]
     assert st["ops"] > 0 and st["kernels"] > 0 and st["timeouts"] == 0
     assert comm.status()["code"] == 0
 

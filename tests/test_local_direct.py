@@ -1,8 +1,8 @@
 """Operations of ranks that all live on one GPU, straight between their buffers (kernels/local_*.cu): every form that they
 accept gives bit for bit what the staging protocol gives, and what they must not take goes through staging.
 
-The kernels that ranks on GPUs of their own run are tested on one GPU in the other files where a call names its path; the tests
-there that leave it open are run again here with ``local_direct`` off.
+The kernels that ranks on GPUs of their own run are tested on one GPU in the other files where a call names its path or (the fixture
+``local_direct``) runs both ways; the other tests there that leave it open are run again here with ``local_direct`` off.
 """
 import random
 

@@ -1,5 +1,6 @@
 """Parallelism helpers (tensor / sequence / Ulysses / expert / context-ring) on emulated ranks of one
-GPU, each checked against the same computation done on a single device."""
+GPU, each checked against the same computation done on a single device, straight between the ranks' buffers and through the flag
+protocol of ranks on GPUs of their own."""
 import math
 
 import pytest
@@ -10,13 +11,14 @@ P = 4
 
 
 @pytest.fixture(scope="module")
-def comm():
+def comm(local_direct):
     if not torch.cuda.is_available():
         pytest.skip("no CUDA device")
     import aluminum_b200 as al
     al.init()
     c = al.DeviceComm(emulate=P)
     yield c
+    assert local_direct or c.stats()["local"] == 0
     c.close()
 
 
