@@ -182,4 +182,10 @@ def test_gradients_are_lent_where_nothing_looks_at_them(calls):
                  lambda n: n[0].register_forward_hook(lambda m, i, o: o.register_hook(lambda g: None) and None), node_hook,
                  lambda n: torch.autograd.graph.register_multi_grad_hook(list(n.parameters()), lambda *a: None)):
         assert not lent(hook)
+
+    def long(x):
+        for k in range(3000):      # (more nodes than the walk's first table holds, met more than once)
+            x = x + x * 1e-6 if k % 100 == 0 else x + 0
+        return x
+    assert lent(use=long) and not lent(lambda n: n[0].weight.register_hook(lambda g: None), long)
     assert not lent(use=Same.apply) and not calls.lend_gradients(None, [], []) and not calls.lend_gradients(torch.zeros(1), [], [])
