@@ -230,6 +230,14 @@ int al_maxpool_backward(int dt, const void* dy, const unsigned char* place, void
  * channel, channel, row, column of the weight. */
 int al_stem_gather(int in_dt, const void* x, int dt, void* out, const float* weight, void* packed, const int* shape, const long long* strides,
                    void* stream);
+/* The same; watch[al_stem_watch_words()] then says where al_stem_repair(), run on the convolution's result, has to look: a value that is not finite
+ * and lies below a result's window meets zeros of the packed weight, and such results are computed again.  Its strides are those of the
+ * result (n, channel, row, column) behind four that are not read. */
+int al_stem_gather_watched(int in_dt, const void* x, int dt, void* out, const float* weight, void* packed, unsigned* watch, const int* shape,
+                           const long long* strides, void* stream);
+size_t al_stem_watch_words(const int* shape);
+int al_stem_repair(int dt, const void* out, const void* packed, const unsigned* watch, void* result, const int* shape, const long long* strides,
+                   void* stream);
 int al_stem_scatter(int dt, const void* packed, float* grad, const int* shape, const long long* strides, void* stream);
 
 #ifdef __cplusplus

@@ -217,7 +217,14 @@ struct StemShape {
   int n, h, w, oh, ow, oc;
   long long xs[4], ws[4];   // strides, in elements, of the images and of the weight (n or oc, channel, row, column)
 };
-void launch_stem_gather(const StemShape& s, const void* x, DType in, void* out, const float* weight, void* packed, DType dt, cudaStream_t stream);
+void launch_stem_gather(const StemShape& s, const void* x, DType in, void* out, const float* weight, void* packed, DType dt, unsigned* watch,
+                        cudaStream_t stream);
+/**
+ * After the convolution y (ws: its strides), from the words (stem_watch_words of them) that the gather left in `watch`: results beside whose window
+ * there is a value that is not finite, computed again without it.
+ */
+void launch_stem_repair(const StemShape& s, const void* seen, const void* packed, const unsigned* watch, void* y, DType dt, cudaStream_t stream);
+size_t stem_watch_words(const StemShape& s);
 void launch_stem_scatter(const StemShape& s, const void* packed, float* grad, DType dt, cudaStream_t stream);
 /** Fill with a 32-bit pattern (used by tests and benchmarks to flush L2). */
 void launch_fill_u32(uint32_t* out, size_t n, uint32_t value, cudaStream_t stream);

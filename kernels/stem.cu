@@ -26,9 +26,18 @@ constexpr int kRow = kSeen * kIn;             // values of one input row
 constexpr int kPairs = 4;                     // row pairs of a CTA: as many rows as it has warps
 static_assert(2 * kPairs == kThreads / 32, "a warp has one row");
 
+/** Is one of two values infinite or NaN? */
+template <typename T>
+__device__ __forceinline__ bool not_finite2(uint32_t w) {
+  constexpr uint32_t top = std::is_same<T, __half>::value ? 0x7c00u : 0x7f80u;
+  return (w & top) == top || (w >> 16 & top) == top;
+}
+
+/** watch (or nullptr): a word per CTA, whether the second row of one of its pairs has a value that is not finite (stem_repair_kernel). */
 template <typename Ti, typename To>
 __global__ void __launch_bounds__(kThreads) stem_gather_kernel(const __grid_constant__ StemShape s, const Ti* __restrict__ x, To* __restrict__ out,
-                                                               const float* __restrict__ weight, To* __restrict__ packed, unsigned rows) {
+                                                               const float* __restrict__ weight, To* __restrict__ packed, unsigned rows,
+                                                               unsigned* __restrict__ watch) {
   auto as = [](Ti v) { return Elem<To>::down((float)Elem<Ti>::up(v)); };
   const To zero = Elem<To>::down(0.f);
   if (blockIdx.x >= rows) {   // the weight: [output][row pair][channel], zero where there is no tap
@@ -90,7 +99,15 @@ __global__ void __launch_bounds__(kThreads) stem_gather_kernel(const __grid_cons
     }
   }
   __syncthreads();
-  // a pixel's 24 values of a row begin 6 values behind its neighbour's: on 4 bytes, not on 16
+  if (watch) {
+    bool odd = false;
+    const unsigned words = (unsigned)cols * kIn / 2;
+    for (unsigned i = threadIdx.x; i < kPairs * words; i += kThreads) odd |= not_finite2<To>(smem[(2 * (i / words) + 1) * words + i % words]);
+    odd = __syncthreads_or(odd);
+    if (threadIdx.x == 0) watch[blockIdx.x] = odd;
+  }
+  // a pixel's 24 values of a row begin 6 values behind its neighbour's: on 4 bytes, not on 16.  The last three are of the column behind its
+  // window: zeros here, so that the weight's zeros there meet nothing that is not finite.
   const int pixels = min(kPairs, s.oh + 3 - r0) * s.ow, k = threadIdx.x % (kCh / 8);
   uint4* dst = (uint4*)out + ((size_t)n * (s.oh + 3) + r0) * s.ow * (kCh / 8);
   int j = threadIdx.x / (kCh / 8) % s.ow, pair = threadIdx.x / (kCh / 8) / s.ow;
@@ -99,9 +116,46 @@ __global__ void __launch_bounds__(kThreads) stem_gather_kernel(const __grid_cons
     if (k < 6) {
       const uint32_t* p = smem + (((2 * pair + k / 3) * cols + 2 * j) * kIn + (k % 3) * 8) / 2;
       v = uint4{p[0], p[1], p[2], p[3]};
+      if (k % 3 == 2) v = uint4{v.x, v.y, v.z & 0xffffu, 0};
     }
     dst[(size_t)i * (kCh / 8) + k] = v;
     for (j += kThreads / (kCh / 8); j >= s.ow; j -= s.ow) ++pair;
+  }
+}
+
+/**
+ * Results whose window ends beside a value that is not finite.  The second row of a result's last pair lies below its window; the weight is zero
+ * there, but that row is in the window of the next result, so its values have to be in the layout, and zero times infinity is NaN.
+ * Those results are computed again without that row, a warp per pixel.  Images are finite nearly always: then the launch
+ * reads a word per eight rows of them and is gone.
+ */
+template <typename T>
+__global__ void __launch_bounds__(kThreads) stem_repair_kernel(const __grid_constant__ StemShape s, const T* __restrict__ seen, const T* __restrict__ packed,
+                                                               const unsigned* __restrict__ watch, unsigned rows, T* __restrict__ y) {
+  __shared__ unsigned found[kThreads];
+  const unsigned from = blockIdx.x * kThreads;
+  found[threadIdx.x] = from + threadIdx.x < rows ? watch[from + threadIdx.x] : 0;
+  if (!__syncthreads_or(found[threadIdx.x])) return;
+  const int groups = (s.oh + 3 + kPairs - 1) / kPairs, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (unsigned t = 0; t < kThreads; ++t) {
+    if (!found[t]) continue;
+    const int n = (int)((from + t) / (unsigned)groups), r0 = (int)((from + t) % (unsigned)groups) * kPairs;
+    const int pixels = min(kPairs, s.oh + 3 - r0) * s.ow;
+    for (int i = warp; i < pixels; i += kThreads / 32) {
+      const int oh = r0 + i / s.ow - 3, ow = i % s.ow;
+      if (oh < 0) continue;
+      const T* first = seen + (((size_t)n * (s.oh + 3) + oh) * s.ow + ow) * kCh;   // of four pairs of rows, s.ow pixels apart
+      const size_t step = (size_t)s.ow * kCh;
+      const bool odd = lane < 7 * kIn && not_finite2<T>(((const uint16_t*)first)[3 * step + kRow + lane]);
+      if (!__any_sync(0xffffffffu, odd)) continue;
+      for (int o = lane; o < s.oc; o += 32) {
+        float sum = 0.f;
+        for (int u = 0; u < 7; ++u)
+          for (int c = 0; c < 7 * kIn; ++c)
+            sum = fmaf(Elem<T>::up(first[u / 2 * step + u % 2 * kRow + c]), Elem<T>::up(packed[(o * 4 + u / 2) * kCh + u % 2 * kRow + c]), sum);
+        y[(size_t)n * s.ws[0] + (size_t)o * s.ws[1] + (size_t)oh * s.ws[2] + (size_t)ow * s.ws[3]] = Elem<T>::down(sum);
+      }
+    }
   }
 }
 
@@ -120,24 +174,41 @@ void check(const StemShape& s) {
     throw_al_exception("first convolution: unsupported shape");
 }
 
+unsigned gather_rows(const StemShape& s) { return (unsigned)(s.n * ((s.oh + 3 + kPairs - 1) / kPairs)); }
+
 template <typename Ti, typename To>
-void gather(const StemShape& s, const void* x, void* out, const float* weight, void* packed, cudaStream_t stream) {
-  const unsigned rows = (unsigned)(s.n * ((s.oh + 3 + kPairs - 1) / kPairs)), more = (unsigned)((s.oc * 4 * kCh + kThreads - 1) / kThreads);
+void gather(const StemShape& s, const void* x, void* out, const float* weight, void* packed, unsigned* watch, cudaStream_t stream) {
+  const unsigned rows = gather_rows(s), more = (unsigned)((s.oc * 4 * kCh + kThreads - 1) / kThreads);
   const size_t smem = (size_t)2 * kPairs * (2 * s.ow + 6) * kIn * sizeof(To);   // (a whole number of 4-byte words: a row is 6 (ow + 3) values)
-  stem_gather_kernel<Ti, To><<<rows + more, kThreads, smem, stream>>>(s, (const Ti*)x, (To*)out, weight, (To*)packed, rows);
+  stem_gather_kernel<Ti, To><<<rows + more, kThreads, smem, stream>>>(s, (const Ti*)x, (To*)out, weight, (To*)packed, rows, watch);
   AL_CHECK_CUDA(cudaGetLastError());
 }
 
 }  // namespace
 
-void launch_stem_gather(const StemShape& s, const void* x, DType in, void* out, const float* weight, void* packed, DType dt, cudaStream_t stream) {
+size_t stem_watch_words(const StemShape& s) {
+  check(s);
+  return gather_rows(s);
+}
+
+void launch_stem_gather(const StemShape& s, const void* x, DType in, void* out, const float* weight, void* packed, DType dt, unsigned* watch,
+                        cudaStream_t stream) {
   using bf = __nv_bfloat16;
   check(s);
-  if (in == DType::f32 && dt == DType::bf16) return gather<float, bf>(s, x, out, weight, packed, stream);
-  if (in == DType::f32 && dt == DType::f16) return gather<float, __half>(s, x, out, weight, packed, stream);
-  if (in == DType::bf16 && dt == DType::bf16) return gather<bf, bf>(s, x, out, weight, packed, stream);
-  if (in == DType::f16 && dt == DType::f16) return gather<__half, __half>(s, x, out, weight, packed, stream);
+  if (in == DType::f32 && dt == DType::bf16) return gather<float, bf>(s, x, out, weight, packed, watch, stream);
+  if (in == DType::f32 && dt == DType::f16) return gather<float, __half>(s, x, out, weight, packed, watch, stream);
+  if (in == DType::bf16 && dt == DType::bf16) return gather<bf, bf>(s, x, out, weight, packed, watch, stream);
+  if (in == DType::f16 && dt == DType::f16) return gather<__half, __half>(s, x, out, weight, packed, watch, stream);
   throw_al_exception("first convolution: unsupported datatypes ", dtype_name(in), ", ", dtype_name(dt));
+}
+
+void launch_stem_repair(const StemShape& s, const void* seen, const void* packed, const unsigned* watch, void* y, DType dt, cudaStream_t stream) {
+  check(s);
+  const unsigned rows = gather_rows(s), blocks = (rows + kThreads - 1) / kThreads;
+  if (dt == DType::bf16) stem_repair_kernel<<<blocks, kThreads, 0, stream>>>(s, (const __nv_bfloat16*)seen, (const __nv_bfloat16*)packed, watch, rows, (__nv_bfloat16*)y);
+  else if (dt == DType::f16) stem_repair_kernel<<<blocks, kThreads, 0, stream>>>(s, (const __half*)seen, (const __half*)packed, watch, rows, (__half*)y);
+  else throw_al_exception("first convolution: unsupported datatype ", dtype_name(dt));
+  AL_CHECK_CUDA(cudaGetLastError());
 }
 
 void launch_stem_scatter(const StemShape& s, const void* packed, float* grad, DType dt, cudaStream_t stream) {

@@ -703,7 +703,23 @@ static device::StemShape stem_shape(const int* s, const long long* t) {
 }
 int al_stem_gather(int in_dt, const void* x, int dt, void* out, const float* weight, void* packed, const int* shape, const long long* strides,
                    void* stream) {
-  return guard([&] { device::launch_stem_gather(stem_shape(shape, strides), x, (DType)in_dt, out, weight, packed, (DType)dt, (cudaStream_t)stream); });
+  return al_stem_gather_watched(in_dt, x, dt, out, weight, packed, nullptr, shape, strides, stream);
+}
+int al_stem_gather_watched(int in_dt, const void* x, int dt, void* out, const float* weight, void* packed, unsigned* watch, const int* shape,
+                           const long long* strides, void* stream) {
+  return guard([&] {
+    device::launch_stem_gather(stem_shape(shape, strides), x, (DType)in_dt, out, weight, packed, (DType)dt, watch, (cudaStream_t)stream);
+  });
+}
+size_t al_stem_watch_words(const int* shape) {
+  const long long none[8] = {};
+  size_t words = 0;   // (of a shape that the gather refuses)
+  guard([&] { words = device::stem_watch_words(stem_shape(shape, none)); });
+  return words;
+}
+int al_stem_repair(int dt, const void* out, const void* packed, const unsigned* watch, void* result, const int* shape, const long long* strides,
+                   void* stream) {
+  return guard([&] { device::launch_stem_repair(stem_shape(shape, strides), out, packed, watch, result, (DType)dt, (cudaStream_t)stream); });
 }
 int al_stem_scatter(int dt, const void* packed, float* grad, const int* shape, const long long* strides, void* stream) {
   return guard([&] { device::launch_stem_scatter(stem_shape(shape, strides), packed, grad, (DType)dt, (cudaStream_t)stream); });

@@ -215,12 +215,21 @@ struct StemConv : public torch::autograd::Function<StemConv> {
     Tensor seen = at::empty({s.sizes[0], 64, s.sizes[3] + 3, s.sizes[4]}, x.options().dtype(type), at::MemoryFormat::ChannelsLast);
     Tensor packed = at::empty({oc, 64, 4, 1}, seen.options(), at::MemoryFormat::ChannelsLast);
     const int in = x.scalar_type() == at::kFloat ? (int)Al::DType::f32 : type_code(x);
-    TORCH_CHECK(al_stem_gather(in, x.data_ptr(), type_code(seen), seen.data_ptr(), weight.data_ptr<float>(), packed.data_ptr(), s.sizes.data(),
-                               s.strides.data(), c10::cuda::getCurrentCUDAStream().stream()) == 0,
+    Tensor watch = at::empty({(int64_t)al_stem_watch_words(s.sizes.data())}, x.options().dtype(at::kInt));
+    void* const stream = c10::cuda::getCurrentCUDAStream().stream();
+    TORCH_CHECK(al_stem_gather_watched(in, x.data_ptr(), type_code(seen), seen.data_ptr(), weight.data_ptr<float>(), packed.data_ptr(),
+                                       (unsigned*)watch.data_ptr<int>(), s.sizes.data(), s.strides.data(), stream) == 0,
                 al_last_error());
     ctx->save_for_backward({seen, packed});
     ctx->saved_data["strides"] = weight.strides().vec();
-    return at::conv2d(seen, packed);
+    Tensor y = at::conv2d(seen, packed);
+    const Shape result(x.sizes(), {0, 0, 0, 0}, y);   // (with y's strides)
+    std::array<int, 6> sizes = result.sizes;
+    sizes[5] = (int)oc;
+    TORCH_CHECK(al_stem_repair(type_code(seen), seen.data_ptr(), packed.data_ptr(), (const unsigned*)watch.data_ptr<int>(), y.data_ptr(), sizes.data(),
+                               result.strides.data(), stream) == 0,
+                al_last_error());
+    return y;
   }
 
   static variable_list backward(AutogradContext* ctx, variable_list grads) {

@@ -52,6 +52,39 @@ def test_against_64_bits(shape, layout, dtype):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("shape", [(1, 1, 1), (2, 8, 9), (3, 9, 12), (2, 33, 30), (2, 64, 225), (300, 16, 16)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_pixels_that_are_not_finite(shape, dtype):
+    """Infinities, NaN and values beyond the 16-bit type reach the results whose windows they lie in and the weight's taps that meet them, no others."""
+    n, h, w = shape
+    for k, count in enumerate((1, 1, 3, 40)):
+        g = torch.Generator(device="cuda").manual_seed(17 * h + k)
+        x = torch.randn(n, 3, h, w, device="cuda", generator=g)
+        special = torch.tensor([float("inf"), -float("inf"), float("nan"), 3.4e38], device="cuda")
+        at = torch.randint(0, x.numel(), (count,), device="cuda", generator=g)
+        x.view(-1)[at] = special[torch.randint(0, 4, (count,), device="cuda", generator=g)]
+        conv = stem(40).cuda()
+        with torch.autocast("cuda", dtype=dtype):
+            y = stem_conv(conv, x)
+        assert "StemConv" in y.grad_fn.name()
+        ref = copy.deepcopy(conv).double()
+        with torch.no_grad():
+            ref.weight.copy_(conv.weight.to(dtype).double())
+        want = ref(x.to(dtype).double())
+        dy = torch.randn(want.shape, device="cuda", generator=g).to(dtype)
+        y.backward(dy)
+        want.backward(dy.double())
+        eps = 2 ** -8 if dtype == torch.bfloat16 else 2 ** -11
+        for got, exact in ((y, want), (conv.weight.grad, ref.weight.grad)):
+            if dtype == torch.float16:     # (the library's convolutions of channels-last fp16 images, the module's too, give 0 for minus infinity)
+                got = torch.where((exact == -float("inf")) & (got == 0), exact, got.double())
+            ok = exact.isfinite()
+            assert torch.equal(got.isfinite(), ok) and torch.equal(got.isnan(), exact.isnan()) and torch.equal(got == float("inf"), exact == float("inf"))
+            got, exact = got[ok].double(), exact[ok]
+            assert (got - exact).norm() <= 0.6 * eps * exact.norm() + 1e-6 * exact.norm()
+
+
+@pytest.mark.gpu
 def test_second_derivative_and_a_weight_that_changes_before_the_backward():
     x, conv = torch.randn(2, 3, 18, 20, device="cuda"), stem(8).cuda()
     with torch.autocast("cuda", dtype=torch.bfloat16):
