@@ -12,7 +12,7 @@ import torch
 from torch import nn
 
 from ..ops.activations import _bare, _modes_off, batch_norm_act, batch_norm_act_twice, max_pool
-from ..ops.convolution import cast_weights, convolve, stem_conv
+from ..ops.convolution import cast_weights, convolve, stem_applies, stem_conv
 
 
 class Bottleneck(nn.Module):
@@ -78,8 +78,6 @@ class Shortcut(nn.Sequential):
 
 
 class ResNet(nn.Module):
-    any_layout = True   # the first convolution takes images of any memory layout: the trainer need not lay them out
-
     def __init__(self, layers=(3, 4, 6, 3), num_classes: int = 1000, width: int = 64):
         super().__init__()
         self.c = width
@@ -112,6 +110,11 @@ class ResNet(nn.Module):
         self.c = width * Bottleneck.expansion
         mods += [Bottleneck(self.c, width) for _ in range(1, blocks)]
         return nn.Sequential(*mods)
+
+    @torch.jit.unused
+    def takes_any_layout(self, x) -> bool:
+        """Does the first convolution lay these images out itself, so that the trainer need not?"""
+        return _bare(self) and stem_applies(self.conv1, x)
 
     @torch.jit.unused
     def _blocks(self, x):

@@ -50,16 +50,22 @@ def convolve(conv: nn.Module, x: torch.Tensor, weight) -> torch.Tensor:
     return torch.conv2d(x, weight, None, conv.stride, conv.padding, conv.dilation, conv.groups)
 
 
-def stem_conv(conv: nn.Module, x: torch.Tensor) -> torch.Tensor:
-    """``conv(x)``."""
+def stem_applies(conv: nn.Module, x: torch.Tensor) -> bool:
+    """Whether :func:`stem_conv` runs its own layout of x, and not the module."""
     # (_modes_off() first: a compiler that traces this function sees a constant there and nothing of what follows)
-    if (_modes_off() and torch.is_grad_enabled() and torch.is_autocast_enabled("cuda") and _plain(conv) and conv.training
+    if not (_modes_off() and torch.is_grad_enabled() and torch.is_autocast_enabled("cuda") and _plain(conv) and conv.training
             and conv.in_channels == 3 and conv.kernel_size == (7, 7) and conv.stride == (2, 2) and conv.padding == (3, 3)
             and conv.dilation == (1, 1) and conv.groups == 1):
-        weight, dtype = conv.weight, torch.get_autocast_dtype("cuda")
-        if (dtype in _TYPES and type(x) is torch.Tensor and x.dim() == 4 and x.is_cuda and x.dtype in (torch.float32, dtype) and not x.requires_grad
-                and not x.is_inference() and x.shape[1] == 3 and 0 < x.shape[0] * (x.shape[2] + 8) < 1 << 30 and 0 < x.shape[2]
-                and 0 < x.shape[3] <= 700 and x.get_device() == torch.cuda.current_device()
-                and _weight_ok(weight, x.get_device()) and weight.shape[1:] == (3, 7, 7) and weight.shape[0] % 8 == 0 and 0 < weight.shape[0] <= 4096):
-            return _lib.torch_ops().stem_conv.default(x, weight, dtype)
+        return False
+    weight, dtype = conv.weight, torch.get_autocast_dtype("cuda")
+    return (dtype in _TYPES and type(x) is torch.Tensor and x.dim() == 4 and x.is_cuda and x.dtype in (torch.float32, dtype) and not x.requires_grad
+            and not x.is_inference() and x.shape[1] == 3 and 0 < x.shape[0] * (x.shape[2] + 8) < 1 << 30 and 0 < x.shape[2]
+            and 0 < x.shape[3] <= 700 and x.get_device() == torch.cuda.current_device()
+            and _weight_ok(weight, x.get_device()) and weight.shape[1:] == (3, 7, 7) and weight.shape[0] % 8 == 0 and 0 < weight.shape[0] <= 4096)
+
+
+def stem_conv(conv: nn.Module, x: torch.Tensor) -> torch.Tensor:
+    """``conv(x)``."""
+    if stem_applies(conv, x):
+        return _lib.torch_ops().stem_conv.default(x, conv.weight, torch.get_autocast_dtype("cuda"))
     return conv(x)

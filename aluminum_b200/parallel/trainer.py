@@ -14,7 +14,6 @@ from typing import Iterable, Iterator, Tuple
 import torch
 from torch import nn
 
-from ..ops.activations import _bare
 from .ddp import DataParallel
 
 
@@ -34,10 +33,11 @@ class Trainer:
 
     # ---- one optimisation step on device-resident data -------------------------------------------
     def step_device(self, x: torch.Tensor, y: torch.Tensor) -> torch.Tensor:
-        m = getattr(self.dp, "module", None)
-        if self.channels_last and x.dim() == 4 and not (type(m).__dict__.get("any_layout", False) and _bare(m)):
-            x = x.contiguous(memory_format=torch.channels_last)  # one device pass; the upload itself stays a plain copy
         with torch.autocast("cuda", dtype=self.autocast_dtype, enabled=self.autocast_dtype is not None):
+            m = getattr(self.dp, "module", None)
+            own = type(m).__dict__.get("takes_any_layout")   # (of the class itself: a subclass may do something else with its images)
+            if self.channels_last and x.dim() == 4 and not (own is not None and own(m, x)):
+                x = x.contiguous(memory_format=torch.channels_last)  # one device pass; the upload itself stays a plain copy
             out = self.dp(x)
             loss = self.loss_fn(out.float(), y)
         if isinstance(self.dp, DataParallel):

@@ -173,3 +173,28 @@ def test_weights_cast_together(dtype):
         with torch.no_grad():
             assert cast_weights(convs, x) is None
     assert cast_weights(convs, x) is None     # no autocast
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("case", ["own", "hook", "fp32", "other", "evaluation", "wide"])
+def test_images_are_laid_out_where_the_first_convolution_does_not(case, monkeypatch):
+    """The trainer's promise of channels-last images holds for every first convolution but the one that takes any layout."""
+    from aluminum_b200.models import resnet
+    from aluminum_b200.parallel import DataParallel, Trainer
+    net, seen = resnet.ResNet((1, 1, 1, 1), 10, width=16).cuda(), []
+    stem_conv = resnet.stem_conv
+
+    def watched(conv, x):
+        seen.append(x.is_contiguous(memory_format=torch.channels_last))
+        return stem_conv(conv, x)
+    monkeypatch.setattr(resnet, "stem_conv", watched)
+    if case == "hook":
+        net.conv1.register_forward_pre_hook(lambda *a: None)
+    elif case == "other":
+        net.conv1 = nn.Sequential(nn.Conv2d(3, 16, 3, stride=2, padding=1, bias=False)).cuda()
+    elif case == "evaluation":
+        net.conv1.eval()
+    trainer = Trainer(DataParallel(net, None, lr=0.01), autocast_dtype=None if case == "fp32" else torch.bfloat16)
+    x = torch.randn(2, 3, 32, 704 if case == "wide" else 40, device="cuda")
+    trainer.step_device(x, torch.tensor([1, 2], device="cuda"))
+    assert seen == [case != "own"]
