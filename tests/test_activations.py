@@ -377,3 +377,39 @@ def test_modules_that_write_to_a_blocks_input(where):
         stage.register_forward_hook(lambda *a: None)     # the stages are called
     for u, v in zip(grads(own), grads(called)):
         assert rel(u, v.double()) < 2e-2
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("shape", [(2, 8, 3, 5), (24, 64, 56, 56)])
+def test_captured_in_a_graph(shape):
+    """Launches behind the previous kernel under stream capture: a replay on other values gives what the calls one by one give."""
+    from aluminum_b200.ops import batch_norm_act_twice
+    torch.manual_seed(0)
+    cl = dict(memory_format=torch.channels_last)
+    rand = lambda: torch.randn(shape, device="cuda").bfloat16().contiguous(**cl)
+    bns, relu = [nn.BatchNorm2d(shape[1]).cuda() for _ in range(2)], nn.ReLU()
+    start = copy.deepcopy(bns)
+    x, r, dy = rand().requires_grad_(), rand().requires_grad_(), rand()
+
+    def step(bns, x, r, dy):
+        y = batch_norm_act(bns[0], x, relu)
+        a, b = batch_norm_act_twice(bns[1], y + 0, relu, r)     # (behind a kernel of the framework's and behind ones of its own)
+        return torch.autograd.grad([a, b], [x, r] + [p for m in bns for p in m.parameters()], [dy, dy]), a
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        step(bns, x, r, dy)
+    torch.cuda.current_stream().wait_stream(side)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        grads, y = step(bns, x, r, dy)
+    for m, s in zip(bns, start):
+        m.load_state_dict(s.state_dict())
+    for _ in range(3):
+        with torch.no_grad():
+            for t in (x, r, dy):
+                t.copy_(rand())
+        graph.replay()
+        want, z = step(start, x.detach().requires_grad_(), r.detach().requires_grad_(), dy)
+        assert torch.equal(y, z) and all(torch.equal(g, w) for g, w in zip(grads, want))
+        assert all(torch.equal(u, v) for m, s in zip(bns, start) for u, v in zip(m.buffers(), s.buffers()))
