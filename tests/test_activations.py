@@ -413,3 +413,26 @@ def test_captured_in_a_graph(shape):
         want, z = step(start, x.detach().requires_grad_(), r.detach().requires_grad_(), dy)
         assert torch.equal(y, z) and all(torch.equal(g, w) for g, w in zip(grads, want))
         assert all(torch.equal(u, v) for m, s in zip(bns, start) for u, v in zip(m.buffers(), s.buffers()))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("shape", [(24, 64, 56), (64, 64, 112), (64, 256, 56), (96, 512, 28)])
+@pytest.mark.parametrize("first", ["image", "rows"])
+def test_statistics_of_rows_that_begin_far_from_the_others(shape, first):
+    """A first image ten times as bright, a first stripe a thousand standard deviations off: the partial sums, and their fold, begin with them."""
+    from aluminum_b200.ops import batch_norm_act
+    n, c, h = shape
+    torch.manual_seed(c)
+    x = torch.randn(n, c, h, h, device="cuda")
+    if first == "image":
+        x[0] = x[0] * 10 + 10
+    else:
+        x[0, :, :8] += 1000
+    x = x.bfloat16().contiguous(memory_format=torch.channels_last).requires_grad_()
+    bn = nn.BatchNorm2d(c, momentum=1.0).cuda()
+    assert "BatchNormAct" in batch_norm_act(bn, x, nn.ReLU()).grad_fn.name()
+    v = x.detach().double().transpose(0, 1).flatten(1)
+    mean, var = v.mean(1), v.var(1)
+    # fp32 (roundings of 2^-24): a quarter of one of the standard deviation, over means of many rows, and two of the mean; eight of the variance
+    assert ((bn.running_mean - mean).abs() <= 2 ** -26 * var.sqrt() + 2 ** -23 * mean.abs()).all()
+    assert ((bn.running_var - var).abs() <= 2 ** -21 * var).all()
