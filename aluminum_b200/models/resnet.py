@@ -46,9 +46,11 @@ class Bottleneck(nn.Module):
     def plain(self) -> bool:
         """Nothing but :meth:`forward`'s own steps happens to a block's input, and nothing in its place writes to it: :meth:`twice` may have it
         as two tensors on the same memory."""
-        shortcut = self.downsample
-        first = [self.conv1] if shortcut is None else [self.conv1, shortcut[0]] if type(shortcut) is Shortcut and len(shortcut) == 2 else [None]
-        return _bare(self) and all(type(c) is nn.Conv2d and _bare(c) for c in first) and (shortcut is None or _bare(shortcut))
+        conv, shortcut = self._modules.get("conv1"), self.downsample
+        if not (type(conv) is nn.Conv2d and _bare(conv) and _bare(self)):
+            return False
+        return shortcut is None or (type(shortcut) is Shortcut and _bare(shortcut) and len(shortcut) == 2 and type(shortcut[0]) is nn.Conv2d
+                                    and _bare(shortcut[0]))
 
     def twice(self, x, same):
         """forward(x) as two tensors, for the next block's first convolution and for its end; ``same`` is x, for the end of this one."""
