@@ -14,10 +14,11 @@
 // Statistics are folded batch by batch with the parallel update of mean and sum of squared deviations (Chan, Golub and
 // LeVeque, "Updating formulae and a pairwise algorithm for computing sample variances", 1979), in fp32 and in a fixed order.
 //
-// Measured, one B200, ResNet-50 training step in bf16: batch 256 53.7 -> 26.2 ms, batch 24 (bound by the host's launches:
-// 1013 -> 795 a step) 10.9 -> 9.0 ms (repeats differ by up to 8 %).  Three CTAs per SM (80 registers, spills in the gradient kernels) took 27.8 ms.
+// Measured, one B200, ResNet-50 training step in bf16 with the modules / when these kernels were new (what came since has it at 20.0 and about
+// 8 ms): batch 256 53.7 / 26.2 ms, batch 24 (bound by the host's launches: 1013 / 795 a step) 10.9 / 9.0 ms (repeats differ by up to 8 %).  Three CTAs per
+// SM (80 registers, spills in the gradient kernels) took 27.8 ms.
 // All 53 of a step, device time before / with sums of deviations, folds in parallel and launches behind the kernel before, us: batch 256 forward 4062 /
-// 3799, backward 5419 / 5293; batch 24 795 / 732 and 829 / 723.  Folding in fp64 took 1.5 us more per fold; errors against 64 bits, over
+// 3799, backward 5419 / 5293; batch 24 795 / 732 and 829 / 723.  Folding in fp64 took 1.5 us more per fold; errors against 64 bits of values around one mean, over
 // fourteen shapes, are 0.67 (means), 1.0 (variances), 0.89 and 0.99 (gradients of weight and bias) of what they were.
 #include <algorithm>
 
@@ -127,9 +128,10 @@ __device__ __forceinline__ void load8(float* v, const float* src, int col) {
 /**
  * part[b][c] = (mean, sum of squared deviations) of channel c over the rows of CTA b.  A thread sums the deviations of its rows from a
  * value near their mean, and their squares: four instructions per element, where updating the mean with every batch of
- * eight rows took seven, and few enough registers for twice the CTAs.  That value is the mean of the first kBnStatRows rows, and whenever the
- * rows have doubled the mean of all so far: with the first rows' mean for good, 256 x 256 x 56 x 56 whose first eight rows of pixels lie a
- * thousand deviations off had errors of the variance of 9.8e-7, now 5.3e-8.
+ * eight rows took seven, and few enough registers for twice the CTAs.  That value is the mean of the first kBnStatRows rows, and whenever there
+ * are four times as many the mean of all so far: with the first rows' mean for good, 256 x 256 x 56 x 56 whose first eight rows of pixels lie a
+ * thousand deviations off had errors of the variance of 9.8e-7, now 5.9e-8.  (All 53 forwards of a step 3652 -> 3705 us at batch 256, 815 -> 829 at 24; moved
+ * at every doubling, behind the rows and not while they are loaded, 3730 and 843.)
  */
 template <typename T>
 __global__ void __launch_bounds__(kBnThreads, kBnStatPerSm) bn_stats_kernel(const T* __restrict__ x, float2* __restrict__ part, const BnGrid g) {
@@ -137,7 +139,7 @@ __global__ void __launch_bounds__(kBnThreads, kBnStatPerSm) bn_stats_kernel(cons
   after_previous_kernel();
   const Place at(g);
   const size_t tile_rows = (size_t)at.TY * U;
-  float ref[8], mean[8], m2[8], n = 0.f, doubled = 2.f * U;
+  float ref[8], mean[8], m2[8], n = 0.f, move_at = 4.f * U;
 #pragma unroll
   for (int k = 0; k < 8; ++k) ref[k] = mean[k] = m2[k] = 0.f;
   if (at.active) {
@@ -154,6 +156,17 @@ __global__ void __launch_bounds__(kBnThreads, kBnStatPerSm) bn_stats_kernel(cons
           nb = i + 1;
         }
       if (nb == 0) break;
+      if (n >= move_at) {   // (while the rows just asked for are on their way)
+        move_at = 4.f * n;
+        const float inv = 1.f / n;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+          const float to = fmaf(mean[k], inv, ref[k]), by = to - ref[k], rest = fmaf(-n, by, mean[k]);
+          m2[k] = fmaf(-by, mean[k] + rest, m2[k]);
+          mean[k] = rest;   // (what rounding left)
+          ref[k] = to;
+        }
+      }
       if (n == 0.f) {
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
@@ -177,17 +190,6 @@ __global__ void __launch_bounds__(kBnThreads, kBnStatPerSm) bn_stats_kernel(cons
         m2[k] += q;
       }
       n += (float)nb;
-      if (n >= doubled) {
-        doubled = 2.f * n;
-        const float inv = 1.f / n;
-#pragma unroll
-        for (int k = 0; k < 8; ++k) {
-          const float to = fmaf(mean[k], inv, ref[k]), by = to - ref[k], rest = fmaf(-n, by, mean[k]);
-          m2[k] = fmaf(-by, mean[k] + rest, m2[k]);
-          mean[k] = rest;   // (what rounding left)
-          ref[k] = to;
-        }
-      }
     }
     if (n > 0.f) {
       const float inv = 1.f / n;
@@ -284,15 +286,15 @@ __global__ void __launch_bounds__(8 * kFinishRows) bn_stats_finish_kernel(const 
   load_partials(p, part, g, c);
   // (what lies above n times the first partial's mean: short sums are as exact as their values are close.  Where that partial lies far
   // from the others, what rounding left of the mean is in the deviations from it, and is summed with their squares: in the case
-  // above 9.2e-10 deviations instead of 5.3e-8.)
-  const float n = (float)g.rows, near = part[c].x;
+  // above 1.5e-9 deviations instead of 5.3e-8.)
+  const float n = (float)g.rows, inv = 1.f / n, near = part[c].x;
   float sum = 0.f, q = 0.f;
 #pragma unroll
   for (int i = 0; i < kFinishEach; ++i) {
     const unsigned b = threadIdx.y + i * kFinishRows;
     if (b < g.nblk) sum = fmaf(rows_of(g, b), p[i].x - near, sum);
   }
-  const float first = near + column_sums(make_float2(sum, 0.f), s, total[0]).x / n;
+  const float first = near + column_sums(make_float2(sum, 0.f), s, total[0]).x * inv;
   sum = 0.f;
 #pragma unroll
   for (int i = 0; i < kFinishEach; ++i) {
@@ -304,7 +306,7 @@ __global__ void __launch_bounds__(8 * kFinishRows) bn_stats_finish_kernel(const 
     }
   }
   const float2 both = column_sums(make_float2(q, sum), s, total[1]);
-  const float by = both.y / n, mean = first + by;
+  const float by = both.y * inv, mean = first + by;
   q = fmaf(-both.y, by, both.x);
   if (threadIdx.y == 0) {
     save_mean[c] = mean;
