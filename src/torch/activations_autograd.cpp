@@ -256,7 +256,11 @@ struct StemConv : public torch::autograd::Function<StemConv> {
   }
 };
 
-/** The weights of a block in a 16-bit type, and their gradients back in fp32, with one launch each way. */
+/**
+ * The weights of a block in a 16-bit type, and their gradients back in fp32, with one launch each way.  The gradients of a block come
+ * together then, when the last of them is there.  For the 25 MB buckets that several ranks average meanwhile, ResNet-50 at batch 256, ms
+ * after backward began: 0.58, 1.31, 1.94, 4.58, 12.69; with a cast per weight 0.59, 1.37, 1.77, 4.70, 12.90.
+ */
 struct CastAll : public torch::autograd::Function<CastAll> {
   /** Every tensor in `to`, dense and in the order of its memory. */
   static std::vector<Tensor> cast(at::TensorList tensors, at::ScalarType from, at::ScalarType to) {
